@@ -41,7 +41,9 @@ extern "C" {
 #define MG_ERR_NAN         -5   /* NaN detected (reference: x .eq. x+1)   */
 
 /* ---- precision modes ----------------------------------------------------- */
-#define MG_FP64   0   /* plain path: every kernel in FP64                 */
+#define MG_FP64   0   /* FP64 data and accuracy; the contractions of large
+                         bases as exact digit products rounded once to FP64,
+                         with a smaller error than a chain of FP64 FMAs    */
 #define MG_MIXED  1   /* tensor-core digit GEMMs, double-float mesh work  */
 
 /* ---- bases --------------------------------------------------------------- */

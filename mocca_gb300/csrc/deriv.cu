@@ -410,7 +410,19 @@ int build_basis_jobs(mg_ctx* c, int b) {
             for (int d = 0; d < 3; ++d) J.slot[d] = (int8_t)lag_slot(d, P, S, TS, l + 1);
         }
     }
+    // the jobs of each axis' matrix slots (deriv_tc.cu)
+    std::vector<int> perm;
+    for (int d = 0; d < 3; ++d) {
+        for (int s = 0; s < 2; ++s)
+            for (int j = 0; j < 4 * nwt; ++j)
+                if (jobs[j].slot[d] == s) perm.push_back(j);
+        B.job_slot0[d] = (int)std::count_if(jobs.begin(), jobs.end(),
+                                            [d](const GridJob& J) { return J.slot[d] == 0; });
+    }
+    if (!B.job_perm) MG_CUDA(cudaMalloc(&B.job_perm, perm.size() * sizeof(int)));
     MG_CUDA(cudaMemcpyAsync(B.jobs, jobs.data(), jobs.size() * sizeof(GridJob),
+                            cudaMemcpyHostToDevice, c->stream));
+    MG_CUDA(cudaMemcpyAsync(B.job_perm, perm.data(), perm.size() * sizeof(int),
                             cudaMemcpyHostToDevice, c->stream));
     MG_CUDA(cudaStreamSynchronize(c->stream));
     return MG_OK;
@@ -520,13 +532,19 @@ int run_jobs(mg_ctx* c, const GridJob* jobs, int njobs, bool out_df) {
 // In the mixed form the basis derivatives stay double-float in HBM (the same
 // 8 bytes per value), so that h.psi and the densities read them without FP64
 // conversions; Basis::der_df records the format.  They come from the tensor
-// cores (deriv_tc.cu) when every line length is at most 32, else from the
-// double-float kernels above.
+// cores (deriv_tc.cu) on lines of up to 48 points (mixed) or 32 (FP64), else
+// from the kernels above.  The tensor-core passes cost about 18 us however
+// small the basis; the FP64 kernels cost 13 us at 8^3 with 20 spwfs (1.0e6 in
+// the units below; tensor cores 18 us), 23 at 8^3 with 60 (2.9e6; 25), 33 at
+// 10^3 with 40 (4.8e6; 29) and 39 at 12^3 with 30 (7.5e6; 31).
+constexpr double kTc64MinWork = 3.0e6;   // grids x points x (nx + ny + nz)
+
 int derive_basis(mg_ctx* c, int b) {
     if (!c->bas[b].have_qn) return MG_ERR_STATE;
     const bool df = c->cur_precision == MG_MIXED;
-    if (df && c->tc_ok)
-        MG_TRY(run_jobs_tc(c, c->bas[b].jobs, 4 * c->p.nwt));
+    const double work = 4.0 * c->p.nwt * c->V * (c->nx + c->ny + c->nz);
+    if (df ? c->tc_ok : c->tc_ok64 && work >= kTc64MinWork)
+        MG_TRY(derive_basis_tc(c, b, !df));
     else
         MG_TRY(run_jobs(c, c->bas[b].jobs, 4 * c->p.nwt, df));
     c->bas[b].der_df = df;

@@ -34,6 +34,7 @@ void free_all(mg_ctx* c) {
     for (int b = 0; b < 2; ++b) {
         Basis& B = c->bas[b];
         F(B.psi); F(B.der); F(B.lap); F(B.qn); F(B.occ); F(B.e); F(B.disp); F(B.jobs);
+        F(B.job_perm);
     }
     F(c->updates); F(c->hbuf);
     F(c->rho); F(c->tau); F(c->nablaj); F(c->derrho); F(c->laprho);

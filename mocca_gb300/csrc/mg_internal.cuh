@@ -62,6 +62,8 @@ struct Basis {
     double* e = nullptr;     // nwt
     double* disp = nullptr;  // nwt
     GridJob* jobs = nullptr; // 4*nwt derivative jobs
+    int* job_perm = nullptr; // per axis: the jobs of matrix slot 0, then those of slot 1
+    int job_slot0[3] = {0, 0, 0};   // jobs of slot 0
     bool der_df = false;     // der / lap hold double-float {hi, lo} pairs (mixed form)
     std::vector<int> h_qn;
     std::vector<double> h_occ, h_e, h_disp;
@@ -232,15 +234,14 @@ struct mg_ctx {
     long mat32_off[3][2][2];
     int cur_precision = MG_FP64;  // precision of the next kernels (MG_FP64 / MG_MIXED)
     // digit planes of the Lagrange blocks for the tensor-core derivatives
-    // (deriv_tc.cu): [axis][slot] blocks of 6 planes x N rows x 32, bf16
+    // (deriv_tc.cu), bf16: per (axis, slot) six planes, for the FP64 form seven
     uint16_t* tcmats = nullptr;
-    int* tc_erow = nullptr;       // [axis][slot][64] row exponents
+    int* tc_erow = nullptr;       // [axis][slot] row exponents
     int* tc_status = nullptr;     // set when an MMA completion wait ran out
-    long tc_off[3][2];
-    int tc_N[3] = {0, 0, 0};
-    bool tc_ok = false;           // every line length <= 32
+    long tc_off[2][3][2];         // [0 mixed, 1 FP64][axis][slot]
+    bool tc_ok = false;           // every line length <= 48: the mixed form's derivatives
+    bool tc_ok64 = false;         // every line length <= 32: the FP64 form's
     bool tc_mesh_ok = false;      // mesh-sized GEMMs on the tensor cores (blocks <= kMeshTcMax)
-    int tc_kp = 32;               // padded K of the tensor-core derivative planes (32 or 48)
     int* h_tc_status = nullptr;   // pinned copy of tc_status, read with the energy's sync
     // largest grid of the persistent tensor-core derivative kernel (0: one CTA
     // per SM); set while it runs beside other work on the side stream
@@ -394,7 +395,7 @@ int build_field_jobs(mg_ctx* c);
 int run_jobs(mg_ctx* c, const GridJob* jobs, int njobs, bool out_df = false);
 int derive_basis(mg_ctx* c, int b);
 int tc_setup(mg_ctx* c);
-int run_jobs_tc(mg_ctx* c, const GridJob* jobs, int njobs);
+int derive_basis_tc(mg_ctx* c, int b, bool f64);
 int tc_check(mg_ctx* c);
 // tc_check in two halves: enqueue the status copy, read it after a later sync
 int tc_status_async(mg_ctx* c);

@@ -137,6 +137,171 @@ __device__ __forceinline__ void digits8(const double (&v)[8], int emax, uint4 (&
     for (int a = 0; a < kDigits; ++a) w[a] = make_uint4(x[a][0], x[a][1], x[a][2], x[a][3]);
 }
 
+// ---- eight digits: operands of 62 bits, results rounded once to FP64 -----------
+//
+// The FP64 form of a contraction over at most 32 terms.  Every entry is
+// rounded to 62 bits of its row's largest (FP64 carries 53 of its own), the
+// 36 digit pairs of weight 0..7 are kept, those of weight 0..5 in six exact
+// accumulators (6 pairs x 32 terms x 2^14 < 2^22) and those of weight 6 and 7
+// in a seventh, rounded near 2^-70 of the row's largest products; the
+// epilogue adds them as one 64-bit integer and rounds it once to FP64.  (An
+// eighth accumulator saves MMAs but not time: 356 us against 336 for DeriveAll
+// at 24^3 with 160 spwfs, the epilogue's loads and registers being the limit.)  A
+// chain of FP64 FMAs rounds every partial sum.  Norm-wise errors against
+// extended-precision sums on Lagrange lines (5 to 32 points, folded and full):
+// first derivatives 0.5e-16 to 1.1e-16 (the chain: 1.3e-16 to 2.8e-16),
+// Laplacians 0.8e-16 to 2.4e-16 (1.5e-16 to 3.0e-16).
+// (Seven digits, 55 bits, were not enough: second derivatives are small
+// differences of large products, and 2.6e-15 came out where the chain has
+// 2.6e-16.)
+
+constexpr int kDigits64 = 8;
+constexpr int kAccs64 = 7;
+// product units: 2^(E_row + E_col - kUnit64), E as above
+constexpr int kUnit64 = 10;
+
+// power g of the fixed-point form round(v * 2^g) of a row with exponent E:
+// one bit fewer than ND digits hold with eight, so that 64-bit integers do
+template <int ND>
+__host__ __device__ constexpr int fixed_power(int E) {
+    return 8 * ND - (ND == kDigits64 ? 3 : 2) - E;
+}
+
+// What turns the values of a row into fixed-point words: per row, from the
+// largest biased exponent emax of the row (rows with emax of 0 or near 2046
+// are for the caller to leave out).
+template <int ND>
+struct FixedRow;
+
+// Six digits: the 47-bit integers of fixed(), rounded half away from zero
+// (one variable shift: floor((m + 2^(s-1)) / 2^s) = floor((floor(m / 2^(s-1)) + 1) / 2)).
+template <>
+struct FixedRow<kDigits> {
+    int emax;
+    __device__ __forceinline__ explicit FixedRow(int e) : emax(e) {}
+    __device__ __forceinline__ unsigned long long biased(double v) const {
+        const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+        const int e = (int)((hi >> 20) & 0x7FFu);
+        const unsigned long long m = ((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo;
+        const long long t = (long long)(((m >> min(53 - 8 * kDigits + emax - e, 63)) + 1) >> 1);
+        const long long X = e == 0 ? 0 : t;
+        return (unsigned long long)(((int)hi < 0 ? -X : X) + kDigitBias);
+    }
+};
+
+// Eight digits: 53 bits shifted up by 9, down by the exponent's distance from
+// the row's largest, in two's complement (so that what the shift drops, below
+// 2^-61 of the largest, is rounded down).
+template <>
+struct FixedRow<kDigits64> {
+    int emax;
+    __device__ __forceinline__ explicit FixedRow(int e) : emax(e) {}
+    __device__ __forceinline__ unsigned long long biased(double v) const {
+        const uint32_t hi = (uint32_t)__double2hiint(v), lo = (uint32_t)__double2loint(v);
+        const int e = (int)((hi >> 20) & 0x7FFu);
+        const long long sgn = (long long)((int)hi >> 31);
+        const long long m = (long long)((((unsigned long long)((hi & 0xFFFFFu) | 0x100000u) << 32) | lo) << 9);
+        const long long X = (m ^ sgn) >> min(emax - e, 63);
+        return (unsigned long long)(e == 0 ? 0 : X) + 0x80808080808080ULL;
+    }
+};
+
+// The pre-scaled digits (top digit first) of a fixed-point value plus the
+// digit bias.
+template <int ND>
+__device__ __forceinline__ void digits_of(unsigned long long Y, uint32_t (&d)[ND]) {
+    static_assert(ND == kDigits || ND == kDigits64, "six or eight digits");
+    const uint32_t ylo = (uint32_t)Y, yhi = (uint32_t)(Y >> 32);
+    // the top digit is Y >> 8 (ND - 1) (arithmetic)
+    const int top = (int)yhi >> (ND == kDigits ? 8 : 24);
+    d[0] = __float_as_uint(__int_as_float(0x4B400000 + top) - 12582912.0f);
+    if constexpr (ND == kDigits) {
+        // digit a (a = 1..5) is byte (5 - a) of Y, biased by 128
+        d[1] = low_digit<1>(yhi, 0x7540);
+        d[2] = low_digit<2>(ylo, 0x7543);
+        d[3] = low_digit<3>(ylo, 0x7542);
+        d[4] = low_digit<4>(ylo, 0x7541);
+        d[5] = low_digit<5>(ylo, 0x7540);
+    } else {
+        // digit a (a = 1..7) is byte (7 - a) of Y
+        d[1] = low_digit<1>(yhi, 0x7542);
+        d[2] = low_digit<2>(yhi, 0x7541);
+        d[3] = low_digit<3>(yhi, 0x7540);
+        d[4] = low_digit<4>(ylo, 0x7543);
+        d[5] = low_digit<5>(ylo, 0x7542);
+        d[6] = low_digit<6>(ylo, 0x7541);
+        d[7] = low_digit<7>(ylo, 0x7540);
+    }
+}
+
+// Digits of 4 values of a row as one 8-byte half of a core-matrix row per
+// digit plane.
+template <int ND>
+__device__ __forceinline__ void digits4(const double (&v)[4], const FixedRow<ND>& row,
+                                        uint2 (&w)[ND]) {
+    uint32_t x[ND][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        uint32_t d0[ND], d1[ND];
+        digits_of<ND>(row.biased(v[2 * h]), d0);
+        digits_of<ND>(row.biased(v[2 * h + 1]), d1);
+#pragma unroll
+        for (int a = 0; a < ND; ++a) x[a][h] = __byte_perm(d0[a], d1[a], 0x7632);
+    }
+#pragma unroll
+    for (int a = 0; a < ND; ++a) w[a] = make_uint2(x[a][0], x[a][1]);
+}
+
+// A float that is a multiple of 2^-P below 2^(22 - P) (or any smaller value,
+// rounded to one) plus the magic number 1.5 * 2^(23 - P): its bits are the
+// integer multiple plus magic_bits(P).
+template <int P>
+__device__ __forceinline__ uint32_t units(uint32_t bits) {
+    constexpr float magic = 12582912.0f / (float)(1ull << P);
+    return __float_as_uint(__fadd_rn(__uint_as_float(bits), magic));
+}
+__host__ __device__ constexpr uint32_t magic_bits(int P) { return 0x4B400000u - ((uint32_t)P << 23); }
+
+// The seven accumulators' sum times 2^x as FP64: a 64-bit integer in units
+// of 2^-44 (top digits are at most 64, so 32 products stay below 2^18 and the
+// integer below 2^62), rounded once with integer instructions (an FP64
+// instruction holds a warp's slot of the FP64 pipe for 16 clocks).  The
+// accumulators' magic numbers are carried along and taken off once.  The
+// caller keeps x between -900 and 900.
+__device__ __forceinline__ double combine64(const uint32_t (&a)[kAccs64], int x) {
+    const uint32_t hi = units<0>(a[0]) * 256u + units<8>(a[1]);     // 2^-8
+    const uint32_t mid = units<16>(a[2]) * 256u + units<24>(a[3]);  // 2^-24, with its magic >= 0
+    const uint32_t low = units<32>(a[4]) * 256u + units<40>(a[5]);  // 2^-40, with its magic >= 0
+    const uint32_t tail = units<44>(a[6]);
+    constexpr uint32_t mhi = magic_bits(0) * 256u + magic_bits(8);
+    constexpr uint32_t mmid = magic_bits(16) * 256u + magic_bits(24);
+    constexpr uint32_t mlow = magic_bits(32) * 256u + magic_bits(40);
+    constexpr unsigned long long off = ((unsigned long long)mhi << 36) +
+                                       ((unsigned long long)mmid << 20) +
+                                       ((unsigned long long)mlow << 4) + magic_bits(44);
+    const unsigned long long I = (unsigned long long)mid * (1ull << 20) +
+                                 ((unsigned long long)low * 16u + tail) +
+                                 ((unsigned long long)(hi << 4) << 32) - off;
+    const uint32_t sgn = (uint32_t)((int)(uint32_t)(I >> 32) >> 31);
+    const unsigned long long s64 = ((unsigned long long)sgn << 32) | sgn;
+    const unsigned long long u = (I ^ s64) - s64;
+    uint32_t h = (uint32_t)(u >> 32), l = (uint32_t)u;
+    int e = 1023 + 63 - 44 + x;
+    if (h == 0) {
+        h = l;
+        l = 0;
+        e -= 32;
+    }
+    const int lz = __clz((int)h);
+    if (h == 0) return 0.0;
+    h = __funnelshift_l(l, h, lz);
+    l <<= lz;
+    // 53 bits with the hidden one, rounded to nearest
+    const unsigned long long r = ((((unsigned long long)h << 32) | l) >> 11) + ((l >> 10) & 1u);
+    const uint32_t rh = (uint32_t)(r >> 32) + ((uint32_t)(e - lz - 1) << 20);
+    return __hiloint2double((int)(rh | (sgn & 0x80000000u)), (int)(uint32_t)r);
+}
+
 // a0 + a1 + a2 + a3 as a normalised double-float.  a0 is an integer below
 // 2^22, a1 a multiple of 2^-8 below 2^15, a2 a multiple of 2^-16 below 2^8
 // (all exact); a3 is the small rounded remainder.  With a1 = i1 + f1
@@ -184,23 +349,72 @@ __device__ __forceinline__ void issue_pairs(uint32_t tmem, int N, uint32_t idesc
     }
 }
 
+// The digit-pair MMAs of a block of COLS columns with ND digits and NACC
+// accumulators side by side at tmem (COLS columns each): A planes at aBase + a
+// aPlane, the B planes of the block stacked row below row at bBase.  Plane a
+// times the stacked planes 0, 1, ... fills accumulators a, a + 1, ..., so one
+// MMA of up to 256 columns serves all pairs of digit a that have an
+// accumulator of their own; the pairs of the last accumulator's weights follow
+// one by one, in order of weight and a.  (An MMA of 32 columns holds the
+// tensor pipe for as long as one of 192: with a pair per MMA and column block
+// the issue of 84 to 144 MMAs per tile bound the derivative kernel.)
+template <int ND, int NACC, int COLS, int KSTEPS>
+__device__ __forceinline__ void issue_stacked(uint32_t tmem, uint32_t aBase, uint32_t aPlane,
+                                              uint32_t bBase, uint32_t sbo) {
+    constexpr uint32_t bPlane = COLS * KSTEPS * 32;
+    constexpr int most = 256 / COLS;   // stacked planes of one MMA
+    // accumulators filled by stacked planes; the FP64 form's last one takes its
+    // own weight that way too (its sums are not exact, but far below the result)
+    constexpr int own = ND == kDigits64 ? NACC : NACC - 1;
+    const uint64_t da = tc::desc_sbo(aBase, sbo), db = tc::desc_sbo(bBase, sbo);
+    // the descriptors' address field counts 16 bytes
+    const auto mma = [&](int a, int b, int ks, int acc, int count, uint32_t add) {
+        tc::mma_bf16(tmem + (uint32_t)(acc * COLS), da + ((a * aPlane + ks * tc::kKStep) >> 4),
+                     db + ((b * bPlane + ks * tc::kKStep) >> 4),
+                     tc::idesc_bf16(128, count * COLS), add);
+    };
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks)
+#pragma unroll
+        for (int a = 0; a < ND; ++a) {
+#pragma unroll
+            for (int b = 0; b < own - a; b += most) {
+                const int left = own - a - b;
+                // digit 0 is the first to reach each of these accumulators
+                mma(a, b, ks, a + b, left < most ? left : most, ks == 0 && a == 0 ? 0u : 1u);
+            }
+            // the pairs past the last weight, between MMAs that do not wait for them
+            if (own == NACC)
+#pragma unroll
+                for (int b = own - a > 0 ? own - a : 0; b < ND - a; ++b) mma(a, b, ks, NACC - 1, 1, 1u);
+        }
+    if (own < NACC) {
+#pragma unroll
+        for (int c = own; c < ND; ++c)
+#pragma unroll
+            for (int a = 0; a <= c; ++a)
+#pragma unroll
+                for (int ks = 0; ks < KSTEPS; ++ks)
+                    mma(a, c - a, ks, NACC - 1, 1, c == own && a == 0 && ks == 0 ? 0u : 1u);
+    }
+}
+
 // Host form of the digits: BF16 bit patterns of the pre-scaled digits of
-// round(x * 2^g), top first.
-inline void host_digits(double x, int g, uint16_t* out) {
-    const long long X = std::llrint(std::ldexp(x, g));
-    const long long Y = X + kDigitBias;
-    for (int b = kDigits - 1; b >= 1; --b) {
-        const int j = kDigits - 1 - b;   // byte position
-        const int d = (int)((Y >> (8 * j)) & 0xFF) - 128;
-        const float f = std::ldexp((float)d, -8 * b);
+// round(x * scale), scale a power of two, top first.
+inline void host_digits(double x, double scale, uint16_t* out, int nd = kDigits) {
+    const long long X = std::llrint(x * scale);
+    long long bias = 0;
+    for (int b = 1; b < nd; ++b) bias = bias * 256 + 128;
+    const long long Y = X + bias;
+    float weight = 1.0f;   // 2^(-8 b)
+    for (int b = 0; b < nd; ++b, weight *= 1.0f / 256.0f) {
+        const int j = nd - 1 - b;   // byte position
+        const float d = b == 0 ? (float)(Y >> (8 * j)) : (float)((int)((Y >> (8 * j)) & 0xFF) - 128);
+        const float f = d * weight;
         uint32_t u;
         std::memcpy(&u, &f, 4);
         out[b] = (uint16_t)(u >> 16);
     }
-    const float f = (float)(Y >> (8 * (kDigits - 1)));
-    uint32_t u;
-    std::memcpy(&u, &f, 4);
-    out[0] = (uint16_t)(u >> 16);
 }
 
 // The power g = 8 kDigits - 2 - E used for a row whose largest |entry| is mx,

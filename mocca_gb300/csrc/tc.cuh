@@ -105,18 +105,22 @@ __device__ __forceinline__ void mbar_init(uint64_t* mbar, uint32_t count) {
 // clocks.  Returns true when the phase completed.
 __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, long long max_cycles) {
     const uint32_t a = smem_u32(mbar);
-    const long long t0 = clock64();
-    while (true) {
-        uint32_t done;
+    const auto done = [a, parity]() {
+        uint32_t d;
+        // the hardware may suspend the thread for up to 20 us per try
         asm volatile(
-            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
             "selp.b32 %0, 1, 0, p;\n}\n"
-            : "=r"(done)
-            : "r"(a), "r"(parity)
+            : "=r"(d)
+            : "r"(a), "r"(parity), "r"(20000u)
             : "memory");
-        if (done) return true;
+        return d != 0;
+    };
+    if (done()) return true;
+    const long long t0 = clock64();
+    while (!done())
         if (clock64() - t0 > max_cycles) return false;
-    }
+    return true;
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
