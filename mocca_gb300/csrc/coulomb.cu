@@ -7,12 +7,29 @@
 //   ConjugGrad (:755-900) with CoulombLaplacian (5-point FD, even mirror at
 //     the low end of each axis, src/CoulombDerivatives.f90:144-281);
 //   Slater exchange -(3/pi)^(1/3) e2 rho_p^(1/3) (:338-344).
-// The CG runs as ONE cooperative kernel: every block owns a slice of the
-// extended box, the two dot products per iteration are block partials summed
-// by every block in the same order (so every block takes the same branch),
-// and blocks meet at a sense-reversing grid barrier whose spin is bounded:
-// a barrier that waits longer than its cap sets the timeout status and the
-// kernel returns instead of hanging.
+// The CG runs as ONE cooperative kernel: every thread owns up to eight points
+// of the stored box and keeps their solution, residual, direction and its
+// Laplacian in registers; only the residual, which the stencil reads at the
+// neighbours, goes to memory.  The recurrences are those of Chronopoulos and
+// Gear (J. Comput. Appl. Math. 25 (1989) 153): w = Lap(r) and the sums r.r and
+// r.w give both coefficients, so an iteration has one meeting of all blocks,
+// where a block posts its partial sums and adds up everybody's in the same
+// order (so every block takes the same branch).  The blocks come in clusters
+// of eight, which add up their partials through distributed shared memory; one
+// block of a cluster sends the sum to a mailbox of every block.  Everything
+// that travels through memory (sums and residuals) is a pair of 64-bit words
+// that carry a running number beside the halves of the value, so a reader sees
+// by itself whether the value is there: no counters, flags or fences.  The
+// waits are bounded: one that runs out of its cap sets the timeout status and
+// the kernel returns instead of hanging.
+// The kernel is a chain of latencies: an FP64 add or FMA takes 64 clocks, a
+// divide 549, a cluster barrier 400, a word written by one block and polled by
+// another about a thousand (but ten thousand where many blocks poll the lines
+// that are to be written: the reason for clusters and mailboxes).  With three
+// meetings through a counter and fences, serial sums of the partials and FP64
+// divides an iteration took 19.8 us on a 24^3 box, 14.1 on 10^3 and 48 on 64^3
+// (solve times over iterations); now 4.8, 3.9 and 20.
+#include <algorithm>
 #include <cmath>
 
 #include "mg_internal.cuh"
@@ -22,50 +39,23 @@ namespace mg {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr long long kSpinCap = 1ll << 22;  // ~0.2 s of 50 ns sleeps per barrier
+constexpr long long kWaitCycles = 4000000000LL;   // ~2 s at the top SM clock
+constexpr int kCluster = 8;       // blocks of a cluster of the CG kernel
+constexpr int kMaxClusters = 32;  // sums of a meeting, one per lane
 
 struct CgArgs {
-    double* sol;
-    double* res;
-    double* p;
-    double* t;
-    const double* src;
-    double* red;          // 2 * gridDim.x
-    unsigned* bar;        // [0] arrival count, [1] generation
-    int* status;          // [0] state, [1] iterations
-    int nx, ny, nz, mx, my, mz;
+    double* sol;            // extended box
+    const double* src;      // extended box
+    ulonglong2* res;        // stored box, tagged
+    ulonglong2* mail;       // [2][blocks][kMaxClusters][2] sums of the clusters, tagged
+    unsigned tag;           // every tag of this launch is above it, every earlier one at most it
+    int* status;            // [0] state, [1] iterations
+    int nx, ny, nz, mx, my;
     double inv_dx2;
     double prec;
-    double rel;           // > 0: stop at |r| <= rel |src| instead of |r|^2 <= prec
+    double rel;             // > 0: stop at |r| <= rel |src| instead of |r|^2 <= prec
     int maxit;
 };
-
-__device__ bool grid_barrier(unsigned* bar, int* status) {
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned* gen = bar + 1;
-        const unsigned g = *gen;
-        __threadfence();
-        const unsigned arrived = atomicAdd(bar, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            atomicExch(bar, 0u);
-            __threadfence();
-            atomicAdd(bar + 1, 1u);
-        } else {
-            long long spins = 0;
-            while (*gen == g) {
-                if (++spins > kSpinCap) {
-                    atomicExch(status, 2);
-                    break;
-                }
-                __nanosleep(50);
-            }
-        }
-        __threadfence();
-    }
-    __syncthreads();
-    return *(volatile int*)status != 2;
-}
 
 __device__ __forceinline__ double lap_at(const double* g, int i, int j, int k, int mx, int my,
                                          double inv_dx2) {
@@ -83,108 +73,366 @@ __device__ __forceinline__ double lap_at(const double* g, int i, int j, int k, i
     return ax * inv_dx2 + ay * inv_dx2 + az * inv_dx2;
 }
 
-__device__ double block_sum(double x, double* sh) {
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = x;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int q = 0; q < kThreads / 32; ++q) s += sh[q];
-    __syncthreads();
-    return s;  // valid in thread 0
+// A double as two words, each half of the value's bits below a 32-bit tag.
+__device__ __forceinline__ void put_tagged(ulonglong2* p, double x, unsigned tag) {
+    const unsigned long long e = (unsigned long long)tag << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p),
+                 "l"(e | (unsigned)__double2hiint(x)), "l"(e | (unsigned)__double2loint(x))
+                 : "memory");
+}
+__device__ __forceinline__ ulonglong2 get_words(const ulonglong2* p) {
+    ulonglong2 w;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(w.x), "=l"(w.y) : "l"(p) : "memory");
+    return w;
+}
+// zero when both words carry the tag
+__device__ __forceinline__ unsigned differs(const ulonglong2& w, unsigned tag) {
+    return ((unsigned)(w.x >> 32) ^ tag) | ((unsigned)(w.y >> 32) ^ tag);
+}
+__device__ __forceinline__ double value_of(const ulonglong2& w) {
+    return __hiloint2double((int)(unsigned)w.x, (int)(unsigned)w.y);
 }
 
-__device__ double grid_total(const double* red, double* bc) {
-    if (threadIdx.x == 0) {
-        double s = 0.0;
-        for (unsigned q = 0; q < gridDim.x; ++q) s += ((volatile const double*)red)[q];
-        *bc = s;
-    }
-    __syncthreads();
-    const double v = *bc;
-    __syncthreads();
+// Sums of x and of y over the warp in one chain of five adds: after the first
+// exchange the lower half-warp carries x, the upper one y.  Lane 0 ends with
+// the sum of x, lane 16 with that of y.
+__device__ __forceinline__ double warp_sum2(double x, double y) {
+    const bool up = (threadIdx.x & 16) != 0;
+    double v = (up ? y : x) + __shfl_xor_sync(0xffffffffu, up ? x : y, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
 }
 
-__global__ void __launch_bounds__(kThreads) k_cg(CgArgs a) {
-    __shared__ double sh[kThreads / 32];
-    __shared__ double bcast;
-    const long M = (long)a.mx * a.my * a.mz;
-    const long stride = (long)gridDim.x * kThreads;
-    const long t0 = (long)blockIdx.x * kThreads + threadIdx.x;
-    double* red1 = a.red;
-    double* red2 = a.red + gridDim.x;
+// 1 / d by Newton's iteration from the float reciprocal (a CG coefficient:
+// right to an ulp or two; an FP64 divide takes 549 clocks).  The float comes
+// and goes by bit moves, as FP64 conversions wait for the FP64 pipe.
+__device__ __forceinline__ double inverse(double d) {
+    const unsigned hi = (unsigned)__double2hiint(d), e = (hi >> 20) & 0x7FFu;
+    if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / d;
+    float f = __uint_as_float((hi & 0x80000000u) | ((hi & 0x7FFFFFFFu) - (896u << 20)) << 3 |
+                              (unsigned)__double2loint(d) >> 29);
+    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(f));
+    const unsigned u = __float_as_uint(f);
+    double x = __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7FFFFFFFu) >> 3) + (896u << 20))),
+                                (int)(u << 29));
+    x = fma(x, fma(-d, x, 1.0), x);
+    return fma(x, fma(-d, x, 1.0), x);
+}
 
-    // r0 = src - Lap(sol); p0 = r0; pnorm = r0.r0
-    double loc = 0.0;
-    for (long o = t0; o < M; o += stride) {
-        const int i = (int)(o % a.mx), j = (int)((o / a.mx) % a.my), k = (int)(o / ((long)a.mx * a.my));
-        double lap = 0.0;
-        if (i < a.nx && j < a.ny && k < a.nz) lap = lap_at(a.sol, i, j, k, a.mx, a.my, a.inv_dx2);
-        const double r = -lap + a.src[o];
-        a.res[o] = r;
-        a.p[o] = r;
-        loc = fma(r, r, loc);
+// What the blocks of a cluster leave in each other's shared memory.
+struct CgShared {
+    double part[2][2][kCluster];   // [turn][x, y][rank]: the ranks' partial sums
+    int bad[2][kCluster];          // a wait of that rank ran out
+    double warp[2][16];
+    double result[2];
+    int fail;
+};
+
+__device__ __forceinline__ uint32_t remote(const void* p, int rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+    return r;
+}
+
+// Sums x and y over the grid; warp 0 of every block applies `then` to the
+// totals (the same bits everywhere) and gives its two results to its threads.
+// `meanwhile` is work of warp 0 for the time that the barrier takes.  `turn`
+// alternates from call to call: what is left for a turn has been read when that
+// turn comes again, because the call in between needed every block.
+template <class Meanwhile, class Then>
+__device__ bool grid_sum(CgShared& S, ulonglong2* mail, int* status, unsigned tag, double x, double y,
+                         double& a, double& b, Meanwhile meanwhile, Then then) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int turn = (int)(tag & 1u);
+    const int rank = (int)(blockIdx.x % kCluster), cluster = (int)(blockIdx.x / kCluster);
+    const int nclusters = (int)(gridDim.x / kCluster);
+    double v = warp_sum2(x, y);
+    if (nw > 1) {
+        if ((lane & 15) == 0) S.warp[lane >> 4][warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            v = (lane & 15) < nw ? S.warp[lane >> 4][lane & 15] : 0.0;
+#pragma unroll
+            for (int o = 8; o > 0; o >>= 1)
+                if (o < nw) v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
     }
-    double s = block_sum(loc, sh);
-    if (threadIdx.x == 0) red2[blockIdx.x] = s;
+    if (warp == 0) {
+        // lane r of the lower half sends x, of the upper half y, to rank r
+        v = __shfl_sync(0xffffffffu, v, lane & 16);
+        if ((lane & 15) < kCluster) {
+            const uint32_t p = remote(&S.part[turn][lane >> 4][rank], lane & 15);
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(p), "d"(v) : "memory");
+            if (lane < kCluster) {
+                const uint32_t f = remote(&S.bad[turn][rank], lane);
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(f), "r"(S.fail) : "memory");
+            }
+        }
+    }
+    // every rank's partials are here after this (threads that have left count
+    // as arrived)
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (warp == 0) meanwhile();
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    int bad = 0;
+#pragma unroll
+    for (int r = 0; r < kCluster; ++r) bad |= S.bad[turn][r];
+    if (bad) {
+        // all ranks of the cluster leave here together
+        if (threadIdx.x == 0) atomicExch(status, 2);
+        return false;
+    }
+    if (warp == 0) {
+        v = S.part[turn][lane >> 4][lane % kCluster];
+#pragma unroll
+        for (int o = kCluster / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        x = __shfl_sync(0xffffffffu, v, 0);
+        y = __shfl_sync(0xffffffffu, v, 16);
+        if (nclusters > 1) {
+            ulonglong2* box = mail + (size_t)turn * gridDim.x * kMaxClusters * 2;
+            if (rank == 0) {
+                for (int q = lane; q < (int)gridDim.x; q += 32) {
+                    ulonglong2* to = box + ((size_t)q * kMaxClusters + cluster) * 2;
+                    put_tagged(to, x, tag);
+                    put_tagged(to + 1, y, tag);
+                }
+            }
+            const ulonglong2* mine = box + ((size_t)blockIdx.x * kMaxClusters + lane) * 2;
+            x = y = 0.0;
+            bool ok = true;
+            if (lane < nclusters) {
+                const long long t0 = clock64();
+                while (true) {
+                    const ulonglong2 w = get_words(mine), z = get_words(mine + 1);
+                    if ((differs(w, tag) | differs(z, tag)) == 0) {
+                        x = value_of(w);
+                        y = value_of(z);
+                        break;
+                    }
+                    if (clock64() - t0 > kWaitCycles) {
+                        ok = false;
+                        break;
+                    }
+                }
+            }
+            if (!ok) S.fail = 1;   // read by warp 0 at the next call
+            __syncwarp();
+            v = warp_sum2(x, y);
+            x = __shfl_sync(0xffffffffu, v, 0);
+            y = __shfl_sync(0xffffffffu, v, 16);
+        }
+        double ra, rb;
+        then(x, y, ra, rb);
+        if (lane == 0) {
+            S.result[0] = ra;
+            S.result[1] = rb;
+        }
+    }
+    __syncthreads();
+    a = S.result[0];
+    b = S.result[1];
+    return true;
+}
+
+// A stored point's twelve neighbours: offsets per axis to -1, +1, -2, +2, the
+// low ones mirrored (-1 to 0, -2 to 1); `have` leaves out the Dirichlet planes,
+// where the residual is zero.
+struct Neighbours {
+    int off[12];
+    unsigned have;
+    __device__ __forceinline__ Neighbours(int i, int j, int k, int nx, int ny, int nz) {
+        const int at[3] = {i, j, k}, n[3] = {nx, ny, nz}, st[3] = {1, nx, nx * ny};
+        have = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const int q = at[d], s = st[d];
+            const bool in[4] = {true, q + 1 < n[d], q > 0 || n[d] > 1, q + 2 < n[d]};
+            const int o[4] = {q >= 1 ? -s : 0, s, q >= 2 ? -2 * s : (q == 1 ? -s : s), 2 * s};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                off[4 * d + u] = in[u] ? o[u] : 0;
+                have |= (in[u] ? 1u : 0u) << (4 * d + u);
+            }
+        }
+    }
+};
+
+// Laplacian of the residual at the point c, whose neighbours carry `tag`.
+__device__ __forceinline__ double lap_res(const ulonglong2* c, double centre, const Neighbours& nb,
+                                          double k0, double k1, double k2, unsigned tag, int* fail) {
+    double v[12];
+    const long long t0 = clock64();
+    while (true) {
+        ulonglong2 w[12];
+#pragma unroll
+        for (int u = 0; u < 12; ++u) w[u] = get_words(c + nb.off[u]);
+        unsigned bad = 0;
+#pragma unroll
+        for (int u = 0; u < 12; ++u) {
+            bad |= differs(w[u], tag);
+            v[u] = nb.have >> u & 1u ? value_of(w[u]) : 0.0;
+        }
+        if (bad == 0) break;
+        if (clock64() - t0 > kWaitCycles) {
+            *fail = 1;
+            break;
+        }
+    }
+    const double one = ((v[0] + v[1]) + (v[4] + v[5])) + (v[8] + v[9]);
+    const double two = ((v[2] + v[3]) + (v[6] + v[7])) + (v[10] + v[11]);
+    return fma(k2, two, fma(k1, one, k0 * centre));
+}
+
+// R points per thread: point q of thread t is t + q * (threads of the grid).
+template <int R>
+__global__ void __launch_bounds__(512, 1) k_cg(CgArgs a) {
+    __shared__ CgShared S;
+    if (threadIdx.x == 0) S.fail = 0;
+    // no rank writes to another's shared memory before that one has started
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    unsigned tag = a.tag;   // of the last sums and of the residual before them
+    const int V = a.nx * a.ny * a.nz;
+    const int stride = (int)(gridDim.x * blockDim.x);
+    const int t0 = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    const double k0 = -7.5 * a.inv_dx2, k1 = 4.0 / 3.0 * a.inv_dx2, k2 = -1.0 / 12.0 * a.inv_dx2;
+    double sol[R], res[R], p[R], s[R];   // s = Lap(p)
+    int ci[R], cj[R], ck[R];
+
+    // r0 = src - Lap(sol)
+    double bb = 0.0, unused;
+    if (a.rel > 0.0) ++tag;
+    ++tag;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int v = t0 + q * stride;
+        sol[q] = res[q] = p[q] = s[q] = 0.0;
+        ci[q] = v % a.nx;
+        cj[q] = (v / a.nx) % a.ny;
+        ck[q] = v / (a.nx * a.ny);
+        if (v >= V) continue;
+        const long o = ci[q] + a.mx * (cj[q] + (long)a.my * ck[q]);
+        sol[q] = a.sol[o];
+        res[q] = a.src[o] - lap_at(a.sol, ci[q], cj[q], ck[q], a.mx, a.my, a.inv_dx2);
+        put_tagged(a.res + v, res[q], tag);
+        bb = fma(a.src[o], a.src[o], bb);
+    }
     double prec = a.prec;
     if (a.rel > 0.0) {
         // |src|^2 over the stored box for the relative test
-        loc = 0.0;
-        for (long o = t0; o < M; o += stride) {
-            const int i = (int)(o % a.mx), j = (int)((o / a.mx) % a.my);
-            const int k = (int)(o / ((long)a.mx * a.my));
-            if (i < a.nx && j < a.ny && k < a.nz) loc = fma(a.src[o], a.src[o], loc);
-        }
-        s = block_sum(loc, sh);
-        if (threadIdx.x == 0) red1[blockIdx.x] = s;
+        if (!grid_sum(S, a.mail, a.status, tag - 1, bb, 0.0, bb, unused, []() {},
+                      [](double x, double, double& u, double& w) { u = x; w = 0.0; }))
+            return;
+        prec = a.rel * a.rel * bb;
     }
-    if (!grid_barrier(a.bar, a.status)) return;
-    double pnorm = grid_total(red2, &bcast);
-    if (a.rel > 0.0) {
-        prec = a.rel * a.rel * grid_total(red1, &bcast);
-        // every block has read red1 before the first iteration rewrites it
-        if (!grid_barrier(a.bar, a.status)) return;
-    }
-    int it;
-    for (it = 1; it <= a.maxit; ++it) {
-        // t = Lap(p), integral = r.t
-        loc = 0.0;
-        for (long o = t0; o < M; o += stride) {
-            const int i = (int)(o % a.mx), j = (int)((o / a.mx) % a.my), k = (int)(o / ((long)a.mx * a.my));
-            double lap = 0.0;
-            if (i < a.nx && j < a.ny && k < a.nz) lap = lap_at(a.p, i, j, k, a.mx, a.my, a.inv_dx2);
-            a.t[o] = lap;
-            loc = fma(a.res[o], lap, loc);
+    const Neighbours nb0(ci[0], cj[0], ck[0], a.nx, a.ny, a.nz);
+    // of warp 0: |r|^2 and |r|^2 / alpha of the iteration before, the inverses
+    // of |r|^2 and alpha
+    double rr_old = 0.0, d_old = 0.0, inv_rr = 0.0, inv_alpha = 0.0;
+    int it = 0;
+    bool done = false;
+    for (;; ++it) {
+        double rr = 0.0, rw = 0.0, lap[R];
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            lap[q] = 0.0;
+            const int v = t0 + q * stride;
+            if (v >= V) continue;
+            lap[q] = lap_res(a.res + v, res[q],
+                             q == 0 ? nb0 : Neighbours(ci[q], cj[q], ck[q], a.nx, a.ny, a.nz), k0, k1, k2,
+                             tag, &S.fail);
+            rr = fma(res[q], res[q], rr);
+            rw = fma(res[q], lap[q], rw);
         }
-        s = block_sum(loc, sh);
-        if (threadIdx.x == 0) red1[blockIdx.x] = s;
-        if (!grid_barrier(a.bar, a.status)) return;
-        const double integral = grid_total(red1, &bcast);
-        const double ak = pnorm / integral;
-        loc = 0.0;
-        for (long o = t0; o < M; o += stride) {
-            a.sol[o] = fma(ak, a.p[o], a.sol[o]);
-            const double r = fma(-ak, a.t[o], a.res[o]);
-            a.res[o] = r;
-            loc = fma(r, r, loc);
+        double alpha, beta;
+        // beta = rr / rr_old, alpha = rr / (rw - beta rr / alpha_old); a negative
+        // beta says that the test is met (rr <= prec)
+        if (!grid_sum(
+                S, a.mail, a.status, tag, rr, rw, alpha, beta,
+                [&]() {
+                    if (it == 0) return;
+                    inv_rr = inverse(rr_old);
+                    inv_alpha = d_old * inv_rr;
+                },
+                [&](double x, double y, double& u, double& w) {
+                    const double b = x * inv_rr;
+                    d_old = fma(-b, x * inv_alpha, y);
+                    rr_old = x;
+                    u = x * inverse(d_old);
+                    w = it > 0 && x <= prec ? -1.0 : b;
+                }))
+            return;
+        done = beta < 0.0;
+        if (done || it == a.maxit) break;
+        ++tag;
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+            s[q] = fma(beta, s[q], lap[q]);
+            const double r = fma(-alpha, s[q], res[q]);
+            if (t0 + q * stride < V) put_tagged(a.res + t0 + q * stride, r, tag);
+            p[q] = fma(beta, p[q], res[q]);
+            sol[q] = fma(alpha, p[q], sol[q]);
+            res[q] = r;
         }
-        s = block_sum(loc, sh);
-        if (threadIdx.x == 0) red2[blockIdx.x] = s;
-        if (!grid_barrier(a.bar, a.status)) return;
-        const double nn = grid_total(red2, &bcast);
-        if (nn <= prec) break;
-        const double ck = nn / pnorm;
-        pnorm = nn;
-        for (long o = t0; o < M; o += stride) a.p[o] = fma(ck, a.p[o], a.res[o]);
-        if (!grid_barrier(a.bar, a.status)) return;
     }
+#pragma unroll
+    for (int q = 0; q < R; ++q)
+        if (t0 + q * stride < V) a.sol[ci[q] + a.mx * (cj[q] + (long)a.my * ck[q])] = sol[q];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        a.status[1] = it > a.maxit ? a.maxit : it;
-        if (it > a.maxit && a.status[0] == 0) a.status[0] = 1;
+        a.status[1] = it;
+        if (!done && a.status[0] == 0) a.status[0] = 1;
     }
 }
+
+// Launch shape of the CG: clusters of eight blocks with up to 128 points each
+// until the card is full, then more threads, then two, four or eight points
+// per thread.  More blocks cost mail, more points per block FP64 issue: per
+// iteration at 10^3 3.9 us with 64 points a block, 3.25 with 128, 4.2 with 256;
+// at 16^3 4.27, 4.29 and 4.8; at 20^3 4.37 with 128 and 5.2 with 256.
+struct CgShape {
+    const void* fn;
+    int blocks, threads;
+};
+constexpr int kCgThreads = 512;
+CgShape cg_shape(const mg_ctx* c) {
+    constexpr long kPer = 128L * kCluster;
+    const int clusters = (int)std::max<long>(1, std::min<long>(c->cg_clusters, (c->V + kPer - 1) / kPer));
+    const int blocks = clusters * kCluster;
+    const long per = (c->V + blocks - 1) / blocks;
+    int r = 1;
+    while (r < 8 && (per + r - 1) / r > 256) r *= 2;
+    const int threads = (int)(((per + r - 1) / r + 31) / 32 * 32);
+    const void* fn = r == 1   ? (const void*)k_cg<1>
+                     : r == 2 ? (const void*)k_cg<2>
+                     : r == 4 ? (const void*)k_cg<4>
+                              : (const void*)k_cg<8>;
+    return CgShape{fn, blocks, threads};
+}
+// the residuals, then the mailboxes
+size_t cg_tagged_bytes(const mg_ctx* c) {
+    return ((size_t)c->V + 4 * (size_t)cg_shape(c).blocks * kMaxClusters) * sizeof(ulonglong2);
+}
+
+// The launch of a CG shape: cooperative (its blocks wait for one another), in
+// clusters.
+struct CgLaunch {
+    cudaLaunchAttribute attr[2];
+    cudaLaunchConfig_t cfg;
+    CgLaunch(int blocks, int threads, cudaStream_t stream) : attr{}, cfg{} {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kCluster;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeCooperative;
+        attr[1].val.cooperative = 1;
+        cfg.gridDim = dim3(blocks);
+        cfg.blockDim = dim3(threads);
+        cfg.stream = stream;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+    }
+};
 
 // Source and multipole Dirichlet values on the extended box.
 __global__ void k_coulomb_bound(const double* __restrict__ rho_p, const double* __restrict__ sh,
@@ -444,16 +692,19 @@ int coulomb_setup(mg_ctx* c) {
     MG_CUDA(cudaMemcpy(c->cpot, guess.data(), M * sizeof(double), cudaMemcpyHostToDevice));
     MG_CUDA(cudaMalloc(&c->cguess, M * sizeof(double)));
     MG_CUDA(cudaMemcpy(c->cguess, guess.data(), M * sizeof(double), cudaMemcpyHostToDevice));
-    MG_CUDA(cudaMalloc(&c->cg_bar, 4 * sizeof(unsigned)));
     MG_CUDA(cudaMalloc(&c->cg_status, 4 * sizeof(int)));
-    int per_sm = 0;
-    MG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg, kThreads, 0));
-    if (per_sm < 1) return MG_ERR_CUDA;
-    // The CG runs 4 grid barriers per iteration on a small box (26^3 for a
-    // 24^3 mesh): about two mesh points per thread and few blocks make the
-    // barriers cheaper than spreading the points over every SM (measured on
-    // GB300: 32 blocks beat 152 by ~1.3 ms per solve at 26^3).
-    c->cg_blocks = std::max(1, std::min(c->num_sms, std::max(8, div_up(M, 2 * kThreads))));
+    // clusters that the card holds at once, whatever the shape
+    c->cg_clusters = kMaxClusters;
+    for (const void* fn : {(const void*)k_cg<1>, (const void*)k_cg<2>, (const void*)k_cg<4>,
+                           (const void*)k_cg<8>}) {
+        CgLaunch L(kCluster, kCgThreads, c->stream);
+        int n = 0;
+        MG_CUDA(cudaOccupancyMaxActiveClusters(&n, fn, &L.cfg));
+        c->cg_clusters = std::min(c->cg_clusters, n);
+    }
+    if (c->cg_clusters < 1 || cg_shape(c).threads > kCgThreads) return MG_ERR_CUDA;
+    MG_CUDA(cudaMalloc(&c->cg_tagged, cg_tagged_bytes(c)));
+    MG_CUDA(cudaMemset(c->cg_tagged, 0, cg_tagged_bytes(c)));
     // eigendecompositions of the three 1-D operators for the direct solve
     {
         const int ns[3] = {nx, ny, nz};
@@ -624,19 +875,30 @@ int coulomb_solve(mg_ctx* c, int* iters) {
         if (iters) *iters = 2;
         return MG_OK;
     }
-    MG_CUDA(cudaMemsetAsync(c->cg_bar, 0, 4 * sizeof(unsigned), c->stream));
     MG_CUDA(cudaMemsetAsync(c->cg_status, 0, 4 * sizeof(int), c->stream));
+    const int maxit = c->p.coulomb_max > 0 ? c->p.coulomb_max : 500;
+    // tags run on from solve to solve, so nothing is cleared between them
+    // until they come near the end of 32 bits
+    const unsigned span = (unsigned)maxit + 8u;
+    if (c->cg_tag > 0xFFFFFFFFu - span) {
+        MG_CUDA(cudaMemsetAsync(c->cg_tagged, 0, cg_tagged_bytes(c), c->stream));
+        c->cg_tag = 0;
+    }
     CgArgs a;
-    a.sol = c->cpot; a.res = c->cres; a.p = c->cp; a.t = c->ct; a.src = c->csource;
-    a.red = c->red; a.bar = c->cg_bar; a.status = c->cg_status;
-    a.nx = c->nx; a.ny = c->ny; a.nz = c->nz; a.mx = c->mx; a.my = c->my; a.mz = c->mz;
+    a.sol = c->cpot; a.src = c->csource;
+    a.res = c->cg_tagged; a.mail = c->cg_tagged + c->V;
+    a.tag = c->cg_tag;
+    c->cg_tag += span;
+    a.status = c->cg_status;
+    a.nx = c->nx; a.ny = c->ny; a.nz = c->nz; a.mx = c->mx; a.my = c->my;
     a.inv_dx2 = 1.0 / (c->p.dx * c->p.dx);
     a.prec = 1.0e-9 / (c->p.dx * c->p.dx * c->p.dx * c->nx * c->ny * c->nz);
     a.rel = c->p.coulomb_prec > 0 ? c->p.coulomb_prec : 0.0;
-    a.maxit = c->p.coulomb_max > 0 ? c->p.coulomb_max : 500;
+    a.maxit = maxit;
     void* args[] = {&a};
-    MG_CUDA(cudaLaunchCooperativeKernel((const void*)k_cg, dim3(c->cg_blocks), dim3(kThreads), args,
-                                        0, c->stream));
+    const CgShape shape = cg_shape(c);
+    CgLaunch L(shape.blocks, shape.threads, c->stream);
+    MG_CUDA(cudaLaunchKernelExC(&L.cfg, shape.fn, args));
     ++c->launches;
     const double pi = 4.0 * std::atan2(1.0, 1.0);
     const double fac = -std::pow(3 / pi, 1 / 3.0) * c->f.e2;

@@ -42,7 +42,7 @@ void free_all(mg_ctx* c) {
     F(c->gs_S); F(c->gs_R); F(c->gs_index);
     F(c->cpot); F(c->csource); F(c->cres); F(c->cp); F(c->ct); F(c->sh_ext); F(c->sh_mesh);
     F(c->coulomb); F(c->coulex); F(c->moment_values); F(c->rpow_ext); F(c->mfac);
-    F(c->cg_bar); F(c->cg_status); F(c->red); F(c->flags); F(c->cfast); F(c->cguess);
+    F(c->cg_tagged); F(c->cg_status); F(c->red); F(c->flags); F(c->cfast); F(c->cguess);
     F(c->dhist); F(c->Uold); F(c->Sold); F(c->Wold); F(c->pc_buf); F(c->pc_jobs); F(c->jmunu); F(c->jmunu_hist);
     F(c->odd); F(c->odd_hist); F(c->Apot); F(c->Spot); F(c->divA); F(c->odd_der); F(c->odd_tmp);
     F(c->odd_jobs);

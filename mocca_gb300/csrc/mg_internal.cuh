@@ -295,10 +295,11 @@ struct mg_ctx {
     double* moment_values = nullptr;   // [n_moments][2]
     double* rpow_ext = nullptr;        // r^(2l+1) on the extended box per moment
     double* mfac = nullptr;            // 4 pi / (2l+1) per moment
-    unsigned* cg_bar = nullptr;        // grid barrier state of the CG kernel
+    ulonglong2* cg_tagged = nullptr;   // the CG kernel's residuals and partial sums
+    unsigned cg_tag = 0;               // last tag its launches may have used
+    int cg_clusters = 0;               // clusters of its blocks that run at once
     int* cg_status = nullptr;          // [state, iterations]
     int* h_cg_status = nullptr;        // pinned host copy
-    int cg_blocks = 0;
     double* red = nullptr;             // reduction scratch
     size_t red_len = 0;
     int* flags = nullptr;              // device status flags
