@@ -32,6 +32,7 @@
 #include <algorithm>
 #include <cmath>
 
+#include "cgsum.cuh"
 #include "mg_internal.cuh"
 
 namespace mg {
@@ -40,7 +41,6 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr long long kWaitCycles = 4000000000LL;   // ~2 s at the top SM clock
-constexpr int kCluster = 8;       // blocks of a cluster of the CG kernel
 constexpr int kMaxClusters = 32;  // sums of a meeting, one per lane
 
 struct CgArgs {
@@ -93,103 +93,24 @@ __device__ __forceinline__ double value_of(const ulonglong2& w) {
     return __hiloint2double((int)(unsigned)w.x, (int)(unsigned)w.y);
 }
 
-// Sums of x and of y over the warp in one chain of five adds: after the first
-// exchange the lower half-warp carries x, the upper one y.  Lane 0 ends with
-// the sum of x, lane 16 with that of y.
-__device__ __forceinline__ double warp_sum2(double x, double y) {
-    const bool up = (threadIdx.x & 16) != 0;
-    double v = (up ? y : x) + __shfl_xor_sync(0xffffffffu, up ? x : y, 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// 1 / d by Newton's iteration from the float reciprocal (a CG coefficient:
-// right to an ulp or two; an FP64 divide takes 549 clocks).  The float comes
-// and goes by bit moves, as FP64 conversions wait for the FP64 pipe.
-__device__ __forceinline__ double inverse(double d) {
-    const unsigned hi = (unsigned)__double2hiint(d), e = (hi >> 20) & 0x7FFu;
-    if (e < 1023 - 100 || e > 1023 + 100) return 1.0 / d;
-    float f = __uint_as_float((hi & 0x80000000u) | ((hi & 0x7FFFFFFFu) - (896u << 20)) << 3 |
-                              (unsigned)__double2loint(d) >> 29);
-    asm("rcp.approx.ftz.f32 %0, %0;" : "+f"(f));
-    const unsigned u = __float_as_uint(f);
-    double x = __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7FFFFFFFu) >> 3) + (896u << 20))),
-                                (int)(u << 29));
-    x = fma(x, fma(-d, x, 1.0), x);
-    return fma(x, fma(-d, x, 1.0), x);
-}
-
-// What the blocks of a cluster leave in each other's shared memory.
-struct CgShared {
-    double part[2][2][kCluster];   // [turn][x, y][rank]: the ranks' partial sums
-    int bad[2][kCluster];          // a wait of that rank ran out
-    double warp[2][16];
-    double result[2];
-    int fail;
-};
-
-__device__ __forceinline__ uint32_t remote(const void* p, int rank) {
-    uint32_t a = (uint32_t)__cvta_generic_to_shared(p), r;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
-    return r;
-}
-
 // Sums x and y over the grid; warp 0 of every block applies `then` to the
 // totals (the same bits everywhere) and gives its two results to its threads.
-// `meanwhile` is work of warp 0 for the time that the barrier takes.  `turn`
-// alternates from call to call: what is left for a turn has been read when that
-// turn comes again, because the call in between needed every block.
+// `meanwhile` is work of warp 0 for the time that the cluster's barrier takes.
+// The tag's parity picks the turn: what is left for a turn has been read when
+// that turn comes again, because the call in between needed every block.
 template <class Meanwhile, class Then>
-__device__ bool grid_sum(CgShared& S, ulonglong2* mail, int* status, unsigned tag, double x, double y,
+__device__ bool grid_sum(ClusterSum& S, ulonglong2* mail, int* status, unsigned tag, double x, double y,
                          double& a, double& b, Meanwhile meanwhile, Then then) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int turn = (int)(tag & 1u);
     const int rank = (int)(blockIdx.x % kCluster), cluster = (int)(blockIdx.x / kCluster);
     const int nclusters = (int)(gridDim.x / kCluster);
-    double v = warp_sum2(x, y);
-    if (nw > 1) {
-        if ((lane & 15) == 0) S.warp[lane >> 4][warp] = v;
-        __syncthreads();
-        if (warp == 0) {
-            v = (lane & 15) < nw ? S.warp[lane >> 4][lane & 15] : 0.0;
-#pragma unroll
-            for (int o = 8; o > 0; o >>= 1)
-                if (o < nw) v += __shfl_xor_sync(0xffffffffu, v, o);
-        }
-    }
-    if (warp == 0) {
-        // lane r of the lower half sends x, of the upper half y, to rank r
-        v = __shfl_sync(0xffffffffu, v, lane & 16);
-        if ((lane & 15) < kCluster) {
-            const uint32_t p = remote(&S.part[turn][lane >> 4][rank], lane & 15);
-            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(p), "d"(v) : "memory");
-            if (lane < kCluster) {
-                const uint32_t f = remote(&S.bad[turn][rank], lane);
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(f), "r"(S.fail) : "memory");
-            }
-        }
-    }
-    // every rank's partials are here after this (threads that have left count
-    // as arrived)
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    if (warp == 0) meanwhile();
-    __syncwarp();
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    int bad = 0;
-#pragma unroll
-    for (int r = 0; r < kCluster; ++r) bad |= S.bad[turn][r];
-    if (bad) {
+    if (!cluster_sum(S, turn, rank, x, y, meanwhile)) {
         // all ranks of the cluster leave here together
         if (threadIdx.x == 0) atomicExch(status, 2);
         return false;
     }
     if (warp == 0) {
-        v = S.part[turn][lane >> 4][lane % kCluster];
-#pragma unroll
-        for (int o = kCluster / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        x = __shfl_sync(0xffffffffu, v, 0);
-        y = __shfl_sync(0xffffffffu, v, 16);
         if (nclusters > 1) {
             ulonglong2* box = mail + (size_t)turn * gridDim.x * kMaxClusters * 2;
             if (rank == 0) {
@@ -219,7 +140,7 @@ __device__ bool grid_sum(CgShared& S, ulonglong2* mail, int* status, unsigned ta
             }
             if (!ok) S.fail = 1;   // read by warp 0 at the next call
             __syncwarp();
-            v = warp_sum2(x, y);
+            const double v = warp_sum2(x, y);
             x = __shfl_sync(0xffffffffu, v, 0);
             y = __shfl_sync(0xffffffffu, v, 16);
         }
@@ -287,12 +208,14 @@ __device__ __forceinline__ double lap_res(const ulonglong2* c, double centre, co
 
 // R points per thread: point q of thread t is t + q * (threads of the grid).
 template <int R>
-__global__ void __launch_bounds__(512, 1) k_cg(CgArgs a) {
-    __shared__ CgShared S;
+__global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(512, 1) k_cg(CgArgs a) {
+    __shared__ ClusterSum S;
+    if (!in_cluster()) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) a.status[0] = 3;
+        return;
+    }
     if (threadIdx.x == 0) S.fail = 0;
-    // no rank writes to another's shared memory before that one has started
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    cluster_barrier();   // no rank writes to another's shared memory before that one has started
     unsigned tag = a.tag;   // of the last sums and of the residual before them
     const int V = a.nx * a.ny * a.nz;
     const int stride = (int)(gridDim.x * blockDim.x);
@@ -414,25 +337,6 @@ CgShape cg_shape(const mg_ctx* c) {
 size_t cg_tagged_bytes(const mg_ctx* c) {
     return ((size_t)c->V + 4 * (size_t)cg_shape(c).blocks * kMaxClusters) * sizeof(ulonglong2);
 }
-
-// The launch of a CG shape: cooperative (its blocks wait for one another), in
-// clusters.
-struct CgLaunch {
-    cudaLaunchAttribute attr[2];
-    cudaLaunchConfig_t cfg;
-    CgLaunch(int blocks, int threads, cudaStream_t stream) : attr{}, cfg{} {
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = kCluster;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeCooperative;
-        attr[1].val.cooperative = 1;
-        cfg.gridDim = dim3(blocks);
-        cfg.blockDim = dim3(threads);
-        cfg.stream = stream;
-        cfg.attrs = attr;
-        cfg.numAttrs = 2;
-    }
-};
 
 // Source and multipole Dirichlet values on the extended box.
 __global__ void k_coulomb_bound(const double* __restrict__ rho_p, const double* __restrict__ sh,
@@ -697,9 +601,17 @@ int coulomb_setup(mg_ctx* c) {
     c->cg_clusters = kMaxClusters;
     for (const void* fn : {(const void*)k_cg<1>, (const void*)k_cg<2>, (const void*)k_cg<4>,
                            (const void*)k_cg<8>}) {
-        CgLaunch L(kCluster, kCgThreads, c->stream);
+        cudaLaunchAttribute attr{};
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kCluster;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kCluster);
+        cfg.blockDim = dim3(kCgThreads);
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
         int n = 0;
-        MG_CUDA(cudaOccupancyMaxActiveClusters(&n, fn, &L.cfg));
+        MG_CUDA(cudaOccupancyMaxActiveClusters(&n, fn, &cfg));
         c->cg_clusters = std::min(c->cg_clusters, n);
     }
     if (c->cg_clusters < 1 || cg_shape(c).threads > kCgThreads) return MG_ERR_CUDA;
@@ -897,8 +809,9 @@ int coulomb_solve(mg_ctx* c, int* iters) {
     a.maxit = maxit;
     void* args[] = {&a};
     const CgShape shape = cg_shape(c);
-    CgLaunch L(shape.blocks, shape.threads, c->stream);
-    MG_CUDA(cudaLaunchKernelExC(&L.cfg, shape.fn, args));
+    // cooperative: its blocks wait for one another
+    MG_CUDA(cudaLaunchCooperativeKernel(shape.fn, dim3(shape.blocks), dim3(shape.threads), args, 0,
+                                        c->stream));
     ++c->launches;
     const double pi = 4.0 * std::atan2(1.0, 1.0);
     const double fac = -std::pow(3 / pi, 1 / 3.0) * c->f.e2;
@@ -911,6 +824,7 @@ int coulomb_solve(mg_ctx* c, int* iters) {
         MG_CUDA(cudaStreamSynchronize(c->stream));
         *iters = c->h_cg_status[1];
         if (c->h_cg_status[0] == 2) return MG_ERR_TIMEOUT;
+        if (c->h_cg_status[0] == 3) return MG_ERR_CUDA;
         if (c->h_cg_status[0] == 1) return MG_NOT_CONVERGED;
     }
     return MG_OK;

@@ -343,6 +343,7 @@ struct mg_ctx {
     bool have_uold = false;            // UpotOld not all zero
     double* pc_buf = nullptr;          // preconditioner CG: res, dir, upd, lap, inv (10V)
     mg::GridJob* pc_jobs = nullptr;    // Laplacians of the two directions
+    int8_t pc_slots[8][3] = {};        // matrix slots of the symmetry classes
 
     double pairing_energy[2] = {0.0, 0.0};
     long long launches = 0;
