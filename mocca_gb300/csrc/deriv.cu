@@ -28,6 +28,14 @@ namespace {
 
 constexpr int kThreads = 256;
 constexpr int kColTile = 32;  // (x,y) columns per k_deriv_z block
+// Fewer grids than this go to k_deriv_few: in FP64 on every mesh (UpdateDensities
+// and ConstructPotentials of two spwfs, 2 and 20 grids: 29 and 57 us against 72
+// and 109 at 24^3, 427 and 859 against 1260 and 2266 at 64^3), in double-float
+// up to so many points in all, since it splits a line's values again for every
+// output (2 grids at 36^3: 77 us against 90, at 48^3: 121 against 124; 20 grids
+// at 18^3: 54 against 60, at 24^3: 74 against 70, at 36^3: 196 against 149)
+constexpr int kFewGrids = 64;
+constexpr long kFewMaxDf = 200000;
 
 struct MatPtrs {
     const double* m[3][2][2];  // [axis][kind][slot]
@@ -328,6 +336,97 @@ MatPtrs32 mat_ptrs32(const mg_ctx* c) {
     return mp;
 }
 
+// ---- few grids (densities, fields, the estimation probe) -----------------------
+//
+// One launch, a thread per point, grid and axis (warp a of a block has axis a
+// of its 32 points, and the Laplacian's three parts meet in shared memory; of a
+// grid with one derivative the block has 96 points), matrices and lines read
+// through L1: a handful of grids gives the plane and
+// column kernels above too few blocks (a plane each) to fill the card, and
+// the sums are chains of latencies (an FP64 FMA takes 64 clocks).  They run in
+// the same order with the same roundings.  grad rho and lap rho of both
+// isospins at 24^3 (under ncu): 13 us against 57 in FP64; at 21 x 23 x 27 in
+// double-float 26 against 62.
+constexpr int kFewPts = 32;
+
+// Axis and point of a thread of k_deriv_few; a point past the grid when it
+// has none.
+__device__ __forceinline__ void few_place(const GridJob& J, int V, int& a, int& v) {
+    const int w = threadIdx.x / kFewPts, lane = threadIdx.x % kFewPts;
+    const bool one = !J.lap && (J.dx != nullptr) + (J.dy != nullptr) + (J.dz != nullptr) == 1;
+    a = one ? (J.dx ? 0 : (J.dy ? 1 : 2)) : w;
+    v = ((int)blockIdx.x * (one ? 3 : 1) + (one ? w : 0)) * kFewPts + lane;
+}
+
+__global__ void __launch_bounds__(3 * kFewPts)
+k_deriv_few(const GridJob* __restrict__ jobs, MatPtrs mp, int nx, int ny, int nz) {
+    __shared__ double part[3][kFewPts];
+    const GridJob J = jobs[blockIdx.y];
+    const int V = nx * ny * nz, lane = threadIdx.x % kFewPts;
+    int a, v;
+    few_place(J, V, a, v);
+    double* const out = a == 0 ? J.dx : (a == 1 ? J.dy : J.dz);
+    if (v < V && (out || J.lap)) {
+        const int n = a == 0 ? nx : (a == 1 ? ny : nz);
+        const int st = a == 0 ? 1 : (a == 1 ? nx : nx * ny);
+        const int at = a == 0 ? v % nx : (a == 1 ? (v / nx) % ny : v / (nx * ny));
+        const int slot = a == 0 ? J.slot[0] : (a == 1 ? J.slot[1] : J.slot[2]);
+        const double* d1 = mp.m[a][0][slot ? 1 : 0] + at;
+        const double* d2 = mp.m[a][1][slot ? 1 : 0] + at;
+        const double* in = J.in + (v - at * st);
+        double s1 = 0.0, s2 = 0.0;
+        if (J.lap) {
+#pragma unroll 8
+            for (int q = 0; q < n; ++q) {
+                const double x = in[q * st];
+                s1 = fma(d1[q * n], x, s1);
+                s2 = fma(d2[q * n], x, s2);
+            }
+        } else {
+#pragma unroll 8
+            for (int q = 0; q < n; ++q) s1 = fma(d1[q * n], in[q * st], s1);
+        }
+        if (out) out[v] = s1;
+        part[a][lane] = s2;
+    }
+    if (!J.lap) return;
+    __syncthreads();
+    if (a == 0 && v < V) J.lap[v] = (part[0][lane] + part[1][lane]) + part[2][lane];
+}
+
+__global__ void __launch_bounds__(3 * kFewPts)
+k_deriv_few_df(const GridJob* __restrict__ jobs, MatPtrs32 mp, int nx, int ny, int nz) {
+    __shared__ float2 part[3][kFewPts];
+    const GridJob J = jobs[blockIdx.y];
+    const int V = nx * ny * nz, lane = threadIdx.x % kFewPts;
+    int a, v;
+    few_place(J, V, a, v);
+    double* const out = a == 0 ? J.dx : (a == 1 ? J.dy : J.dz);
+    if (v < V && (out || J.lap)) {
+        const int n = a == 0 ? nx : (a == 1 ? ny : nz);
+        const int st = a == 0 ? 1 : (a == 1 ? nx : nx * ny);
+        const int at = a == 0 ? v % nx : (a == 1 ? (v / nx) % ny : v / (nx * ny));
+        const int slot = a == 0 ? J.slot[0] : (a == 1 ? J.slot[1] : J.slot[2]);
+        const int ld = mp.ld4[a], lo = n * ld;
+        const float* d1 = mp.m[a][0][slot ? 1 : 0] + at;
+        const float* d2 = mp.m[a][1][slot ? 1 : 0] + at;
+        const double* in = J.in + (v - at * st);
+        float h1 = 0.f, l1 = 0.f, h2 = 0.f, l2 = 0.f;
+#pragma unroll 8
+        for (int q = 0; q < n; ++q) {
+            const dfl x = df_split(in[q * st]);
+            df_acc(h1, l1, dfl{d1[q * ld], d1[lo + q * ld]}, x);
+            if (J.lap) df_acc(h2, l2, dfl{d2[q * ld], d2[lo + q * ld]}, x);
+        }
+        if (out) out[v] = df_to(df_norm(dfl{h1, l1}));
+        df_st(&part[a][lane], df_norm(dfl{h2, l2}));
+    }
+    if (!J.lap) return;
+    __syncthreads();
+    if (a == 0 && v < V)
+        J.lap[v] = df_to(df_add(df_ld(&part[0][lane]), df_ld(&part[1][lane]))) + df_to(df_ld(&part[2][lane]));
+}
+
 MatPtrs mat_ptrs(const mg_ctx* c) {
     MatPtrs mp;
     for (int a = 0; a < 3; ++a)
@@ -468,6 +567,16 @@ static int tuned_planes(mg_ctx* c, int& slot, Launch launch_xy) {
 int run_jobs(mg_ctx* c, const GridJob* jobs, int njobs, bool out_df) {
     if (njobs <= 0) return MG_OK;
     const int nx = c->nx, ny = c->ny, nz = c->nz;
+    const bool mixed = c->cur_precision == MG_MIXED;
+    if (njobs < kFewGrids && !out_df && (!mixed || njobs * c->V <= kFewMaxDf)) {
+        const dim3 grid(div_up(c->V, kFewPts), njobs);
+        if (mixed)
+            k_deriv_few_df<<<grid, 3 * kFewPts, 0, c->stream>>>(jobs, mat_ptrs32(c), nx, ny, nz);
+        else
+            k_deriv_few<<<grid, 3 * kFewPts, 0, c->stream>>>(jobs, mat_ptrs(c), nx, ny, nz);
+        MG_LAUNCHED(c);
+        return MG_OK;
+    }
     // z planes per k_deriv_xy block, tuned per (form, grid-count class):
     // few grids (densities, fields) and whole bases
     int& ppb = c->deriv_planes[c->cur_precision == MG_MIXED ? 1 : 0][njobs < 64 ? 0 : 1];
