@@ -5,7 +5,7 @@
 // src/HFB.f90:5880-6087) at a small fraction of that, so the FP64 work is
 // arranged as batched GEMMs and the sequential part runs in FP32:
 //
-//   1. k_jacobi32: cyclic two-sided Jacobi in FP32, one CTA per matrix, the
+//   1. k_jacobi32: cyclic two-sided Jacobi in FP32, two CTAs per matrix, the
 //      n/2 rotations of a round-robin round applied in parallel (rows, then
 //      columns and vectors), optionally warm-started from earlier vectors
 //      (B = X^T A X).  Eigenpairs sorted ascending.
@@ -127,7 +127,7 @@ __device__ void smem_mm32(const float* A, const float* B, float* C, int n, int l
     }
 }
 
-// One matrix per CTA.  A: FP64 n x n (lda) input; Xw: optional FP64 warm
+// One matrix per CTA pair.  A: FP64 n x n (lda) input; Xw: optional FP64 warm
 // start (n x n, ldx); X: FP64 output vectors (n x n, ldx, column k <-> w[k]);
 // w: eigenvalues ascending.  n <= kEigMax.  Above kJSmemMax the warm start's
 // product A V goes through X (FP64) instead of a third shared-memory plane;
@@ -141,17 +141,73 @@ __device__ void smem_mm32(const float* A, const float* B, float* C, int n, int l
 // kJacobiSkip |A| (FP32 rounding of the matrix entries is ~6e-8 |A|); a
 // round without such a pair is skipped, which makes the later sweeps of a
 // warm start cheap.
-__global__ void __launch_bounds__(kJThreads)
+//
+// A matrix has a cluster of two CTAs.  One CTA's rounds are bound by instruction
+// issue and its barriers (60% of the slots at n = 92), and half of that work is
+// V, which the rounds never read: side 0 rotates A and hands each round's (c, s)
+// through a ring to side 1, which rotates V some rounds behind.  Four matrices of
+// 92 from a cold start: 357 us, 534 in one CTA each.
+constexpr int kRing = 4;
+struct JacobiRing {
+    float2 cs[kRing][kEigMax / 2];
+    int round[kRing];       // the round's number, -1: no more
+    uint64_t full[kRing];   // of side 1: the bytes of a round have come
+    uint64_t empty[kRing];  // of side 0: side 1 has used the slot
+};
+
+__device__ __forceinline__ uint32_t shared_addr(const void* p) {
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ uint32_t peer_addr(const void* p, int side) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(shared_addr(p)), "r"(side));
+    return r;
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(shared_addr(bar)), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(bar)),
+                 "r"(bytes)
+                 : "memory");
+}
+// Arrival (release) at a barrier of the other CTA.
+__device__ __forceinline__ void peer_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Wait (acquire) for phase `parity` of an own barrier, ~2 s at most.
+__device__ __forceinline__ bool ring_wait(uint64_t* bar, uint32_t parity) {
+    const long long t0 = clock64();
+    while (true) {
+        uint32_t done;
+        asm volatile(
+            "{\n.reg .pred p;\n"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+            "selp.b32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(shared_addr(bar)), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if (clock64() - t0 > 4000000000LL) return false;
+    }
+}
+__device__ __forceinline__ void pair_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kJThreads)
 k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __restrict__ nsz,
            const double* Xw, double* X, long xstride, int ldx,
            double* __restrict__ w, long wstride, int max_sweeps, int* __restrict__ flag) {
     extern __shared__ float smf[];
     __shared__ float red[32];
-    __shared__ float4 prm[kEigMax / 2];   // c, s, p, q (index bits) of the round's pairs
+    __shared__ float2 prm[kEigMax / 2];   // c, s of the round's pairs
     __shared__ int perm[kEigMax];
-    const int b = blockIdx.x;
+    __shared__ JacobiRing ring;
+    const int b = blockIdx.x >> 1, side = blockIdx.x & 1;
     const int n0 = nsz[b];
-    if (n0 == 0) return;
+    if (n0 == 0) return;   // both sides
     const int n = n0 + (n0 & 1);  // pad odd sizes with an isolated zero row
     const int ld = n + 1;
     float* a = smf;             // n x ld
@@ -159,6 +215,17 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
     float* t = n <= kJSmemMax ? v + n * ld : nullptr;   // n x ld scratch
     const double* Ab = A + b * astride;
     const int tid = threadIdx.x;
+    const int half = n / 2;
+    const uint32_t msg = half * sizeof(float2) + sizeof(int);
+    if (tid == 0) {
+        for (int q = 0; q < kRing; ++q) {
+            mbar_init(&ring.full[q], 1);
+            mbar_init(&ring.empty[q], 1);
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (side == 1)
+            for (int q = 0; q < kRing; ++q) mbar_expect_tx(&ring.full[q], msg);
+    }
     for (int q = tid; q < n * n; q += kJThreads) {
         const int i = q / n, j = q % n;
         a[i * ld + j] = (i < n0 && j < n0) ? (float)Ab[(long)i * lda + j] : 0.0f;
@@ -166,7 +233,48 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
         if (Xw && i < n0 && j < n0) vv = (float)Xw[b * xstride + (long)i * ldx + j];
         v[i * ld + j] = vv;
     }
-    __syncthreads();
+    // both sides' barriers exist, and side 1 has read its V before side 0 writes X
+    pair_barrier();
+    // ceil(2^32 / d): exact quotients of u < 2^32 / d by a multiply (n >= 2; d = 1
+    // is its own case)
+    const uint32_t inv_half = half > 1 ? 0xFFFFFFFFu / half + 1u : 0xFFFFFFFFu;
+    const uint32_t inv_n = 0xFFFFFFFFu / n + 1u;
+    // rr_player with j - 1 + r < 2 (n - 1) taken modulo by one subtraction
+    const auto player = [n](int j, int r) {
+        const int t = j - 1 + r;
+        return j == 0 ? 0 : 1 + (t >= n - 1 ? t - (n - 1) : t);
+    };
+    if (side == 1) {
+        // V <- V J, round by round as they come
+        bool ok = true;
+        for (int k = 0;; ++k) {
+            const int slot = k % kRing;
+            ok = ring_wait(&ring.full[slot], (k / kRing) & 1);
+            const int r = ok ? ring.round[slot] : -1;
+            if (r < 0) break;
+            for (int u = tid; u < n * half; u += kJThreads) {
+                const int pair = (int)__umulhi((uint32_t)u, inv_n), row = u - pair * n;
+                const float2 Cc = ring.cs[slot][pair];
+                float* vr = v + row * ld;
+                const int jp = player(pair, r), jq = player(n - 1 - pair, r);
+                const float vp = vr[jp], vq = vr[jq];
+                vr[jp] = Cc.x * vp - Cc.y * vq;
+                vr[jq] = Cc.y * vp + Cc.x * vq;
+            }
+            __syncthreads();
+            if (tid == 0) {
+                mbar_expect_tx(&ring.full[slot], msg);
+                peer_arrive(peer_addr(&ring.empty[slot], 0));
+            }
+        }
+        if (!ok && flag) atomicExch(flag, 1);
+        pair_barrier();   // side 0 has written perm
+        for (int q = tid; q < n0 * n0; q += kJThreads) {
+            const int i = q / n0, col = q % n0;
+            X[b * xstride + (long)i * ldx + col] = (double)v[i * ld + perm[col]];
+        }
+        return;
+    }
     if (Xw && t) {
         // a <- V^T A V
         smem_mm32(a, v, t, n, ld, false);
@@ -204,7 +312,6 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
         }
         __syncthreads();
     }
-    const int half = n / 2;
     float part = 0.0f;
     for (int q = tid; q < n * n; q += kJThreads) {
         const float x = a[(q / n) * ld + q % n];
@@ -213,6 +320,31 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
     const float norm2 = cta_sumf(part, red);
     const float tol2 = 1e-11f * norm2;  // off-diagonal <= 3e-6 |A|: an FP32-level seed
     const float thr = kJacobiSkip * sqrtf(norm2);
+    // hands round r (-1: the end) to side 1; the stores need no fence, each
+    // counts its bytes on the slot's barrier
+    int sent = 0;
+    bool sending = true;   // side 1 keeps up
+    const auto send = [&](int r, float c, float s) {
+        const int slot = sent % kRing;
+        if (tid <= half) {
+            if (sent >= kRing && sending)
+                sending = ring_wait(&ring.empty[slot], (sent / kRing - 1) & 1);
+            const uint32_t bar = peer_addr(&ring.full[slot], 1);
+            if (sending && tid < half)
+                asm volatile(
+                    "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 "
+                    "[%0], {%1, %2}, [%3];" ::"r"(peer_addr(&ring.cs[slot][tid], 1)),
+                    "f"(c), "f"(s), "r"(bar)
+                    : "memory");
+            if (sending && tid == half)
+                asm volatile(
+                    "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.s32 "
+                    "[%0], %1, [%2];" ::"r"(peer_addr(&ring.round[slot], 1)),
+                    "r"(r), "r"(bar)
+                    : "memory");
+        }
+        ++sent;
+    };
     int sweep = 0;
     for (; sweep < max_sweeps; ++sweep) {
         part = 0.0f;
@@ -224,10 +356,10 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
         if (off <= tol2) break;
         for (int r = 0; r < n - 1; ++r) {
             int on = 0;
+            float c = 1.0f, s = 0.0f;
             if (tid < half) {
-                const int p = rr_player(tid, r, n), q = rr_player(n - 1 - tid, r, n);
+                const int p = player(tid, r), q = player(n - 1 - tid, r);
                 const float apq = a[p * ld + q];
-                float c = 1.0f, s = 0.0f;
                 if (fabsf(apq) > thr) {
                     const float th = (a[q * ld + q] - a[p * ld + p]) / (2.0f * apq);
                     const float tt = (th >= 0.0f ? 1.0f : -1.0f) / (fabsf(th) + sqrtf(th * th + 1.0f));
@@ -235,14 +367,16 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
                     s = tt * c;
                     on = 1;
                 }
-                prm[tid] = make_float4(c, s, __int_as_float(p), __int_as_float(q));
+                prm[tid] = make_float2(c, s);
             }
             if (!__syncthreads_or(on)) continue;
+            send(r, c, s);
             for (int u = tid; u < half * half; u += kJThreads) {
-                const float4 R = prm[u / half], Cc = prm[u % half];
-                float* ap = a + __float_as_int(R.z) * ld;
-                float* aq = a + __float_as_int(R.w) * ld;
-                const int jp = __float_as_int(Cc.z), jq = __float_as_int(Cc.w);
+                const int i = (int)__umulhi((uint32_t)u, inv_half), j = u - i * half;
+                const float2 R = prm[i], Cc = prm[j];
+                float* ap = a + player(i, r) * ld;
+                float* aq = a + player(n - 1 - i, r) * ld;
+                const int jp = player(j, r), jq = player(n - 1 - j, r);
                 const float x00 = ap[jp], x01 = ap[jq], x10 = aq[jp], x11 = aq[jq];
                 // rows of pair i, then columns of pair j
                 const float r00 = R.x * x00 - R.y * x10, r10 = R.y * x00 + R.x * x10;
@@ -252,18 +386,11 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
                 aq[jp] = Cc.x * r10 - Cc.y * r11;
                 aq[jq] = Cc.y * r10 + Cc.x * r11;
             }
-            for (int u = tid; u < n * half; u += kJThreads) {
-                const float4 Cc = prm[u / n];
-                float* vr = v + (u % n) * ld;
-                const int jp = __float_as_int(Cc.z), jq = __float_as_int(Cc.w);
-                const float vp = vr[jp], vq = vr[jq];
-                vr[jp] = Cc.x * vp - Cc.y * vq;
-                vr[jq] = Cc.y * vp + Cc.x * vq;
-            }
             __syncthreads();
         }
     }
-    if (sweep == max_sweeps && tid == 0 && flag) atomicExch(flag, 1);
+    send(-1, 1.0f, 0.0f);
+    if ((sweep == max_sweeps && tid == 0 || !sending) && flag) atomicExch(flag, 1);
     // sort the n0 real eigenpairs ascending, ties by index (the padding row
     // stays last): rank of each diagonal entry; perm starts as the identity
     // so that it stays a valid index table whatever the values
@@ -279,11 +406,12 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
         if (rank < n0) perm[rank] = i;
     }
     __syncthreads();
-    for (int q = tid; q < n0 * n0; q += kJThreads) {
-        const int i = q / n0, col = q % n0;
-        X[b * xstride + (long)i * ldx + col] = (double)v[i * ld + perm[col]];
-    }
+    // side 1 writes the vectors in this order
+    for (int i = tid; i < n0; i += kJThreads)
+        asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(peer_addr(&perm[i], 1)), "r"(perm[i])
+                     : "memory");
     for (int k = tid; k < n0; k += kJThreads) w[b * wstride + k] = (double)a[perm[k] * ld + perm[k]];
+    pair_barrier();
 }
 
 // Early exit of the refinement steps (EigBatch::skip_tol).  Step s of
@@ -896,9 +1024,9 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
     if (seed != kSeedRefine) {
         const bool warm = seed == kSeedJacobiWarm;
         const size_t sm = jacobi_smem(E.nmax);
-        k_jacobi32<<<E.nb, kJThreads, sm, c->stream>>>(E.A, E.stride, E.ld, E.nsz,
-                                                      warm ? E.X : nullptr, E.X, E.stride, E.ld,
-                                                      E.w, E.wstride, warm ? 12 : 30, c->flags + 4);
+        k_jacobi32<<<2 * E.nb, kJThreads, sm, c->stream>>>(
+            E.A, E.stride, E.ld, E.nsz, warm ? E.X : nullptr, E.X, E.stride, E.ld, E.w, E.wstride,
+            warm ? 12 : 30, c->flags + 4);
         MG_LAUNCHED(c);
     }
     k_frob<<<E.nb, 1024, 0, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm);
@@ -935,7 +1063,7 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
     // of near-degenerate eigenvalues (density-matrix occupations ~1e-8 apart
     // near 0 or 1) can leave R ~ 1e-2, which one pass only brings to 1e-7.
     for (int pass = 0; pass < (polish ? 2 : 1); ++pass) {
-        launch_gemm(c, dfg, dim3(tiles, 2 * E.nb), E.d_sg, none);
+        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg + E.nb, none);   // G alone
         MG_LAUNCHED(c);
         k_orth_prep<<<dim3(div_up((long)E.nmax * E.nmax, kThreads), E.nb), kThreads, 0,
                       c->stream>>>(E.G, E.AX, E.G, E.stride, E.ld, E.nsz);
@@ -1069,8 +1197,8 @@ int eig_setup(mg_ctx* c, EigBatch& E, int nb, int nmax, const int* nsz_dev, doub
         const int n = hn[b];
         const long o = (long)b * stride;
         ax[b] = GemmDesc{A + o, E.X + o, E.AX + o, n, n, n, ld, ld, ld, 0, 0, 1.0, 0.0, b};
-        sg[2 * b] = GemmDesc{E.X + o, E.AX + o, E.S + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
-        sg[2 * b + 1] = GemmDesc{E.X + o, E.X + o, E.G + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
+        sg[b] = GemmDesc{E.X + o, E.AX + o, E.S + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
+        sg[nb + b] = GemmDesc{E.X + o, E.X + o, E.G + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
         xf[b] = GemmDesc{E.X + o, E.G + o, E.X2 + o, n, n, n, ld, ld, ld, 0, 0, 1.0, 0.0, b};
         rr[b] = GemmDesc{E.AX + o, E.AX + o, E.G + o, n, n, n, ld, ld, ld, 0, 0, 0.375, 1.0, b, 1};
     }
@@ -1186,8 +1314,8 @@ __global__ void k_eig_noalloc_tables(NoAllocArgs a, int* nsz, GemmDesc* ax, Gemm
     const long o = (long)b * ld * ld;
     nsz[b] = n;
     ax[b] = GemmDesc{a.A + o, a.X + o, a.AX + o, n, n, n, ld, ld, ld, 0, 0, 1.0, 0.0, b};
-    sg[2 * b] = GemmDesc{a.X + o, a.AX + o, a.S + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
-    sg[2 * b + 1] = GemmDesc{a.X + o, a.X + o, a.G + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
+    sg[b] = GemmDesc{a.X + o, a.AX + o, a.S + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
+    sg[a.nb + b] = GemmDesc{a.X + o, a.X + o, a.G + o, n, n, n, ld, ld, ld, 1, 0, 1.0, 0.0, b, 1};
     xf[b] = GemmDesc{a.X + o, a.G + o, a.X2 + o, n, n, n, ld, ld, ld, 0, 0, 1.0, 0.0, b};
     rr[b] = GemmDesc{a.AX + o, a.AX + o, a.G + o, n, n, n, ld, ld, ld, 0, 0, 0.375, 1.0, b, 1};
 }
