@@ -32,7 +32,8 @@ namespace mg {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kTile = 16;
+constexpr int kTile = 8;           // GEMM tile, one thread per entry
+constexpr int kGemmThreads = kTile * kTile;
 // Jacobi kernels: one CTA per matrix, so the whole SM's warps work on its
 // rounds (128 lanes for the columns / rows x 8 groups of rotation pairs)
 constexpr int kJThreads = 1024;
@@ -436,101 +437,107 @@ __device__ __forceinline__ bool skip_step(const SkipCtl& k, int b) {
     return true;
 }
 
-// Batched FP64 GEMM, C = alpha op(A) op(B) + beta C, k <= kEigMax, row-major.
+// Batched GEMM, C = alpha op(A) op(B) + beta C, k <= kEigMax, row-major.
 // With g.sym (C symmetric, and C itself when beta != 0) only the upper
 // triangle is computed and written to both halves, which also makes C
 // exactly symmetric.
-__global__ void __launch_bounds__(kThreads) k_gemm64(const GemmDesc* __restrict__ descs,
-                                                     SkipCtl sk) {
-    __shared__ double sA[kTile][kEigMax + 1];
-    __shared__ double sB[kEigMax + 1][kTile + 1];
+//
+// DF = false: FP64, one chain of FMAs in k order per entry.
+// DF = true: double-float for the mixed form: operands split into FP32 pairs
+// after the load (integer instructions, df_split), products and sums with the
+// exact FP32 error terms (df_acc, ~11 FP32 instructions per term), one FP64 add
+// per output.  ~1e-14 relative like the mixed form's Jacobi polish, at several
+// times the rate of the FP64 pipe.
+//
+// Four matrices of a few dozen rows fill a fraction of the chip and a launch
+// lasts a few microseconds: it is bound by the latency of the operands and of one
+// entry's chain (64 clocks per FP64 FMA), from n ~ 90 on by the FP64 pipe (16
+// clocks per warp and FMA).  So a CTA has the smallest tile that still loads
+// whole sectors, 8 x 8, one entry per thread: four times the CTAs of 16 x 16, an
+// even share of the pipe's work (the half grid of a symmetric C left SMs with
+// twice their neighbours' work); and all operand words are in flight at once,
+// copied to shared memory without passing through registers.  A launch over four
+// matrices of 92 takes 11.2 us from a cold L2 (16.1 with 16 x 16 tiles loaded word
+// by word), over four of ~48 5.9 (8.5).
+template <bool DF>
+__global__ void __launch_bounds__(kGemmThreads) k_gemm(const GemmDesc* __restrict__ descs,
+                                                       SkipCtl sk) {
+    constexpr int T = kTile;
+    __shared__ __align__(8) double sA[T][kEigMax + 1];
+    __shared__ __align__(8) double sB[kEigMax][T];
     const GemmDesc g = descs[blockIdx.y];
     if (skip_step(sk, g.mat)) return;
-    const int tiles_n = (g.n + kTile - 1) / kTile;
+    const int tiles_n = (g.n + T - 1) / T;
     const int ti = blockIdx.x / tiles_n, tj = blockIdx.x % tiles_n;
-    if (ti * kTile >= g.m || (g.sym && ti > tj)) return;
-    const int r = threadIdx.x / kTile, cidx = threadIdx.x % kTile;
-    // tile loads with the fastest thread index along the operand's contiguous
-    // dimension (transposed operands included), so that a warp reads
-    // consecutive words
-    for (int q = threadIdx.x; q < kTile * g.k; q += kThreads) {
-        int i, kk;
-        if (g.ta) { i = q % kTile; kk = q / kTile; }
-        else { i = q / g.k; kk = q % g.k; }
-        const int gi = ti * kTile + i;
-        double x = 0.0;
-        if (gi < g.m) x = g.ta ? g.A[(long)kk * g.lda + gi] : g.A[(long)gi * g.lda + kk];
-        sA[i][kk] = x;
-    }
-    for (int q = threadIdx.x; q < kTile * g.k; q += kThreads) {
-        int kk, j;
-        if (g.tb) { kk = q % g.k; j = q / g.k; }
-        else { kk = q / kTile; j = q % kTile; }
-        const int gj = tj * kTile + j;
-        double x = 0.0;
-        if (gj < g.n) x = g.tb ? g.B[(long)gj * g.ldb + kk] : g.B[(long)kk * g.ldb + gj];
-        sB[kk][j] = x;
-    }
+    if (ti * T >= g.m || (g.sym && ti > tj)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int r = tid / T, col = tid % T;
+    const int gi = ti * T + r, gj = tj * T + col;
+    // the fastest thread index runs along the operand's contiguous dimension
+    // (transposed operands included); rows past the edge are zero.  f(word,
+    // source or null) for the words of this thread
+    const auto words = [&](auto f) {
+        if (g.ta) {
+            const int i = ti * T + col;
+            for (int kk = r; kk < g.k; kk += T)
+                f(&sA[col][kk], i < g.m ? g.A + (long)kk * g.lda + i : nullptr);
+        } else {
+#pragma unroll
+            for (int q = 0; q < T; q += kGemmThreads / 32) {
+                const int i = ti * T + q + warp;
+                const double* row = g.A + (long)i * g.lda;
+                for (int kk = lane; kk < g.k; kk += 32)
+                    f(&sA[q + warp][kk], i < g.m ? row + kk : nullptr);
+            }
+        }
+        if (g.tb) {
+#pragma unroll
+            for (int q = 0; q < T; q += kGemmThreads / 32) {
+                const int j = tj * T + q + warp;
+                const double* row = g.B + (long)j * g.ldb;
+                for (int kk = lane; kk < g.k; kk += 32)
+                    f(&sB[kk][q + warp], j < g.n ? row + kk : nullptr);
+            }
+        } else {
+            const int j = tj * T + col;
+            for (int kk = r; kk < g.k; kk += T)
+                f(&sB[kk][col], j < g.n ? g.B + (long)kk * g.ldb + j : nullptr);
+        }
+    };
+    words([](double* dst, const double* src) {
+        if (src)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(shared_addr(dst)), "l"(src)
+                         : "memory");
+        else
+            *dst = 0.0;
+    });
+    const bool mine = gi < g.m && gj < g.n && !(g.sym && gi > gj);   // else the mirror's
+    double* c = g.C + (long)gi * g.ldc + gj;
+    double old = 0.0;
+    if (mine && g.beta != 0.0) old = *c;
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    if constexpr (DF)
+        words([](double* dst, const double*) {
+            const dfl d = df_split(*dst);
+            *reinterpret_cast<float2*>(dst) = make_float2(d.h, d.l);
+        });
     __syncthreads();
-    const int gi = ti * kTile + r, gj = tj * kTile + cidx;
-    if (gi >= g.m || gj >= g.n) return;
-    if (g.sym && gi > gj) return;   // the mirror of an entry another thread writes
+    if (!mine) return;
     double s = 0.0;
-    for (int kk = 0; kk < g.k; ++kk) s = fma(sA[r][kk], sB[kk][cidx], s);
-    double* c = g.C + (long)gi * g.ldc + gj;
-    const double v = g.beta == 0.0 ? g.alpha * s : fma(g.alpha, s, g.beta * *c);
-    *c = v;
-    if (g.sym && gi < gj) g.C[(long)gj * g.ldc + gi] = v;
-}
-
-// The same GEMMs in double-float arithmetic for the mixed form: operands
-// split into FP32 pairs at the tile load (integer instructions, df_split),
-// products and sums with the exact FP32 error terms (df_acc, ~11 FP32
-// instructions per term), one FP64 add per output.  ~1e-14 relative like
-// the mixed form's Jacobi polish, at several times the rate of the FP64
-// pipe, which bounds k_gemm64 on GB300.
-__global__ void __launch_bounds__(kThreads) k_gemm_df(const GemmDesc* __restrict__ descs,
-                                                      SkipCtl sk) {
-    __shared__ float2 sA[kTile][kEigMax + 1];
-    __shared__ float2 sB[kEigMax + 1][kTile + 1];
-    const GemmDesc g = descs[blockIdx.y];
-    if (skip_step(sk, g.mat)) return;
-    const int tiles_n = (g.n + kTile - 1) / kTile;
-    const int ti = blockIdx.x / tiles_n, tj = blockIdx.x % tiles_n;
-    if (ti * kTile >= g.m || (g.sym && ti > tj)) return;
-    const int r = threadIdx.x / kTile, cidx = threadIdx.x % kTile;
-    for (int q = threadIdx.x; q < kTile * g.k; q += kThreads) {
-        int i, kk;
-        if (g.ta) { i = q % kTile; kk = q / kTile; }
-        else { i = q / g.k; kk = q % g.k; }
-        const int gi = ti * kTile + i;
-        double x = 0.0;
-        if (gi < g.m) x = g.ta ? g.A[(long)kk * g.lda + gi] : g.A[(long)gi * g.lda + kk];
-        const dfl d = df_split(x);
-        sA[i][kk] = make_float2(d.h, d.l);
+    if constexpr (DF) {
+        float sh = 0.0f, sl = 0.0f;
+#pragma unroll 8
+        for (int kk = 0; kk < g.k; ++kk) {
+            const float2 a = reinterpret_cast<const float2&>(sA[r][kk]);
+            const float2 b = reinterpret_cast<const float2&>(sB[kk][col]);
+            df_acc(sh, sl, dfl{a.x, a.y}, dfl{b.x, b.y});
+        }
+        s = df_to_fast(dfl{sh, sl});
+    } else {
+#pragma unroll 8
+        for (int kk = 0; kk < g.k; ++kk) s = fma(sA[r][kk], sB[kk][col], s);
     }
-    for (int q = threadIdx.x; q < kTile * g.k; q += kThreads) {
-        int kk, j;
-        if (g.tb) { kk = q % g.k; j = q / g.k; }
-        else { kk = q / kTile; j = q % kTile; }
-        const int gj = tj * kTile + j;
-        double x = 0.0;
-        if (gj < g.n) x = g.tb ? g.B[(long)gj * g.ldb + kk] : g.B[(long)kk * g.ldb + gj];
-        const dfl d = df_split(x);
-        sB[kk][j] = make_float2(d.h, d.l);
-    }
-    __syncthreads();
-    const int gi = ti * kTile + r, gj = tj * kTile + cidx;
-    if (gi >= g.m || gj >= g.n) return;
-    if (g.sym && gi > gj) return;
-    float sh = 0.0f, sl = 0.0f;
-    for (int kk = 0; kk < g.k; ++kk) {
-        const float2 a = sA[r][kk], b = sB[kk][cidx];
-        df_acc(sh, sl, dfl{a.x, a.y}, dfl{b.x, b.y});
-    }
-    const double s = df_to_fast(dfl{sh, sl});
-    double* c = g.C + (long)gi * g.ldc + gj;
-    const double v = g.beta == 0.0 ? g.alpha * s : fma(g.alpha, s, g.beta * *c);
+    const double v = g.beta == 0.0 ? g.alpha * s : fma(g.alpha, s, g.beta * old);
     *c = v;
     if (g.sym && gi < gj) g.C[(long)gj * g.ldc + gi] = v;
 }
@@ -999,9 +1006,9 @@ size_t jacobi_smem(int n) {
 // One launch of a GEMM table: double-float in the mixed form, FP64 otherwise.
 static void launch_gemm(mg_ctx* c, bool df, dim3 grid, const GemmDesc* descs, SkipCtl sk) {
     if (df)
-        k_gemm_df<<<grid, kThreads, 0, c->stream>>>(descs, sk);
+        k_gemm<true><<<grid, kGemmThreads, 0, c->stream>>>(descs, sk);
     else
-        k_gemm64<<<grid, kThreads, 0, c->stream>>>(descs, sk);
+        k_gemm<false><<<grid, kGemmThreads, 0, c->stream>>>(descs, sk);
 }
 
 // Eigen-decomposition of a batch (nb <= 64: the GEMM grids hold 2 nb
@@ -1149,7 +1156,7 @@ int eig_jacobi_fp64(mg_ctx* c, EigBatch& E) {
 int gemm_batched_skip(mg_ctx* c, const GemmDesc* descs, int ndesc, int maxdim, int* done) {
     const SkipCtl sk{done, nullptr, 0, 0, 0.0};
     const int tiles = div_up(maxdim, kTile) * div_up(maxdim, kTile);
-    k_gemm64<<<dim3(tiles, ndesc), kThreads, 0, c->stream>>>(descs, sk);
+    k_gemm<false><<<dim3(tiles, ndesc), kGemmThreads, 0, c->stream>>>(descs, sk);
     MG_LAUNCHED(c);
     return MG_OK;
 }
@@ -1337,7 +1344,7 @@ int noalloc_setup(int dev, unsigned char** base) {
         MG_CUDA(cudaFuncGetAttributes(&fa, k_jacobi32));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_jacobi64_polish));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_sort_cols));
-        MG_CUDA(cudaFuncGetAttributes(&fa, k_gemm64));
+        MG_CUDA(cudaFuncGetAttributes(&fa, k_gemm<false>));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_oa_rows));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_oa_apply));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_orth_prep));

@@ -21,7 +21,7 @@
 // then modified Gram-Schmidt of the columns of [Ua; Va] and of [Vb; Ub]; an
 // isospin stops when |Gradient|, sqrt|sum G_ij G_ji|, and |N - N0| are below
 // FermiPrec in both its blocks.  The matrix products are batched FP64 GEMMs
-// (eig.cu's k_gemm64, a converged isospin's blocks skipped), the Fermi
+// (eig.cu's k_gemm, a converged isospin's blocks skipped), the Fermi
 // update and the convergence test one small kernel, the orthonormalisation
 // one CTA per block and column set.  Iterations replay in chunks of kChunk
 // as one CUDA graph; the host reads the state after each chunk.
