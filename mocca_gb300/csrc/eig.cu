@@ -128,6 +128,17 @@ __device__ void smem_mm32(const float* A, const float* B, float* C, int n, int l
     }
 }
 
+// |A|_F of the n x n matrix at A, on thread 0 of kJThreads.
+__device__ __forceinline__ double frobenius(const double* __restrict__ A, int ld, int n, double* red) {
+    double p = 0.0;
+#pragma unroll 4
+    for (int q = threadIdx.x; q < n * n; q += kJThreads) {
+        const double x = A[(long)(q / n) * ld + q % n];
+        p += x * x;
+    }
+    return sqrt(cta_sumd(p, red));
+}
+
 // One matrix per CTA pair.  A: FP64 n x n (lda) input; Xw: optional FP64 warm
 // start (n x n, ldx); X: FP64 output vectors (n x n, ldx, column k <-> w[k]);
 // w: eigenvalues ascending.  n <= kEigMax.  Above kJSmemMax the warm start's
@@ -200,15 +211,20 @@ __device__ __forceinline__ void pair_barrier() {
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kJThreads)
 k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __restrict__ nsz,
            const double* Xw, double* X, long xstride, int ldx,
-           double* __restrict__ w, long wstride, int max_sweeps, int* __restrict__ flag) {
+           double* __restrict__ w, long wstride, int max_sweeps, int* __restrict__ flag,
+           double* __restrict__ anorm) {
     extern __shared__ float smf[];
     __shared__ float red[32];
+    __shared__ double redd[32];
     __shared__ float2 prm[kEigMax / 2];   // c, s of the round's pairs
     __shared__ int perm[kEigMax];
     __shared__ JacobiRing ring;
     const int b = blockIdx.x >> 1, side = blockIdx.x & 1;
     const int n0 = nsz[b];
-    if (n0 == 0) return;   // both sides
+    if (n0 == 0) {   // both sides
+        if (side == 0 && threadIdx.x == 0) anorm[b] = 0.0;
+        return;
+    }
     const int n = n0 + (n0 & 1);  // pad odd sizes with an isolated zero row
     const int ld = n + 1;
     float* a = smf;             // n x ld
@@ -246,6 +262,8 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
         return j == 0 ? 0 : 1 + (t >= n - 1 ? t - (n - 1) : t);
     };
     if (side == 1) {
+        const double f = frobenius(A + b * astride, lda, n0, redd);
+        if (tid == 0) anorm[b] = f;
         // V <- V J, round by round as they come
         bool ok = true;
         for (int k = 0;; ++k) {
@@ -415,6 +433,32 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
     pair_barrier();
 }
 
+// The kernels of the refinement chain last a few microseconds each, about as long
+// as it takes to start one.  They are launched while the kernel before them runs
+// (launch_early): chain_wait() holds them until that one has ended and its writes
+// are visible, and lets the one after them start.  With the copies back from X2
+// gone too (Flip), four matrices of 92 went from 771 to 702 us, the pairing step
+// of 18^3 from 1068 to 1010.
+__device__ __forceinline__ void chain_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// X <- X F writes the other of the two vector buffers X and X2 instead of being
+// copied back: with `on`, the tables' pointers into one mean the other.
+struct Flip {
+    const double *x, *x2;
+    long len;
+    bool on;
+    template <class P>
+    __device__ __forceinline__ P* at(P* p) const {
+        if (!on) return p;
+        if (p >= x && p < x + len) return p + (x2 - x);
+        if (p >= x2 && p < x2 + len) return p - (x2 - x);
+        return p;
+    }
+};
+
 // Early exit of the refinement steps (EigBatch::skip_tol).  Step s of
 // matrix b is skipped when done[b] <= s.  The first launch of step s (decide)
 // sets done[b] = s when step s - 1 saw |S - diag S|_F <= tol |A|_F: its
@@ -461,12 +505,16 @@ __device__ __forceinline__ bool skip_step(const SkipCtl& k, int b) {
 // by word), over four of ~48 5.9 (8.5).
 template <bool DF>
 __global__ void __launch_bounds__(kGemmThreads) k_gemm(const GemmDesc* __restrict__ descs,
-                                                       SkipCtl sk) {
+                                                       SkipCtl sk, Flip flip) {
     constexpr int T = kTile;
     __shared__ __align__(8) double sA[T][kEigMax + 1];
     __shared__ __align__(8) double sB[kEigMax][T];
-    const GemmDesc g = descs[blockIdx.y];
+    chain_wait();
+    GemmDesc g = descs[blockIdx.y];
     if (skip_step(sk, g.mat)) return;
+    g.A = flip.at(g.A);
+    g.B = flip.at(g.B);
+    g.C = flip.at(g.C);
     const int tiles_n = (g.n + T - 1) / T;
     const int ti = blockIdx.x / tiles_n, tj = blockIdx.x % tiles_n;
     if (ti * T >= g.m || (g.sym && ti > tj)) return;
@@ -558,6 +606,7 @@ k_oa_rows(const double* __restrict__ S, const double* __restrict__ G, long strid
           const int* __restrict__ nsz, double* __restrict__ w, long wstride,
           double* __restrict__ part, SkipCtl sk) {
     __shared__ double red[32];
+    chain_wait();
     const int b = blockIdx.y, i = blockIdx.x, n = nsz[b];
     if (i >= n || skip_step(sk, b)) return;
     const double* Sr = S + b * stride + (long)i * ld;
@@ -585,6 +634,7 @@ k_oa_apply(const double* __restrict__ S, double* __restrict__ G, long stride, in
            const double* __restrict__ w, long wstride, const double* __restrict__ part,
            double* __restrict__ emax, double* __restrict__ offrel, SkipCtl sk) {
     __shared__ double red[32];
+    chain_wait();
     const int b = blockIdx.y, i = blockIdx.x, n = nsz[b];
     if (i >= n || skip_step(sk, b)) return;
     double ps = 0.0, pr = 0.0;
@@ -928,6 +978,7 @@ k_jacobi_df_polish(const double* __restrict__ S, long stride, int ld, const int*
 __global__ void k_orth_prep(const double* __restrict__ G, double* __restrict__ Rm,
                             double* __restrict__ F, long stride, int ld,
                             const int* __restrict__ nsz) {
+    chain_wait();
     const int b = blockIdx.y, n = nsz[b];
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n * n) return;
@@ -941,9 +992,10 @@ __global__ void k_orth_prep(const double* __restrict__ G, double* __restrict__ R
 // Ascending order after a refinement that started from earlier vectors (the
 // eigenvalue estimates keep the column order of the start, which need not be
 // sorted any more): rank each eigenvalue (ties by index), move column j of X
-// to column rank(j) of X2 and reorder w.  Grid (row chunks, matrices): every
-// CTA ranks the eigenvalues itself (integer compares of order-preserving
-// keys of the FP64 bit patterns) and moves kSortRows rows.
+// to column rank(j) of out, which may be X, and reorder w into w2, which may not
+// be w.  Grid (row chunks, matrices): every CTA ranks the eigenvalues itself
+// (integer compares of order-preserving keys of the FP64 bit patterns) and moves
+// kSortRows rows through shared memory.
 constexpr int kSortRows = 8;
 
 __device__ __forceinline__ unsigned long long order_key(double x) {
@@ -952,15 +1004,20 @@ __device__ __forceinline__ unsigned long long order_key(double x) {
 }
 
 __global__ void __launch_bounds__(128)
-k_sort_cols(const double* __restrict__ X, double* __restrict__ X2, const double* __restrict__ w,
+k_sort_cols(const double* X, double* out, const double* __restrict__ w,
             double* __restrict__ w2, long stride, int ld, long wstride,
             const int* __restrict__ nsz) {
     __shared__ unsigned long long key[kEigMax];
     __shared__ double sw[kEigMax];
     __shared__ int rank[kEigMax];
+    __shared__ double rows[kSortRows][kEigMax];
+    chain_wait();
     const int b = blockIdx.y, n = nsz[b];
     const int r0 = blockIdx.x * kSortRows;
     if (r0 >= n) return;
+    const int r1 = min(n, r0 + kSortRows);
+    for (int t = threadIdx.x; t < (r1 - r0) * n; t += blockDim.x)
+        rows[t / n][t % n] = X[b * stride + (long)(r0 + t / n) * ld + t % n];
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         sw[i] = w[b * wstride + i];
         key[i] = order_key(sw[i]);
@@ -973,29 +1030,37 @@ k_sort_cols(const double* __restrict__ X, double* __restrict__ X2, const double*
         rank[i] = r < n ? r : n - 1;
     }
     __syncthreads();
-    const int r1 = min(n, r0 + kSortRows);
-    for (int t = threadIdx.x; t < (r1 - r0) * n; t += blockDim.x) {
-        const int r = r0 + t / n, j = t % n;
-        X2[b * stride + (long)r * ld + rank[j]] = X[b * stride + (long)r * ld + j];
-    }
+    for (int t = threadIdx.x; t < (r1 - r0) * n; t += blockDim.x)
+        out[b * stride + (long)(r0 + t / n) * ld + rank[t % n]] = rows[t / n][t % n];
     // every CTA holds the same values; the first writes the sorted w (to a
     // second buffer: the other CTAs may still be reading w)
     if (blockIdx.x == 0)
         for (int i = threadIdx.x; i < n; i += blockDim.x) w2[b * wstride + rank[i]] = sw[i];
 }
 
-// Frobenius norms of the batch matrices (delta of the refinement uses ||A||).
-__global__ void k_frob(const double* __restrict__ A, long stride, int ld, const int* __restrict__ nsz,
-                       double* __restrict__ out) {
+// Vectors of the matrices that an early exit left in X2, into X: those with an odd
+// number of refinement steps run.
+__global__ void __launch_bounds__(kThreads)
+k_settle(double* __restrict__ X, const double* __restrict__ X2, long stride, int ld,
+         const int* __restrict__ nsz, const int* __restrict__ done, int nref) {
+    chain_wait();
+    const int b = blockIdx.y, n = nsz[b];
+    if (!(min(done[b], nref) & 1)) return;
+    const int t = blockIdx.x * kThreads + threadIdx.x;
+    if (t >= n * n) return;
+    const long o = b * stride + (long)(t / n) * ld + t % n;
+    X[o] = X2[o];
+}
+
+// Frobenius norms of the batch matrices (delta of the refinement uses ||A||),
+// where no Jacobi seed has left them.
+__global__ void __launch_bounds__(kJThreads)
+k_frob(const double* __restrict__ A, long stride, int ld, const int* __restrict__ nsz,
+       double* __restrict__ out) {
     __shared__ double red[32];
     const int b = blockIdx.x, n = nsz[b];
-    double p = 0.0;
-    for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
-        const double x = A[b * stride + (long)(q / n) * ld + q % n];
-        p += x * x;
-    }
-    const double s = cta_sumd(p, red);
-    if (threadIdx.x == 0) out[b] = sqrt(s);
+    const double s = frobenius(A + b * stride, ld, n, red);
+    if (threadIdx.x == 0) out[b] = s;
 }
 
 size_t jacobi_smem(int n) {
@@ -1003,12 +1068,27 @@ size_t jacobi_smem(int n) {
     return (size_t)(np <= kJSmemMax ? 3 : 2) * np * (np + 1) * sizeof(float);
 }
 
+// A launch of a kernel that begins with chain_wait().
+template <class... P, class... V>
+static int launch_early(mg_ctx* c, void (*kernel)(P...), dim3 grid, int threads, V... args) {
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.stream = c->stream;
+    cfg.attrs = &early;
+    cfg.numAttrs = 1;
+    MG_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    MG_LAUNCHED(c);
+    return MG_OK;
+}
+
 // One launch of a GEMM table: double-float in the mixed form, FP64 otherwise.
-static void launch_gemm(mg_ctx* c, bool df, dim3 grid, const GemmDesc* descs, SkipCtl sk) {
-    if (df)
-        k_gemm<true><<<grid, kGemmThreads, 0, c->stream>>>(descs, sk);
-    else
-        k_gemm<false><<<grid, kGemmThreads, 0, c->stream>>>(descs, sk);
+static int launch_gemm(mg_ctx* c, bool df, dim3 grid, const GemmDesc* descs, SkipCtl sk,
+                       Flip flip = Flip{}) {
+    return launch_early(c, df ? k_gemm<true> : k_gemm<false>, grid, kGemmThreads, descs, sk, flip);
 }
 
 // Eigen-decomposition of a batch (nb <= 64: the GEMM grids hold 2 nb
@@ -1033,35 +1113,37 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
         const size_t sm = jacobi_smem(E.nmax);
         k_jacobi32<<<2 * E.nb, kJThreads, sm, c->stream>>>(
             E.A, E.stride, E.ld, E.nsz, warm ? E.X : nullptr, E.X, E.stride, E.ld, E.w, E.wstride,
-            warm ? 12 : 30, c->flags + 4);
+            warm ? 12 : 30, c->flags + 4, E.anorm);
         MG_LAUNCHED(c);
     }
-    k_frob<<<E.nb, 1024, 0, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm);
-    MG_LAUNCHED(c);
+    if (seed == kSeedRefine) {
+        k_frob<<<E.nb, kJThreads, 0, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm);
+        MG_LAUNCHED(c);
+    }
     const int tiles = div_up(E.nmax, kTile) * div_up(E.nmax, kTile);
+    const dim3 rows(E.nmax, E.nb), elems(div_up((long)E.nmax * E.nmax, kThreads), E.nb);
     const bool dfg = c->cur_precision == MG_MIXED;
     const SkipCtl none{nullptr, nullptr, 0, 0, 0.0};
+    Flip flip{E.X, E.X2, (long)E.nb * E.stride, false};   // on: the vectors are in X2
     if (E.skip_tol >= 0.0)
         MG_CUDA(cudaMemsetAsync(E.done, 0x7f, (size_t)E.nb * sizeof(int), c->stream));
     for (int s = 0; s < nref; ++s) {
-        // AX = A X ; S = X^T AX ; G = X^T X ; F = I + E ; X2 = X F ; X <- X2
+        // AX = A X ; S = X^T AX ; G = X^T X ; F = I + E ; X <- X F
         SkipCtl sk{E.skip_tol >= 0.0 ? E.done : nullptr, E.offrel, s, 1, E.skip_tol};
-        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, sk);
-        MG_LAUNCHED(c);
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, sk, flip));
         sk.decide = 0;
-        launch_gemm(c, dfg, dim3(tiles, 2 * E.nb), E.d_sg, sk);
-        MG_LAUNCHED(c);
-        k_oa_rows<<<dim3(E.nmax, E.nb), 128, 0, c->stream>>>(E.S, E.G, E.stride, E.ld, E.nsz,
-                                                             E.w, E.wstride, E.part, sk);
-        MG_LAUNCHED(c);
-        k_oa_apply<<<dim3(E.nmax, E.nb), 128, 0, c->stream>>>(E.S, E.G, E.stride, E.ld, E.nsz,
-                                                              E.anorm, E.w, E.wstride, E.part,
-                                                              E.emax, E.offrel, sk);
-        MG_LAUNCHED(c);
-        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, sk);
-        MG_LAUNCHED(c);
-        MG_CUDA(cudaMemcpyAsync(E.X, E.X2, (size_t)E.nb * E.stride * sizeof(double),
-                                cudaMemcpyDeviceToDevice, c->stream));
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, 2 * E.nb), E.d_sg, sk, flip));
+        MG_TRY(launch_early(c, k_oa_rows, rows, 128, E.S, E.G, E.stride, E.ld, E.nsz, E.w,
+                            E.wstride, E.part, sk));
+        MG_TRY(launch_early(c, k_oa_apply, rows, 128, E.S, E.G, E.stride, E.ld, E.nsz, E.anorm, E.w,
+                            E.wstride, E.part, E.emax, E.offrel, sk));
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, sk, flip));
+        flip.on = !flip.on;
+    }
+    if (E.skip_tol >= 0.0) {
+        MG_TRY(launch_early(c, k_settle, elems, kThreads, E.X, E.X2, E.stride, E.ld, E.nsz, E.done,
+                            nref));
+        flip.on = false;
     }
     // re-orthonormalise: G = X^T X, F = I + R/2 + 3/8 R^2, X <- X F, leaving
     // ~(5/16) R^3.  With the polish a second pass follows: the polish
@@ -1070,48 +1152,41 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
     // of near-degenerate eigenvalues (density-matrix occupations ~1e-8 apart
     // near 0 or 1) can leave R ~ 1e-2, which one pass only brings to 1e-7.
     for (int pass = 0; pass < (polish ? 2 : 1); ++pass) {
-        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg + E.nb, none);   // G alone
-        MG_LAUNCHED(c);
-        k_orth_prep<<<dim3(div_up((long)E.nmax * E.nmax, kThreads), E.nb), kThreads, 0,
-                      c->stream>>>(E.G, E.AX, E.G, E.stride, E.ld, E.nsz);
-        MG_LAUNCHED(c);
-        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_rr, none);
-        MG_LAUNCHED(c);
-        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, none);
-        MG_LAUNCHED(c);
-        MG_CUDA(cudaMemcpyAsync(E.X, E.X2, (size_t)E.nb * E.stride * sizeof(double),
-                                cudaMemcpyDeviceToDevice, c->stream));
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg + E.nb, none, flip));   // G alone
+        MG_TRY(launch_early(c, k_orth_prep, elems, kThreads, E.G, E.AX, E.G, E.stride, E.ld,
+                            E.nsz));
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_rr, none));
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, none, flip));
+        flip.on = !flip.on;
     }
     if (polish) {
         const int np = E.nmax + (E.nmax & 1);
         const size_t psm = (size_t)np * (np + 1) * sizeof(double);
         if (psm > (size_t)kSmemOptIn) return MG_ERR_ARG;
-        // Rayleigh-Ritz matrix and the FP64 Jacobi polish
-        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, none);
-        MG_LAUNCHED(c);
-        launch_gemm(c, dfg, dim3(tiles, 2 * E.nb), E.d_sg, none);
-        MG_LAUNCHED(c);
+        // Rayleigh-Ritz matrix and the FP64 Jacobi polish, its eigenvalues in E.part
+        // (2 * nb * ld doubles, free after the refinement) until they are sorted
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, none, flip));
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg, none, flip));   // S alone
         if (c->cur_precision == MG_MIXED && E.nmax <= kDfPolishMax)
             k_jacobi_df_polish<<<E.nb, kJThreads, df_polish_smem(E.nmax), c->stream>>>(
-                E.S, E.stride, E.ld, E.nsz, E.anorm, E.G, E.w, E.wstride, E.pfail, 12);
+                E.S, E.stride, E.ld, E.nsz, E.anorm, E.G, E.part, E.wstride, E.pfail, 12);
         else
             k_jacobi64_polish<<<E.nb, kJThreads, psm, c->stream>>>(
-                E.S, E.stride, E.ld, E.nsz, E.anorm, E.G, E.w, E.wstride, E.pfail, 12);
+                E.S, E.stride, E.ld, E.nsz, E.anorm, E.G, E.part, E.wstride, E.pfail, 12);
         MG_LAUNCHED(c);
-        launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, none);
-        MG_LAUNCHED(c);
-        MG_CUDA(cudaMemcpyAsync(E.X, E.X2, (size_t)E.nb * E.stride * sizeof(double),
-                                cudaMemcpyDeviceToDevice, c->stream));
+        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, none, flip));
+        flip.on = !flip.on;
     }
     // ascending order: the refinement keeps the column order of its start and
     // the polish leaves diag(S) in place
     if (seed == kSeedRefine || polish) {
-        // E.part (2 * nb * ld doubles, free after the refinement) takes the sorted w
-        k_sort_cols<<<dim3(div_up(E.nmax, kSortRows), E.nb), 128, 0, c->stream>>>(
-            E.X, E.X2, E.w, E.part, E.stride, E.ld, E.wstride, E.nsz);
-        MG_LAUNCHED(c);
-        MG_CUDA(cudaMemcpyAsync(E.w, E.part, (size_t)E.nb * E.wstride * sizeof(double),
-                                cudaMemcpyDeviceToDevice, c->stream));
+        MG_TRY(launch_early(c, k_sort_cols, dim3(div_up(E.nmax, kSortRows), E.nb), 128,
+                            flip.on ? E.X2 : E.X, E.X, polish ? E.part : E.w,
+                            polish ? E.w : E.part, E.stride, E.ld, E.wstride, E.nsz));
+        if (!polish)
+            MG_CUDA(cudaMemcpyAsync(E.w, E.part, (size_t)E.nb * E.wstride * sizeof(double),
+                                    cudaMemcpyDeviceToDevice, c->stream));
+    } else if (flip.on) {
         MG_CUDA(cudaMemcpyAsync(E.X, E.X2, (size_t)E.nb * E.stride * sizeof(double),
                                 cudaMemcpyDeviceToDevice, c->stream));
     }
@@ -1136,18 +1211,13 @@ int eig_jacobi_fp64(mg_ctx* c, EigBatch& E) {
                                      (int)df_polish_smem(kDfPolishMax)));
         E.attr_done = true;
     }
-    k_frob<<<E.nb, 1024, 0, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm);
+    k_frob<<<E.nb, kJThreads, 0, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm);
     MG_LAUNCHED(c);
     k_jacobi64_polish<<<E.nb, kJThreads, psm, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm,
-                                                           E.X, E.w, E.wstride, E.pfail, 40);
+                                                           E.X, E.part, E.wstride, E.pfail, 40);
     MG_LAUNCHED(c);
-    k_sort_cols<<<dim3(div_up(E.nmax, kSortRows), E.nb), 128, 0, c->stream>>>(
-        E.X, E.X2, E.w, E.part, E.stride, E.ld, E.wstride, E.nsz);
-    MG_LAUNCHED(c);
-    MG_CUDA(cudaMemcpyAsync(E.w, E.part, (size_t)E.nb * E.wstride * sizeof(double),
-                            cudaMemcpyDeviceToDevice, c->stream));
-    MG_CUDA(cudaMemcpyAsync(E.X, E.X2, (size_t)E.nb * E.stride * sizeof(double),
-                            cudaMemcpyDeviceToDevice, c->stream));
+    MG_TRY(launch_early(c, k_sort_cols, dim3(div_up(E.nmax, kSortRows), E.nb), 128, E.X, E.X,
+                        E.part, E.w, E.stride, E.ld, E.wstride, E.nsz));
     E.have_vectors = true;
     return MG_OK;
 }
@@ -1156,9 +1226,7 @@ int eig_jacobi_fp64(mg_ctx* c, EigBatch& E) {
 int gemm_batched_skip(mg_ctx* c, const GemmDesc* descs, int ndesc, int maxdim, int* done) {
     const SkipCtl sk{done, nullptr, 0, 0, 0.0};
     const int tiles = div_up(maxdim, kTile) * div_up(maxdim, kTile);
-    k_gemm<false><<<dim3(tiles, ndesc), kGemmThreads, 0, c->stream>>>(descs, sk);
-    MG_LAUNCHED(c);
-    return MG_OK;
+    return launch_gemm(c, false, dim3(tiles, ndesc), descs, sk);
 }
 
 // ndesc FP64 GEMMs of at most maxdim x maxdim from a device descriptor
@@ -1166,9 +1234,7 @@ int gemm_batched_skip(mg_ctx* c, const GemmDesc* descs, int ndesc, int maxdim, i
 int gemm_batched(mg_ctx* c, const GemmDesc* descs, int ndesc, int maxdim, bool df) {
     const SkipCtl none{nullptr, nullptr, 0, 0, 0.0};
     const int tiles = div_up(maxdim, kTile) * div_up(maxdim, kTile);
-    launch_gemm(c, df, dim3(tiles, ndesc), descs, none);
-    MG_LAUNCHED(c);
-    return MG_OK;
+    return launch_gemm(c, df, dim3(tiles, ndesc), descs, none);
 }
 
 // Workspace and GEMM descriptor tables for a batch.
@@ -1408,10 +1474,10 @@ extern "C" int mg_eigh_batched_noalloc(int nb, const int* n, int ld, const doubl
     E.d_rr = desc + 4 * nb;
     E.attr_done = true;
 
-    // Must start at zero on every call: the flags, and X2, whose padding
-    // (outside each leading n x n block) is copied into z.
+    // Must start at zero on every call: the flags, and z, whose padding (outside
+    // each leading n x n block) nothing writes.
     MG_CUDA(cudaMemsetAsync(tmp.flags, 0, 256, tmp.stream));
-    MG_CUDA(cudaMemsetAsync(E.X2, 0, (size_t)nb * E.stride * sizeof(double), tmp.stream));
+    MG_CUDA(cudaMemsetAsync(E.X, 0, (size_t)nb * E.stride * sizeof(double), tmp.stream));
     NoAllocArgs args{};
     for (int b = 0; b < nb; ++b) args.n[b] = n[b];
     args.nb = nb;
