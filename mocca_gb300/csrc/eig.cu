@@ -25,6 +25,7 @@
 #include <mutex>
 
 #include "df.cuh"
+#include "chain.cuh"
 #include "mg_internal.cuh"
 
 namespace mg {
@@ -433,19 +434,11 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
     pair_barrier();
 }
 
-// The kernels of the refinement chain last a few microseconds each, about as long
-// as it takes to start one.  They are launched while the kernel before them runs
-// (launch_early): chain_wait() holds them until that one has ended and its writes
-// are visible, and lets the one after them start.  With the copies back from X2
-// gone too (Flip), four matrices of 92 went from 771 to 702 us, the pairing step
-// of 18^3 from 1068 to 1010.
-__device__ __forceinline__ void chain_wait() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
 // X <- X F writes the other of the two vector buffers X and X2 instead of being
 // copied back: with `on`, the tables' pointers into one mean the other.
+//
+// With this and early launches (chain.cuh), four matrices of 92 went from 771 to
+// 702 us, the pairing step of 18^3 from 1068 to 1010.
 struct Flip {
     const double *x, *x2;
     long len;
@@ -1068,27 +1061,11 @@ size_t jacobi_smem(int n) {
     return (size_t)(np <= kJSmemMax ? 3 : 2) * np * (np + 1) * sizeof(float);
 }
 
-// A launch of a kernel that begins with chain_wait().
-template <class... P, class... V>
-static int launch_early(mg_ctx* c, void (*kernel)(P...), dim3 grid, int threads, V... args) {
-    cudaLaunchAttribute early{};
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.stream = c->stream;
-    cfg.attrs = &early;
-    cfg.numAttrs = 1;
-    MG_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
-    MG_LAUNCHED(c);
-    return MG_OK;
-}
-
 // One launch of a GEMM table: double-float in the mixed form, FP64 otherwise.
 static int launch_gemm(mg_ctx* c, bool df, dim3 grid, const GemmDesc* descs, SkipCtl sk,
                        Flip flip = Flip{}) {
-    return launch_early(c, df ? k_gemm<true> : k_gemm<false>, grid, kGemmThreads, descs, sk, flip);
+    return launch_early(c, df ? k_gemm<true> : k_gemm<false>, grid, kGemmThreads, 0,
+                        descs, sk, flip);
 }
 
 // Eigen-decomposition of a batch (nb <= 64: the GEMM grids hold 2 nb
@@ -1133,15 +1110,15 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, sk, flip));
         sk.decide = 0;
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, 2 * E.nb), E.d_sg, sk, flip));
-        MG_TRY(launch_early(c, k_oa_rows, rows, 128, E.S, E.G, E.stride, E.ld, E.nsz, E.w,
+        MG_TRY(launch_early(c, k_oa_rows, rows, 128, 0, E.S, E.G, E.stride, E.ld, E.nsz, E.w,
                             E.wstride, E.part, sk));
-        MG_TRY(launch_early(c, k_oa_apply, rows, 128, E.S, E.G, E.stride, E.ld, E.nsz, E.anorm, E.w,
+        MG_TRY(launch_early(c, k_oa_apply, rows, 128, 0, E.S, E.G, E.stride, E.ld, E.nsz, E.anorm, E.w,
                             E.wstride, E.part, E.emax, E.offrel, sk));
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, sk, flip));
         flip.on = !flip.on;
     }
     if (E.skip_tol >= 0.0) {
-        MG_TRY(launch_early(c, k_settle, elems, kThreads, E.X, E.X2, E.stride, E.ld, E.nsz, E.done,
+        MG_TRY(launch_early(c, k_settle, elems, kThreads, 0, E.X, E.X2, E.stride, E.ld, E.nsz, E.done,
                             nref));
         flip.on = false;
     }
@@ -1153,7 +1130,7 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
     // near 0 or 1) can leave R ~ 1e-2, which one pass only brings to 1e-7.
     for (int pass = 0; pass < (polish ? 2 : 1); ++pass) {
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg + E.nb, none, flip));   // G alone
-        MG_TRY(launch_early(c, k_orth_prep, elems, kThreads, E.G, E.AX, E.G, E.stride, E.ld,
+        MG_TRY(launch_early(c, k_orth_prep, elems, kThreads, 0, E.G, E.AX, E.G, E.stride, E.ld,
                             E.nsz));
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_rr, none));
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, none, flip));
@@ -1180,7 +1157,7 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
     // ascending order: the refinement keeps the column order of its start and
     // the polish leaves diag(S) in place
     if (seed == kSeedRefine || polish) {
-        MG_TRY(launch_early(c, k_sort_cols, dim3(div_up(E.nmax, kSortRows), E.nb), 128,
+        MG_TRY(launch_early(c, k_sort_cols, dim3(div_up(E.nmax, kSortRows), E.nb), 128, 0,
                             flip.on ? E.X2 : E.X, E.X, polish ? E.part : E.w,
                             polish ? E.w : E.part, E.stride, E.ld, E.wstride, E.nsz));
         if (!polish)
@@ -1216,7 +1193,7 @@ int eig_jacobi_fp64(mg_ctx* c, EigBatch& E) {
     k_jacobi64_polish<<<E.nb, kJThreads, psm, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm,
                                                            E.X, E.part, E.wstride, E.pfail, 40);
     MG_LAUNCHED(c);
-    MG_TRY(launch_early(c, k_sort_cols, dim3(div_up(E.nmax, kSortRows), E.nb), 128, E.X, E.X,
+    MG_TRY(launch_early(c, k_sort_cols, dim3(div_up(E.nmax, kSortRows), E.nb), 128, 0, E.X, E.X,
                         E.part, E.w, E.stride, E.ld, E.wstride, E.nsz));
     E.have_vectors = true;
     return MG_OK;
