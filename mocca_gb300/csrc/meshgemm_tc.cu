@@ -3,7 +3,7 @@
 // Gram-Schmidt overlap and apply, and the canonical-basis transform.
 //
 // Blocks of up to kMeshTcMax (80) spinors; above 64, four accumulators take
-// 512 TMEM columns and the kernels run one CTA per SM.
+// 512 TMEM columns and the overlap and gaps kernels run one CTA per SM.
 //
 // Gram-Schmidt (gs.cu; GramSchmidt, src/SpwfStorage.f90:372-480, as
 // Q = Psi R^{-1} with S = R^T R per (isospin, parity, signature) block in
@@ -17,7 +17,7 @@
 // Block apply, out_l(p) = sum_k C[k][l] in_k(p) per block of spinors:
 //   k_coef_digits   : digit planes of C (rows: output l, K: input k), one
 //                     power of two per row;
-//   k_apply_tc      : 128 points per CTA (MMA M), K = the block's spinors, FP64
+//   k_apply_tc      : tiles of 128 points (MMA M), K = the block's spinors, FP64
 //                     output.  Gram-Schmidt: C = R^{-1}, in place, plus the
 //                     GradDesc history upd_l = out_l - upd_l.  Canonical basis
 //                     (HFBOccupations, src/HFB.f90:3448-3487): C = CanTransfo,
@@ -200,214 +200,281 @@ k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
     if (warp == 0) tc::dealloc(tmem, tcols);
 }
 
-// Digit planes of C (per block: kDigits planes of Np rows x Np, row l = output
-// l, K = input k; C[k][l] = coef[b * bstride + k * ld + l], ld = nb when 0) and
-// the row exponents (biased).
-__global__ void k_coef_digits(const double* __restrict__ coef, long bstride, int ld, BlockIdx bi,
-                              uint16_t* __restrict__ xd, int* __restrict__ xe) {
+// Digit planes of C (per block: ND planes of NP rows x NP, row l = output l, K =
+// input k; C[k][l] = coef[b * bstride + k * ld + l], ld = nb when 0) and the row
+// exponents (biased).  Thread (l, y): entries k = y, y + kCoefRows, ...
+constexpr int kCoefRows = 8;
+
+template <int ND, int NP>
+__global__ void __launch_bounds__(NP * kCoefRows)
+k_coef_digits(const double* __restrict__ coef, long bstride, int ld, BlockIdx bi,
+              uint16_t* __restrict__ xd, int* __restrict__ xe) {
+    __shared__ int se[kCoefRows][NP];
     const int b = blockIdx.x;
     const int nb = bi.nb(b);
-    const int Np = max(16, (nb + 15) / 16 * 16);
-    const int l = threadIdx.x;
-    if (nb == 0 || l >= Np) return;
+    const int l = threadIdx.x, y = threadIdx.y;
+    if (nb == 0) return;
     const int ldc = ld > 0 ? ld : nb;
     const double* X = coef + (long)b * bstride;
-    uint16_t* out = xd + (long)b * kDigits * kXdStride;
+    uint16_t* out = xd + (long)b * ND * kXdStride;
+    double v[NP / kCoefRows];
     int emax = 0;
-    if (l < nb)
-        for (int k = 0; k < nb; ++k) emax = max(emax, oz::bexp(X[k * ldc + l]));
-    xe[b * kMeshTcMax + l] = emax;
-    for (int k = 0; k < Np; ++k) {
-        const double v = (l < nb && k < nb) ? X[k * ldc + l] : 0.0;
-        uint32_t d[kDigits];
-        oz::digits(v, emax, d);
-        const uint32_t o = tc::kmajor_off_g(l, k, Np / 8) / 2;
 #pragma unroll
-        for (int a = 0; a < kDigits; ++a) out[(long)a * Np * Np + o] = (uint16_t)(d[a] >> 16);
+    for (int q = 0; q < NP / kCoefRows; ++q) {
+        const int k = y + q * kCoefRows;
+        v[q] = (l < nb && k < nb) ? X[k * ldc + l] : 0.0;
+        emax = max(emax, oz::bexp(v[q]));
+    }
+    se[y][l] = emax;
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < kCoefRows; ++q) emax = max(emax, se[q][l]);
+    if (y == 0) xe[b * kMeshTcMax + l] = emax;
+    const oz::FixedRow<ND> fixed(emax);
+#pragma unroll
+    for (int q = 0; q < NP / kCoefRows; ++q) {
+        uint32_t d[ND];
+        oz::digits_of<ND>(fixed.biased(v[q]), d);
+        const uint32_t o = tc::kmajor_off_g(l, y + q * kCoefRows, NP / 8) / 2;
+#pragma unroll
+        for (int a = 0; a < ND; ++a) out[(long)a * NP * NP + o] = (uint16_t)(d[a] >> 16);
     }
 }
 
 // out_l = sum_k C[k][l] in_k over 128 points (in_k = in[in_list[off + k]],
 // out_l = out[out_list[off + l]] or out[out_base[b] + l]); when upd is given,
 // upd_l = out_l - upd_l.  in and out may be the same array (in place).
-// Thread t: point row = t % 128, K groups h, h + 2, h + 4, ... (h = t / 128);
-// up to 48 spinors the point's values stay in registers between the
-// exponent and the digits, above they are read twice.
-__global__ void __launch_bounds__(256, 2)
+//
+// One CTA per SM takes a run of the (block, 128 points) tiles.  Three roles work on
+// different tiles at a time: the slicers hold a tile's values (two threads a point)
+// and cut them once the planes of the tile before are free, one thread issues the
+// MMAs, the epilogue takes the accumulators to registers, gives them back and
+// writes.  The integer and FP32 work of cutting and combining bounds it (about 160
+// instructions per entry, 51% of the issue slots), the MMAs come next (one of up to
+// 256 columns holds the tensor pipe ~130 clocks: 54 of them for a tile of 48
+// spinors, 90 for 80).  A CTA per tile went through the same steps one after the
+// other: 1628 us for the 300 spwfs of 36^3 (blocks of 75), now 573; 110 for the 160
+// of 24^3 (40), now 82.
+constexpr int kRoleWarps = 8;                       // epilogue: warps 0-7, slicers: 8-15
+constexpr int kApplyThreads = 2 * kRoleWarps * 32 + 32;   // and the MMA warp
+constexpr int kSmemCap = 225 * 1024;
+
+__host__ __device__ constexpr int apply_accs(int nd) { return nd == oz::kDigits64 ? oz::kAccs64 : (int)oz::kAccs; }
+__host__ __device__ constexpr int apply_plane(int np) { return kRows * np * 2; }
+__host__ __device__ constexpr int apply_coef(int nd, int np) { return nd * np * np * 2; }
+// operand and accumulator buffers that fit
+__host__ __device__ constexpr int apply_bufs(int nd, int np) {
+    return 2 * nd * apply_plane(np) + apply_coef(nd, np) + 128 <= kSmemCap ? 2 : 1;
+}
+__host__ __device__ constexpr int apply_tbufs(int nd, int np) {
+    return 2 * apply_accs(nd) * np <= 512 ? 2 : 1;
+}
+__host__ __device__ constexpr size_t apply_smem(int nd, int np) {
+    return (size_t)apply_bufs(nd, np) * nd * apply_plane(np) + apply_coef(nd, np) + 128;
+}
+
+__device__ __forceinline__ bool wait_warp(uint64_t* mbar, uint32_t parity) {
+    return __all_sync(0xffffffffu, tc::mbar_wait(mbar, parity, kWaitCycles)) != 0;
+}
+__device__ __forceinline__ void arrive_warp(uint64_t* mbar, int lane) {
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(mbar);
+}
+
+template <int ND, int NP>
+__global__ void __launch_bounds__(kApplyThreads, 1)
 k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
            const int* __restrict__ in_list, const int* __restrict__ out_list,
            const int* __restrict__ out_base, const uint16_t* __restrict__ xd,
-           const int* __restrict__ xe, long V4, int* __restrict__ status) {
+           const int* __restrict__ xe, long V4, int tpb, int ntiles, int* __restrict__ status) {
+    constexpr int NACC = apply_accs(ND), NBUF = apply_bufs(ND, NP), NTB = apply_tbufs(ND, NP);
+    constexpr int kg = NP / 8, kPlane = apply_plane(NP);
     extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t fullA[2], emptyA[2], fullT[2], emptyT[2], emaxReady[4];
     __shared__ uint32_t tmem_slot;
-    __shared__ int sEmax[256];
-    __shared__ int sXe[kMeshTcMax];
-    __shared__ int sIdx[kMeshTcMax];
-    __shared__ int sOut[kMeshTcMax];
-    const int b = blockIdx.y;
-    const int s0 = bi.off(b), nb = bi.nb(b);
-    if (nb == 0) return;
-    const int Np = max(16, (nb + 15) / 16 * 16);
-    const int kg = Np / 8;
-    const uint32_t tcols = tmem_cols(Np);
+    __shared__ int sEx[2][2 * kRows];          // the two slicers of a point
+    __shared__ int sEmax[4][kRows];            // of the last tiles
+    __shared__ int sXe[NP], sIdx[NP], sOut[NP];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int row = tid & (kRows - 1), half = tid >> 7;
-    const long p = (long)blockIdx.x * kRows + row;
-    const bool live = p < V4;
-
     const uint32_t s0a = tc::smem_u32(smraw);
-    uint8_t* base = smraw + ((128u - (s0a & 127u)) & 127u);
-    const int aPlane = kRows * Np * 2, bPlane = Np * Np * 2;
-    uint8_t* sA = base;
-    uint8_t* sB = sA + kDigits * aPlane;
-    if (warp == 0) tc::alloc(&tmem_slot, tcols);
-    if (tid == 0) tc::mbar_init(&mbar, 1);
-    {
-        const uint4* src = reinterpret_cast<const uint4*>(xd + (long)b * kDigits * kXdStride);
-        uint4* dst = reinterpret_cast<uint4*>(sB);
-        for (int t = tid; t < kDigits * bPlane / 16; t += 256) dst[t] = src[t];
-        if (tid < kMeshTcMax) {
-            sXe[tid] = tid < Np ? xe[b * kMeshTcMax + tid] : 0;
-            sIdx[tid] = tid < nb ? in_list[s0 + tid] : 0;
-            sOut[tid] = tid < nb ? (out_list ? out_list[s0 + tid] : out_base[b] + tid) : 0;
-        }
-    }
-    __syncthreads();
-    if (kg <= 6) {
-        // the point's values psi_k(p) for this thread's K groups
-        double v[24];
-#pragma unroll
-        for (int u = 0; u < 24; ++u) {
-            const int k = 8 * (half + 2 * (u >> 3)) + (u & 7);
-            v[u] = (live && k < nb) ? in[(long)sIdx[k] * V4 + p] : 0.0;
-        }
-        int emax = 0;
-#pragma unroll
-        for (int u = 0; u < 24; ++u) emax = max(emax, oz::bexp(v[u]));
-        sEmax[tid] = emax;
-        __syncthreads();
-        emax = max(sEmax[row], sEmax[row + kRows]);
-#pragma unroll
-        for (int gg = 0; gg < 3; ++gg) {
-            const int g = half + 2 * gg;
-            if (g >= kg) continue;
-            uint4 w[kDigits];
-            if (8 * g < nb) {
-                double v8[8];
-#pragma unroll
-                for (int h = 0; h < 8; ++h) v8[h] = v[8 * gg + h];
-                oz::digits8(v8, emax, w);
-            } else {
-#pragma unroll
-                for (int a = 0; a < kDigits; ++a) w[a] = make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int a = 0; a < kDigits; ++a)
-                *reinterpret_cast<uint4*>(sA + a * aPlane + tc::kmajor_off_g(row, 8 * g, kg)) = w[a];
-        }
-    } else {
-        // blocks of 49 to kMeshTcMax spinors: the exponent pass, then the
-        // digits pass over the same values
-        int emax = 0;
-        for (int g = half; g < kg; g += 2)
-#pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                const int k = 8 * g + h;
-                if (live && k < nb) emax = max(emax, oz::bexp(in[(long)sIdx[k] * V4 + p]));
-            }
-        sEmax[tid] = emax;
-        __syncthreads();
-        emax = max(sEmax[row], sEmax[row + kRows]);
-        for (int g = half; g < kg; g += 2) {
-            uint4 w[kDigits];
-            if (8 * g < nb) {
-                double v8[8];
-#pragma unroll
-                for (int h = 0; h < 8; ++h) {
-                    const int k = 8 * g + h;
-                    v8[h] = (live && k < nb) ? in[(long)sIdx[k] * V4 + p] : 0.0;
-                }
-                oz::digits8(v8, emax, w);
-            } else {
-#pragma unroll
-                for (int a = 0; a < kDigits; ++a) w[a] = make_uint4(0u, 0u, 0u, 0u);
-            }
-#pragma unroll
-            for (int a = 0; a < kDigits; ++a)
-                *reinterpret_cast<uint4*>(sA + a * aPlane + tc::kmajor_off_g(row, 8 * g, kg)) = w[a];
-        }
-    }
-    tc::fence_proxy_async();
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = tmem_slot;
+    uint8_t* sA = smraw + ((128u - (s0a & 127u)) & 127u);
+    uint8_t* sB = sA + NBUF * ND * kPlane;
+    if (warp == 0) tc::alloc(&tmem_slot, 512u);
     if (tid == 0) {
-        const uint32_t idesc = tc::idesc_bf16(kRows, Np);
-        const uint32_t sbo = (uint32_t)kg * 128u;
-        const uint32_t aB = tc::smem_u32(sA), bB = tc::smem_u32(sB);
-        if (kg == 2)
-            oz::issue_pairs<1>(tmem, Np, idesc, aB, aPlane, sbo, bB, bPlane, sbo, false);
-        else if (kg == 4)
-            oz::issue_pairs<2>(tmem, Np, idesc, aB, aPlane, sbo, bB, bPlane, sbo, false);
-        else if (kg == 6)
-            oz::issue_pairs<3>(tmem, Np, idesc, aB, aPlane, sbo, bB, bPlane, sbo, false);
-        else if (kg == 8)
-            oz::issue_pairs<4>(tmem, Np, idesc, aB, aPlane, sbo, bB, bPlane, sbo, false);
-        else
-            oz::issue_pairs<5>(tmem, Np, idesc, aB, aPlane, sbo, bB, bPlane, sbo, false);
-        tc::commit(&mbar);
+        for (int q = 0; q < 2; ++q) {
+            tc::mbar_init(&fullA[q], kRoleWarps);
+            tc::mbar_init(&emptyA[q], 1);
+            tc::mbar_init(&fullT[q], 1);
+            tc::mbar_init(&emptyT[q], kRoleWarps);
+        }
+        for (int q = 0; q < 4; ++q) tc::mbar_init(&emaxReady[q], kRoleWarps);
     }
-    bool ok = tc::mbar_wait(&mbar, 0, kWaitCycles);
-    ok = __syncthreads_and(ok) != 0;
-    tc::fence_after();
-    if (ok) {
-        const int quarter = warp & 3, colh = warp >> 2;
-        const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-        // the epilogue's lane is point (quarter * 32 + lane) of the tile
-        const int erow = quarter * 32 + lane;
-        const long pe = (long)blockIdx.x * kRows + erow;
-        const int ep = max(sEmax[erow], sEmax[erow + kRows]) - 1023;
-        const bool elive = pe < V4 && max(sEmax[erow], sEmax[erow + kRows]) > 0;
-        for (int q = 0; q < Np / 16; ++q) {
-            const int c0 = 16 * q + 8 * colh;
-            uint32_t r0[8], r1[8], r2[8], r3[8];
-            __syncwarp();
-            tc::ld8(trow + (uint32_t)(0 * Np + c0), r0);
-            tc::ld8(trow + (uint32_t)(1 * Np + c0), r1);
-            tc::ld8(trow + (uint32_t)(2 * Np + c0), r2);
-            tc::ld8(trow + (uint32_t)(3 * Np + c0), r3);
-            tc::wait_ld(r0);
-            tc::wait_ld(r1);
-            tc::wait_ld(r2);
-            tc::wait_ld(r3);
-            if (pe >= V4) continue;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int l = c0 + u;
-                if (l >= nb) break;
-                double val = 0.0;
-                if (elive) {
-                    dfl o = oz::combine4(__uint_as_float(r0[u]), __uint_as_float(r1[u]),
-                                         __uint_as_float(r2[u]), __uint_as_float(r3[u]));
-                    const float sc = oz::pow2f(ep + sXe[l] - 1023 - 12);
-                    o.h = __fmul_rn(o.h, sc);
-                    o.l = __fmul_rn(o.l, sc);
-                    val = f2d_bits(o.h) + f2d_bits(o.l);
-                }
-                const long o = (long)sOut[l] * V4 + pe;
-                out[o] = val;
-                if (upd) upd[o] = val - upd[o];
+    const int t0 = (int)((long)ntiles * blockIdx.x / gridDim.x);
+    const int t1 = (int)((long)ntiles * (blockIdx.x + 1) / gridDim.x);
+    bool ok = true;
+    int k0 = 0;   // tiles of this CTA before the block at hand
+    uint32_t tmem = 0;
+    for (int ta = t0; ta < t1;) {
+        const int b = ta / tpb, te = min(t1, (b + 1) * tpb);
+        const int off = bi.off(b), nb = bi.nb(b);
+        const long first = (long)(ta - b * tpb) * kRows;
+        const int count = nb > 0 ? te - ta : 0;
+        ta = te;
+        if (count == 0) continue;
+        {
+            const uint4* src = reinterpret_cast<const uint4*>(xd + (long)b * ND * kXdStride);
+            uint4* dst = reinterpret_cast<uint4*>(sB);
+            for (int t = tid; t < apply_coef(ND, NP) / 16; t += kApplyThreads) dst[t] = src[t];
+            // K groups past the block's spinors stay zero
+            uint4* a = reinterpret_cast<uint4*>(sA);
+            for (int t = tid; t < NBUF * ND * kPlane / 16; t += kApplyThreads)
+                a[t] = make_uint4(0u, 0u, 0u, 0u);
+            if (tid < NP) {
+                sXe[tid] = xe[b * kMeshTcMax + tid];
+                sIdx[tid] = tid < nb ? in_list[off + tid] : 0;
+                sOut[tid] = tid < nb ? (out_list ? out_list[off + tid] : out_base[b] + tid) : 0;
             }
         }
-    } else {
-        if (tid == 0) atomicExch(status, 1);
-        tc::mbar_wait(&mbar, 0, kWaitCycles);
+        tc::fence_proxy_async();
+        tc::fence_before();
+        __syncthreads();
+        tc::fence_after();
+        tmem = tmem_slot;
+        if (warp >= kRoleWarps && warp < 2 * kRoleWarps) {
+            // ---------------- slicers ----------------
+            // thread: point `row`, K groups half, half + 2, ...
+            const int st = tid - 32 * kRoleWarps, row = st & (kRows - 1), half = st >> 7;
+            constexpr int own = (kg + 1) / 2;
+            for (int q = 0, k = k0; q < count; ++q, ++k) {
+                const int buf = k % NBUF;
+                const long p = first + (long)q * kRows + row;
+                double v[8 * own];
+                int emax = 0;
+#pragma unroll
+                for (int u = 0; u < 8 * own; ++u) {
+                    const int kk = 8 * (half + 2 * (u >> 3)) + (u & 7);
+                    v[u] = (p < V4 && kk < nb) ? in[(long)sIdx[kk] * V4 + p] : 0.0;
+                }
+#pragma unroll
+                for (int u = 0; u < 8 * own; ++u) emax = max(emax, oz::bexp(v[u]));
+                sEx[k & 1][st] = emax;
+                asm volatile("bar.sync 1, %0;" ::"n"(32 * kRoleWarps) : "memory");
+                emax = max(sEx[k & 1][row], sEx[k & 1][row + kRows]);
+                if (k >= NBUF) {
+                    ok = wait_warp(&emptyA[buf], ((k - NBUF) / NBUF) & 1);
+                    if (!ok) break;
+                }
+                if (half == 0) sEmax[k & 3][row] = emax;
+                arrive_warp(&emaxReady[k & 3], lane);
+                const oz::FixedRow<ND> fixed(emax);
+                uint8_t* planes = sA + buf * ND * kPlane;
+#pragma unroll
+                for (int gg = 0; gg < own; ++gg) {
+                    const int g = half + 2 * gg;
+                    if (8 * g >= nb) continue;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const double v4[4] = {v[8 * gg + 4 * h], v[8 * gg + 4 * h + 1],
+                                              v[8 * gg + 4 * h + 2], v[8 * gg + 4 * h + 3]};
+                        uint2 w[ND];
+                        oz::digits4<ND>(v4, fixed, w);
+#pragma unroll
+                        for (int a = 0; a < ND; ++a)
+                            *reinterpret_cast<uint2*>(planes + a * kPlane +
+                                                      tc::kmajor_off_g(row, 8 * g + 4 * h, kg)) = w[a];
+                    }
+                }
+                tc::fence_proxy_async();
+                arrive_warp(&fullA[buf], lane);
+            }
+        } else if (warp == 2 * kRoleWarps) {
+            // ---------------- MMA issue ----------------
+            if (lane == 0) {
+                int k = k0;
+                for (int q = 0; q < count; ++q, ++k) {
+                    const int buf = k % NBUF, tb = k % NTB;
+                    ok = tc::mbar_wait(&fullA[buf], (k / NBUF) & 1, kWaitCycles);
+                    if (ok && k >= NTB)
+                        ok = tc::mbar_wait(&emptyT[tb], ((k - NTB) / NTB) & 1, kWaitCycles);
+                    if (!ok) break;
+                    tc::fence_after();
+                    oz::issue_stacked<ND, NACC, NP, NP / 16>(
+                        tmem + (uint32_t)(tb * NACC * NP), tc::smem_u32(sA + buf * ND * kPlane),
+                        kPlane, tc::smem_u32(sB), (uint32_t)kg * 128u);
+                    tc::commit(&emptyA[buf]);
+                    tc::commit(&fullT[tb]);
+                }
+                // the last commit covers every MMA of this CTA
+                if (k > k0) ok &= tc::mbar_wait(&fullT[(k - 1) % NTB], ((k - 1) / NTB) & 1, kWaitCycles);
+            }
+            __syncwarp();
+        } else {
+            // ---------------- epilogue ----------------
+            // lane: point quarter * 32 + lane of the tile; columns 16 q + 8 colh + ...
+            const int quarter = warp & 3, colh = warp >> 2, erow = quarter * 32 + lane;
+            for (int q = 0, k = k0; q < count; ++q, ++k) {
+                const int tb = k % NTB;
+                const long pe = first + (long)q * kRows + erow;
+                ok = wait_warp(&emaxReady[k & 3], (k >> 2) & 1);
+                if (ok) ok = wait_warp(&fullT[tb], (k / NTB) & 1);
+                if (!ok) break;
+                tc::fence_after();
+                const int emax = sEmax[k & 3][erow];
+                const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) +
+                                      (uint32_t)(tb * NACC * NP + 8 * colh);
+                const int nch = max(0, (nb - 8 * colh + 15) / 16);   // chunks of 8 columns
+                if (nch == 0) {
+                    tc::fence_before();
+                    arrive_warp(&emptyT[tb], lane);
+                }
+#pragma unroll 1
+                for (int c = 0; c < nch; ++c) {
+                    const int l0 = 16 * c + 8 * colh;
+                    uint32_t r[NACC][8];
+                    __syncwarp();
+#pragma unroll
+                    for (int g = 0; g < NACC; ++g) tc::ld8(trow + (uint32_t)(g * NP + 16 * c), r[g]);
+                    double was[8];
+                    if (upd && pe < V4)
+#pragma unroll
+                        for (int u = 0; u < 8; ++u)
+                            if (l0 + u < nb) was[u] = upd[(long)sOut[l0 + u] * V4 + pe];
+#pragma unroll
+                    for (int g = 0; g < NACC; ++g) tc::wait_ld(r[g]);
+                    if (c == nch - 1) {
+                        // the last accumulators of this tile are in registers
+                        tc::fence_before();
+                        arrive_warp(&emptyT[tb], lane);
+                    }
+                    if (pe >= V4) continue;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        if (l0 + u >= nb) break;
+                        const int ex = sXe[l0 + u];
+                        double x = 0.0;
+                        if (emax > 0) {
+                            dfl o = oz::combine4(__uint_as_float(r[0][u]), __uint_as_float(r[1][u]),
+                                                 __uint_as_float(r[2][u]), __uint_as_float(r[3][u]));
+                            const float sc = oz::pow2f(emax - 1023 + ex - 1023 - 12);
+                            o.h = __fmul_rn(o.h, sc);
+                            o.l = __fmul_rn(o.l, sc);
+                            x = f2d_bits(o.h) + f2d_bits(o.l);
+                        }
+                        const long o = (long)sOut[l0 + u] * V4 + pe;
+                        out[o] = x;
+                        if (upd) upd[o] = x - was[u];
+                    }
+                }
+            }
+        }
+        k0 += count;
+        ok = __syncthreads_and(ok) != 0;
+        if (!ok) break;
     }
+    if (!ok && tid == 0) atomicExch(status, 1);
     tc::fence_before();
     __syncthreads();
-    if (warp == 0) tc::dealloc(tmem, tcols);
+    if (warp == 0) tc::dealloc(tmem_slot, 512u);
 }
 
 // Pairing gaps, HFBGaps (src/HFB.f90:520-632), per block b (isospin b / 2):
@@ -664,8 +731,6 @@ bool gs_tc_prepare(mg_ctx* c) {
             return false;
         cudaFuncSetAttribute(k_gs_overlap_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              200 * 1024);
-        cudaFuncSetAttribute(k_apply_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024);
     }
     return true;
 }
@@ -681,20 +746,32 @@ int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d
     return MG_OK;
 }
 
-static int apply_tc(mg_ctx* c, int nblk, int nbmax, const double* coef, long bstride, int ld,
-                    BlockIdx bi, const double* in, double* out, double* upd, const int* in_list,
-                    const int* out_list, const int* out_base, uint16_t* xd, int* xe) {
-    k_coef_digits<<<nblk, 96, 0, c->stream>>>(coef, bstride, ld, bi, xd, xe);
+template <int ND, int NP>
+static int apply_launch(mg_ctx* c, int nblk, const double* coef, long bstride, int ld, BlockIdx bi,
+                        const double* in, double* out, double* upd, const int* in_list,
+                        const int* out_list, const int* out_base, uint16_t* xd, int* xe) {
+    k_coef_digits<ND, NP><<<nblk, dim3(NP, kCoefRows), 0, c->stream>>>(coef, bstride, ld, bi, xd, xe);
     MG_LAUNCHED(c);
-    const int Np = std::max(16, (nbmax + 15) / 16 * 16);
-    size_t sm = 128 + (size_t)kDigits * (kRows * Np * 2 + Np * Np * 2);
-    // at most two CTAs per SM (2 x 256 TMEM columns), one above N = 64
-    sm = std::max(sm, tmem_cols(Np) > 256 ? kOneCtaSmem : (size_t)80 * 1024);
+    MG_CUDA(cudaFuncSetAttribute(k_apply_tc<ND, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)apply_smem(ND, NP)));
     const long V4 = 4 * c->V;
-    k_apply_tc<<<dim3(div_up(V4, kRows), nblk), 256, sm, c->stream>>>(
-        in, out, upd, bi, in_list, out_list, out_base, xd, xe, V4, c->tc_status);
+    const int tpb = div_up(V4, kRows), ntiles = tpb * nblk;
+    const int sms = c->tc_grid_cap > 0 ? std::min(c->tc_grid_cap, c->num_sms) : c->num_sms;
+    k_apply_tc<ND, NP><<<std::min(sms, ntiles), kApplyThreads, apply_smem(ND, NP), c->stream>>>(
+        in, out, upd, bi, in_list, out_list, out_base, xd, xe, V4, tpb, ntiles, c->tc_status);
     MG_LAUNCHED(c);
     return MG_OK;
+}
+
+template <class... A>
+static int apply_tc(mg_ctx* c, int nblk, int nbmax, A... args) {
+    switch (std::max(1, div_up(nbmax, 16))) {
+        case 1: return apply_launch<kDigits, 16>(c, nblk, args...);
+        case 2: return apply_launch<kDigits, 32>(c, nblk, args...);
+        case 3: return apply_launch<kDigits, 48>(c, nblk, args...);
+        case 4: return apply_launch<kDigits, 64>(c, nblk, args...);
+        default: return apply_launch<kDigits, 80>(c, nblk, args...);
+    }
 }
 
 int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const int* d_ordered) {
@@ -713,8 +790,6 @@ int can_transform_tc(mg_ctx* c) {
         MG_CUDA(cudaMalloc(&c->can_xd, (size_t)4 * kDigits * kXdStride * sizeof(uint16_t)));
         MG_CUDA(cudaMemset(c->can_xd, 0, (size_t)4 * kDigits * kXdStride * sizeof(uint16_t)));
         MG_CUDA(cudaMalloc(&c->can_xe, (size_t)4 * kMeshTcMax * sizeof(int)));
-        MG_CUDA(cudaFuncSetAttribute(k_apply_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     200 * 1024));
     }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
     return apply_tc(c, 4, H.hmax, H.cantr, (long)H.hmax * H.hmax, 0, bi,
@@ -762,8 +837,6 @@ int pair_field_tc(mg_ctx* c) {
         MG_CUDA(cudaMalloc(&c->field_ybase, 4 * sizeof(int)));
         const int yb[4] = {0, H.hmax, 2 * H.hmax, 3 * H.hmax};
         MG_CUDA(cudaMemcpy(c->field_ybase, yb, sizeof(yb), cudaMemcpyHostToDevice));
-        MG_CUDA(cudaFuncSetAttribute(k_apply_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     200 * 1024));
     }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
     MG_TRY(apply_tc(c, 4, H.hmax, H.ktil, (long)H.hmax * H.hmax, 0, bi,
