@@ -45,8 +45,11 @@ __device__ __forceinline__ void pauli(const double* p, int dir, double* o) {
     else { o[0] = p[0]; o[1] = p[1]; o[2] = -p[2]; o[3] = -p[3]; }
 }
 
+// Bound by the FP64 pipe (a warp's instruction takes 16 clocks of the SM): 83 FP64
+// instructions a point, 95 with the GradDesc step.  200 spwfs at 32^3: 916 us (1180
+// with 101, the terms summed one by one), 160 at 24^3 with the step 495 (510).
 template <bool kGradStep>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 3)
 k_hpsi(double* __restrict__ psi, const double* __restrict__ der,
        const double* __restrict__ lap, const int* __restrict__ qn, Fields F,
        double* __restrict__ hout, double* __restrict__ upd, double* __restrict__ partial,
@@ -73,37 +76,32 @@ k_hpsi(double* __restrict__ psi, const double* __restrict__ der,
         const double nb0 = F.nablaB[(it * 3 + 0) * V + v];
         const double nb1 = F.nablaB[(it * 3 + 1) * V + v];
         const double nb2 = F.nablaB[(it * 3 + 2) * V + v];
-        double w[4] = {0.0, 0.0, 0.0, 0.0};
+        // one chain of FMAs per component: U, B, then W
+        double h[4];
+        const double bk = -(Bq + kin);
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+            h[l] = fma(bk, L[l], Uq * p[l]);
+            h[l] = fma(-nb0, d[0][l], h[l]);
+            h[l] = fma(-nb1, d[1][l], h[l]);
+            h[l] = fma(-nb2, d[2][l], h[l]);
+        }
+        // -i c sigma_n psi: (re, im) of a component from (im, -re)
+        const auto spin = [&](const double* q, int n, double c) {
+            double t[4];
+            pauli(q, n, t);
+            h[0] = fma(c, t[1], h[0]);
+            h[1] = fma(-c, t[0], h[1]);
+            h[2] = fma(c, t[3], h[2]);
+            h[3] = fma(-c, t[2], h[3]);
+        };
 #pragma unroll
         for (int mu = 0; mu < 3; ++mu)
 #pragma unroll
-            for (int nu = 0; nu < 3; ++nu) {
-                double s[4];
-                pauli(d[mu], nu + 1, s);
-                const double wv = F.W[((it * 3 + nu) * 3 + mu) * V + v];
+            for (int nu = 0; nu < 3; ++nu)
+                spin(d[mu], nu + 1, F.W[((it * 3 + nu) * 3 + mu) * V + v]);
 #pragma unroll
-                for (int l = 0; l < 4; ++l) w[l] = fma(wv, s[l], w[l]);
-            }
-#pragma unroll
-        for (int nu = 0; nu < 3; ++nu) {
-            double s[4];
-            pauli(p, nu + 1, s);
-            const double hv = 0.5 * F.divW[(it * 3 + nu) * V + v];
-#pragma unroll
-            for (int l = 0; l < 4; ++l) w[l] = fma(hv, s[l], w[l]);
-        }
-        const double wf[4] = {w[1], -w[0], w[3], -w[2]};
-        double h[4];
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            double t = -(Bq * L[l]);
-            t = t - kin * L[l];
-            double sd = fma(nb1, d[1][l], nb0 * d[0][l]);
-            sd = fma(nb2, d[2][l], sd);
-            const double b = t - sd;
-            const double u = Uq * p[l];
-            h[l] = (b + u) + wf[l];
-        }
+        for (int nu = 0; nu < 3; ++nu) spin(p, nu + 1, 0.5 * F.divW[(it * 3 + nu) * V + v]);
         if (F.A) {
             // ActionOfS: sum_m S_m sigma_m psi; ActionOfA: -i (sum_m A_m d_m psi
             // + 1/2 div A psi) (src/MeanFields.f90:1107-1147)
@@ -151,21 +149,20 @@ k_hpsi(double* __restrict__ psi, const double* __restrict__ der,
             for (int l = 0; l < 4; ++l) ho[l * V + v] = h[l];
         }
     }
-    // block reduction of (s_eh, s_hh)
-    __shared__ double red[2][kThreads / 32];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        s_eh += __shfl_xor_sync(0xffffffffu, s_eh, o);
-        s_hh += __shfl_xor_sync(0xffffffffu, s_hh, o);
-    }
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    if (lane == 0) { red[0][warp] = s_eh; red[1][warp] = s_hh; }
+    // block sums of (s_eh, s_hh): warps 0 and 1 add 8 values a lane and then the
+    // lanes (shuffles in every warp would be a tenth of the kernel's FP64 work)
+    __shared__ double red[2][kThreads];
+    red[0][threadIdx.x] = s_eh;
+    red[1][threadIdx.x] = s_hh;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0.0, b = 0.0;
-        for (int q = 0; q < kThreads / 32; ++q) { a += red[0][q]; b += red[1][q]; }
-        partial[((long)i * gridDim.x + blockIdx.x) * 2 + 0] = a;
-        partial[((long)i * gridDim.x + blockIdx.x) * 2 + 1] = b;
+    if (threadIdx.x < 64) {
+        const int q = threadIdx.x / 32, lane = threadIdx.x % 32;
+        double a = red[q][lane];
+#pragma unroll
+        for (int u = 1; u < kThreads / 32; ++u) a += red[q][lane + 32 * u];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+        if (lane == 0) partial[((long)i * gridDim.x + blockIdx.x) * 2 + q] = a;
     }
 }
 
