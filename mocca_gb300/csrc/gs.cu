@@ -14,9 +14,10 @@
 //   k_gs_factor   : S = R^T R, X = R^{-1} (one block per CTA, in smem)
 //   k_gs_apply    : psi'_l = sum_{k<=l} X_kl psi_k in place (+ update history)
 // For the near-orthonormal input of an imaginary-time step cond(S) ~ 1, so
-// the Cholesky form keeps full FP64 accuracy.  In the mixed form the overlap
-// and the apply run on the tensor cores instead (meshgemm_tc.cu); the sum, the
-// factorisation and the order stay these FP64 kernels.
+// the Cholesky form keeps full FP64 accuracy.  In the mixed form and, for blocks of
+// 24 to 64 spinors, in the FP64 form the overlap and the apply run on the tensor cores
+// instead (meshgemm_tc.cu); the sum, the factorisation and the order stay these FP64
+// kernels.
 #include "mg_internal.cuh"
 
 namespace mg {
@@ -260,17 +261,18 @@ int gram_schmidt_impl(mg_ctx* c, double* upd) {
                                                                  d_ordered);
     MG_LAUNCHED(c);
     const size_t sm_f = (size_t)(2 * nbmax * nbmax) * sizeof(double);
-    if (c->cur_precision == MG_MIXED && gs_tc_prepare(c)) {
-        // mixed form: the overlap and the apply on the tensor cores (meshgemm_tc.cu)
-        const int nct = c->gs_nchunk_tc;
-        MG_TRY(gs_overlap_tc(c, B.psi, d_lists, d_ordered));
+    const bool f64 = c->cur_precision != MG_MIXED;
+    if (gs_tc_prepare(c, f64)) {
+        // the overlap and the apply on the tensor cores (meshgemm_tc.cu)
+        int nct = 0;
+        MG_TRY(gs_overlap_tc(c, B.psi, d_lists, d_ordered, f64, &nct));
         k_gs_sum<<<dim3(div_up((long)nbmax * nbmax, kThreads / 32), nblk), kThreads, 0,
                    c->stream>>>(c->gs_Stc, nbmax, nct);
         MG_LAUNCHED(c);
         k_gs_factor<<<nblk, kThreads, sm_f, c->stream>>>(c->gs_Stc, d_lists, nbmax, nct, c->dv,
                                                          c->gs_R, c->flags);
         MG_LAUNCHED(c);
-        return gs_apply_tc(c, B.psi, upd, d_lists, d_ordered);
+        return gs_apply_tc(c, B.psi, upd, d_lists, d_ordered, f64);
     }
     const int npair_max = nbmax * (nbmax + 1) / 2;
     const size_t sm_ov = (size_t)(nbmax * kPts + npair_max) * sizeof(double);

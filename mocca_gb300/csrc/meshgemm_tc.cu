@@ -1,19 +1,23 @@
-// meshgemm_tc.cu -- the mesh-sized contractions of the mixed form on the
-// tcgen05 tensor cores (exact BF16 digit products, ozaki.cuh): the
-// Gram-Schmidt overlap and apply, and the canonical-basis transform.
+// meshgemm_tc.cu -- the mesh-sized contractions on the tcgen05 tensor cores
+// (exact BF16 digit products, ozaki.cuh): the Gram-Schmidt overlap and apply,
+// in the mixed form with six digits and in the FP64 form with eight, and the
+// mixed form's canonical-basis transform and pairing contractions.
 //
-// Blocks of up to kMeshTcMax (80) spinors; above 64, four accumulators take
-// 512 TMEM columns and the overlap and gaps kernels run one CTA per SM.
+// Blocks of up to kMeshTcMax (80) spinors in the mixed form, kMeshTcMin64 to
+// kMeshTcMax64 (24 to 64) in the FP64 form, whose results are rounded once to FP64
+// (norm-wise errors of the Gram-Schmidt of blocks of 22 to 50, mean over the spinors:
+// 1.27e-16 to 1.49e-16, with FP64 FMAs 1.31e-16 to 1.59e-16).  Above 64, four
+// accumulators take 512 TMEM columns and the gaps kernel runs one CTA per SM.
 //
 // Gram-Schmidt (gs.cu; GramSchmidt, src/SpwfStorage.f90:372-480, as
 // Q = Psi R^{-1} with S = R^T R per (isospin, parity, signature) block in
 // energy order):
-//   k_gs_overlap_tc : S partial sums over 256-point chunks.  Rows of the
-//                     MMA are the block's spinors (zero beyond nb), K the
-//                     chunk's points; A and B are the same digit planes.  Each
-//                     (spinor, chunk) row gets its own power of two.  The
-//                     partials go to the same table as the FP64 kernel, so
-//                     k_gs_sum / k_gs_factor (gs.cu) finish the job.
+//   k_gs_overlap_tc : S partial sums over chunks of 256 points (128).  Rows of
+//                     the MMA are the block's spinors, K the chunk's points; A
+//                     and B are the same digit planes.  Each (spinor, chunk) row
+//                     gets its own power of two.  The partials go to the same
+//                     kind of table as the FP64 kernel's, so k_gs_sum /
+//                     k_gs_factor (gs.cu) finish the job.
 // Block apply, out_l(p) = sum_k C[k][l] in_k(p) per block of spinors:
 //   k_coef_digits   : digit planes of C (rows: output l, K: input k), one
 //                     power of two per row;
@@ -22,8 +26,9 @@
 //                     GradDesc history upd_l = out_l - upd_l.  Canonical basis
 //                     (HFBOccupations, src/HFB.f90:3448-3487): C = CanTransfo,
 //                     HF basis in, canonical basis out.
-// A 256-point chunk keeps every digit-weight group of the overlap below 2^24
-// (at most 3 pairs x 256 points x 2^14), so its FP32 sums are exact.
+// A chunk keeps the digit-weight groups of the overlap that have an accumulator of
+// their own below 2^24 (at most 3 pairs x 256 points x 2^14, in the FP64 form 6 x 128),
+// so their FP32 sums are exact.
 #include <algorithm>
 #include <vector>
 
@@ -63,141 +68,250 @@ __device__ __forceinline__ double pow2d(int x) {
     return x < -1022 ? 0.0 : __longlong_as_double((long long)(min(x, 1023) + 1023) << 52);
 }
 
-__global__ void __launch_bounds__(256, 2)
-k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
-                const int* __restrict__ ordered, int nbmax, long V4, int nchunk,
-                double* __restrict__ part, int* __restrict__ status) {
-    extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t mbar[2];
-    __shared__ uint32_t tmem_slot;
-    __shared__ int sE[kRows];
-    const int b = blockIdx.y, chunk = blockIdx.x;
-    const int s0 = starts[b], nb = starts[b + 1] - s0;
-    if (nb == 0) return;
-    const int N = max(16, (nb + 15) / 16 * 16);
-    const uint32_t tcols = tmem_cols(N);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // rows row0 and row0 + 64 (blocks above 64 spinors); a row's 4 K groups
-    // sit on 4 neighbouring lanes
-    const int row0 = tid >> 2, g = tid & 3;
+// Sum over a chunk of points of psi_k psi_l for the pairs k <= l of a block, to part.
+//
+// A unit is a chunk of one block, 256 points in the mixed form, 128 in the FP64 form
+// (what keeps the sums of a weight exact).  One CTA per SM takes a run of units with
+// the roles of k_apply_tc: the slicers cut stages of kStage points into a ring of
+// plane buffers, one thread issues a stage's MMAs, the epilogue writes a unit's sums
+// while the next unit's stages go on.  A's rows are the planes' own, one after the
+// other, so that the planes are B's stacked columns too; what A reads past a plane's
+// NP rows gives rows of D that nothing reads.  The tensor pipe bounds it (36 MMAs of
+// ~130 clocks a stage of 32 points): 300 spwfs of 36^3 (blocks of 75) 566 us, 834
+// with a CTA per chunk; the FP64 form for 160 of 24^3 (40) 156, 512 by FP64 FMAs.
+constexpr int kRoleWarps = 8;                       // epilogue: warps 0-7, slicers: 8-15
+constexpr int kRoleThreads = 2 * kRoleWarps * 32 + 32;   // and the MMA warp
+constexpr int kSmemCap = 225 * 1024;
+constexpr int kNone = 255;
 
+__host__ __device__ constexpr int accs_for(int nd) { return nd == oz::kDigits64 ? oz::kAccs64 : (int)oz::kAccs; }
+__host__ __device__ constexpr int chunk_for(int nd) { return nd == oz::kDigits64 ? 128 : kChunk; }
+__host__ __device__ constexpr int tbufs_for(int nd, int np) { return 2 * accs_for(nd) * np <= 512 ? 2 : 1; }
+__host__ __device__ constexpr int overlap_stage(int nd, int np) { return nd * np * kStage * 2; }
+constexpr int kOverlapTail = kRows * kStage * 2;    // A's reads past the last plane
+__host__ __device__ constexpr int overlap_bufs(int nd, int np) {
+    return (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np) >= 6
+               ? 6 : (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np);
+}
+__host__ __device__ constexpr size_t overlap_smem(int nd, int np) {
+    return (size_t)overlap_bufs(nd, np) * overlap_stage(nd, np) + kOverlapTail + 128;
+}
+
+__device__ __forceinline__ bool wait_warp(uint64_t* mbar, uint32_t parity) {
+    return __all_sync(0xffffffffu, tc::mbar_wait(mbar, parity, kWaitCycles)) != 0;
+}
+__device__ __forceinline__ void arrive_warp(uint64_t* mbar, int lane) {
+    __syncwarp();
+    if (lane == 0) tc::mbar_arrive(mbar);
+}
+
+template <int ND, int NP>
+__global__ void __launch_bounds__(kRoleThreads, 1)
+k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
+                const int* __restrict__ ordered, int nbmax, long V4, int nchunk, int nunits,
+                double* __restrict__ part, int* __restrict__ status) {
+    constexpr int NACC = accs_for(ND), NBUF = overlap_bufs(ND, NP), NTB = tbufs_for(ND, NP);
+    constexpr int CH = chunk_for(ND), kPlane = NP * kStage * 2, kBuf = overlap_stage(ND, NP);
+    constexpr int kPasses = (NP + 63) / 64;   // rows of a slicer: row0, row0 + 64
+    extern __shared__ uint8_t smraw[];
+    __shared__ __align__(8) uint64_t full[6], empty[6], fullT[2], emptyT[2], expReady[8];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int sE[8][NP];   // of the last units
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t s0a = tc::smem_u32(smraw);
     uint8_t* base = smraw + ((128u - (s0a & 127u)) & 127u);
-    // two stage buffers of kDigits planes; rows >= nb stay zero
-    for (int t = tid; t < 2 * kDigits * kStagePlane / 16; t += 256)
+    for (int t = tid; t < (NBUF * kBuf + kOverlapTail) / 16; t += kRoleThreads)
         reinterpret_cast<uint4*>(base)[t] = make_uint4(0u, 0u, 0u, 0u);
-    if (warp == 0) tc::alloc(&tmem_slot, tcols);
+    if (warp == 0) tc::alloc(&tmem_slot, 512u);
     if (tid == 0) {
-        tc::mbar_init(&mbar[0], 1);
-        tc::mbar_init(&mbar[1], 1);
-    }
-    const long p0 = (long)chunk * kChunk;
-    const int npts = (int)min((long)kChunk, V4 - p0);
-    const int nst = (npts + kStage - 1) / kStage;
-    bool live[2];
-    const double* src[2];
-    int emax[2] = {0, 0};
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int row = row0 + 64 * r;
-        live[r] = row < nb;
-        src[r] = live[r] ? psi + (long)ordered[s0 + row] * V4 + p0 : psi;
-        // largest exponent of the row over the chunk
-        if (live[r]) {
-            for (int s = 0; s < nst; ++s) {
-#pragma unroll
-                for (int h = 0; h < 8; ++h) {
-                    const int q = s * kStage + 8 * g + h;
-                    if (q < npts) emax[r] = max(emax[r], oz::bexp(src[r][q]));
-                }
-            }
+        for (int q = 0; q < NBUF; ++q) {
+            tc::mbar_init(&full[q], kRoleWarps);
+            tc::mbar_init(&empty[q], 1);
         }
-        emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 1));
-        emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 2));
-        if (live[r] && g == 0) sE[row] = emax[r];
+        for (int q = 0; q < 2; ++q) {
+            tc::mbar_init(&fullT[q], 1);
+            tc::mbar_init(&emptyT[q], kRoleWarps);
+        }
+        for (int q = 0; q < 8; ++q) tc::mbar_init(&expReady[q], kRoleWarps);
     }
-
+    tc::fence_proxy_async();
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = tc::idesc_bf16(kRows, N);
+    const int u0 = (int)((long)nunits * blockIdx.x / gridDim.x);
+    const int u1 = (int)((long)nunits * (blockIdx.x + 1) / gridDim.x);
     bool ok = true;
-    for (int s = 0; s < nst; ++s) {
-        const int buf = s & 1;
-        uint8_t* planes = base + buf * kDigits * kStagePlane;
-        if (s >= 2) ok &= tc::mbar_wait(&mbar[buf], ((s - 2) >> 1) & 1, kWaitCycles);
+    // units of empty blocks are passed over by every role
+    const auto stages_of = [&](int unit, int& b, int& s0, int& nb, long& p0, int& npts) {
+        b = unit / nchunk;
+        s0 = starts[b];
+        nb = starts[b + 1] - s0;
+        p0 = (long)(unit - b * nchunk) * CH;
+        npts = (int)min((long)CH, V4 - p0);
+        return nb > 0 ? (npts + kStage - 1) / kStage : 0;
+    };
+    int b, s0, nb, npts;
+    long p0;
+    if (warp >= kRoleWarps && warp < 2 * kRoleWarps) {
+        // ---------------- slicers ----------------
+        // a row's 4 K groups sit on 4 neighbouring lanes
+        const int st = tid - 32 * kRoleWarps, row0 = st >> 2, g = st & 3;
+        int stage = 0;   // stages of this CTA so far
+        for (int unit = u0, k = 0; unit < u1 && ok; ++unit) {
+            const int nst = stages_of(unit, b, s0, nb, p0, npts);
+            if (nst == 0) continue;
+            const double* src[kPasses];
+            int emax[kPasses];
 #pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            if (!live[r]) continue;
-            double v[8];
+            for (int r = 0; r < kPasses; ++r) {
+                const int row = row0 + 64 * r;
+                src[r] = row < nb ? psi + (long)ordered[s0 + row] * V4 + p0 : nullptr;
+                emax[r] = 0;
+                if (src[r])
+                    for (int s = 0; s < nst; ++s) {
 #pragma unroll
-            for (int h = 0; h < 8; ++h) {
-                const int q = s * kStage + 8 * g + h;
-                v[h] = q < npts ? src[r][q] : 0.0;
+                        for (int h = 0; h < 8; ++h) {
+                            const int q = s * kStage + 8 * g + h;
+                            if (q < npts) emax[r] = max(emax[r], oz::bexp(src[r][q]));
+                        }
+                    }
+                emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 1));
+                emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 2));
             }
-            uint4 w[kDigits];
-            oz::digits8(v, emax[r], w);
+            // (the epilogue of unit k - 8 has read its slot: the ring's stages and the
+            // accumulators let the slicers run at most five units ahead)
 #pragma unroll
-            for (int a = 0; a < kDigits; ++a)
-                *reinterpret_cast<uint4*>(planes + a * kStagePlane +
-                                          tc::kmajor_off(row0 + 64 * r, 8 * g)) = w[a];
+            for (int r = 0; r < kPasses; ++r)
+                if (src[r] && g == 0) sE[k & 7][row0 + 64 * r] = emax[r];
+            arrive_warp(&expReady[k & 7], lane);
+            ++k;
+            for (int s = 0; s < nst; ++s, ++stage) {
+                const int buf = stage % NBUF;
+                double v[kPasses][8];
+#pragma unroll
+                for (int r = 0; r < kPasses; ++r)
+#pragma unroll
+                    for (int h = 0; h < 8; ++h) {
+                        const int q = s * kStage + 8 * g + h;
+                        v[r][h] = src[r] && q < npts ? src[r][q] : 0.0;
+                    }
+                if (stage >= NBUF) {
+                    ok = wait_warp(&empty[buf], ((stage - NBUF) / NBUF) & 1);
+                    if (!ok) break;
+                }
+                uint8_t* planes = base + buf * kBuf;
+#pragma unroll
+                for (int r = 0; r < kPasses; ++r) {
+                    const int row = row0 + 64 * r;
+                    if (row >= NP) continue;
+                    const oz::FixedRow<ND> fixed(emax[r]);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const double v4[4] = {v[r][4 * h], v[r][4 * h + 1], v[r][4 * h + 2],
+                                              v[r][4 * h + 3]};
+                        uint2 w[ND];
+                        oz::digits4<ND>(v4, fixed, w);
+#pragma unroll
+                        for (int a = 0; a < ND; ++a)
+                            *reinterpret_cast<uint2*>(planes + a * kPlane +
+                                                      tc::kmajor_off(row, 8 * g + 4 * h)) = w[a];
+                    }
+                }
+                tc::fence_proxy_async();
+                arrive_warp(&full[buf], lane);
+            }
         }
-        tc::fence_proxy_async();
-        tc::fence_before();
-        __syncthreads();
-        tc::fence_after();
-        if (tid == 0) {
-            const uint32_t pa = tc::smem_u32(planes);
-            oz::issue_pairs<2>(tmem, N, idesc, pa, kStagePlane, tc::kSbo, pa, kStagePlane,
-                               tc::kSbo, s > 0);
-            tc::commit(&mbar[buf]);
+    } else if (warp == 2 * kRoleWarps) {
+        // ---------------- MMA issue ----------------
+        if (lane == 0) {
+            int stage = 0, k = 0;
+            for (int unit = u0; unit < u1 && ok; ++unit) {
+                const int nst = stages_of(unit, b, s0, nb, p0, npts);
+                if (nst == 0) continue;
+                const int tb = k % NTB;
+                if (k >= NTB) ok = tc::mbar_wait(&emptyT[tb], ((k - NTB) / NTB) & 1, kWaitCycles);
+                for (int s = 0; s < nst && ok; ++s, ++stage) {
+                    const int buf = stage % NBUF;
+                    ok = tc::mbar_wait(&full[buf], (stage / NBUF) & 1, kWaitCycles);
+                    if (!ok) break;
+                    tc::fence_after();
+                    const uint32_t pa = tc::smem_u32(base + buf * kBuf);
+                    oz::issue_stacked<ND, NACC, NP, kStage / 16>(
+                        tmem + (uint32_t)(tb * NACC * NP), pa, kPlane, pa, tc::kSbo, s > 0);
+                    tc::commit(&empty[buf]);
+                }
+                if (!ok) break;
+                tc::commit(&fullT[tb]);
+                ++k;
+            }
+            // the last commit covers every MMA of this CTA (after a timeout: the
+            // buffers' last ones)
+            if (k > 0) ok &= tc::mbar_wait(&fullT[(k - 1) % NTB], ((k - 1) / NTB) & 1, kWaitCycles);
+            if (!ok && stage > 0)
+                tc::mbar_wait(&empty[(stage - 1) % NBUF], ((stage - 1) / NBUF) & 1, kWaitCycles);
         }
-    }
-    const int last = nst - 1;
-    ok &= tc::mbar_wait(&mbar[last & 1], (last >> 1) & 1, kWaitCycles);
-    ok = __syncthreads_and(ok) != 0;
-    tc::fence_after();
-    if (ok) {
+        __syncwarp();
+    } else {
+        // ---------------- epilogue ----------------
         // D[k][l], k = TMEM lane (row), l = column; warps w and w + 4 share lane quarter w % 4
-        const int quarter = warp & 3, colh = warp >> 2;
-        const int k = quarter * 32 + lane;
-        const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-        double* out = part + ((long)b * nchunk + chunk) * nbmax * nbmax;
-        const int ek = k < nb ? sE[k] - 1023 : 0;
-        for (int q = 0; q < N / 16; ++q) {
-            const int c0 = 16 * q + 8 * colh;
-            uint32_t r0[8], r1[8], r2[8], r3[8];
-            __syncwarp();
-            tc::ld8(trow + (uint32_t)(0 * N + c0), r0);
-            tc::ld8(trow + (uint32_t)(1 * N + c0), r1);
-            tc::ld8(trow + (uint32_t)(2 * N + c0), r2);
-            tc::ld8(trow + (uint32_t)(3 * N + c0), r3);
-            tc::wait_ld(r0);
-            tc::wait_ld(r1);
-            tc::wait_ld(r2);
-            tc::wait_ld(r3);
-            if (k >= nb) continue;
+        const int quarter = warp & 3, colh = warp >> 2, kr = quarter * 32 + lane;
+        for (int unit = u0, k = 0; unit < u1; ++unit) {
+            const int nst = stages_of(unit, b, s0, nb, p0, npts);
+            if (nst == 0) continue;
+            const int tb = k % NTB;
+            ok = wait_warp(&expReady[k & 7], (k >> 3) & 1);
+            if (ok) ok = wait_warp(&fullT[tb], (k / NTB) & 1);
+            if (!ok) break;
+            tc::fence_after();
+            const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) +
+                                  (uint32_t)(tb * NACC * NP + 8 * colh);
+            double* out = part + (long)unit * nbmax * nbmax;
+            const int* se = sE[k & 7];
+            const int ek = kr < nb ? se[kr] : 0;
+            // rows past the block have nothing to write
+            const int nch = quarter * 32 < nb ? (nb - 8 * colh + 15) / 16 : 0;
+#pragma unroll 1
+            for (int c = 0; c < nch; ++c) {
+                const int l0 = 16 * c + 8 * colh;
+                uint32_t r[NACC][8];
+                __syncwarp();
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int l = c0 + u;
-                if (l >= nb || l < k) continue;
-                const dfl o = oz::combine4(__uint_as_float(r0[u]), __uint_as_float(r1[u]),
-                                           __uint_as_float(r2[u]), __uint_as_float(r3[u]));
-                const double val = (f2d_bits(o.h) + f2d_bits(o.l)) * pow2d(ek + sE[l] - 1023 - 12);
-                out[k * nbmax + l] = val;
+                for (int q = 0; q < NACC; ++q) tc::ld8(trow + (uint32_t)(q * NP + 16 * c), r[q]);
+#pragma unroll
+                for (int q = 0; q < NACC; ++q) tc::wait_ld(r[q]);
+                if (kr >= nb) continue;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int l = l0 + u;
+                    if (l >= nb || l < kr) continue;
+                    double val;
+                    if constexpr (ND == oz::kDigits64) {
+                        uint32_t acc[NACC];
+#pragma unroll
+                        for (int q = 0; q < NACC; ++q) acc[q] = r[q][u];
+                        val = oz::combine64_any(acc, ek - 1023 + se[l] - 1023 - oz::kUnit64);
+                        if (ek == 0 || se[l] == 0) val = 0.0;
+                        if (ek == 2047 || se[l] == 2047)
+                            val = __longlong_as_double(0x7FF8000000000000ll);
+                    } else {
+                        const dfl o = oz::combine4(__uint_as_float(r[0][u]), __uint_as_float(r[1][u]),
+                                                   __uint_as_float(r[2][u]), __uint_as_float(r[3][u]));
+                        val = (f2d_bits(o.h) + f2d_bits(o.l)) * pow2d(ek - 1023 + se[l] - 1023 - 12);
+                    }
+                    out[kr * nbmax + l] = val;
+                }
             }
+            tc::fence_before();
+            arrive_warp(&emptyT[tb], lane);
+            ++k;
         }
-    } else if (tid == 0) {
-        atomicExch(status, 1);
     }
-    if (!ok) {
-        tc::mbar_wait(&mbar[0], 0, kWaitCycles);   // let the MMAs drain before the columns go
-        tc::mbar_wait(&mbar[1], 0, kWaitCycles);
-    }
+    ok = __syncthreads_and(ok) != 0;
+    if (!ok && tid == 0) atomicExch(status, 1);
     tc::fence_before();
     __syncthreads();
-    if (warp == 0) tc::dealloc(tmem, tcols);
+    if (warp == 0) tc::dealloc(tmem_slot, 512u);
 }
 
 // Digit planes of C (per block: ND planes of NP rows x NP, row l = output l, K =
@@ -255,39 +369,23 @@ k_coef_digits(const double* __restrict__ coef, long bstride, int ld, BlockIdx bi
 // spinors, 90 for 80).  A CTA per tile went through the same steps one after the
 // other: 1628 us for the 300 spwfs of 36^3 (blocks of 75), now 573; 110 for the 160
 // of 24^3 (40), now 82.
-constexpr int kRoleWarps = 8;                       // epilogue: warps 0-7, slicers: 8-15
-constexpr int kApplyThreads = 2 * kRoleWarps * 32 + 32;   // and the MMA warp
-constexpr int kSmemCap = 225 * 1024;
-
-__host__ __device__ constexpr int apply_accs(int nd) { return nd == oz::kDigits64 ? oz::kAccs64 : (int)oz::kAccs; }
 __host__ __device__ constexpr int apply_plane(int np) { return kRows * np * 2; }
 __host__ __device__ constexpr int apply_coef(int nd, int np) { return nd * np * np * 2; }
 // operand and accumulator buffers that fit
 __host__ __device__ constexpr int apply_bufs(int nd, int np) {
     return 2 * nd * apply_plane(np) + apply_coef(nd, np) + 128 <= kSmemCap ? 2 : 1;
 }
-__host__ __device__ constexpr int apply_tbufs(int nd, int np) {
-    return 2 * apply_accs(nd) * np <= 512 ? 2 : 1;
-}
 __host__ __device__ constexpr size_t apply_smem(int nd, int np) {
     return (size_t)apply_bufs(nd, np) * nd * apply_plane(np) + apply_coef(nd, np) + 128;
 }
 
-__device__ __forceinline__ bool wait_warp(uint64_t* mbar, uint32_t parity) {
-    return __all_sync(0xffffffffu, tc::mbar_wait(mbar, parity, kWaitCycles)) != 0;
-}
-__device__ __forceinline__ void arrive_warp(uint64_t* mbar, int lane) {
-    __syncwarp();
-    if (lane == 0) tc::mbar_arrive(mbar);
-}
-
 template <int ND, int NP>
-__global__ void __launch_bounds__(kApplyThreads, 1)
+__global__ void __launch_bounds__(kRoleThreads, 1)
 k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
            const int* __restrict__ in_list, const int* __restrict__ out_list,
            const int* __restrict__ out_base, const uint16_t* __restrict__ xd,
            const int* __restrict__ xe, long V4, int tpb, int ntiles, int* __restrict__ status) {
-    constexpr int NACC = apply_accs(ND), NBUF = apply_bufs(ND, NP), NTB = apply_tbufs(ND, NP);
+    constexpr int NACC = accs_for(ND), NBUF = apply_bufs(ND, NP), NTB = tbufs_for(ND, NP);
     constexpr int kg = NP / 8, kPlane = apply_plane(NP);
     extern __shared__ uint8_t smraw[];
     __shared__ __align__(8) uint64_t fullA[2], emptyA[2], fullT[2], emptyT[2], emaxReady[4];
@@ -324,10 +422,10 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
         {
             const uint4* src = reinterpret_cast<const uint4*>(xd + (long)b * ND * kXdStride);
             uint4* dst = reinterpret_cast<uint4*>(sB);
-            for (int t = tid; t < apply_coef(ND, NP) / 16; t += kApplyThreads) dst[t] = src[t];
+            for (int t = tid; t < apply_coef(ND, NP) / 16; t += kRoleThreads) dst[t] = src[t];
             // K groups past the block's spinors stay zero
             uint4* a = reinterpret_cast<uint4*>(sA);
-            for (int t = tid; t < NBUF * ND * kPlane / 16; t += kApplyThreads)
+            for (int t = tid; t < NBUF * ND * kPlane / 16; t += kRoleThreads)
                 a[t] = make_uint4(0u, 0u, 0u, 0u);
             if (tid < NP) {
                 sXe[tid] = xe[b * kMeshTcMax + tid];
@@ -357,14 +455,30 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                 }
 #pragma unroll
                 for (int u = 0; u < 8 * own; ++u) emax = max(emax, oz::bexp(v[u]));
-                sEx[k & 1][st] = emax;
+                int bad = kNone;   // FP64 form: the first spinor with an infinity or a NaN
+                if (ND == oz::kDigits64 && emax == 2047) {
+                    emax = 0;
+#pragma unroll
+                    for (int u = 0; u < 8 * own; ++u) {
+                        if (oz::bexp(v[u]) == 2047) {
+                            bad = min(bad, 8 * (half + 2 * (u >> 3)) + (u & 7));
+                            v[u] = 0.0;
+                        }
+                        emax = max(emax, oz::bexp(v[u]));
+                    }
+                }
+                sEx[k & 1][st] = emax * 256 + bad;
                 asm volatile("bar.sync 1, %0;" ::"n"(32 * kRoleWarps) : "memory");
-                emax = max(sEx[k & 1][row], sEx[k & 1][row + kRows]);
+                {
+                    const int e0 = sEx[k & 1][row], e1 = sEx[k & 1][row + kRows];
+                    emax = max(e0 >> 8, e1 >> 8);
+                    bad = min(e0 & 255, e1 & 255);
+                }
                 if (k >= NBUF) {
                     ok = wait_warp(&emptyA[buf], ((k - NBUF) / NBUF) & 1);
                     if (!ok) break;
                 }
-                if (half == 0) sEmax[k & 3][row] = emax;
+                if (half == 0) sEmax[k & 3][row] = emax * 256 + bad;
                 arrive_warp(&emaxReady[k & 3], lane);
                 const oz::FixedRow<ND> fixed(emax);
                 uint8_t* planes = sA + buf * ND * kPlane;
@@ -419,7 +533,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                 if (ok) ok = wait_warp(&fullT[tb], (k / NTB) & 1);
                 if (!ok) break;
                 tc::fence_after();
-                const int emax = sEmax[k & 3][erow];
+                const int emax = sEmax[k & 3][erow] >> 8, bad = sEmax[k & 3][erow] & 255;
                 const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) +
                                       (uint32_t)(tb * NACC * NP + 8 * colh);
                 const int nch = max(0, (nb - 8 * colh + 15) / 16);   // chunks of 8 columns
@@ -452,7 +566,19 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                         if (l0 + u >= nb) break;
                         const int ex = sXe[l0 + u];
                         double x = 0.0;
-                        if (emax > 0) {
+                        if constexpr (ND == oz::kDigits64) {
+                            uint32_t acc[NACC];
+#pragma unroll
+                            for (int g = 0; g < NACC; ++g) acc[g] = r[g][u];
+                            const int e = emax - 1023 + ex - 1023 - oz::kUnit64;
+                            // 6 pairs x 42 x 2^14 < 2^22: the magic numbers' range
+                            if (nb <= 42 && e >= -900 && e <= 900)
+                                x = oz::combine64(acc, e);
+                            else
+                                x = oz::combine64_any(acc, e);
+                            if (emax == 0 || ex == 0) x = 0.0;
+                            if (l0 + u >= bad || ex == 2047) x = __longlong_as_double(0x7FF8000000000000ll);
+                        } else if (emax > 0) {
                             dfl o = oz::combine4(__uint_as_float(r[0][u]), __uint_as_float(r[1][u]),
                                                  __uint_as_float(r[2][u]), __uint_as_float(r[3][u]));
                             const float sc = oz::pow2f(emax - 1023 + ex - 1023 - 12);
@@ -714,36 +840,63 @@ k_field_contract(const double* __restrict__ Y, const double* __restrict__ psi,
 
 }  // namespace
 
-// Buffers and attributes of the tensor-core Gram-Schmidt (blocks of at most
-// kMeshTcMax spinors).  Returns false when the blocks are larger.
-bool gs_tc_prepare(mg_ctx* c) {
-    if (!c->tc_mesh_ok || c->gs_nbmax > kMeshTcMax) return false;
+// Largest and smallest blocks of the FP64 form.  Above 64 its seven accumulators do
+// not fit the 512 TMEM columns.  Below 24 the FP64 kernels of gs.cu are as fast or
+// faster; the whole Gram-Schmidt of four blocks at 10^3 / 16^3 / 24^3 in us, there and
+// here: blocks of 16: 54 / 83 / 167 and 64 / 89 / 166, of 24: 83 / 149 / 336 and
+// 83 / 119 / 216, of 40: 155 / 318 / 785 and 130 / 193 / 360, of 64: 317 / 709 / 1851
+// and 217 / 301 / 546.
+constexpr int kMeshTcMax64 = 64, kMeshTcMin64 = 24;
+
+// Buffers of the tensor-core Gram-Schmidt.  Returns false where the FP64 kernels of
+// gs.cu are the ones to run.
+bool gs_tc_prepare(mg_ctx* c, bool f64) {
+    if (!c->tc_mesh_ok || c->gs_nbmax > (f64 ? kMeshTcMax64 : kMeshTcMax)) return false;
+    if (f64 && c->gs_nbmax < kMeshTcMin64) return false;
     if (c->gs_xd == nullptr) {
         const int nblk = c->gs_nblk;
-        c->gs_nchunk_tc = div_up(4 * c->V, kChunk);
-        if (cudaMalloc(&c->gs_Stc, (size_t)nblk * c->gs_nchunk_tc * c->gs_nbmax * c->gs_nbmax *
+        const bool both = c->gs_nbmax <= kMeshTcMax64;   // the FP64 form's chunks are smaller
+        const long chunks = div_up(4 * c->V, chunk_for(both ? oz::kDigits64 : kDigits));
+        if (cudaMalloc(&c->gs_Stc, (size_t)nblk * chunks * c->gs_nbmax * c->gs_nbmax *
                                        sizeof(double)) != cudaSuccess ||
-            cudaMalloc(&c->gs_xd, (size_t)nblk * kDigits * kXdStride * sizeof(uint16_t)) !=
+            cudaMalloc(&c->gs_xd, (size_t)nblk * oz::kDigits64 * kXdStride * sizeof(uint16_t)) !=
                 cudaSuccess ||
-            cudaMalloc(&c->gs_xe, (size_t)nblk * kMeshTcMax * sizeof(int)) != cudaSuccess ||
-            cudaMemset(c->gs_xd, 0, (size_t)nblk * kDigits * kXdStride * sizeof(uint16_t)) !=
-                cudaSuccess)
+            cudaMalloc(&c->gs_xe, (size_t)nblk * kMeshTcMax * sizeof(int)) != cudaSuccess)
             return false;
-        cudaFuncSetAttribute(k_gs_overlap_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024);
     }
     return true;
 }
 
-int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered) {
-    size_t sm = 128 + 2 * (size_t)kDigits * kStagePlane;
-    const int N = std::max(16, (c->gs_nbmax + 15) / 16 * 16);
-    if (tmem_cols(N) > 256) sm = std::max(sm, kOneCtaSmem);
-    k_gs_overlap_tc<<<dim3(c->gs_nchunk_tc, c->gs_nblk), 256, sm, c->stream>>>(
-        psi, d_lists, d_ordered, c->gs_nbmax, 4 * c->V, c->gs_nchunk_tc, c->gs_Stc,
-        c->tc_status);
+template <int ND, int NP>
+static int overlap_launch(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered,
+                          int nchunk) {
+    MG_CUDA(cudaFuncSetAttribute(k_gs_overlap_tc<ND, NP>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)overlap_smem(ND, NP)));
+    const int nunits = nchunk * c->gs_nblk;
+    k_gs_overlap_tc<ND, NP><<<std::min(c->num_sms, nunits), kRoleThreads, overlap_smem(ND, NP),
+                              c->stream>>>(psi, d_lists, d_ordered, c->gs_nbmax, 4 * c->V, nchunk,
+                                           nunits, c->gs_Stc, c->tc_status);
     MG_LAUNCHED(c);
     return MG_OK;
+}
+
+// Chunk partials of the blocks' overlaps in gs_Stc, *nchunk of them.
+int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered, bool f64,
+                  int* nchunk) {
+    *nchunk = div_up(4 * c->V, chunk_for(f64 ? oz::kDigits64 : kDigits));
+    const auto run = [&](auto launch) { return launch(c, psi, d_lists, d_ordered, *nchunk); };
+    const int steps = std::max(1, div_up(c->gs_nbmax, 16));
+    if (f64) return steps <= 2   ? run(overlap_launch<oz::kDigits64, 32>)
+                    : steps == 3 ? run(overlap_launch<oz::kDigits64, 48>)
+                                 : run(overlap_launch<oz::kDigits64, 64>);
+    switch (steps) {
+        case 1: return run(overlap_launch<kDigits, 16>);
+        case 2: return run(overlap_launch<kDigits, 32>);
+        case 3: return run(overlap_launch<kDigits, 48>);
+        case 4: return run(overlap_launch<kDigits, 64>);
+        default: return run(overlap_launch<kDigits, 80>);
+    }
 }
 
 template <int ND, int NP>
@@ -757,15 +910,19 @@ static int apply_launch(mg_ctx* c, int nblk, const double* coef, long bstride, i
     const long V4 = 4 * c->V;
     const int tpb = div_up(V4, kRows), ntiles = tpb * nblk;
     const int sms = c->tc_grid_cap > 0 ? std::min(c->tc_grid_cap, c->num_sms) : c->num_sms;
-    k_apply_tc<ND, NP><<<std::min(sms, ntiles), kApplyThreads, apply_smem(ND, NP), c->stream>>>(
+    k_apply_tc<ND, NP><<<std::min(sms, ntiles), kRoleThreads, apply_smem(ND, NP), c->stream>>>(
         in, out, upd, bi, in_list, out_list, out_base, xd, xe, V4, tpb, ntiles, c->tc_status);
     MG_LAUNCHED(c);
     return MG_OK;
 }
 
 template <class... A>
-static int apply_tc(mg_ctx* c, int nblk, int nbmax, A... args) {
-    switch (std::max(1, div_up(nbmax, 16))) {
+static int apply_tc(mg_ctx* c, int nblk, int nbmax, bool f64, A... args) {
+    const int steps = std::max(1, div_up(nbmax, 16));
+    if (f64) return steps <= 2   ? apply_launch<oz::kDigits64, 32>(c, nblk, args...)
+                    : steps == 3 ? apply_launch<oz::kDigits64, 48>(c, nblk, args...)
+                                 : apply_launch<oz::kDigits64, 64>(c, nblk, args...);
+    switch (steps) {
         case 1: return apply_launch<kDigits, 16>(c, nblk, args...);
         case 2: return apply_launch<kDigits, 32>(c, nblk, args...);
         case 3: return apply_launch<kDigits, 48>(c, nblk, args...);
@@ -774,9 +931,10 @@ static int apply_tc(mg_ctx* c, int nblk, int nbmax, A... args) {
     }
 }
 
-int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const int* d_ordered) {
+int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const int* d_ordered,
+                bool f64) {
     const BlockIdx bi{d_lists, nullptr, 0};
-    return apply_tc(c, c->gs_nblk, c->gs_nbmax, c->gs_R, (long)c->gs_nbmax * c->gs_nbmax,
+    return apply_tc(c, c->gs_nblk, c->gs_nbmax, f64, c->gs_R, (long)c->gs_nbmax * c->gs_nbmax,
                     c->gs_nbmax, bi, psi, psi, upd, d_ordered, d_ordered, nullptr, c->gs_xd,
                     c->gs_xe);
 }
@@ -792,7 +950,7 @@ int can_transform_tc(mg_ctx* c) {
         MG_CUDA(cudaMalloc(&c->can_xe, (size_t)4 * kMeshTcMax * sizeof(int)));
     }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
-    return apply_tc(c, 4, H.hmax, H.cantr, (long)H.hmax * H.hmax, 0, bi,
+    return apply_tc(c, 4, H.hmax, false, H.cantr, (long)H.hmax * H.hmax, 0, bi,
                     c->bas[MG_HF_BASIS].psi, c->bas[MG_CAN_BASIS].psi, nullptr, H.members,
                     nullptr, H.cstart, c->can_xd, c->can_xe);
 }
@@ -839,7 +997,7 @@ int pair_field_tc(mg_ctx* c) {
         MG_CUDA(cudaMemcpy(c->field_ybase, yb, sizeof(yb), cudaMemcpyHostToDevice));
     }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
-    MG_TRY(apply_tc(c, 4, H.hmax, H.ktil, (long)H.hmax * H.hmax, 0, bi,
+    MG_TRY(apply_tc(c, 4, H.hmax, false, H.ktil, (long)H.hmax * H.hmax, 0, bi,
                     c->bas[MG_HF_BASIS].psi, c->field_y, nullptr, H.members, nullptr,
                     c->field_ybase, c->field_xd, c->field_xe));
     k_field_contract<<<dim3(div_up(V, 64), 4), 256, 0, c->stream>>>(

@@ -275,7 +275,6 @@ struct mg_ctx {
     double* gs_Stc = nullptr;
     uint16_t* gs_xd = nullptr;
     int* gs_xe = nullptr;
-    int gs_nchunk_tc = 0;
     uint16_t* can_xd = nullptr;   // digit planes of CanTransfo (tensor-core canonical basis)
     int* can_xe = nullptr;
     double* gap_part = nullptr;   // tensor-core gaps: partials per 64-point chunk
@@ -409,9 +408,11 @@ int hpsi_single(mg_ctx* c, double* psi, const double* der, const double* lap, co
 int estimate_parameters(mg_ctx* c);
 int gram_schmidt(mg_ctx* c);
 int gram_schmidt_impl(mg_ctx* c, double* upd);
-bool gs_tc_prepare(mg_ctx* c);
-int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered);
-int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const int* d_ordered);
+bool gs_tc_prepare(mg_ctx* c, bool f64);
+int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered, bool f64,
+                  int* nchunk);
+int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const int* d_ordered,
+                bool f64);
 int can_transform_tc(mg_ctx* c);
 int gaps_tc(mg_ctx* c, double* gsum);
 int pair_field_tc(mg_ctx* c);

@@ -262,26 +262,10 @@ __device__ __forceinline__ uint32_t units(uint32_t bits) {
 }
 __host__ __device__ constexpr uint32_t magic_bits(int P) { return 0x4B400000u - ((uint32_t)P << 23); }
 
-// The seven accumulators' sum times 2^x as FP64: a 64-bit integer in units
-// of 2^-44 (top digits are at most 64, so 32 products stay below 2^18 and the
-// integer below 2^62), rounded once with integer instructions (an FP64
-// instruction holds a warp's slot of the FP64 pipe for 16 clocks).  The
-// accumulators' magic numbers are carried along and taken off once.  The
-// caller keeps x between -900 and 900.
-__device__ __forceinline__ double combine64(const uint32_t (&a)[kAccs64], int x) {
-    const uint32_t hi = units<0>(a[0]) * 256u + units<8>(a[1]);     // 2^-8
-    const uint32_t mid = units<16>(a[2]) * 256u + units<24>(a[3]);  // 2^-24, with its magic >= 0
-    const uint32_t low = units<32>(a[4]) * 256u + units<40>(a[5]);  // 2^-40, with its magic >= 0
-    const uint32_t tail = units<44>(a[6]);
-    constexpr uint32_t mhi = magic_bits(0) * 256u + magic_bits(8);
-    constexpr uint32_t mmid = magic_bits(16) * 256u + magic_bits(24);
-    constexpr uint32_t mlow = magic_bits(32) * 256u + magic_bits(40);
-    constexpr unsigned long long off = ((unsigned long long)mhi << 36) +
-                                       ((unsigned long long)mmid << 20) +
-                                       ((unsigned long long)mlow << 4) + magic_bits(44);
-    const unsigned long long I = (unsigned long long)mid * (1ull << 20) +
-                                 ((unsigned long long)low * 16u + tail) +
-                                 ((unsigned long long)(hi << 4) << 32) - off;
+// I 2^(x - 44) as FP64, rounded once with integer instructions (an FP64
+// instruction holds a warp's slot of the FP64 pipe for 16 clocks).  The caller keeps
+// x between -900 and 900.
+__device__ __forceinline__ double round64(unsigned long long I, int x) {
     const uint32_t sgn = (uint32_t)((int)(uint32_t)(I >> 32) >> 31);
     const unsigned long long s64 = ((unsigned long long)sgn << 32) | sgn;
     const unsigned long long u = (I ^ s64) - s64;
@@ -300,6 +284,47 @@ __device__ __forceinline__ double combine64(const uint32_t (&a)[kAccs64], int x)
     const unsigned long long r = ((((unsigned long long)h << 32) | l) >> 11) + ((l >> 10) & 1u);
     const uint32_t rh = (uint32_t)(r >> 32) + ((uint32_t)(e - lz - 1) << 20);
     return __hiloint2double((int)(rh | (sgn & 0x80000000u)), (int)(uint32_t)r);
+}
+
+// The seven accumulators' sum times 2^x as FP64: a 64-bit integer in units
+// of 2^-44 (top digits are at most 64, so 32 products stay below 2^18 and the
+// integer below 2^62), rounded once.  The accumulators' magic numbers are carried
+// along and taken off once.
+__device__ __forceinline__ double combine64(const uint32_t (&a)[kAccs64], int x) {
+    const uint32_t hi = units<0>(a[0]) * 256u + units<8>(a[1]);     // 2^-8
+    const uint32_t mid = units<16>(a[2]) * 256u + units<24>(a[3]);  // 2^-24, with its magic >= 0
+    const uint32_t low = units<32>(a[4]) * 256u + units<40>(a[5]);  // 2^-40, with its magic >= 0
+    const uint32_t tail = units<44>(a[6]);
+    constexpr uint32_t mhi = magic_bits(0) * 256u + magic_bits(8);
+    constexpr uint32_t mmid = magic_bits(16) * 256u + magic_bits(24);
+    constexpr uint32_t mlow = magic_bits(32) * 256u + magic_bits(40);
+    constexpr unsigned long long off = ((unsigned long long)mhi << 36) +
+                                       ((unsigned long long)mmid << 20) +
+                                       ((unsigned long long)mlow << 4) + magic_bits(44);
+    const unsigned long long I = (unsigned long long)mid * (1ull << 20) +
+                                 ((unsigned long long)low * 16u + tail) +
+                                 ((unsigned long long)(hi << 4) << 32) - off;
+    return round64(I, x);
+}
+
+// The same for sums of up to 128 products (6 pairs x 128 x 2^14 < 2^24 are exact in
+// FP32 but past the magic numbers' range; the whole sum is below 2^63 units), and for
+// any x.
+__device__ __forceinline__ double combine64_any(const uint32_t (&a)[kAccs64], int x) {
+    const auto part = [&a](int g, int up, int shift) {
+        // a multiple of 2^-up below 2^(31 - up) as an integer, shifted
+        const float f = __uint_as_float(a[g]) * __int_as_float((up + 127) << 23);
+        return (unsigned long long)(long long)__float2int_rn(f) << shift;
+    };
+    const unsigned long long I = part(0, 0, 44) + part(1, 8, 36) + part(2, 16, 28) +
+                                 part(3, 24, 20) + part(4, 32, 12) + part(5, 40, 4) +
+                                 part(6, 44, 0);
+    if (x >= -900 && x <= 900) return round64(I, x);
+    // past the exponent range of one step: two exact ones and a rounding
+    const int first = x < 0 ? max(x, -1960) / 2 : min(x, 1960) / 2;
+    const int rest = (x < 0 ? max(x, -1960) : min(x, 1960)) - first;
+    return round64(I, 0) * __longlong_as_double((long long)(first + 1023) << 52) *
+           __longlong_as_double((long long)(rest + 1023) << 52);
 }
 
 // a0 + a1 + a2 + a3 as a normalised double-float.  a0 is an integer below
@@ -360,7 +385,8 @@ __device__ __forceinline__ void issue_pairs(uint32_t tmem, int N, uint32_t idesc
 // the issue of 84 to 144 MMAs per tile bound the derivative kernel.)
 template <int ND, int NACC, int COLS, int KSTEPS>
 __device__ __forceinline__ void issue_stacked(uint32_t tmem, uint32_t aBase, uint32_t aPlane,
-                                              uint32_t bBase, uint32_t sbo) {
+                                              uint32_t bBase, uint32_t sbo,
+                                              bool accumulate = false) {
     constexpr uint32_t bPlane = COLS * KSTEPS * 32;
     constexpr int most = 256 / COLS;   // stacked planes of one MMA
     // accumulators filled by stacked planes; the FP64 form's last one takes its
@@ -381,7 +407,7 @@ __device__ __forceinline__ void issue_stacked(uint32_t tmem, uint32_t aBase, uin
             for (int b = 0; b < own - a; b += most) {
                 const int left = own - a - b;
                 // digit 0 is the first to reach each of these accumulators
-                mma(a, b, ks, a + b, left < most ? left : most, ks == 0 && a == 0 ? 0u : 1u);
+                mma(a, b, ks, a + b, left < most ? left : most, ks == 0 && a == 0 && !accumulate ? 0u : 1u);
             }
             // the pairs past the last weight, between MMAs that do not wait for them
             if (own == NACC)
@@ -395,7 +421,7 @@ __device__ __forceinline__ void issue_stacked(uint32_t tmem, uint32_t aBase, uin
             for (int a = 0; a <= c; ++a)
 #pragma unroll
                 for (int ks = 0; ks < KSTEPS; ++ks)
-                    mma(a, c - a, ks, NACC - 1, 1, c == own && a == 0 && ks == 0 ? 0u : 1u);
+                    mma(a, c - a, ks, NACC - 1, 1, c == own && a == 0 && ks == 0 && !accumulate ? 0u : 1u);
     }
 }
 
