@@ -117,15 +117,21 @@ __global__ void k_gs_sum(double* __restrict__ part, int nbmax, int nchunk) {
 }
 
 // Cholesky S = R^T R (R upper), X = R^{-1}; X to xout[b].
-__global__ void __launch_bounds__(kThreads)
+//
+// S = L D L^T by symmetric elimination (L unit lower, D the pivots), so that
+// R = D^(1/2) L^T; the same row operations applied to the identity leave
+// W = L^(-1), and X = R^(-1) = W^T D^(-1/2) needs no back substitution.  Step j
+// takes u_k = S_jk / S_jj times row j from every row k below: S from column k on, W up
+// to column j.  GB300 issues a warp's FP64 instruction over ~16 clocks and a divide is
+// a chain of ~550, so the entries of a step are dealt out to 15 warps without gaps, one
+// thread of the first makes the next pivot and its reciprocal meanwhile, and the
+// square roots wait until the end.  Blocks of 40: 82 us with a warp per row and the square root in
+// the chain, now 36; of 75: 196 and 96.
+constexpr int kFactorThreads = 512;
+
+__global__ void __launch_bounds__(kFactorThreads)
 k_gs_factor(const double* __restrict__ part, const int* __restrict__ starts, int nbmax,
             int nchunk, double dv, double* __restrict__ xout, int* __restrict__ flag) {
-    // S = L D L^T by symmetric elimination (L unit lower, D the pivots), so
-    // that R = D^(1/2) L^T; the same row operations applied to the identity
-    // leave W = L^(-1), and X = R^(-1) = W^T D^(-1/2) needs no back
-    // substitution.  GB300 issues a warp's FP64 instruction over ~16 clocks
-    // and a divide or square root is a sequence of them, so each pivot's
-    // reciprocal and reciprocal square root are taken once, by one thread.
     extern __shared__ double sm[];
     const int b = blockIdx.x;
     const int nb = starts[b + 1] - starts[b];
@@ -135,38 +141,59 @@ k_gs_factor(const double* __restrict__ part, const int* __restrict__ starts, int
     __shared__ double rsq[256];  // D^(-1/2)
     __shared__ double u[256];
     __shared__ double inv_d;
-    const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    constexpr int kWarps = kThreads / 32;
-    for (int t = threadIdx.x; t < nb * nb; t += kThreads) {
+    const int tid = threadIdx.x;
+    for (int t = tid; t < nb * nb; t += kFactorThreads) {
         const int k = t / nb, l = t % nb;
         S[t] = k <= l ? part[(long)b * nchunk * nbmax * nbmax + k * nbmax + l] * dv : 0.0;
         W[t] = k == l ? 1.0 : 0.0;
     }
     __syncthreads();
-    for (int j = 0; j < nb; ++j) {
-        if (threadIdx.x == 0) {
-            const double d = S[j * nb + j];
-            if (!(d > 0.0)) atomicExch(flag, 1);
-            const double dd = fmax(d, 1e-300);
-            inv_d = 1.0 / dd;
-            rsq[j] = 1.0 / sqrt(dd);
-        }
+    const auto pivot = [&](double d) {
+        if (!(d > 0.0)) atomicExch(flag, 1);
+        inv_d = 1.0 / fmax(d, 1e-300);
+    };
+    if (tid == 0) pivot(S[0]);
+    __syncthreads();
+    for (int j = 0; j + 1 < nb; ++j) {
+        const double* Sj = S + j * nb;
+        const double* Wj = W + j * nb;
+        const int R = nb - 1 - j;
+        for (int m = 1 + tid; m <= R; m += kFactorThreads) u[m] = Sj[j + m] * inv_d;
         __syncthreads();
-        // pivot row scaled once (u_k = S_jk / S_jj), then one FMA per entry
-        // of the trailing upper triangle and of W's rows below j, a warp per row
-        const double id = inv_d;
-        for (int k = j + 1 + threadIdx.x; k < nb; k += kThreads) u[k] = S[j * nb + k] * id;
-        __syncthreads();
-        for (int k = j + 1 + warp; k < nb; k += kWarps) {
-            const double uk = u[k];
-            for (int l = k + lane; l < nb; l += 32) S[k * nb + l] = fma(-uk, S[j * nb + l], S[k * nb + l]);
-            for (int l = lane; l <= j; l += 32) W[k * nb + l] = fma(-uk, W[j * nb + l], W[k * nb + l]);
+        if (tid < 32) {
+            if (tid == 0) {
+                double* d = S + (j + 1) * nb + j + 1;
+                const double v = fma(-u[1], Sj[j + 1], *d);
+                *d = v;
+                pivot(v);
+            }
+        } else {
+            // row j + m (m = 1 .. R) has nb + 1 - m entries: rows m and R + 1 - m
+            // together `width`, whatever m
+            const int width = 2 * nb + 1 - R, pairs = (R + 1) / 2;
+            const float inv = 1.0f / (float)width;
+            for (int e = tid - 32; e < pairs * width; e += kFactorThreads - 32) {
+                const int q = (int)(((float)e + 0.5f) * inv);
+                int m = q + 1, x = e - q * width;
+                if (x >= nb + 1 - m) {
+                    x -= nb + 1 - m;
+                    if (R - q == m) continue;   // the middle row has no partner
+                    m = R - q;
+                }
+                const int k = j + m, l = x <= j ? x : k + x - (j + 1);
+                if (m == 1 && l == k) continue;   // the next pivot
+                const double* src = x <= j ? Wj : Sj;
+                double* dst = (x <= j ? W : S) + k * nb + l;
+                *dst = fma(-u[m], src[l], *dst);
+            }
         }
         __syncthreads();
     }
+    for (int j = tid; j < nb; j += kFactorThreads) rsq[j] = 1.0 / sqrt(fmax(S[j * nb + j], 1e-300));
+    __syncthreads();
     // X[i][j] = W[j][i] d_j^(-1/2) (i <= j), zero below the diagonal
     double* xo = xout + (long)b * nbmax * nbmax;
-    for (int t = threadIdx.x; t < nb * nb; t += kThreads) {
+    for (int t = tid; t < nb * nb; t += kFactorThreads) {
         const int i = t / nb, j = t % nb;
         xo[i * nbmax + j] = i <= j ? W[j * nb + i] * rsq[j] : 0.0;
     }
@@ -269,7 +296,7 @@ int gram_schmidt_impl(mg_ctx* c, double* upd) {
         k_gs_sum<<<dim3(div_up((long)nbmax * nbmax, kThreads / 32), nblk), kThreads, 0,
                    c->stream>>>(c->gs_Stc, nbmax, nct);
         MG_LAUNCHED(c);
-        k_gs_factor<<<nblk, kThreads, sm_f, c->stream>>>(c->gs_Stc, d_lists, nbmax, nct, c->dv,
+        k_gs_factor<<<nblk, kFactorThreads, sm_f, c->stream>>>(c->gs_Stc, d_lists, nbmax, nct, c->dv,
                                                          c->gs_R, c->flags);
         MG_LAUNCHED(c);
         return gs_apply_tc(c, B.psi, upd, d_lists, d_ordered, f64);
@@ -283,7 +310,7 @@ int gram_schmidt_impl(mg_ctx* c, double* upd) {
     k_gs_sum<<<dim3(div_up((long)nbmax * nbmax, kThreads / 32), nblk), kThreads, 0,
                c->stream>>>(c->gs_S, nbmax, nchunk);
     MG_LAUNCHED(c);
-    k_gs_factor<<<nblk, kThreads, sm_f, c->stream>>>(c->gs_S, d_lists, nbmax, nchunk, c->dv,
+    k_gs_factor<<<nblk, kFactorThreads, sm_f, c->stream>>>(c->gs_S, d_lists, nbmax, nchunk, c->dv,
                                                      c->gs_R, c->flags);
     MG_LAUNCHED(c);
     k_gs_apply<<<dim3(div_up(V4, kPts), nblk), kThreads, sm_ap, c->stream>>>(
