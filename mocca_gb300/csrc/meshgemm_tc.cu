@@ -1,7 +1,7 @@
 // meshgemm_tc.cu -- the mesh-sized contractions on the tcgen05 tensor cores
 // (exact BF16 digit products, ozaki.cuh): the Gram-Schmidt overlap and apply,
-// in the mixed form with six digits and in the FP64 form with eight, and the
-// mixed form's canonical-basis transform and pairing contractions.
+// and the canonical-basis transform, in the mixed form with six digits and in the
+// FP64 form with eight, and the mixed form's pairing contractions.
 //
 // Blocks of up to kMeshTcMax (80) spinors in the mixed form, kMeshTcMin64 to
 // kMeshTcMax64 (24 to 64) in the FP64 form, whose results are rounded once to FP64
@@ -379,12 +379,13 @@ __host__ __device__ constexpr size_t apply_smem(int nd, int np) {
     return (size_t)apply_bufs(nd, np) * nd * apply_plane(np) + apply_coef(nd, np) + 128;
 }
 
-template <int ND, int NP>
+template <int ND, int NP, bool kInPlace>
 __global__ void __launch_bounds__(kRoleThreads, 1)
 k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
            const int* __restrict__ in_list, const int* __restrict__ out_list,
            const int* __restrict__ out_base, const uint16_t* __restrict__ xd,
-           const int* __restrict__ xe, long V4, int tpb, int ntiles, int* __restrict__ status) {
+           const int* __restrict__ xe, const double* __restrict__ coef, long bstride, int ld,
+           long V4, int tpb, int ntiles, int* __restrict__ status) {
     constexpr int NACC = accs_for(ND), NBUF = apply_bufs(ND, NP), NTB = tbufs_for(ND, NP);
     constexpr int kg = NP / 8, kPlane = apply_plane(NP);
     extern __shared__ uint8_t smraw[];
@@ -435,7 +436,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
         }
         tc::fence_proxy_async();
         tc::fence_before();
-        __syncthreads();
+        const bool xbad = __syncthreads_or(tid < NP && xe[b * kMeshTcMax + tid] == 2047) != 0;
         tc::fence_after();
         tmem = tmem_slot;
         if (warp >= kRoleWarps && warp < 2 * kRoleWarps) {
@@ -577,6 +578,8 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                             else
                                 x = oz::combine64_any(acc, e);
                             if (emax == 0 || ex == 0) x = 0.0;
+                            // in place C is triangular, and NaN from a spinor with an
+                            // infinity or a NaN on (else: below)
                             if (l0 + u >= bad || ex == 2047) x = __longlong_as_double(0x7FF8000000000000ll);
                         } else if (emax > 0) {
                             dfl o = oz::combine4(__uint_as_float(r[0][u]), __uint_as_float(r[1][u]),
@@ -591,6 +594,16 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                         if (upd) upd[o] = x - was[u];
                     }
                 }
+                if (ND == oz::kDigits64 && !kInPlace && pe < V4 && (bad != kNone || xbad))
+                    // an infinity or a NaN at this point or in C: the plain sums
+                    for (int l = 8 * colh; l < nb; l += (l & 7) == 7 ? 9 : 1) {
+                        const double* C = coef + (long)b * bstride + l;
+                        double x = 0.0;
+#pragma unroll 1
+                        for (int q2 = 0; q2 < nb; ++q2)
+                            x = fma(C[q2 * (ld > 0 ? ld : nb)], in[(long)sIdx[q2] * V4 + pe], x);
+                        out[(long)sOut[l] * V4 + pe] = x;
+                    }
             }
         }
         k0 += count;
@@ -848,11 +861,16 @@ k_field_contract(const double* __restrict__ Y, const double* __restrict__ psi,
 // and 217 / 301 / 546.
 constexpr int kMeshTcMax64 = 64, kMeshTcMin64 = 24;
 
+// Whether blocks of up to nbmax spinors go to the kernels of this file.
+bool mesh_tc_serves(const mg_ctx* c, int nbmax, bool f64) {
+    return c->tc_mesh_ok &&
+           (f64 ? nbmax >= kMeshTcMin64 && nbmax <= kMeshTcMax64 : nbmax <= kMeshTcMax);
+}
+
 // Buffers of the tensor-core Gram-Schmidt.  Returns false where the FP64 kernels of
 // gs.cu are the ones to run.
 bool gs_tc_prepare(mg_ctx* c, bool f64) {
-    if (!c->tc_mesh_ok || c->gs_nbmax > (f64 ? kMeshTcMax64 : kMeshTcMax)) return false;
-    if (f64 && c->gs_nbmax < kMeshTcMin64) return false;
+    if (!mesh_tc_serves(c, c->gs_nbmax, f64)) return false;
     if (c->gs_xd == nullptr) {
         const int nblk = c->gs_nblk;
         const bool both = c->gs_nbmax <= kMeshTcMax64;   // the FP64 form's chunks are smaller
@@ -905,13 +923,18 @@ static int apply_launch(mg_ctx* c, int nblk, const double* coef, long bstride, i
                         const int* out_list, const int* out_base, uint16_t* xd, int* xe) {
     k_coef_digits<ND, NP><<<nblk, dim3(NP, kCoefRows), 0, c->stream>>>(coef, bstride, ld, bi, xd, xe);
     MG_LAUNCHED(c);
-    MG_CUDA(cudaFuncSetAttribute(k_apply_tc<ND, NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    // (in place matters to the FP64 form's treatment of infinities alone)
+    auto kernel = k_apply_tc<ND, NP, true>;
+    if constexpr (ND == oz::kDigits64)
+        if (in != out) kernel = k_apply_tc<ND, NP, false>;
+    MG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)apply_smem(ND, NP)));
     const long V4 = 4 * c->V;
     const int tpb = div_up(V4, kRows), ntiles = tpb * nblk;
     const int sms = c->tc_grid_cap > 0 ? std::min(c->tc_grid_cap, c->num_sms) : c->num_sms;
-    k_apply_tc<ND, NP><<<std::min(sms, ntiles), kRoleThreads, apply_smem(ND, NP), c->stream>>>(
-        in, out, upd, bi, in_list, out_list, out_base, xd, xe, V4, tpb, ntiles, c->tc_status);
+    kernel<<<std::min(sms, ntiles), kRoleThreads, apply_smem(ND, NP), c->stream>>>(
+        in, out, upd, bi, in_list, out_list, out_base, xd, xe, coef, bstride, ld, V4, tpb, ntiles,
+        c->tc_status);
     MG_LAUNCHED(c);
     return MG_OK;
 }
@@ -941,16 +964,15 @@ int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const i
 
 // Canonical basis of the four pairing blocks (hsz[b] <= kMeshTcMax):
 // CanTransfo is stored densely per block (ld = h) at b * hmax^2.
-int can_transform_tc(mg_ctx* c) {
+int can_transform_tc(mg_ctx* c, bool f64) {
     Hfb& H = c->hfb;
-    if (!c->tc_mesh_ok || H.hmax > kMeshTcMax) return MG_ERR_STATE;
+    if (!mesh_tc_serves(c, H.hmax, f64)) return MG_ERR_STATE;
     if (c->can_xd == nullptr) {
-        MG_CUDA(cudaMalloc(&c->can_xd, (size_t)4 * kDigits * kXdStride * sizeof(uint16_t)));
-        MG_CUDA(cudaMemset(c->can_xd, 0, (size_t)4 * kDigits * kXdStride * sizeof(uint16_t)));
+        MG_CUDA(cudaMalloc(&c->can_xd, (size_t)4 * oz::kDigits64 * kXdStride * sizeof(uint16_t)));
         MG_CUDA(cudaMalloc(&c->can_xe, (size_t)4 * kMeshTcMax * sizeof(int)));
     }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
-    return apply_tc(c, 4, H.hmax, false, H.cantr, (long)H.hmax * H.hmax, 0, bi,
+    return apply_tc(c, 4, H.hmax, f64, H.cantr, (long)H.hmax * H.hmax, 0, bi,
                     c->bas[MG_HF_BASIS].psi, c->bas[MG_CAN_BASIS].psi, nullptr, H.members,
                     nullptr, H.cstart, c->can_xd, c->can_xe);
 }

@@ -408,12 +408,13 @@ int hpsi_single(mg_ctx* c, double* psi, const double* der, const double* lap, co
 int estimate_parameters(mg_ctx* c);
 int gram_schmidt(mg_ctx* c);
 int gram_schmidt_impl(mg_ctx* c, double* upd);
+bool mesh_tc_serves(const mg_ctx* c, int nbmax, bool f64);
 bool gs_tc_prepare(mg_ctx* c, bool f64);
 int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered, bool f64,
                   int* nchunk);
 int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const int* d_ordered,
                 bool f64);
-int can_transform_tc(mg_ctx* c);
+int can_transform_tc(mg_ctx* c, bool f64);
 int gaps_tc(mg_ctx* c, double* gsum);
 int pair_field_tc(mg_ctx* c);
 int densities(mg_ctx* c);

@@ -52,3 +52,31 @@ def test_blocks(built, precision, bar, n, sizes):
         want = np.linalg.solve(np.linalg.cholesky(s), psi[rows])
         err = np.linalg.norm(got[rows] - want, axis=1) / np.linalg.norm(want, axis=1)
         assert err.max() <= bar, (b, len(rows), err.max())
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("nb", [20, 30, 50])
+def test_not_a_number_stays_behind(built, nb, value):
+    """A NaN or an infinity in one spinor of an FP64 block: the spinors before it
+    in energy are what they are without it, those from it on are not finite there
+    (blocks of 20 go to the FP64 kernels, the others to the tensor cores)."""
+    p = RunParams(nx=6, ny=7, nz=5, dx=0.8, nwt=nb, neutrons=2, protons=2, precision=MG_FP64)
+    rng = np.random.default_rng(nb)
+    npts = 4 * 6 * 7 * 5
+    q, _ = np.linalg.qr(rng.normal(size=(npts, nb)))
+    psi = q.T / np.sqrt(p.dv)
+    qn = np.ones((nb, 4), dtype=np.int32)
+    out = []
+    for bad in (False, True):
+        x = psi.copy()
+        if bad:
+            x[12, 17] = value
+        g = MeshState(p, SLY4)
+        g.set_spinors(x, qn)
+        g.set_energies(np.arange(nb, dtype=float))
+        g.GramSchmidt()
+        out.append(g.get_spinors().reshape(nb, npts))
+        g.close()
+    clean, got = out
+    assert np.array_equal(got[:12], clean[:12])
+    assert not np.isfinite(got[12:, 17]).any()
