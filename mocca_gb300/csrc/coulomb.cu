@@ -404,6 +404,9 @@ static dim3 bound_blocks(const mg_ctx* c) {
     return dim3(div_up(c->M - c->V, kBoundPoints) + div_up(c->V, kBoundThreads));
 }
 
+// (blocks of two warps: the power is FP64 work, spread over all SMs)
+constexpr int kOutThreads = 64;
+
 __global__ void k_coulomb_out(const double* __restrict__ sol, const double* __restrict__ rho_p,
                               int nx, int ny, int nz, int mx, int my, double fac,
                               double* __restrict__ coul, double* __restrict__ coulex) {
@@ -811,7 +814,7 @@ int coulomb_solve(mg_ctx* c, int* iters) {
         const int st = coulomb_multigrid(c, c->p.coulomb_prec > 0 ? c->p.coulomb_prec : 1e-10,
                                          maxit, iters);
         if (st < 0) return st;
-        k_coulomb_out<<<div_up(c->V, kThreads), kThreads, 0, c->stream>>>(
+        k_coulomb_out<<<div_up(c->V, kOutThreads), kOutThreads, 0, c->stream>>>(
             c->cpot, c->rho + c->V, c->nx, c->ny, c->nz, c->mx, c->my,
             -std::pow(3 / pi_, 1 / 3.0) * c->f.e2, c->coulomb, c->coulex);
         MG_LAUNCHED(c);
@@ -821,7 +824,7 @@ int coulomb_solve(mg_ctx* c, int* iters) {
         MG_TRY(coulomb_direct(c));
         const double pi = 4.0 * std::atan2(1.0, 1.0);
         const double fac = -std::pow(3 / pi, 1 / 3.0) * c->f.e2;
-        k_coulomb_out<<<div_up(c->V, kThreads), kThreads, 0, c->stream>>>(
+        k_coulomb_out<<<div_up(c->V, kOutThreads), kOutThreads, 0, c->stream>>>(
             c->cpot, c->rho + c->V, c->nx, c->ny, c->nz, c->mx, c->my, fac, c->coulomb,
             c->coulex);
         MG_LAUNCHED(c);
@@ -856,7 +859,7 @@ int coulomb_solve(mg_ctx* c, int* iters) {
     ++c->launches;
     const double pi = 4.0 * std::atan2(1.0, 1.0);
     const double fac = -std::pow(3 / pi, 1 / 3.0) * c->f.e2;
-    k_coulomb_out<<<div_up(c->V, kThreads), kThreads, 0, c->stream>>>(
+    k_coulomb_out<<<div_up(c->V, kOutThreads), kOutThreads, 0, c->stream>>>(
         c->cpot, c->rho + c->V, c->nx, c->ny, c->nz, c->mx, c->my, fac, c->coulomb, c->coulex);
     MG_LAUNCHED(c);
     MG_CUDA(cudaMemcpyAsync(c->h_cg_status, c->cg_status, 4 * sizeof(int), cudaMemcpyDeviceToHost,

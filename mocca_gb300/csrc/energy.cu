@@ -55,7 +55,13 @@ struct ECoef {
     double B4, B6, B8a, B8b, B9q, byt3a, byt3b, B7b;
 };
 
-__global__ void __launch_bounds__(kThreads)
+// A row of partials is the sum over kThreads threads' points, by eight blocks of one
+// warp in a cluster: the powers and the 26 sums are FP64 work that one SM's pipe takes
+// 16 clocks a warp and instruction for.  24^3: 42 us with a block of eight warps, its
+// sums one after the other, now 16; the sums keep their order.
+constexpr int kEnergyCtas = kThreads / 32;
+
+__global__ void __cluster_dims__(kEnergyCtas, 1, 1) __launch_bounds__(32)
 k_energy_partial(const double* __restrict__ rho, const double* __restrict__ tau,
                  const double* __restrict__ laprho, const double* __restrict__ nablaj,
                  const double* __restrict__ coul, const double* __restrict__ jm, ECoef k, long V,
@@ -63,7 +69,8 @@ k_energy_partial(const double* __restrict__ rho, const double* __restrict__ tau,
     double acc[kTerms];
 #pragma unroll
     for (int q = 0; q < kTerms; ++q) acc[q] = 0.0;
-    for (long v = (long)blockIdx.x * kThreads + threadIdx.x; v < V; v += (long)gridDim.x * kThreads) {
+    // (32 blockIdx.x + lane: row blockIdx.x / kEnergyCtas, thread 32 w + lane of it)
+    for (long v = (long)blockIdx.x * 32 + threadIdx.x; v < V; v += (long)gridDim.x * 32) {
         const double rn = rho[v], rp = rho[V + v];
         const double rt = rn + rp;
         const double tt = tau[v] + tau[V + v];
@@ -109,18 +116,33 @@ k_energy_partial(const double* __restrict__ rho, const double* __restrict__ tau,
             acc[23] += tr[0] * tr[0] + tr[1] * tr[1];
         }
     }
-    __shared__ double red[kThreads / 32];
-    for (int q = 0; q < kTerms; ++q) {
-        double s = acc[q];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        __syncthreads();
-        if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = s;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-            for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-            part[(long)blockIdx.x * kTerms + q] = t;
+    // lane q: the sum of term q over the lanes, halves exchanged so that a step adds
+    // for two terms at once (the pairs of a shuffle tree 16, 8, 4, 2, 1 per term)
+    double x[32];
+#pragma unroll
+    for (int q = 0; q < 32; ++q) x[q] = q < kTerms ? acc[q] : 0.0;
+    const int lane = threadIdx.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < o; ++q) {
+            const bool up = (lane & o) != 0;
+            const double give = up ? x[q] : x[q + o], keep = up ? x[q + o] : x[q];
+            x[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
         }
+    __shared__ double red[kEnergyCtas][32];   // of the row's first block
+    const int w = blockIdx.x % kEnergyCtas;
+    uint32_t to;
+    asm("mapa.shared::cluster.u32 %0, %1, 0;"
+        : "=r"(to)
+        : "r"((uint32_t)__cvta_generic_to_shared(&red[w][lane])));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(x[0]) : "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (w == 0 && lane < kTerms) {
+        double t = 0.0;
+        for (int u = 0; u < kEnergyCtas; ++u) t += red[u][lane];
+        part[(long)(blockIdx.x / kEnergyCtas) * kTerms + lane] = t;
     }
 }
 
@@ -176,7 +198,7 @@ int energy(mg_ctx* c, mg_energy_terms* out) {
     const int nblk = std::max(1, std::min(2 * c->num_sms, div_up(V, kThreads)));
     if (ndots + (size_t)nblk * kTerms > c->red_len) return MG_ERR_STATE;
     ECoef k{B.B4, B.B6, B.B8a, B.B8b, B.B9q, B.byt3a, B.byt3b, B.B7b};
-    k_energy_partial<<<nblk, kThreads, 0, c->stream>>>(c->rho, c->tau, c->laprho, c->nablaj,
+    k_energy_partial<<<nblk * kEnergyCtas, 32, 0, c->stream>>>(c->rho, c->tau, c->laprho, c->nablaj,
                                                        c->coulomb,
                                                        c->tensor ? c->jmunu : nullptr, k, V,
                                                        c->red + ndots);

@@ -316,19 +316,35 @@ k_hfb_mix(double* rho, double* kappa, double* oldrho, double* oldkappa, const do
     const int N = 2 * hsz[b];
     const long o0 = (long)b * nmax * nmax;
     double part = 0.0;
-    for (int t = threadIdx.x; t < N * N; t += kThreads) {
-        const long o = o0 + t;
-        double r = rho[o], k = kappa[o];
-        const double ro = oldrho[o], ko = oldkappa[o];
-        bak_rho[o] = ro;     // the history as it was, for a redo of the step
-        bak_kappa[o] = ko;
-        if (mix_rho) r = mix * r + (1.0 - mix) * ro;
-        if (mix_kappa) k = mix * k + (1.0 - mix) * ko;
-        rho[o] = r;
-        kappa[o] = k;
-        oldrho[o] = r;
-        oldkappa[o] = k;
-        part = part - delta[o] * k;
+    // a thread's words kAhead at a time (the arrays do not overlap)
+    constexpr int kAhead = 8;
+    for (int t0 = threadIdx.x; t0 < N * N; t0 += kAhead * kThreads) {
+        double r[kAhead], k[kAhead], ro[kAhead], ko[kAhead], d[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const long o = o0 + t0 + u * kThreads;
+            if (t0 + u * kThreads < N * N) {
+                r[u] = rho[o];
+                k[u] = kappa[o];
+                ro[u] = oldrho[o];
+                ko[u] = oldkappa[o];
+                d[u] = delta[o];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const long o = o0 + t0 + u * kThreads;
+            if (t0 + u * kThreads >= N * N) break;
+            bak_rho[o] = ro[u];     // the history as it was, for a redo of the step
+            bak_kappa[o] = ko[u];
+            if (mix_rho) r[u] = mix * r[u] + (1.0 - mix) * ro[u];
+            if (mix_kappa) k[u] = mix * k[u] + (1.0 - mix) * ko[u];
+            rho[o] = r[u];
+            kappa[o] = k[u];
+            oldrho[o] = r[u];
+            oldkappa[o] = k[u];
+            part = part - d[u] * k[u];
+        }
     }
     const double s = cta_sum(part, red);
     if (threadIdx.x == 0) scal[b] = s;

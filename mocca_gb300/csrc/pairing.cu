@@ -196,6 +196,21 @@ k_pair_gaps(const double* __restrict__ psi, const int* __restrict__ members,
 }
 
 // Delta(i, j+h) = dv f_i f_j sum_chunks, Delta(j+h, i) = -Delta(i, j+h); rest 0
+// x[0] + x[stride] + ... in order, the words loaded sixteen at a time.
+__device__ __forceinline__ double chunk_sum(const double* __restrict__ x, int count, long stride) {
+    double s = 0.0;
+    int q = 0;
+    for (; q + 16 <= count; q += 16) {
+        double y[16];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) y[u] = x[(q + u) * stride];
+#pragma unroll
+        for (int u = 0; u < 16; ++u) s += y[u];
+    }
+    for (; q < count; ++q) s += x[q * stride];
+    return s;
+}
+
 __global__ void k_gaps_finish(const double* __restrict__ gpart, const int* __restrict__ members,
                               const int* __restrict__ hsz, int hmax, int nmax, int nchunk,
                               const double* __restrict__ f, double dv, double* __restrict__ delta) {
@@ -209,16 +224,16 @@ __global__ void k_gaps_finish(const double* __restrict__ gpart, const int* __res
         const int i = r, j = c - h;
         const double fi = f[members[b * hmax + i]], fj = f[members[b * hmax + j]];
         if (fi * fj >= kNumCut) {
-            double s = 0.0;
-            for (int q = 0; q < nchunk; ++q) s += gpart[((long)b * nchunk + q) * hmax * hmax + i * h + j];
+            const double s = chunk_sum(gpart + (long)b * nchunk * hmax * hmax + i * h + j, nchunk,
+                                       (long)hmax * hmax);
             val = dv * fi * fj * s;
         }
     } else if (r >= h && c < h) {
         const int i = c, j = r - h;
         const double fi = f[members[b * hmax + i]], fj = f[members[b * hmax + j]];
         if (fi * fj >= kNumCut) {
-            double s = 0.0;
-            for (int q = 0; q < nchunk; ++q) s += gpart[((long)b * nchunk + q) * hmax * hmax + i * h + j];
+            const double s = chunk_sum(gpart + (long)b * nchunk * hmax * hmax + i * h + j, nchunk,
+                                       (long)hmax * hmax);
             val = -(dv * fi * fj * s);
         }
     }
