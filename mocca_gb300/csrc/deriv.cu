@@ -20,6 +20,7 @@
 
 #include "df.cuh"
 
+#include "chain.cuh"
 #include "mg_internal.cuh"
 
 namespace mg {
@@ -361,6 +362,7 @@ __device__ __forceinline__ void few_place(const GridJob& J, int V, int& a, int& 
 __global__ void __launch_bounds__(3 * kFewPts)
 k_deriv_few(const GridJob* __restrict__ jobs, MatPtrs mp, int nx, int ny, int nz) {
     __shared__ double part[3][kFewPts];
+    chain_wait();
     const GridJob J = jobs[blockIdx.y];
     const int V = nx * ny * nz, lane = threadIdx.x % kFewPts;
     int a, v;
@@ -573,7 +575,7 @@ int run_jobs(mg_ctx* c, const GridJob* jobs, int njobs, bool out_df) {
         if (mixed)
             k_deriv_few_df<<<grid, 3 * kFewPts, 0, c->stream>>>(jobs, mat_ptrs32(c), nx, ny, nz);
         else
-            k_deriv_few<<<grid, 3 * kFewPts, 0, c->stream>>>(jobs, mat_ptrs(c), nx, ny, nz);
+            return launch_early(c, k_deriv_few, grid, 3 * kFewPts, 0, jobs, mat_ptrs(c), nx, ny, nz);
         MG_LAUNCHED(c);
         return MG_OK;
     }

@@ -16,9 +16,11 @@
 //      dt = 0.9 hbar 4 / (maxE + relE + 2 sqrt(maxE relE)).
 // The reference fills the start with Fortran's random_number (unseeded); this
 // uses a fixed-seed splitmix64 stream instead, so that runs repeat.
+#include <climits>
 #include <cmath>
 #include <vector>
 
+#include "chain.cuh"
 #include "mg_internal.cuh"
 
 namespace mg {
@@ -37,16 +39,33 @@ inline double start_value(unsigned long long k) {
     return (double)(z >> 11) * (1.0 / 9007199254740992.0);
 }
 
+constexpr double kEstTol = 1e-2;   // of the probe's energy from one iteration to the next
+constexpr int kEstChunk = 4;       // iterations between host reads
+
+// Device side of the stopping test: the last energy and the iteration that met it.
+struct EstState {
+    double prev;
+    int stop;
+};
+
 // update = fac (h psi - maxE psi) + mu update ; psi += update ; block partials of psi^2
 __global__ void __launch_bounds__(kThreads)
 k_est_step(double* __restrict__ psi, const double* __restrict__ hp, double* __restrict__ up,
-           const double* __restrict__ e_dev, double fac, double mom, long n,
+           const double* __restrict__ e_dev, EstState* state, int it, double fac, double mom, long n,
            double* __restrict__ part) {
     __shared__ double red[kThreads / 32];
+    chain_wait();
+    if (it > 0 && state->stop < it) return;
     const long t = (long)blockIdx.x * kThreads + threadIdx.x;
     double s = 0.0;
+    const double maxE = e_dev[0];
+    if (t == 0) {
+        // (no block of this iteration is stopped by what is written here)
+        if (it == 0) state->stop = INT_MAX;
+        if (it > 0 && fabs(state->prev - maxE) < kEstTol) state->stop = it;
+        state->prev = maxE;
+    }
     if (t < n) {
-        const double maxE = e_dev[0];
         const double u = fac * (hp[t] - maxE * psi[t]) + mom * up[t];
         up[t] = u;
         const double x = psi[t] + u;
@@ -65,13 +84,20 @@ k_est_step(double* __restrict__ psi, const double* __restrict__ hp, double* __re
 
 // psi /= sqrt(norm), norm = dv * (partials added in block order)
 __global__ void k_est_normalise(double* __restrict__ psi, const double* __restrict__ part,
-                                int nblk, double dv, long n) {
-    __shared__ double scale;
-    if (threadIdx.x == 0) {
-        double a = 0.0;
-        for (int q = 0; q < nblk; ++q) a += part[q];
-        scale = 1.0 / std::sqrt(a * dv);
+                                int nblk, double dv, long n, const EstState* __restrict__ state,
+                                int it) {
+    __shared__ double scale, red[kThreads];
+    chain_wait();
+    if (state->stop < it) return;
+    double a = 0.0;
+    for (int q0 = 0; q0 < nblk; q0 += kThreads) {
+        if (q0 + (int)threadIdx.x < nblk) red[threadIdx.x] = part[q0 + threadIdx.x];
+        __syncthreads();
+        if (threadIdx.x == 0)
+            for (int q = 0; q < min(kThreads, nblk - q0); ++q) a += red[q];
+        __syncthreads();
     }
+    if (threadIdx.x == 0) scale = 1.0 / std::sqrt(a * dv);
     __syncthreads();
     for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (long)gridDim.x * blockDim.x)
         psi[t] *= scale;
@@ -86,7 +112,8 @@ int estimate_parameters(mg_ctx* c) {
     const int nwt = c->p.nwt;
     double* psi = nullptr;
     if (!c->est) {
-        MG_CUDA(cudaMalloc(&c->est, (28 * V + 2) * sizeof(double)));
+        MG_CUDA(cudaMalloc(&c->est, (28 * V + 2 * kEstChunk) * sizeof(double) + sizeof(EstState)));
+        MG_CUDA(cudaMallocHost(&c->h_est, 2 * kEstChunk * sizeof(double)));
         MG_CUDA(cudaMalloc(&c->est_jobs, 4 * sizeof(GridJob)));
         MG_CUDA(cudaMalloc(&c->est_qn, 4 * sizeof(int)));
     }
@@ -95,7 +122,8 @@ int estimate_parameters(mg_ctx* c) {
     double* lap = der + 12 * V;
     double* hp = lap + V4;
     double* up = hp + V4;
-    double* e_dev = up + V4;
+    double* e_dev = up + V4;   // energy and dispersion of a chunk's iterations
+    EstState* state = reinterpret_cast<EstState*>(e_dev + 2 * kEstChunk);
     ++c->est_iter;
     if (c->est_iter == 1) {
         // maxspwf: quantum numbers of HFBasis(nwt), or of the last neutron
@@ -137,20 +165,30 @@ int estimate_parameters(mg_ctx* c) {
     MG_CUDA(cudaMemsetAsync(up, 0, V4 * sizeof(double), c->stream));
     const double fac = c->step_dt / c->f.hbar, mom = c->step_mom;
     const int nblk = div_up(V4, kThreads);
+    // kEstChunk iterations are launched before their energies are read; those after
+    // the one that has converged leave the probe as it is
     double maxE = 0.0, prev = NAN, con = NAN;
-    for (int it = 0; it < 500; ++it) {
-        MG_TRY(hpsi_single(c, psi, der, lap, c->est_qn, hp, e_dev));
-        MG_CUDA(cudaMemcpyAsync(&maxE, e_dev, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-        k_est_step<<<nblk, kThreads, 0, c->stream>>>(psi, hp, up, e_dev, fac, mom, V4, c->red);
-        MG_LAUNCHED(c);
-        k_est_normalise<<<std::min(nblk, 4 * c->num_sms), kThreads, 0, c->stream>>>(psi, c->red,
-                                                                                  nblk, c->dv, V4);
-        MG_LAUNCHED(c);
-        MG_TRY(run_jobs(c, c->est_jobs, 4, false));
+    bool found = false;
+    for (int it0 = 0; it0 < 500 && !found; it0 += kEstChunk) {
+        const int count = std::min(kEstChunk, 500 - it0);
+        for (int it = it0; it < it0 + count; ++it) {
+            double* e = e_dev + 2 * (it - it0);
+            MG_TRY(hpsi_single(c, psi, der, lap, c->est_qn, hp, e));
+            MG_TRY(launch_early(c, k_est_step, dim3(nblk), kThreads, 0, psi, hp, up, e, state, it,
+                                fac, mom, V4, c->red));
+            MG_TRY(launch_early(c, k_est_normalise, dim3(std::min(nblk, 4 * c->num_sms)), kThreads,
+                                0, psi, c->red, nblk, c->dv, V4, state, it));
+            MG_TRY(run_jobs(c, c->est_jobs, 4, false));
+        }
+        MG_CUDA(cudaMemcpyAsync(c->h_est, e_dev, 2 * kEstChunk * sizeof(double),
+                                cudaMemcpyDeviceToHost, c->stream));
         MG_CUDA(cudaStreamSynchronize(c->stream));
-        con = prev - maxE;
-        prev = maxE;
-        if (std::fabs(con) < 1e-2) break;
+        for (int it = 0; it < count && !found; ++it) {
+            maxE = c->h_est[2 * it];
+            con = prev - maxE;
+            prev = maxE;
+            found = std::fabs(con) < kEstTol;
+        }
     }
     if (std::isnan(maxE)) return MG_ERR_NAN;   // src/ImaginaryTime.f90:190-192
     // the smallest excitation

@@ -54,6 +54,7 @@ void free_all(mg_ctx* c) {
     constraints_free(c);
     if (c->h_cg_status) cudaFreeHost(c->h_cg_status);
     if (c->h_tc_status) cudaFreeHost(c->h_tc_status);
+    if (c->h_est) cudaFreeHost(c->h_est);
     if (c->cfast_graph) cudaGraphExecDestroy(c->cfast_graph);
     if (c->ev_fork) cudaEventDestroy(c->ev_fork);
     if (c->ev_join) cudaEventDestroy(c->ev_join);
@@ -268,7 +269,7 @@ extern "C" int mg_create(const mg_params* p, const mg_force* f, void* stream, mg
     if (ok && c->tensor) ok = A(&c->jmunu, 18 * V) && A(&c->jmunu_hist, 18 * V);
     if (!ok) return fail(MG_ERR_CUDA);
     // reduction scratch: the largest of the per-kernel partial tables
-    const long hp = nwt * div_up(V, 256) * 2;
+    const long hp = nwt * div_up(V, 64) * 2;
     const long dens = (long)density_groups(c) * 6 * V;
     const long dots = 64 * nwt;
     const long en = 2L * c->num_sms * 26 + 4L * c->num_sms;

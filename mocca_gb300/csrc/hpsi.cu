@@ -14,6 +14,7 @@
 // h.psi never goes to HBM.  The per-spwf sums <psi|h psi> and <h psi|h psi>
 // are reduced per block into a partial table and finished in block order
 // (deterministic).
+#include "chain.cuh"
 #include "df.cuh"
 #include "mg_internal.cuh"
 
@@ -21,7 +22,9 @@ namespace mg {
 
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 256;     // mixed form
+constexpr int kThreads64 = 128;   // FP64 form
+constexpr int kThreads1 = 64;     // ... of one spinor
 
 struct Fields {
     const double* U;
@@ -46,16 +49,18 @@ __device__ __forceinline__ void pauli(const double* p, int dir, double* o) {
 }
 
 // Bound by the FP64 pipe (a warp's instruction takes 16 clocks of the SM): 83 FP64
-// instructions a point, 95 with the GradDesc step.  200 spwfs at 32^3: 916 us (1180
-// with 101, the terms summed one by one), 160 at 24^3 with the step 495 (510).
-template <bool kGradStep>
-__global__ void __launch_bounds__(kThreads, 3)
+// instructions a point, 95 with the GradDesc step.  200 spwfs at 32^3: 927 us (1180
+// with 101, the terms summed one by one), 160 at 24^3 with the step 466 (510).
+// Blocks of kT threads: 128, or 64 for the few points of a single spinor.
+template <bool kGradStep, int kT>
+__global__ void __launch_bounds__(kT, 768 / kT)
 k_hpsi(double* __restrict__ psi, const double* __restrict__ der,
        const double* __restrict__ lap, const int* __restrict__ qn, Fields F,
        double* __restrict__ hout, double* __restrict__ upd, double* __restrict__ partial,
        long V, double kin0, double kin1, double fac, double mom) {
+    chain_wait();
     const int i = blockIdx.y;
-    const long v = (long)blockIdx.x * kThreads + threadIdx.x;
+    const long v = (long)blockIdx.x * kT + threadIdx.x;
     double s_eh = 0.0, s_hh = 0.0;
     if (v < V) {
         const int it = (qn[4 * i] + 3) / 2 - 1;
@@ -149,9 +154,9 @@ k_hpsi(double* __restrict__ psi, const double* __restrict__ der,
             for (int l = 0; l < 4; ++l) ho[l * V + v] = h[l];
         }
     }
-    // block sums of (s_eh, s_hh): warps 0 and 1 add 8 values a lane and then the
-    // lanes (shuffles in every warp would be a tenth of the kernel's FP64 work)
-    __shared__ double red[2][kThreads];
+    // block sums of (s_eh, s_hh): warps 0 and 1 add a value of each warp per lane and
+    // then the lanes (shuffles in every warp would be a tenth of the kernel's FP64 work)
+    __shared__ double red[2][kT];
     red[0][threadIdx.x] = s_eh;
     red[1][threadIdx.x] = s_hh;
     __syncthreads();
@@ -159,7 +164,7 @@ k_hpsi(double* __restrict__ psi, const double* __restrict__ der,
         const int q = threadIdx.x / 32, lane = threadIdx.x % 32;
         double a = red[q][lane];
 #pragma unroll
-        for (int u = 1; u < kThreads / 32; ++u) a += red[q][lane + 32 * u];
+        for (int u = 1; u < kT / 32; ++u) a += red[q][lane + 32 * u];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
         if (lane == 0) partial[((long)i * gridDim.x + blockIdx.x) * 2 + q] = a;
@@ -321,18 +326,62 @@ k_hpsi_df(double* __restrict__ psi, const float2* __restrict__ der,
 }
 
 // e[i] = dv * sum <psi|h psi>, disp[i] = dv * sum <h psi|h psi> - e^2
+// Mixed form: a thread per spwf adds its chunks in order, eight loads ahead of the
+// sums' chains.
 __global__ void k_finish_energies(const double* __restrict__ partial, int nchunk, int nwt,
                                   double dv, double* __restrict__ e, double* __restrict__ disp) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nwt) return;
     double a = 0.0, b = 0.0;
-    for (int q = 0; q < nchunk; ++q) {
-        a += partial[((long)i * nchunk + q) * 2 + 0];
-        b += partial[((long)i * nchunk + q) * 2 + 1];
+    const double2* p = reinterpret_cast<const double2*>(partial) + (long)i * nchunk;
+    int q = 0;
+    for (; q + 8 <= nchunk; q += 8) {
+        double2 x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = p[q + u];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            a += x[u].x;
+            b += x[u].y;
+        }
+    }
+    for (; q < nchunk; ++q) {
+        a += p[q].x;
+        b += p[q].y;
     }
     const double en = a * dv;
     e[i] = en;
     disp[i] = b * dv - en * en;
+}
+
+// FP64 form: a warp per spwf, its lanes every 32nd chunk and then the lanes (fewer
+// roundings in a row, and no chain of as many adds as there are chunks: 41 -> 4.6 us
+// for 200 spwfs of 256 chunks).
+constexpr int kFinishWarps = 4;
+
+__global__ void __launch_bounds__(32 * kFinishWarps)
+k_finish_energies64(const double* __restrict__ partial, int nchunk, int nwt, double dv,
+                    double* __restrict__ e, double* __restrict__ disp) {
+    chain_wait();
+    const int i = blockIdx.x * kFinishWarps + threadIdx.x / 32, lane = threadIdx.x % 32;
+    if (i >= nwt) return;
+    double a = 0.0, b = 0.0;
+    const double2* p = reinterpret_cast<const double2*>(partial) + (long)i * nchunk;
+#pragma unroll 4
+    for (int q = lane; q < nchunk; q += 32) {
+        a += p[q].x;
+        b += p[q].y;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+        const double en = a * dv;
+        e[i] = en;
+        disp[i] = b * dv - en * en;
+    }
 }
 
 double reduced_mass(const mg_ctx* c, int it) {
@@ -351,7 +400,8 @@ int hpsi_basis(mg_ctx* c, int b, double* out, bool grad_step, double fac, double
     Basis& B = c->bas[b];
     if (!B.have_qn) return MG_ERR_STATE;
     const long V = c->V;
-    const int nchunk = div_up(V, kThreads);
+    const int threads = B.der_df ? kThreads : kThreads64;
+    const int nchunk = div_up(V, threads);
     Fields F{c->U, c->Bp, c->nablaB, c->W, c->divW, c->Apot, c->Spot, c->divA};
     const double kin0 = c->f.hbm / 2.0 * reduced_mass(c, 0);
     const double kin1 = c->f.hbm / 2.0 * reduced_mass(c, 1);
@@ -383,14 +433,18 @@ int hpsi_basis(mg_ctx* c, int b, double* out, bool grad_step, double fac, double
                                                            c->fields_df, out, nullptr, c->red, V,
                                                            0.0, 0.0);
     else if (grad_step)
-        k_hpsi<true><<<grid, kThreads, 0, c->stream>>>(B.psi, B.der, B.lap, B.qn, F, nullptr,
-                                                       c->updates, c->red, V, kin0, kin1, fac, mom);
+        k_hpsi<true, kThreads64><<<grid, kThreads64, 0, c->stream>>>(
+            B.psi, B.der, B.lap, B.qn, F, nullptr, c->updates, c->red, V, kin0, kin1, fac, mom);
     else
-        k_hpsi<false><<<grid, kThreads, 0, c->stream>>>(B.psi, B.der, B.lap, B.qn, F, out,
-                                                        nullptr, c->red, V, kin0, kin1, 0.0, 0.0);
+        k_hpsi<false, kThreads64><<<grid, kThreads64, 0, c->stream>>>(
+            B.psi, B.der, B.lap, B.qn, F, out, nullptr, c->red, V, kin0, kin1, 0.0, 0.0);
     MG_LAUNCHED(c);
-    k_finish_energies<<<div_up(c->p.nwt, 128), 128, 0, c->stream>>>(c->red, nchunk, c->p.nwt,
-                                                                     c->dv, B.e, B.disp);
+    if (mixed)
+        k_finish_energies<<<div_up(c->p.nwt, 32), 32, 0, c->stream>>>(c->red, nchunk, c->p.nwt,
+                                                                      c->dv, B.e, B.disp);
+    else
+        k_finish_energies64<<<div_up(c->p.nwt, kFinishWarps), 32 * kFinishWarps, 0, c->stream>>>(
+            c->red, nchunk, c->p.nwt, c->dv, B.e, B.disp);
     MG_LAUNCHED(c);
     return MG_OK;
 }
@@ -400,7 +454,7 @@ int hpsi_basis(mg_ctx* c, int b, double* out, bool grad_step, double fac, double
 int hpsi_single(mg_ctx* c, double* psi, const double* der, const double* lap, const int* qn_dev,
                 double* out, double* e_dev) {
     const long V = c->V;
-    const int nchunk = div_up(V, kThreads);
+    const int nchunk = div_up(V, kThreads1);
     Fields F{c->U, c->Bp, c->nablaB, c->W, c->divW, c->Apot, c->Spot, c->divA};
     const double kin0 = c->f.hbm / 2.0 * reduced_mass(c, 0);
     const double kin1 = c->f.hbm / 2.0 * reduced_mass(c, 1);
@@ -409,13 +463,10 @@ int hpsi_single(mg_ctx* c, double* psi, const double* der, const double* lap, co
         MG_TRY(tensor_odd_action(c, der, c->est_h_qn, qn_dev, 1, c->todd_x));
         F.X = c->todd_x;
     }
-    k_hpsi<false><<<dim3(nchunk, 1), kThreads, 0, c->stream>>>(psi, der, lap, qn_dev, F, out,
-                                                               nullptr, c->red, V, kin0, kin1,
-                                                               0.0, 0.0);
-    MG_LAUNCHED(c);
-    k_finish_energies<<<1, 128, 0, c->stream>>>(c->red, nchunk, 1, c->dv, e_dev, e_dev + 1);
-    MG_LAUNCHED(c);
-    return MG_OK;
+    MG_TRY(launch_early(c, k_hpsi<false, kThreads1>, dim3(nchunk, 1), kThreads1, 0, psi, der, lap,
+                        qn_dev, F, out, nullptr, c->red, V, kin0, kin1, 0.0, 0.0));
+    return launch_early(c, k_finish_energies64, dim3(1), 32, 0, c->red, nchunk, 1, c->dv, e_dev,
+                        e_dev + 1);
 }
 
 }  // namespace mg

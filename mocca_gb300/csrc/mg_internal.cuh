@@ -371,6 +371,7 @@ struct mg_ctx {
     double* est = nullptr;              // psi 4V, der 12V, lap 4V, hpsi 4V, update 4V, (e, disp)
     mg::GridJob* est_jobs = nullptr;
     int* est_qn = nullptr;
+    double* h_est = nullptr;   // pinned: the probe's energies of a few iterations
     int est_h_qn[4] = {0, 0, 0, 0};   // the probe's quantum numbers on the host
     int est_iter = 0;
     bool step_set = false;
