@@ -1045,6 +1045,187 @@ k_settle(double* __restrict__ X, const double* __restrict__ X2, long stride, int
     X[o] = X2[o];
 }
 
+// The refinement chain for small matrices (FP64 form), one launch: the steps, the
+// re-orthonormalisation and, for the polish, S = X^T A X, which else are some 25
+// launches of ~3 us for a few thousand FMAs each.  A matrix has a cluster of eight
+// CTAs; every CTA holds all matrices of the chain in shared memory, computes an eighth
+// of a product's entries and stores them into all eight.  An entry's sum is shared by
+// as many threads as there are to spare (2, 4, ... of them, four k or more each: fewer
+// roundings in a row, mean errors 0 to 20% below the launches').  Up to kRefineMax:
+// beyond, an eighth of a product is more FP64 work than a launch over all SMs has.  A
+// cold decomposition of four matrices of 20 / 32 / 40 / 48: 143 / 224 / 293 / 395 us,
+// by launches 177 / 250 / 304 / 358; five HFB iterations at 10^3 (matrices of 20 and
+// less): 5313 -> 4942 us.
+constexpr int kRefineCtas = 8;
+constexpr int kRefineThreads = 256;
+constexpr int kRefineMax = 40;
+constexpr int kRefineTri = kRefineMax * (kRefineMax + 1) / 2;
+
+size_t refine_smem(int n) { return 6 * (size_t)n * n * sizeof(double); }
+
+__device__ __forceinline__ void store_all(double* p, double x, int first, int step) {
+    for (int c = first; c < kRefineCtas; c += step)
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(peer_addr(p, c)), "d"(x) : "memory");
+}
+
+// Sum of kRefineThreads values, the same in all threads.
+__device__ __forceinline__ double refine_sum(double x, double* sh) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    __syncthreads();
+    if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = x;
+    __syncthreads();
+    double s = 0.0;
+#pragma unroll
+    for (int q = 0; q < kRefineThreads / 32; ++q) s += sh[q];
+    return s;
+}
+
+__global__ void __cluster_dims__(kRefineCtas, 1, 1) __launch_bounds__(kRefineThreads)
+k_refine(const double* __restrict__ Ag, double* Xg, double* __restrict__ Sg, long stride, int ld,
+         const int* __restrict__ nsz, double* __restrict__ w, long wstride,
+         double* __restrict__ anorm, double* __restrict__ emax, double* __restrict__ offrel,
+         int nref, double skip_tol, int polish) {
+    extern __shared__ double smr[];
+    __shared__ double lam[kRefineMax], red[kRefineThreads / 32];
+    __shared__ unsigned short tri[kRefineTri];
+    chain_wait();
+    const int b = blockIdx.x / kRefineCtas, rank = blockIdx.x % kRefineCtas, tid = threadIdx.x;
+    const int n = nsz[b];
+    if (n == 0) return;   // the whole cluster
+    const int m = n * n, nt = n * (n + 1) / 2;
+    double *A = smr, *X = A + m, *Xn = X + m, *P = Xn + m, *S = P + m, *G = S + m;
+    double part = 0.0;
+    for (int e = tid; e < m; e += kRefineThreads) {
+        const long o = b * stride + (long)(e / n) * ld + e % n;
+        A[e] = Ag[o];
+        X[e] = Xg[o];
+        part = fma(A[e], A[e], part);
+    }
+    for (int e = tid; e < m; e += kRefineThreads) {
+        const int i = e / n, j = e % n;
+        if (i <= j) tri[i * n - i * (i - 1) / 2 + j - i] = (unsigned short)(i * 256 + j);
+    }
+    const double norm = sqrt(refine_sum(part, red));
+    if (rank == 0 && tid == 0) anorm[b] = norm;
+    pair_barrier();   // every CTA has started and holds its copies
+
+    // the entries [e0, e1) of `total` for this CTA; `tpo` threads each
+    int tpo = 1;
+    while (8 * tpo <= n && 2 * tpo * ((m + kRefineCtas - 1) / kRefineCtas) <= kRefineThreads) tpo *= 2;
+    const int q0 = tid % tpo;
+    const auto share = [&](int total, auto fn) {
+        const int e0 = total * rank / kRefineCtas, e1 = total * (rank + 1) / kRefineCtas;
+        // (all lanes of a group take part in its shuffles)
+        for (int base = e0; base < e1; base += kRefineThreads / tpo) {
+            const int e = base + tid / tpo;
+            fn(e < e1 ? e : -1);
+        }
+    };
+    const auto over_k = [&](auto term) {
+        double s = 0.0;
+        for (int k = q0; k < n; k += tpo) s = term(k, s);
+        for (int o = 1; o < tpo; o *= 2) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
+    // C <- U V in all CTAs, an entry through out(e, sum)
+    const auto product = [&](const double* U, const double* V, double* C, auto out) {
+        share(m, [&](int e) {
+            const int i = max(e, 0) / n, j = max(e, 0) % n;
+            const double s = over_k([&](int k, double x) { return fma(U[i * n + k], V[k * n + j], x); });
+            if (e >= 0) store_all(C + e, out(e, s), q0, tpo);
+        });
+        pair_barrier();
+    };
+    // C <- X^T V, symmetric; count entries of the upper triangle from `first` on go to C1
+    const auto gram = [&](const double* V0, double* C0, const double* V1, double* C1) {
+        share(V1 ? 2 * nt : nt, [&](int e) {
+            const int t = tri[max(e, 0) >= nt ? e - nt : max(e, 0)], i = t >> 8, j = t & 255;
+            const double* V = e >= nt ? V1 : V0;
+            double* C = e >= nt ? C1 : C0;
+            const double s = over_k([&](int k, double x) { return fma(X[k * n + i], V[k * n + j], x); });
+            if (e >= 0) {
+                store_all(C + i * n + j, s, q0, tpo);
+                if (i != j) store_all(C + j * n + i, s, q0, tpo);
+            }
+        });
+        pair_barrier();
+    };
+    const auto plain = [](int, double s) { return s; };
+    for (int step = 0; step < nref; ++step) {
+        product(A, X, P, plain);
+        gram(P, S, X, G);
+        if (tid < n) lam[tid] = S[tid * n + tid] / G[tid * n + tid];
+        __syncthreads();
+        double ps = 0.0, pr = 0.0;
+        for (int e = tid; e < m; e += kRefineThreads) {
+            const int i = e / n, j = e % n;
+            const double sd = S[e] - (i == j ? lam[i] : 0.0), rd = (i == j ? 1.0 : 0.0) - G[e];
+            ps = fma(sd, sd, ps);
+            pr = fma(rd, rd, pr);
+        }
+        ps = sqrt(refine_sum(ps, red));
+        pr = sqrt(refine_sum(pr, red));
+        const double delta = 2.0 * (ps + norm * pr), off = ps / norm;
+        const bool last = step == nref - 1 || (skip_tol >= 0.0 && off <= skip_tol);
+        // F = I + E over A X
+        share(m, [&](int e) {
+            if (e < 0 || q0 != 0) return;
+            const int i = e / n, j = e % n;
+            const double r = (i == j ? 1.0 : 0.0) - G[e], d = lam[j] - lam[i];
+            const double x = i != j && fabs(d) > delta ? (S[e] + lam[j] * r) / d : 0.5 * r;
+            store_all(P + e, (i == j ? 1.0 : 0.0) + x, 0, 1);
+        });
+        if (last) {
+            // the largest angle of a row's pairs of opposite sign
+            for (int i = rank + kRefineCtas * (tid / 32); i < n;
+                 i += kRefineCtas * (kRefineThreads / 32)) {
+                double em = 0.0;
+                for (int j = tid % 32; j < n; j += 32)
+                    if (lam[j] * lam[i] < 0.0) em = fmax(em, fabs(S[i * n + j]) / fabs(lam[j] - lam[i]));
+                for (int o = 16; o > 0; o >>= 1) em = fmax(em, __shfl_xor_sync(0xffffffffu, em, o));
+                if (tid % 32 == 0) emax[(long)b * ld + i] = em;
+            }
+            if (rank == 0) {
+                if (tid < n) w[b * wstride + tid] = lam[tid];
+                if (tid == 0) offrel[b] = off;
+            }
+        }
+        pair_barrier();
+        product(X, P, Xn, plain);
+        double* t = X;
+        X = Xn;
+        Xn = t;
+        if (last) break;
+    }
+    for (int pass = 0; pass < (polish ? 2 : 1); ++pass) {
+        // F = I + R / 2 + 3/8 R^2, R = I - X^T X (in S, each CTA its own)
+        gram(X, G, nullptr, nullptr);
+        for (int e = tid; e < m; e += kRefineThreads) S[e] = (e / n == e % n ? 1.0 : 0.0) - G[e];
+        __syncthreads();
+        product(S, S, P, [&](int e, double s) {
+            return fma(0.375, s, fma(0.5, S[e], e / n == e % n ? 1.0 : 0.0));
+        });
+        product(X, P, Xn, plain);
+        double* t = X;
+        X = Xn;
+        Xn = t;
+    }
+    share(m, [&](int e) {
+        if (e >= 0 && q0 == 0) Xg[b * stride + (long)(e / n) * ld + e % n] = X[e];
+    });
+    if (polish) {
+        product(A, X, P, plain);
+        share(nt, [&](int e) {
+            const int t = tri[max(e, 0)], i = t >> 8, j = t & 255;
+            const double s = over_k([&](int k, double x) { return fma(X[k * n + i], P[k * n + j], x); });
+            if (e >= 0 && q0 == 0) {
+                Sg[b * stride + (long)i * ld + j] = s;
+                Sg[b * stride + (long)j * ld + i] = s;
+            }
+        });
+    }
+}
+
 // Frobenius norms of the batch matrices (delta of the refinement uses ||A||),
 // where no Jacobi seed has left them.
 __global__ void __launch_bounds__(kJThreads)
@@ -1083,6 +1264,8 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
         MG_CUDA(cudaFuncSetAttribute(k_jacobi_df_polish,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)df_polish_smem(kDfPolishMax)));
+        MG_CUDA(cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)refine_smem(kRefineMax)));
         E.attr_done = true;
     }
     if (seed != kSeedRefine) {
@@ -1093,18 +1276,23 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
             warm ? 12 : 30, c->flags + 4, E.anorm);
         MG_LAUNCHED(c);
     }
-    if (seed == kSeedRefine) {
+    const bool dfg = c->cur_precision == MG_MIXED;
+    const bool fused = !dfg && E.nmax <= kRefineMax;
+    if (seed == kSeedRefine && !fused) {
         k_frob<<<E.nb, kJThreads, 0, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm);
         MG_LAUNCHED(c);
     }
     const int tiles = div_up(E.nmax, kTile) * div_up(E.nmax, kTile);
     const dim3 rows(E.nmax, E.nb), elems(div_up((long)E.nmax * E.nmax, kThreads), E.nb);
-    const bool dfg = c->cur_precision == MG_MIXED;
     const SkipCtl none{nullptr, nullptr, 0, 0, 0.0};
     Flip flip{E.X, E.X2, (long)E.nb * E.stride, false};   // on: the vectors are in X2
-    if (E.skip_tol >= 0.0)
+    if (fused)
+        MG_TRY(launch_early(c, k_refine, dim3(E.nb * kRefineCtas), kRefineThreads,
+                            refine_smem(E.nmax), E.A, E.X, E.S, E.stride, E.ld, E.nsz, E.w,
+                            E.wstride, E.anorm, E.emax, E.offrel, nref, E.skip_tol, polish ? 1 : 0));
+    else if (E.skip_tol >= 0.0)
         MG_CUDA(cudaMemsetAsync(E.done, 0x7f, (size_t)E.nb * sizeof(int), c->stream));
-    for (int s = 0; s < nref; ++s) {
+    for (int s = 0; s < nref && !fused; ++s) {
         // AX = A X ; S = X^T AX ; G = X^T X ; F = I + E ; X <- X F
         SkipCtl sk{E.skip_tol >= 0.0 ? E.done : nullptr, E.offrel, s, 1, E.skip_tol};
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, sk, flip));
@@ -1117,7 +1305,7 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_xf, sk, flip));
         flip.on = !flip.on;
     }
-    if (E.skip_tol >= 0.0) {
+    if (E.skip_tol >= 0.0 && !fused) {
         MG_TRY(launch_early(c, k_settle, elems, kThreads, 0, E.X, E.X2, E.stride, E.ld, E.nsz, E.done,
                             nref));
         flip.on = false;
@@ -1128,7 +1316,7 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
     // non-orthogonality of X, and a refinement that stops inside a cluster
     // of near-degenerate eigenvalues (density-matrix occupations ~1e-8 apart
     // near 0 or 1) can leave R ~ 1e-2, which one pass only brings to 1e-7.
-    for (int pass = 0; pass < (polish ? 2 : 1); ++pass) {
+    for (int pass = 0; pass < (polish ? 2 : 1) && !fused; ++pass) {
         MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg + E.nb, none, flip));   // G alone
         MG_TRY(launch_early(c, k_orth_prep, elems, kThreads, 0, E.G, E.AX, E.G, E.stride, E.ld,
                             E.nsz));
@@ -1142,8 +1330,10 @@ int eig_batched(mg_ctx* c, EigBatch& E, int seed, int nref, bool polish) {
         if (psm > (size_t)kSmemOptIn) return MG_ERR_ARG;
         // Rayleigh-Ritz matrix and the FP64 Jacobi polish, its eigenvalues in E.part
         // (2 * nb * ld doubles, free after the refinement) until they are sorted
-        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, none, flip));
-        MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg, none, flip));   // S alone
+        if (!fused) {
+            MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_ax, none, flip));
+            MG_TRY(launch_gemm(c, dfg, dim3(tiles, E.nb), E.d_sg, none, flip));   // S alone
+        }
         if (c->cur_precision == MG_MIXED && E.nmax <= kDfPolishMax)
             k_jacobi_df_polish<<<E.nb, kJThreads, df_polish_smem(E.nmax), c->stream>>>(
                 E.S, E.stride, E.ld, E.nsz, E.anorm, E.G, E.part, E.wstride, E.pfail, 12);
@@ -1186,6 +1376,8 @@ int eig_jacobi_fp64(mg_ctx* c, EigBatch& E) {
         MG_CUDA(cudaFuncSetAttribute(k_jacobi_df_polish,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)df_polish_smem(kDfPolishMax)));
+        MG_CUDA(cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)refine_smem(kRefineMax)));
         E.attr_done = true;
     }
     k_frob<<<E.nb, kJThreads, 0, c->stream>>>(E.A, E.stride, E.ld, E.nsz, E.anorm);
@@ -1383,7 +1575,10 @@ int noalloc_setup(int dev, unsigned char** base) {
                                      kSmemOptIn));
         MG_CUDA(cudaFuncSetAttribute(k_jacobi64_polish, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      kSmemOptIn));
+        MG_CUDA(cudaFuncSetAttribute(k_refine, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)refine_smem(kRefineMax)));
         cudaFuncAttributes fa;
+        MG_CUDA(cudaFuncGetAttributes(&fa, k_refine));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_jacobi32));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_jacobi64_polish));
         MG_CUDA(cudaFuncGetAttributes(&fa, k_sort_cols));
