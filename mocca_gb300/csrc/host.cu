@@ -28,7 +28,7 @@ void free_all(mg_ctx* c) {
     F(c->tcmats);
     F(c->tc_erow);
     F(c->tc_status);
-    F(c->gs_Stc); F(c->gs_xd); F(c->gs_xe); F(c->can_xd); F(c->can_xe); F(c->gap_part); F(c->fields_df);
+    F(c->gs_Stc); F(c->gs_xd); F(c->gs_xe); F(c->can_xd); F(c->can_xe); F(c->gap_part); F(c->gap_part64); F(c->fields_df);
     F(c->field_y); F(c->field_xd); F(c->field_xe); F(c->field_ybase);
     F(c->est); F(c->est_jobs); F(c->est_qn);
     for (int b = 0; b < 2; ++b) {

@@ -1,7 +1,7 @@
 // meshgemm_tc.cu -- the mesh-sized contractions on the tcgen05 tensor cores
-// (exact BF16 digit products, ozaki.cuh): the Gram-Schmidt overlap and apply,
-// and the canonical-basis transform, in the mixed form with six digits and in the
-// FP64 form with eight, and the mixed form's pairing contractions.
+// (exact BF16 digit products, ozaki.cuh), in the mixed form with six digits and
+// in the FP64 form with eight: the Gram-Schmidt overlap and apply, the
+// canonical-basis transform and the contractions of the pairing field and gaps.
 //
 // Blocks of up to kMeshTcMax (80) spinors in the mixed form, kMeshTcMin64 to
 // kMeshTcMax64 (24 to 64) in the FP64 form, whose results are rounded once to FP64
@@ -68,7 +68,8 @@ __device__ __forceinline__ double pow2d(int x) {
     return x < -1022 ? 0.0 : __longlong_as_double((long long)(min(x, 1023) + 1023) << 52);
 }
 
-// Sum over a chunk of points of psi_k psi_l for the pairs k <= l of a block, to part.
+// Sum over a chunk of points of psi_k psi_l for the pairs k <= l of a block, or of
+// psi_k z_l for all pairs (kTwo), to part.
 //
 // A unit is a chunk of one block, 256 points in the mixed form, 128 in the FP64 form
 // (what keeps the sums of a weight exact).  One CTA per SM takes a run of units with
@@ -87,14 +88,16 @@ constexpr int kNone = 255;
 __host__ __device__ constexpr int accs_for(int nd) { return nd == oz::kDigits64 ? oz::kAccs64 : (int)oz::kAccs; }
 __host__ __device__ constexpr int chunk_for(int nd) { return nd == oz::kDigits64 ? 128 : kChunk; }
 __host__ __device__ constexpr int tbufs_for(int nd, int np) { return 2 * accs_for(nd) * np <= 512 ? 2 : 1; }
-__host__ __device__ constexpr int overlap_stage(int nd, int np) { return nd * np * kStage * 2; }
-constexpr int kOverlapTail = kRows * kStage * 2;    // A's reads past the last plane
-__host__ __device__ constexpr int overlap_bufs(int nd, int np) {
-    return (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np) >= 6
-               ? 6 : (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np);
+__host__ __device__ constexpr int overlap_stage(int nd, int np, bool two) {
+    return (two ? 2 : 1) * nd * np * kStage * 2;
 }
-__host__ __device__ constexpr size_t overlap_smem(int nd, int np) {
-    return (size_t)overlap_bufs(nd, np) * overlap_stage(nd, np) + kOverlapTail + 128;
+constexpr int kOverlapTail = kRows * kStage * 2;    // A's reads past the last plane
+__host__ __device__ constexpr int overlap_bufs(int nd, int np, bool two) {
+    return (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np, two) >= 6
+               ? 6 : (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np, two);
+}
+__host__ __device__ constexpr size_t overlap_smem(int nd, int np, bool two) {
+    return (size_t)overlap_bufs(nd, np, two) * overlap_stage(nd, np, two) + kOverlapTail + 128;
 }
 
 __device__ __forceinline__ bool wait_warp(uint64_t* mbar, uint32_t parity) {
@@ -105,18 +108,20 @@ __device__ __forceinline__ void arrive_warp(uint64_t* mbar, int lane) {
     if (lane == 0) tc::mbar_arrive(mbar);
 }
 
-template <int ND, int NP>
+// psi_k = psi[list[off + k]], z_l = z[b nbmax + l]; part[chunk of b][k ldo + l].
+template <int ND, int NP, bool kTwo>
 __global__ void __launch_bounds__(kRoleThreads, 1)
-k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
-                const int* __restrict__ ordered, int nbmax, long V4, int nchunk, int nunits,
+k_gs_overlap_tc(const double* __restrict__ psi, const double* __restrict__ z, BlockIdx bi,
+                const int* __restrict__ list, int nbmax, long V4, int nchunk, int nunits,
                 double* __restrict__ part, int* __restrict__ status) {
-    constexpr int NACC = accs_for(ND), NBUF = overlap_bufs(ND, NP), NTB = tbufs_for(ND, NP);
-    constexpr int CH = chunk_for(ND), kPlane = NP * kStage * 2, kBuf = overlap_stage(ND, NP);
+    constexpr int NACC = accs_for(ND), NBUF = overlap_bufs(ND, NP, kTwo), NTB = tbufs_for(ND, NP);
+    constexpr int CH = chunk_for(ND), kPlane = NP * kStage * 2, kBuf = overlap_stage(ND, NP, kTwo);
+    constexpr int kArr = kTwo ? 2 : 1;
     constexpr int kPasses = (NP + 63) / 64;   // rows of a slicer: row0, row0 + 64
     extern __shared__ uint8_t smraw[];
     __shared__ __align__(8) uint64_t full[6], empty[6], fullT[2], emptyT[2], expReady[8];
     __shared__ uint32_t tmem_slot;
-    __shared__ int sE[8][NP];   // of the last units
+    __shared__ int sE[8][kArr * NP];   // of the last units
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t s0a = tc::smem_u32(smraw);
     uint8_t* base = smraw + ((128u - (s0a & 127u)) & 127u);
@@ -145,8 +150,8 @@ k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
     // units of empty blocks are passed over by every role
     const auto stages_of = [&](int unit, int& b, int& s0, int& nb, long& p0, int& npts) {
         b = unit / nchunk;
-        s0 = starts[b];
-        nb = starts[b + 1] - s0;
+        s0 = bi.off(b);
+        nb = bi.nb(b);
         p0 = (long)(unit - b * nchunk) * CH;
         npts = (int)min((long)CH, V4 - p0);
         return nb > 0 ? (npts + kStage - 1) / kStage : 0;
@@ -161,63 +166,73 @@ k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
         for (int unit = u0, k = 0; unit < u1 && ok; ++unit) {
             const int nst = stages_of(unit, b, s0, nb, p0, npts);
             if (nst == 0) continue;
-            const double* src[kPasses];
-            int emax[kPasses];
+            const double* src[kArr][kPasses];
+            int emax[kArr][kPasses];
 #pragma unroll
-            for (int r = 0; r < kPasses; ++r) {
-                const int row = row0 + 64 * r;
-                src[r] = row < nb ? psi + (long)ordered[s0 + row] * V4 + p0 : nullptr;
-                emax[r] = 0;
-                if (src[r])
-                    for (int s = 0; s < nst; ++s) {
+            for (int y = 0; y < kArr; ++y)
 #pragma unroll
-                        for (int h = 0; h < 8; ++h) {
-                            const int q = s * kStage + 8 * g + h;
-                            if (q < npts) emax[r] = max(emax[r], oz::bexp(src[r][q]));
+                for (int r = 0; r < kPasses; ++r) {
+                    const int row = row0 + 64 * r;
+                    src[y][r] = row >= nb ? nullptr
+                                : y == 0  ? psi + (long)list[s0 + row] * V4 + p0
+                                          : z + ((long)b * nbmax + row) * V4 + p0;
+                    int e = 0;
+                    if (src[y][r])
+                        for (int s = 0; s < nst; ++s) {
+#pragma unroll
+                            for (int h = 0; h < 8; ++h) {
+                                const int q = s * kStage + 8 * g + h;
+                                if (q < npts) e = max(e, oz::bexp(src[y][r][q]));
+                            }
                         }
-                    }
-                emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 1));
-                emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 2));
-            }
+                    e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+                    emax[y][r] = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+                }
             // (the epilogue of unit k - 8 has read its slot: the ring's stages and the
             // accumulators let the slicers run at most five units ahead)
 #pragma unroll
-            for (int r = 0; r < kPasses; ++r)
-                if (src[r] && g == 0) sE[k & 7][row0 + 64 * r] = emax[r];
+            for (int y = 0; y < kArr; ++y)
+#pragma unroll
+                for (int r = 0; r < kPasses; ++r)
+                    if (src[y][r] && g == 0) sE[k & 7][y * NP + row0 + 64 * r] = emax[y][r];
             arrive_warp(&expReady[k & 7], lane);
             ++k;
             for (int s = 0; s < nst; ++s, ++stage) {
                 const int buf = stage % NBUF;
-                double v[kPasses][8];
-#pragma unroll
-                for (int r = 0; r < kPasses; ++r)
-#pragma unroll
-                    for (int h = 0; h < 8; ++h) {
-                        const int q = s * kStage + 8 * g + h;
-                        v[r][h] = src[r] && q < npts ? src[r][q] : 0.0;
-                    }
-                if (stage >= NBUF) {
-                    ok = wait_warp(&empty[buf], ((stage - NBUF) / NBUF) & 1);
-                    if (!ok) break;
-                }
                 uint8_t* planes = base + buf * kBuf;
 #pragma unroll
-                for (int r = 0; r < kPasses; ++r) {
-                    const int row = row0 + 64 * r;
-                    if (row >= NP) continue;
-                    const oz::FixedRow<ND> fixed(emax[r]);
+                for (int y = 0; y < kArr; ++y) {
+                    double v[kPasses][8];
 #pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        const double v4[4] = {v[r][4 * h], v[r][4 * h + 1], v[r][4 * h + 2],
-                                              v[r][4 * h + 3]};
-                        uint2 w[ND];
-                        oz::digits4<ND>(v4, fixed, w);
+                    for (int r = 0; r < kPasses; ++r)
 #pragma unroll
-                        for (int a = 0; a < ND; ++a)
-                            *reinterpret_cast<uint2*>(planes + a * kPlane +
-                                                      tc::kmajor_off(row, 8 * g + 4 * h)) = w[a];
+                        for (int h = 0; h < 8; ++h) {
+                            const int q = s * kStage + 8 * g + h;
+                            v[r][h] = src[y][r] && q < npts ? src[y][r][q] : 0.0;
+                        }
+                    if (y == 0 && stage >= NBUF) {
+                        ok = wait_warp(&empty[buf], ((stage - NBUF) / NBUF) & 1);
+                        if (!ok) break;
+                    }
+#pragma unroll
+                    for (int r = 0; r < kPasses; ++r) {
+                        const int row = row0 + 64 * r;
+                        if (row >= NP) continue;
+                        const oz::FixedRow<ND> fixed(emax[y][r]);
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const double v4[4] = {v[r][4 * h], v[r][4 * h + 1], v[r][4 * h + 2],
+                                                  v[r][4 * h + 3]};
+                            uint2 w[ND];
+                            oz::digits4<ND>(v4, fixed, w);
+#pragma unroll
+                            for (int a = 0; a < ND; ++a)
+                                *reinterpret_cast<uint2*>(planes + (y * ND + a) * kPlane +
+                                                          tc::kmajor_off(row, 8 * g + 4 * h)) = w[a];
+                        }
                     }
                 }
+                if (!ok) break;
                 tc::fence_proxy_async();
                 arrive_warp(&full[buf], lane);
             }
@@ -238,7 +253,8 @@ k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
                     tc::fence_after();
                     const uint32_t pa = tc::smem_u32(base + buf * kBuf);
                     oz::issue_stacked<ND, NACC, NP, kStage / 16>(
-                        tmem + (uint32_t)(tb * NACC * NP), pa, kPlane, pa, tc::kSbo, s > 0);
+                        tmem + (uint32_t)(tb * NACC * NP), pa, kPlane,
+                        kTwo ? pa + ND * kPlane : pa, tc::kSbo, s > 0);
                     tc::commit(&empty[buf]);
                 }
                 if (!ok) break;
@@ -267,8 +283,9 @@ k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
             const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) +
                                   (uint32_t)(tb * NACC * NP + 8 * colh);
             double* out = part + (long)unit * nbmax * nbmax;
-            const int* se = sE[k & 7];
-            const int ek = kr < nb ? se[kr] : 0;
+            const int* se = sE[k & 7] + (kTwo ? NP : 0);   // of the columns
+            const int ldo = kTwo ? nb : nbmax;
+            const int ek = kr < nb ? sE[k & 7][kr] : 0;
             // rows past the block have nothing to write
             const int nch = quarter * 32 < nb ? (nb - 8 * colh + 15) / 16 : 0;
 #pragma unroll 1
@@ -284,7 +301,7 @@ k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     const int l = l0 + u;
-                    if (l >= nb || l < kr) continue;
+                    if (l >= nb || (!kTwo && l < kr)) continue;
                     double val;
                     if constexpr (ND == oz::kDigits64) {
                         uint32_t acc[NACC];
@@ -299,7 +316,7 @@ k_gs_overlap_tc(const double* __restrict__ psi, const int* __restrict__ starts,
                                                    __uint_as_float(r[2][u]), __uint_as_float(r[3][u]));
                         val = (f2d_bits(o.h) + f2d_bits(o.l)) * pow2d(ek - 1023 + se[l] - 1023 - 12);
                     }
-                    out[kr * nbmax + l] = val;
+                    out[kr * ldo + l] = val;
                 }
             }
             tc::fence_before();
@@ -813,6 +830,7 @@ __global__ void k_gaps_sum(const double* __restrict__ gpart, const int* __restri
 // in double-float, as k_pair_field (pairing.cu) forms it; part[b][0|1][V].
 // Four lanes per point (spinors i = sub, sub + 4, ...), combined by a fixed
 // shuffle order.
+template <bool kF64>
 __global__ void __launch_bounds__(256)
 k_field_contract(const double* __restrict__ Y, const double* __restrict__ psi,
                  const int* __restrict__ members, const int* __restrict__ hsz, int hmax, long V,
@@ -820,6 +838,30 @@ k_field_contract(const double* __restrict__ Y, const double* __restrict__ psi,
     const int b = blockIdx.y, h = hsz[b];
     const long v = (long)blockIdx.x * (blockDim.x / 4) + threadIdx.x / 4;
     const int sub = threadIdx.x & 3;
+    if constexpr (kF64) {
+        double fr = 0.0, fi = 0.0;
+        for (int i = sub; i < h && v < V; i += 4) {
+            const double* y = Y + (long)(b * hmax + i) * 4 * V + v;
+            const double* p = psi + (long)members[b * hmax + i] * 4 * V + v;
+            const double y0 = y[0], y1 = y[V], y2 = y[2 * V], y3 = y[3 * V];
+            const double a0 = p[0], a1 = p[V], a2 = p[2 * V], a3 = p[3 * V];
+            fr = fma(y0, a0, fr);
+            fr = fma(y1, a1, fr);
+            fr = fma(y2, a2, fr);
+            fr = fma(y3, a3, fr);
+            fi = fi - (y0 * a1 - y1 * a0 + y2 * a3 - y3 * a2);
+        }
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            fr += __shfl_xor_sync(0xffffffffu, fr, o);
+            fi += __shfl_xor_sync(0xffffffffu, fi, o);
+        }
+        if (sub == 0 && v < V) {
+            part[((long)b * 2 + 0) * V + v] = fr;
+            part[((long)b * 2 + 1) * V + v] = fi;
+        }
+        return;
+    }
     float rh = 0.f, rl = 0.f, ih = 0.f, il = 0.f;
     for (int i = sub; i < h && v < V; i += 4) {
         const double* y = Y + (long)(b * hmax + i) * 4 * V + v;
@@ -849,6 +891,26 @@ k_field_contract(const double* __restrict__ Y, const double* __restrict__ psi,
         part[((long)b * 2 + 0) * V + v] = df_to_fast(re);
         part[((long)b * 2 + 1) * V + v] = df_to_fast(im);
     }
+}
+
+// The gaps' right factors in FP64, as k_pair_gaps (pairing.cu) forms them:
+// Z_j0 = -Fr psi_j0 + Fi psi_j1, Z_j1 = -Fi psi_j0 - Fr psi_j1 (same for 2, 3), to
+// z[b hmax + j].
+__global__ void __launch_bounds__(128)
+k_gaps_factor(const double* __restrict__ psi, const int* __restrict__ members,
+              const int* __restrict__ hsz, int hmax, const double* __restrict__ fre,
+              const double* __restrict__ fim, long V, double* __restrict__ z) {
+    const int b = blockIdx.z, j = blockIdx.y, it = b / 2;
+    const long v = (long)blockIdx.x * 128 + threadIdx.x;
+    if (j >= hsz[b] || v >= V) return;
+    const double* a = psi + (long)members[b * hmax + j] * 4 * V + v;
+    double* o = z + ((long)b * hmax + j) * 4 * V + v;
+    const double r = fre[it * V + v], m = fim[it * V + v];
+    const double a0 = a[0], a1 = a[V], a2 = a[2 * V], a3 = a[3 * V];
+    o[0] = fma(m, a1, -r * a0);
+    o[V] = fma(-m, a0, -r * a1);
+    o[2 * V] = fma(m, a3, -r * a2);
+    o[3 * V] = fma(-m, a2, -r * a3);
 }
 
 }  // namespace
@@ -885,16 +947,15 @@ bool gs_tc_prepare(mg_ctx* c, bool f64) {
     return true;
 }
 
-template <int ND, int NP>
-static int overlap_launch(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered,
-                          int nchunk) {
-    MG_CUDA(cudaFuncSetAttribute(k_gs_overlap_tc<ND, NP>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)overlap_smem(ND, NP)));
-    const int nunits = nchunk * c->gs_nblk;
-    k_gs_overlap_tc<ND, NP><<<std::min(c->num_sms, nunits), kRoleThreads, overlap_smem(ND, NP),
-                              c->stream>>>(psi, d_lists, d_ordered, c->gs_nbmax, 4 * c->V, nchunk,
-                                           nunits, c->gs_Stc, c->tc_status);
+template <int ND, int NP, bool kTwo>
+static int overlap_launch(mg_ctx* c, const double* psi, const double* z, BlockIdx bi,
+                          const int* list, int nblk, int nbmax, int nchunk, double* part) {
+    const auto kernel = k_gs_overlap_tc<ND, NP, kTwo>;
+    constexpr size_t sm = overlap_smem(ND, NP, kTwo);
+    MG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    const int nunits = nchunk * nblk;
+    kernel<<<std::min(c->num_sms, nunits), kRoleThreads, sm, c->stream>>>(
+        psi, z, bi, list, nbmax, 4 * c->V, nchunk, nunits, part, c->tc_status);
     MG_LAUNCHED(c);
     return MG_OK;
 }
@@ -903,17 +964,20 @@ static int overlap_launch(mg_ctx* c, const double* psi, const int* d_lists, cons
 int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d_ordered, bool f64,
                   int* nchunk) {
     *nchunk = div_up(4 * c->V, chunk_for(f64 ? oz::kDigits64 : kDigits));
-    const auto run = [&](auto launch) { return launch(c, psi, d_lists, d_ordered, *nchunk); };
+    const auto run = [&](auto launch) {
+        return launch(c, psi, nullptr, BlockIdx{d_lists, nullptr, 0}, d_ordered, c->gs_nblk,
+                      c->gs_nbmax, *nchunk, c->gs_Stc);
+    };
     const int steps = std::max(1, div_up(c->gs_nbmax, 16));
-    if (f64) return steps <= 2   ? run(overlap_launch<oz::kDigits64, 32>)
-                    : steps == 3 ? run(overlap_launch<oz::kDigits64, 48>)
-                                 : run(overlap_launch<oz::kDigits64, 64>);
+    if (f64) return steps <= 2   ? run(overlap_launch<oz::kDigits64, 32, false>)
+                    : steps == 3 ? run(overlap_launch<oz::kDigits64, 48, false>)
+                                 : run(overlap_launch<oz::kDigits64, 64, false>);
     switch (steps) {
-        case 1: return run(overlap_launch<kDigits, 16>);
-        case 2: return run(overlap_launch<kDigits, 32>);
-        case 3: return run(overlap_launch<kDigits, 48>);
-        case 4: return run(overlap_launch<kDigits, 64>);
-        default: return run(overlap_launch<kDigits, 80>);
+        case 1: return run(overlap_launch<kDigits, 16, false>);
+        case 2: return run(overlap_launch<kDigits, 32, false>);
+        case 3: return run(overlap_launch<kDigits, 48, false>);
+        case 4: return run(overlap_launch<kDigits, 64, false>);
+        default: return run(overlap_launch<kDigits, 80, false>);
     }
 }
 
@@ -1005,25 +1069,53 @@ int gaps_tc(mg_ctx* c, double* gsum) {
 
 // Pairing-field partials of the four blocks: Y = block apply of Ktilde
 // (tensor cores) into the scratch basis, then the pointwise contraction.
-int pair_field_tc(mg_ctx* c) {
+int pair_field_tc(mg_ctx* c, bool f64) {
     Hfb& H = c->hfb;
-    if (!c->tc_mesh_ok || H.hmax > kMeshTcMax) return MG_ERR_STATE;
+    if (!mesh_tc_serves(c, H.hmax, f64)) return MG_ERR_STATE;
     const long V = c->V;
     if (c->field_y == nullptr) {
         MG_CUDA(cudaMalloc(&c->field_y, (size_t)4 * H.hmax * 4 * V * sizeof(double)));
-        MG_CUDA(cudaMalloc(&c->field_xd, (size_t)4 * kDigits * kXdStride * sizeof(uint16_t)));
-        MG_CUDA(cudaMemset(c->field_xd, 0, (size_t)4 * kDigits * kXdStride * sizeof(uint16_t)));
+        MG_CUDA(cudaMalloc(&c->field_xd, (size_t)4 * oz::kDigits64 * kXdStride * sizeof(uint16_t)));
         MG_CUDA(cudaMalloc(&c->field_xe, (size_t)4 * kMeshTcMax * sizeof(int)));
         MG_CUDA(cudaMalloc(&c->field_ybase, 4 * sizeof(int)));
         const int yb[4] = {0, H.hmax, 2 * H.hmax, 3 * H.hmax};
         MG_CUDA(cudaMemcpy(c->field_ybase, yb, sizeof(yb), cudaMemcpyHostToDevice));
     }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
-    MG_TRY(apply_tc(c, 4, H.hmax, false, H.ktil, (long)H.hmax * H.hmax, 0, bi,
+    MG_TRY(apply_tc(c, 4, H.hmax, f64, H.ktil, (long)H.hmax * H.hmax, 0, bi,
                     c->bas[MG_HF_BASIS].psi, c->field_y, nullptr, H.members, nullptr,
                     c->field_ybase, c->field_xd, c->field_xe));
-    k_field_contract<<<dim3(div_up(V, 64), 4), 256, 0, c->stream>>>(
+    const auto contract = f64 ? k_field_contract<true> : k_field_contract<false>;
+    contract<<<dim3(div_up(V, 64), 4), 256, 0, c->stream>>>(
         c->field_y, c->bas[MG_HF_BASIS].psi, H.members, H.hsz, H.hmax, V, H.fpart);
+    MG_LAUNCHED(c);
+    return MG_OK;
+}
+
+// The same in the FP64 form, behind pair_field_tc, whose scratch basis takes the
+// factors Z.  Pairing field and gaps of 108 spwfs at 18^3 (blocks of 26 and 28): 136
+// and 152 us by FP64 FMAs, here 65 and 100.
+int gaps_tc64(mg_ctx* c, double* gsum) {
+    Hfb& H = c->hfb;
+    if (!mesh_tc_serves(c, H.hmax, true) || c->field_y == nullptr) return MG_ERR_STATE;
+    const long V = c->V;
+    const int nchunk = div_up(4 * V, chunk_for(oz::kDigits64));
+    if (c->gap_part64 == nullptr)
+        MG_CUDA(cudaMalloc(&c->gap_part64, (size_t)4 * nchunk * H.hmax * H.hmax * sizeof(double)));
+    const double* psi = c->bas[MG_HF_BASIS].psi;
+    k_gaps_factor<<<dim3(div_up(V, 128), H.hmax, 4), 128, 0, c->stream>>>(
+        psi, H.members, H.hsz, H.hmax, H.fre, H.fim, V, c->field_y);
+    MG_LAUNCHED(c);
+    const auto run = [&](auto launch) {
+        return launch(c, psi, c->field_y, BlockIdx{nullptr, H.hsz, H.hmax}, H.members, 4, H.hmax,
+                      nchunk, c->gap_part64);
+    };
+    const int steps = div_up(H.hmax, 16);
+    MG_TRY(steps <= 2   ? run(overlap_launch<oz::kDigits64, 32, true>)
+           : steps == 3 ? run(overlap_launch<oz::kDigits64, 48, true>)
+                        : run(overlap_launch<oz::kDigits64, 64, true>));
+    k_gaps_sum<<<dim3(div_up((long)H.hmax * H.hmax, 8), 4), 256, 0, c->stream>>>(
+        c->gap_part64, H.hsz, H.hmax, nchunk, gsum);
     MG_LAUNCHED(c);
     return MG_OK;
 }

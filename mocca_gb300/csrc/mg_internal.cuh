@@ -279,6 +279,7 @@ struct mg_ctx {
     int* can_xe = nullptr;
     double* gap_part = nullptr;   // tensor-core gaps: partials per 64-point chunk
     double* field_y = nullptr;    // tensor-core pairing field: Y = Psi Ktilde per block (4 hmax x 4V)
+    double* gap_part64 = nullptr;
     uint16_t* field_xd = nullptr;
     int* field_xe = nullptr;
     int* field_ybase = nullptr;   // first row of each block in field_y
@@ -417,7 +418,8 @@ int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const i
                 bool f64);
 int can_transform_tc(mg_ctx* c, bool f64);
 int gaps_tc(mg_ctx* c, double* gsum);
-int pair_field_tc(mg_ctx* c);
+int gaps_tc64(mg_ctx* c, double* gsum);
+int pair_field_tc(mg_ctx* c, bool f64);
 int densities(mg_ctx* c);
 int moments(mg_ctx* c);
 int coulomb_setup(mg_ctx* c);

@@ -430,22 +430,23 @@ int pairing_mesh(mg_ctx* c) {
     MG_LAUNCHED(c);
     const size_t sm_f = (size_t)(hmax * hmax + hmax * 4 * kPts + 2 * kThreads) * sizeof(double);
     const bool mixed = c->cur_precision == MG_MIXED;
-    if (mixed && c->tc_mesh_ok && hmax <= kMeshTcMax)
-        MG_TRY(pair_field_tc(c));   // tensor cores (meshgemm_tc.cu)
+    const bool tensor = mesh_tc_serves(c, hmax, !mixed);   // meshgemm_tc.cu
+    if (tensor)
+        MG_TRY(pair_field_tc(c, !mixed));
     else if (mixed)
         k_pair_field_df<<<dim3(div_up(V, kPts), 4), kThreads, sm_f, c->stream>>>(
             B.psi, H.members, H.hsz, hmax, H.ktil, V, H.fpart);
     else
         k_pair_field<<<dim3(div_up(V, kPts), 4), kThreads, sm_f, c->stream>>>(
             B.psi, H.members, H.hsz, hmax, H.ktil, V, H.fpart);
-    if (!(mixed && c->tc_mesh_ok && hmax <= kMeshTcMax)) MG_LAUNCHED(c);
+    if (!tensor) MG_LAUNCHED(c);
     k_pair_field_finish<<<div_up(2 * V, kThreads), kThreads, 0, c->stream>>>(H.fpart, H.dfac, V,
                                                                            H.fre, H.fim);
     MG_LAUNCHED(c);
     const size_t sm_g = (size_t)(2 * hmax * (4 * kGPts + 1) + hmax * hmax) * sizeof(double);
-    if (mixed && c->tc_mesh_ok && hmax <= kMeshTcMax) {
-        // tensor cores (meshgemm_tc.cu): the summed partials go to chunk slot 0
-        MG_TRY(gaps_tc(c, H.gpart));
+    if (tensor) {
+        // the summed partials go to chunk slot 0
+        MG_TRY(mixed ? gaps_tc(c, H.gpart) : gaps_tc64(c, H.gpart));
         k_gaps_finish<<<dim3(div_up(nmax * nmax, 128), 4), 128, 0, c->stream>>>(
             H.gpart, H.members, H.hsz, hmax, nmax, 1, H.pcut, c->dv, H.delta);
         MG_LAUNCHED(c);
