@@ -6,8 +6,7 @@
 // Blocks of up to kMeshTcMax (80) spinors in the mixed form, kMeshTcMin64 to
 // kMeshTcMax64 (24 to 64) in the FP64 form, whose results are rounded once to FP64
 // (norm-wise errors of the Gram-Schmidt of blocks of 22 to 50, mean over the spinors:
-// 1.27e-16 to 1.49e-16, with FP64 FMAs 1.31e-16 to 1.59e-16).  Above 64, four
-// accumulators take 512 TMEM columns and the gaps kernel runs one CTA per SM.
+// 1.27e-16 to 1.49e-16, with FP64 FMAs 1.31e-16 to 1.59e-16).
 //
 // Gram-Schmidt (gs.cu; GramSchmidt, src/SpwfStorage.f90:372-480, as
 // Q = Psi R^{-1} with S = R^T R per (isospin, parity, signature) block in
@@ -45,13 +44,7 @@ using oz::kDigits;
 constexpr int kRows = 128;            // MMA M
 constexpr int kChunk = 256;           // overlap points per CTA
 constexpr int kStage = 32;            // overlap points per MMA stage (K)
-constexpr int kStagePlane = kRows * kStage * 2;   // bytes of one digit plane of a stage
-// TMEM columns for four accumulators of N columns: 256 up to N = 64, 512 above
-// (one CTA per SM then; the launches keep the shared memory above half of the
-// SM's so that a second CTA never waits in tcgen05.alloc)
-__host__ __device__ constexpr uint32_t tmem_cols(int N) { return 4 * N <= 256 ? 256u : 512u; }
 constexpr long kXdStride = (long)kMeshTcMax * kMeshTcMax;   // per block in the coefficient planes
-constexpr size_t kOneCtaSmem = 116 * 1024;
 constexpr long long kWaitCycles = 4000000000LL;
 
 // Block sizes and list offsets: Gram-Schmidt blocks come from a start table,
@@ -93,8 +86,9 @@ __host__ __device__ constexpr int overlap_stage(int nd, int np, bool two) {
 }
 constexpr int kOverlapTail = kRows * kStage * 2;    // A's reads past the last plane
 __host__ __device__ constexpr int overlap_bufs(int nd, int np, bool two) {
-    return (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np, two) >= 6
-               ? 6 : (kSmemCap - 128 - kOverlapTail) / overlap_stage(nd, np, two);
+    // (8 KB left for the kernels' static shared memory)
+    return (kSmemCap - 8192 - 128 - kOverlapTail) / overlap_stage(nd, np, two) >= 6
+               ? 6 : (kSmemCap - 8192 - 128 - kOverlapTail) / overlap_stage(nd, np, two);
 }
 __host__ __device__ constexpr size_t overlap_smem(int nd, int np, bool two) {
     return (size_t)overlap_bufs(nd, np, two) * overlap_stage(nd, np, two) + kOverlapTail + 128;
@@ -640,169 +634,234 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
 // stage s covers 8 points, K group c = component c.  A rows are the spinors
 // (one power of two per spinor and chunk), B rows their Z, formed in
 // double-float and cut into digits through the fixed-point form with the
-// exponent bound 2 max|F| max|psi_j| of the chunk.  One plane buffer per
-// stage, two CTAs per SM.
+// exponent bound 2 max|F| max|psi_j| of the chunk.  Units, roles and rings as in
+// k_gs_overlap_tc.  160 spwfs of 24^3 (blocks of 40): 225 us with a CTA per chunk and
+// its stages one after the other, now 178 (298 with eight slicer warps).
 constexpr int kGapPts = 64;
+constexpr int kGapSlicers = 16;   // forming and cutting Z is most of the work
+constexpr int kGapThreads = 32 * (kRoleWarps + kGapSlicers + 1);
 
-__global__ void __launch_bounds__(256, 2)
+template <int NP>
+__global__ void __launch_bounds__(kGapThreads, 1)
 k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
           const int* __restrict__ hsz, int hmax, const double* __restrict__ fre,
           const double* __restrict__ fim, long V, int nchunk, double* __restrict__ gpart,
           int* __restrict__ status) {
+    constexpr int NACC = oz::kAccs, NBUF = overlap_bufs(kDigits, NP, true),
+                  NTB = tbufs_for(kDigits, NP);
+    constexpr int kPlane = NP * kStage * 2, kBuf = 2 * kDigits * kPlane, nst = kGapPts / 8;
+    constexpr int kPasses = (NP + 63) / 64;   // rows of a slicer: row0, row0 + 64
     extern __shared__ uint8_t smraw[];
-    __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(8) uint64_t full[6], empty[6], fullT[2], emptyT[2], expReady[8];
     __shared__ uint32_t tmem_slot;
-    __shared__ int sE[kRows], sEz[kRows], sFe[kGapPts];
-    __shared__ float4 sF[kGapPts];   // (Fr hi, Fr lo, Fi hi, Fi lo)
-    const int b = blockIdx.y, it = b >> 1, chunk = blockIdx.x;
-    const int h = hsz[b];
-    if (h == 0) return;
-    const int N = max(16, (h + 15) / 16 * 16);
-    const uint32_t tcols = tmem_cols(N);
+    __shared__ int sE[8][2 * NP];      // of the last units: psi, then Z
+    __shared__ int sFe[2][kGapPts];
+    __shared__ float4 sF[2][kGapPts];  // (Fr hi, Fr lo, Fi hi, Fi lo)
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    // rows row0 and row0 + 64 (blocks above 64 spinors), component c
-    const int row0 = tid >> 2, c = tid & 3;
-    const int bPlane = N * tc::kRowBytes;
-
     const uint32_t s0a = tc::smem_u32(smraw);
     uint8_t* base = smraw + ((128u - (s0a & 127u)) & 127u);
-    uint8_t* sA = base;                          // kDigits planes of 128 x 32
-    uint8_t* sB = sA + kDigits * kStagePlane;    // kDigits planes of N x 32
-    for (int t = tid; t < (kDigits * kStagePlane + kDigits * bPlane) / 16; t += 256)
+    for (int t = tid; t < (NBUF * kBuf + kOverlapTail) / 16; t += kGapThreads)
         reinterpret_cast<uint4*>(base)[t] = make_uint4(0u, 0u, 0u, 0u);
-    if (warp == 0) tc::alloc(&tmem_slot, tcols);
-    if (tid == 0) tc::mbar_init(&mbar, 1);
-    const long p0 = (long)chunk * kGapPts;
-    const int npts = (int)min((long)kGapPts, V - p0);
-    // the pairing field of the chunk, double-float, and its largest exponent
-    if (tid < kGapPts) {
-        double fr = 0.0, fi = 0.0;
-        if (tid < npts) {
-            fr = fre[(long)it * V + p0 + tid];
-            fi = fim[(long)it * V + p0 + tid];
+    if (warp == 0) tc::alloc(&tmem_slot, 512u);
+    if (tid == 0) {
+        for (int q = 0; q < NBUF; ++q) {
+            tc::mbar_init(&full[q], kGapSlicers);
+            tc::mbar_init(&empty[q], 1);
         }
-        const dfl a = df_split(fr), d = df_split(fi);
-        sF[tid] = make_float4(a.h, a.l, d.h, d.l);
-        sFe[tid] = max(oz::bexp(fr), oz::bexp(fi));
-    }
-    const int pc = c ^ 1;   // the partner component of Z
-    bool live[2];
-    const double *src[2], *srp[2];
-    int emax[2] = {0, 0}, ez[2];
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int row = row0 + 64 * r;
-        live[r] = row < h;
-        src[r] = live[r] ? psi + ((long)members[b * hmax + row] * 4 + c) * V + p0 : psi;
-        srp[r] = live[r] ? psi + ((long)members[b * hmax + row] * 4 + pc) * V + p0 : psi;
-        if (live[r])
-            for (int q = 0; q < npts; ++q) emax[r] = max(emax[r], oz::bexp(src[r][q]));
-        emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 1));
-        emax[r] = max(emax[r], __shfl_xor_sync(0xffffffffu, emax[r], 2));
-    }
-    __syncthreads();
-    int efmax = 0;
-    for (int q = 0; q < kGapPts; ++q) efmax = max(efmax, sFe[q]);
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        // |Z| <= |F| (|psi_c| + |psi_c'|) < 2^(E_F + E_psi + 3)
-        ez[r] = (emax[r] == 0 || efmax == 0) ? 0 : emax[r] + efmax - 1023 + 2;
-        if (live[r] && c == 0) {
-            sE[row0 + 64 * r] = emax[r];
-            sEz[row0 + 64 * r] = ez[r];
+        for (int q = 0; q < 2; ++q) {
+            tc::mbar_init(&fullT[q], 1);
+            tc::mbar_init(&emptyT[q], kRoleWarps);
         }
+        for (int q = 0; q < 8; ++q) tc::mbar_init(&expReady[q], kGapSlicers);
     }
+    tc::fence_proxy_async();
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
     const uint32_t tmem = tmem_slot;
-    const uint32_t idesc = tc::idesc_bf16(kRows, N);
+    const int nunits = 4 * nchunk;
+    const int u0 = (int)((long)nunits * blockIdx.x / gridDim.x);
+    const int u1 = (int)((long)nunits * (blockIdx.x + 1) / gridDim.x);
     bool ok = true;
-    const int nst = kGapPts / 8;
-    for (int s = 0; s < nst; ++s) {
-        if (s > 0) ok &= tc::mbar_wait(&mbar, (s - 1) & 1, kWaitCycles);
-#pragma unroll
-        for (int r = 0; r < 2; ++r) {
-            if (!live[r]) continue;
-            const int row = row0 + 64 * r;
-            double a[8];
-            long long zx[8];
-#pragma unroll
-            for (int hh = 0; hh < 8; ++hh) {
-                const int q = 8 * s + hh;
-                const bool in = q < npts;
-                a[hh] = in ? src[r][q] : 0.0;
-                const double ap = in ? srp[r][q] : 0.0;
-                const float4 f = sF[q];
-                const dfl fr = {f.x, f.y}, fi = {f.z, f.w};
-                const dfl ac = df_split(a[hh]), ao = df_split(ap);
-                // c even: Z = -Fr a_c + Fi a_c' ; c odd: Z = -Fi a_c' - Fr a_c
-                const dfl t1 = df_mul(fr, ac), t2 = df_mul(fi, ao);
-                const dfl z = (c & 1) ? df_neg(df_add(t1, t2)) : df_sub(t2, t1);
-                zx[hh] = ez[r] ? oz::fixed_f(z.h, ez[r]) + oz::fixed_f(z.l, ez[r]) : 0ll;
-            }
-            uint4 w[kDigits];
-            oz::digits8(a, emax[r], w);
-#pragma unroll
-            for (int d = 0; d < kDigits; ++d)
-                *reinterpret_cast<uint4*>(sA + d * kStagePlane + tc::kmajor_off(row, 8 * c)) = w[d];
-            oz::digits8_fixed(zx, w);
-#pragma unroll
-            for (int d = 0; d < kDigits; ++d)
-                *reinterpret_cast<uint4*>(sB + d * bPlane + tc::kmajor_off(row, 8 * c)) = w[d];
-        }
-        tc::fence_proxy_async();
-        tc::fence_before();
-        __syncthreads();
-        tc::fence_after();
-        if (tid == 0) {
-            oz::issue_pairs<2>(tmem, N, idesc, tc::smem_u32(sA), kStagePlane, tc::kSbo,
-                               tc::smem_u32(sB), bPlane, tc::kSbo, s > 0);
-            tc::commit(&mbar);
-        }
-    }
-    ok &= tc::mbar_wait(&mbar, (nst - 1) & 1, kWaitCycles);
-    ok = __syncthreads_and(ok) != 0;
-    tc::fence_after();
-    if (ok) {
-        const int quarter = warp & 3, colh = warp >> 2;
-        const int i = quarter * 32 + lane;
-        const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16);
-        double* out = gpart + ((long)b * nchunk + chunk) * hmax * hmax;
-        const int ei = i < h ? sE[i] - 1023 : 0;
-        for (int q = 0; q < N / 16; ++q) {
-            const int c0 = 16 * q + 8 * colh;
-            uint32_t r0[8], r1[8], r2[8], r3[8];
-            __syncwarp();
-            tc::ld8(trow + (uint32_t)(0 * N + c0), r0);
-            tc::ld8(trow + (uint32_t)(1 * N + c0), r1);
-            tc::ld8(trow + (uint32_t)(2 * N + c0), r2);
-            tc::ld8(trow + (uint32_t)(3 * N + c0), r3);
-            tc::wait_ld(r0);
-            tc::wait_ld(r1);
-            tc::wait_ld(r2);
-            tc::wait_ld(r3);
-            if (i >= h) continue;
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int j = c0 + u;
-                if (j >= h) break;
-                double val = 0.0;
-                if (sE[i] != 0 && sEz[j] != 0) {
-                    const dfl o = oz::combine4(__uint_as_float(r0[u]), __uint_as_float(r1[u]),
-                                               __uint_as_float(r2[u]), __uint_as_float(r3[u]));
-                    val = (f2d_bits(o.h) + f2d_bits(o.l)) * pow2d(ei + sEz[j] - 1023 - 12);
+    if (warp >= kRoleWarps && warp < kRoleWarps + kGapSlicers) {
+        // ------- slicers: rows row0 and row0 + 64, component c, half of the points -------
+        const int st = tid - 32 * kRoleWarps, row0 = st >> 3, c = (st >> 1) & 3, half = st & 1;
+        int stage = 0;
+        for (int unit = u0, k = 0; unit < u1 && ok; ++unit) {
+            const int b = unit / nchunk, it = b >> 1, h = hsz[b];
+            if (h == 0) continue;
+            const long p0 = (long)(unit - b * nchunk) * kGapPts;
+            const int npts = (int)min((long)kGapPts, V - p0);
+            // the pairing field of the chunk, double-float, and its largest exponent
+            if (st < kGapPts) {
+                double fr = 0.0, fi = 0.0;
+                if (st < npts) {
+                    fr = fre[(long)it * V + p0 + st];
+                    fi = fim[(long)it * V + p0 + st];
                 }
-                out[i * h + j] = val;
+                const dfl a = df_split(fr), d = df_split(fi);
+                sF[k & 1][st] = make_float4(a.h, a.l, d.h, d.l);
+                sFe[k & 1][st] = max(oz::bexp(fr), oz::bexp(fi));
+            }
+            const double *src[kPasses], *srp[kPasses];   // psi_c and its partner component
+            int emax[kPasses], ez[kPasses];
+#pragma unroll
+            for (int r = 0; r < kPasses; ++r) {
+                const int row = row0 + 64 * r;
+                const bool live = row < h;
+                const double* p = psi + (long)members[b * hmax + (live ? row : 0)] * 4 * V + p0;
+                src[r] = live ? p + c * V : nullptr;
+                srp[r] = p + (c ^ 1) * V;
+                int e = 0;
+                if (live)
+#pragma unroll 8
+                    for (int q = half; q < npts; q += 2) e = max(e, oz::bexp(src[r][q]));
+                e = max(e, __shfl_xor_sync(0xffffffffu, e, 1));
+                e = max(e, __shfl_xor_sync(0xffffffffu, e, 2));
+                emax[r] = max(e, __shfl_xor_sync(0xffffffffu, e, 4));
+            }
+            asm volatile("bar.sync 1, %0;" ::"n"(32 * kGapSlicers) : "memory");
+            int efmax = 0;
+            for (int q = 0; q < kGapPts; ++q) efmax = max(efmax, sFe[k & 1][q]);
+#pragma unroll
+            for (int r = 0; r < kPasses; ++r) {
+                // |Z| <= |F| (|psi_c| + |psi_c'|) < 2^(E_F + E_psi + 3)
+                ez[r] = (emax[r] == 0 || efmax == 0) ? 0 : emax[r] + efmax - 1023 + 2;
+                if (src[r] && c == 0 && half == 0) {
+                    sE[k & 7][row0 + 64 * r] = emax[r];
+                    sE[k & 7][NP + row0 + 64 * r] = ez[r];
+                }
+            }
+            arrive_warp(&expReady[k & 7], lane);
+            const float4* F = sF[k & 1];
+            ++k;
+            for (int s = 0; s < nst; ++s, ++stage) {
+                const int buf = stage % NBUF;
+                uint8_t* planes = base + buf * kBuf;
+                double a[kPasses][4], ap[kPasses][4];
+#pragma unroll
+                for (int r = 0; r < kPasses; ++r)
+#pragma unroll
+                    for (int hh = 0; hh < 4; ++hh) {
+                        const int q = 8 * s + 4 * half + hh;
+                        const bool in = src[r] && q < npts;
+                        a[r][hh] = in ? src[r][q] : 0.0;
+                        ap[r][hh] = in ? srp[r][q] : 0.0;
+                    }
+                if (stage >= NBUF) {
+                    ok = wait_warp(&empty[buf], ((stage - NBUF) / NBUF) & 1);
+                    if (!ok) break;
+                }
+#pragma unroll
+                for (int r = 0; r < kPasses; ++r) {
+                    const int row = row0 + 64 * r;
+                    if (row >= NP) continue;
+                    long long zx[4];
+#pragma unroll
+                    for (int hh = 0; hh < 4; ++hh) {
+                        const float4 f = F[8 * s + 4 * half + hh];
+                        const dfl fr = {f.x, f.y}, fi = {f.z, f.w};
+                        const dfl ac = df_split(a[r][hh]), ao = df_split(ap[r][hh]);
+                        // c even: Z = -Fr a_c + Fi a_c' ; c odd: Z = -Fi a_c' - Fr a_c
+                        const dfl t1 = df_mul(fr, ac), t2 = df_mul(fi, ao);
+                        const dfl z = (c & 1) ? df_neg(df_add(t1, t2)) : df_sub(t2, t1);
+                        zx[hh] = ez[r] ? oz::fixed_f(z.h, ez[r]) + oz::fixed_f(z.l, ez[r]) : 0ll;
+                    }
+                    uint2 w[kDigits];
+                    const uint32_t o = tc::kmajor_off(row, 8 * c + 4 * half);
+                    oz::digits4<kDigits>(a[r], oz::FixedRow<kDigits>(emax[r]), w);
+#pragma unroll
+                    for (int d = 0; d < kDigits; ++d)
+                        *reinterpret_cast<uint2*>(planes + d * kPlane + o) = w[d];
+                    oz::digits4_fixed(zx, w);
+#pragma unroll
+                    for (int d = 0; d < kDigits; ++d)
+                        *reinterpret_cast<uint2*>(planes + (kDigits + d) * kPlane + o) = w[d];
+                }
+                tc::fence_proxy_async();
+                arrive_warp(&full[buf], lane);
             }
         }
+    } else if (warp == kRoleWarps + kGapSlicers) {
+        // ---------------- MMA issue ----------------
+        if (lane == 0) {
+            int stage = 0, k = 0;
+            for (int unit = u0; unit < u1 && ok; ++unit) {
+                if (hsz[unit / nchunk] == 0) continue;
+                const int tb = k % NTB;
+                if (k >= NTB) ok = tc::mbar_wait(&emptyT[tb], ((k - NTB) / NTB) & 1, kWaitCycles);
+                for (int s = 0; s < nst && ok; ++s, ++stage) {
+                    const int buf = stage % NBUF;
+                    ok = tc::mbar_wait(&full[buf], (stage / NBUF) & 1, kWaitCycles);
+                    if (!ok) break;
+                    tc::fence_after();
+                    const uint32_t pa = tc::smem_u32(base + buf * kBuf);
+                    oz::issue_stacked<kDigits, NACC, NP, kStage / 16>(
+                        tmem + (uint32_t)(tb * NACC * NP), pa, kPlane, pa + kDigits * kPlane,
+                        tc::kSbo, s > 0);
+                    tc::commit(&empty[buf]);
+                }
+                if (!ok) break;
+                tc::commit(&fullT[tb]);
+                ++k;
+            }
+            // the last commit covers every MMA of this CTA (after a timeout: the
+            // buffers' last ones)
+            if (k > 0) ok &= tc::mbar_wait(&fullT[(k - 1) % NTB], ((k - 1) / NTB) & 1, kWaitCycles);
+            if (!ok && stage > 0)
+                tc::mbar_wait(&empty[(stage - 1) % NBUF], ((stage - 1) / NBUF) & 1, kWaitCycles);
+        }
+        __syncwarp();
     } else {
-        if (tid == 0) atomicExch(status, 1);
-        tc::mbar_wait(&mbar, 0, kWaitCycles);
+        // ---------------- epilogue: G[i][j], i = TMEM lane, j = column ----------------
+        const int quarter = warp & 3, colh = warp >> 2, i = quarter * 32 + lane;
+        for (int unit = u0, k = 0; unit < u1; ++unit) {
+            const int h = hsz[unit / nchunk];
+            if (h == 0) continue;
+            const int tb = k % NTB;
+            ok = wait_warp(&expReady[k & 7], (k >> 3) & 1);
+            if (ok) ok = wait_warp(&fullT[tb], (k / NTB) & 1);
+            if (!ok) break;
+            tc::fence_after();
+            const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) +
+                                  (uint32_t)(tb * NACC * NP + 8 * colh);
+            double* out = gpart + (long)unit * hmax * hmax;
+            const int ei = i < h ? sE[k & 7][i] : 0;
+            const int* sz = sE[k & 7] + NP;
+            const int nch = quarter * 32 < h ? (h - 8 * colh + 15) / 16 : 0;
+#pragma unroll 1
+            for (int c = 0; c < nch; ++c) {
+                const int l0 = 16 * c + 8 * colh;
+                uint32_t r[NACC][8];
+                __syncwarp();
+#pragma unroll
+                for (int q = 0; q < NACC; ++q) tc::ld8(trow + (uint32_t)(q * NP + 16 * c), r[q]);
+#pragma unroll
+                for (int q = 0; q < NACC; ++q) tc::wait_ld(r[q]);
+                if (i >= h) continue;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int j = l0 + u;
+                    if (j >= h) break;
+                    double val = 0.0;
+                    if (ei != 0 && sz[j] != 0) {
+                        const dfl o = oz::combine4(__uint_as_float(r[0][u]), __uint_as_float(r[1][u]),
+                                                   __uint_as_float(r[2][u]), __uint_as_float(r[3][u]));
+                        val = (f2d_bits(o.h) + f2d_bits(o.l)) * pow2d(ei - 1023 + sz[j] - 1023 - 12);
+                    }
+                    out[i * h + j] = val;
+                }
+            }
+            tc::fence_before();
+            arrive_warp(&emptyT[tb], lane);
+            ++k;
+        }
     }
+    ok = __syncthreads_and(ok) != 0;
+    if (!ok && tid == 0) atomicExch(status, 1);
     tc::fence_before();
     __syncthreads();
-    if (warp == 0) tc::dealloc(tmem, tcols);
+    if (warp == 0) tc::dealloc(tmem_slot, 512u);
 }
 
 // Chunk partials of the gaps summed per entry, one warp each (fixed order):
@@ -1041,26 +1100,33 @@ int can_transform_tc(mg_ctx* c, bool f64) {
                     nullptr, H.cstart, c->can_xd, c->can_xe);
 }
 
+template <int NP>
+static int gaps_launch(mg_ctx* c, int nchunk) {
+    Hfb& H = c->hfb;
+    constexpr size_t sm = overlap_smem(kDigits, NP, true);
+    MG_CUDA(cudaFuncSetAttribute(k_gaps_tc<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_gaps_tc<NP><<<std::min(c->num_sms, 4 * nchunk), kGapThreads, sm, c->stream>>>(
+        c->bas[MG_HF_BASIS].psi, H.members, H.hsz, H.hmax, H.fre, H.fim, c->V, nchunk, c->gap_part,
+        c->tc_status);
+    MG_LAUNCHED(c);
+    return MG_OK;
+}
+
 // Gaps partial sums of the four pairing blocks on the tensor cores into
 // gsum[b][i * h + j] (to be finished by k_gaps_finish with one chunk).
 int gaps_tc(mg_ctx* c, double* gsum) {
     Hfb& H = c->hfb;
-    if (!c->tc_mesh_ok || H.hmax > kMeshTcMax) return MG_ERR_STATE;
-    const long V = c->V;
-    const int nchunk = div_up(V, kGapPts);
-    if (c->gap_part == nullptr) {
+    if (!mesh_tc_serves(c, H.hmax, false)) return MG_ERR_STATE;
+    const int nchunk = div_up(c->V, kGapPts);
+    if (c->gap_part == nullptr)
         MG_CUDA(cudaMalloc(&c->gap_part, (size_t)4 * nchunk * H.hmax * H.hmax * sizeof(double)));
-        MG_CUDA(cudaFuncSetAttribute(k_gaps_tc, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     200 * 1024));
+    switch (std::max(1, div_up(H.hmax, 16))) {
+        case 1: MG_TRY(gaps_launch<16>(c, nchunk)); break;
+        case 2: MG_TRY(gaps_launch<32>(c, nchunk)); break;
+        case 3: MG_TRY(gaps_launch<48>(c, nchunk)); break;
+        case 4: MG_TRY(gaps_launch<64>(c, nchunk)); break;
+        default: MG_TRY(gaps_launch<80>(c, nchunk)); break;
     }
-    const int Np = std::max(16, (H.hmax + 15) / 16 * 16);
-    size_t sm = 128 + (size_t)kDigits * kStagePlane + (size_t)kDigits * Np * tc::kRowBytes;
-    // two CTAs per SM (2 x 256 TMEM columns), one above N = 64
-    sm = std::max(sm, tmem_cols(Np) > 256 ? kOneCtaSmem : (size_t)80 * 1024);
-    k_gaps_tc<<<dim3(nchunk, 4), 256, sm, c->stream>>>(c->bas[MG_HF_BASIS].psi, H.members, H.hsz,
-                                                      H.hmax, H.fre, H.fim, V, nchunk, c->gap_part,
-                                                      c->tc_status);
-    MG_LAUNCHED(c);
     k_gaps_sum<<<dim3(div_up((long)H.hmax * H.hmax, 8), 4), 256, 0, c->stream>>>(
         c->gap_part, H.hsz, H.hmax, nchunk, gsum);
     MG_LAUNCHED(c);

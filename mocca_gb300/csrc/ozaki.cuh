@@ -34,7 +34,6 @@ namespace oz {
 constexpr int kDigits = 6;                       // digits per operand entry
 constexpr int kCmax = 5;                         // largest kept digit weight a + b
 constexpr long long kDigitBias = 0x8080808080LL; // 128 in each of the five lower digits
-constexpr int kPairs = 21;                       // pairs with a + b <= kCmax
 constexpr uint32_t kAccs = 4;                    // accumulators per output
 
 // float bit pattern of (u - 128) * 2^(-8A) for byte u of w, selected by sel
@@ -51,23 +50,9 @@ __device__ __forceinline__ int bexp(double v) {
     return (int)(((unsigned long long)__double_as_longlong(v) >> 52) & 0x7FF);
 }
 
-// round(v * 2^f) for a row whose largest biased exponent is emax, with
-// f = 8 kDigits - 2 - (emax - 1023): |result| <= 2^47.  Zero and subnormal v
-// give 0, as do values 2^62 below the row's largest.
-__device__ __forceinline__ long long fixed(double v, int emax) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-    const int e = (int)((b >> 52) & 0x7FF);
-    const int sh = (54 - 8 * kDigits) + (emax - e);   // >= 6
-    long long X = 0;
-    if (e != 0 && sh < 62) {
-        const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-        X = (long long)((m + (1ull << (sh - 1))) >> sh);
-        if (b >> 63) X = -X;
-    }
-    return X;
-}
-
-// The same fixed-point value of a float (part of a double-float), exact when
+// A row's entries become signed integers round(v * 2^f), f = 8 kDigits - 2 -
+// (emax - 1023) for its largest biased exponent emax: |result| <= 2^47 (FixedRow).
+// The fixed-point value of a float (part of a double-float), exact when
 // the float's bits lie above 2^-f, rounded otherwise.
 __device__ __forceinline__ long long fixed_f(float v, int emax) {
     const uint32_t u = __float_as_uint(v);
@@ -99,18 +84,12 @@ __device__ __forceinline__ void digits_fixed(long long X, uint32_t (&d)[kDigits]
     d[5] = low_digit<5>(ylo, 0x7540);
 }
 
-// The pre-scaled digits of v (top digit first) for a row whose largest
-// biased exponent is emax.
-__device__ __forceinline__ void digits(double v, int emax, uint32_t (&d)[kDigits]) {
-    digits_fixed(fixed(v, emax), d);
-}
-
-// Digits of 8 fixed-point values of a row as one 16-byte core-matrix row per
-// digit plane.
-__device__ __forceinline__ void digits8_fixed(const long long (&X)[8], uint4 (&w)[kDigits]) {
-    uint32_t x[kDigits][4];
+// Digits of 4 fixed-point values of a row as one 8-byte half of a core-matrix row
+// per digit plane.
+__device__ __forceinline__ void digits4_fixed(const long long (&X)[4], uint2 (&w)[kDigits]) {
+    uint32_t x[kDigits][2];
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
+    for (int h = 0; h < 2; ++h) {
         uint32_t d0[kDigits], d1[kDigits];
         digits_fixed(X[2 * h], d0);
         digits_fixed(X[2 * h + 1], d1);
@@ -118,23 +97,7 @@ __device__ __forceinline__ void digits8_fixed(const long long (&X)[8], uint4 (&w
         for (int a = 0; a < kDigits; ++a) x[a][h] = __byte_perm(d0[a], d1[a], 0x7632);
     }
 #pragma unroll
-    for (int a = 0; a < kDigits; ++a) w[a] = make_uint4(x[a][0], x[a][1], x[a][2], x[a][3]);
-}
-
-// Digits of 8 consecutive values of a row, packed as one 16-byte core-matrix
-// row per digit plane.
-__device__ __forceinline__ void digits8(const double (&v)[8], int emax, uint4 (&w)[kDigits]) {
-    uint32_t x[kDigits][4];
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-        uint32_t d0[kDigits], d1[kDigits];
-        digits(v[2 * h], emax, d0);
-        digits(v[2 * h + 1], emax, d1);
-#pragma unroll
-        for (int a = 0; a < kDigits; ++a) x[a][h] = __byte_perm(d0[a], d1[a], 0x7632);
-    }
-#pragma unroll
-    for (int a = 0; a < kDigits; ++a) w[a] = make_uint4(x[a][0], x[a][1], x[a][2], x[a][3]);
+    for (int a = 0; a < kDigits; ++a) w[a] = make_uint2(x[a][0], x[a][1]);
 }
 
 // ---- eight digits: operands of 62 bits, results rounded once to FP64 -----------
@@ -173,7 +136,7 @@ __host__ __device__ constexpr int fixed_power(int E) {
 template <int ND>
 struct FixedRow;
 
-// Six digits: the 47-bit integers of fixed(), rounded half away from zero
+// Six digits: 47-bit integers, rounded half away from zero
 // (one variable shift: floor((m + 2^(s-1)) / 2^s) = floor((floor(m / 2^(s-1)) + 1) / 2)).
 template <>
 struct FixedRow<kDigits> {
@@ -344,34 +307,6 @@ __device__ __forceinline__ dfl combine4(float a0, float a1, float a2, float a3) 
 // dropped; they are far below the grid values)
 __device__ __forceinline__ float pow2f(int x) {
     return x < -126 ? 0.0f : __int_as_float((min(x, 127) + 127) << 23);
-}
-
-// Issue the kPairs digit-pair MMAs of one K stage: A planes at aBase +
-// a * aPlane, B planes at bBase + b * bPlane, KSTEPS MMAs of K = 16 each,
-// accumulators at tmem + g * N (g = min(a + b, 3)).  accumulate: the first
-// MMA of each accumulator adds to what it holds (later K stages).
-template <int KSTEPS>
-__device__ __forceinline__ void issue_pairs(uint32_t tmem, int N, uint32_t idesc, uint32_t aBase,
-                                            uint32_t aPlane, uint32_t aSbo, uint32_t bBase,
-                                            uint32_t bPlane, uint32_t bSbo, bool accumulate) {
-    bool started[4] = {accumulate, accumulate, accumulate, accumulate};
-#pragma unroll
-    for (int c = 0; c <= kCmax; ++c) {
-        const int g = c < 3 ? c : 3;
-#pragma unroll
-        for (int a = 0; a < kDigits; ++a) {
-            const int b = c - a;
-            if (b < 0 || b >= kDigits) continue;
-#pragma unroll
-            for (int ks = 0; ks < KSTEPS; ++ks) {
-                tc::mma_bf16(tmem + (uint32_t)(g * N),
-                             tc::desc_sbo(aBase + a * aPlane + ks * tc::kKStep, aSbo),
-                             tc::desc_sbo(bBase + b * bPlane + ks * tc::kKStep, bSbo), idesc,
-                             started[g] ? 1u : 0u);
-                started[g] = true;
-            }
-        }
-    }
 }
 
 // The digit-pair MMAs of a block of COLS columns with ND digits and NACC
