@@ -32,7 +32,6 @@ namespace mg {
 namespace oz {
 
 constexpr int kDigits = 6;                       // digits per operand entry
-constexpr int kCmax = 5;                         // largest kept digit weight a + b
 constexpr long long kDigitBias = 0x8080808080LL; // 128 in each of the five lower digits
 constexpr uint32_t kAccs = 4;                    // accumulators per output
 
