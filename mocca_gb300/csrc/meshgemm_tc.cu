@@ -379,7 +379,14 @@ k_coef_digits(const double* __restrict__ coef, long bstride, int ld, BlockIdx bi
 // 256 columns holds the tensor pipe ~130 clocks: 54 of them for a tile of 48
 // spinors, 90 for 80).  A CTA per tile went through the same steps one after the
 // other: 1628 us for the 300 spwfs of 36^3 (blocks of 75), now 573; 110 for the 160
-// of 24^3 (40), now 82.
+// of 24^3 (40), now 77.
+// Epilogue warps.  Up to 48 spinors a slicer's values leave the registers for sixteen:
+// 160 spwfs of 24^3 77 us, FP64 form 102, with eight 87 and 150.  Above them not: 300
+// of 36^3 573 us with eight of each, 709 with sixteen slicer warps and eight.
+__host__ __device__ constexpr int apply_epilogue(int np) { return np <= 48 ? 16 : 8; }
+__host__ __device__ constexpr int apply_threads(int np) { return 32 * (apply_epilogue(np) + kRoleWarps + 1); }
+__device__ __forceinline__ void tmem_load(uint32_t t, uint32_t (&r)[4]) { tc::ld4(t, r); }
+__device__ __forceinline__ void tmem_load(uint32_t t, uint32_t (&r)[8]) { tc::ld8(t, r); }
 __host__ __device__ constexpr int apply_plane(int np) { return kRows * np * 2; }
 __host__ __device__ constexpr int apply_coef(int nd, int np) { return nd * np * np * 2; }
 // operand and accumulator buffers that fit
@@ -391,14 +398,15 @@ __host__ __device__ constexpr size_t apply_smem(int nd, int np) {
 }
 
 template <int ND, int NP, bool kInPlace>
-__global__ void __launch_bounds__(kRoleThreads, 1)
+__global__ void __launch_bounds__(apply_threads(NP), 1)
 k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
            const int* __restrict__ in_list, const int* __restrict__ out_list,
            const int* __restrict__ out_base, const uint16_t* __restrict__ xd,
            const int* __restrict__ xe, const double* __restrict__ coef, long bstride, int ld,
            long V4, int tpb, int ntiles, int* __restrict__ status) {
     constexpr int NACC = accs_for(ND), NBUF = apply_bufs(ND, NP), NTB = tbufs_for(ND, NP);
-    constexpr int kg = NP / 8, kPlane = apply_plane(NP);
+    constexpr int kg = NP / 8, kPlane = apply_plane(NP), EW = apply_epilogue(NP);
+    constexpr int W = 64 / EW;   // columns of an epilogue chunk, 16 / W warps side by side
     extern __shared__ uint8_t smraw[];
     __shared__ __align__(8) uint64_t fullA[2], emptyA[2], fullT[2], emptyT[2], emaxReady[4];
     __shared__ uint32_t tmem_slot;
@@ -415,7 +423,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
             tc::mbar_init(&fullA[q], kRoleWarps);
             tc::mbar_init(&emptyA[q], 1);
             tc::mbar_init(&fullT[q], 1);
-            tc::mbar_init(&emptyT[q], kRoleWarps);
+            tc::mbar_init(&emptyT[q], EW);
         }
         for (int q = 0; q < 4; ++q) tc::mbar_init(&emaxReady[q], kRoleWarps);
     }
@@ -434,10 +442,10 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
         {
             const uint4* src = reinterpret_cast<const uint4*>(xd + (long)b * ND * kXdStride);
             uint4* dst = reinterpret_cast<uint4*>(sB);
-            for (int t = tid; t < apply_coef(ND, NP) / 16; t += kRoleThreads) dst[t] = src[t];
+            for (int t = tid; t < apply_coef(ND, NP) / 16; t += apply_threads(NP)) dst[t] = src[t];
             // K groups past the block's spinors stay zero
             uint4* a = reinterpret_cast<uint4*>(sA);
-            for (int t = tid; t < NBUF * ND * kPlane / 16; t += kRoleThreads)
+            for (int t = tid; t < NBUF * ND * kPlane / 16; t += apply_threads(NP))
                 a[t] = make_uint4(0u, 0u, 0u, 0u);
             if (tid < NP) {
                 sXe[tid] = xe[b * kMeshTcMax + tid];
@@ -450,10 +458,10 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
         const bool xbad = __syncthreads_or(tid < NP && xe[b * kMeshTcMax + tid] == 2047) != 0;
         tc::fence_after();
         tmem = tmem_slot;
-        if (warp >= kRoleWarps && warp < 2 * kRoleWarps) {
+        if (warp >= EW && warp < EW + kRoleWarps) {
             // ---------------- slicers ----------------
             // thread: point `row`, K groups half, half + 2, ...
-            const int st = tid - 32 * kRoleWarps, row = st & (kRows - 1), half = st >> 7;
+            const int st = tid - 32 * EW, row = st & (kRows - 1), half = st >> 7;
             constexpr int own = (kg + 1) / 2;
             for (int q = 0, k = k0; q < count; ++q, ++k) {
                 const int buf = k % NBUF;
@@ -513,7 +521,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                 tc::fence_proxy_async();
                 arrive_warp(&fullA[buf], lane);
             }
-        } else if (warp == 2 * kRoleWarps) {
+        } else if (warp == EW + kRoleWarps) {
             // ---------------- MMA issue ----------------
             if (lane == 0) {
                 int k = k0;
@@ -536,7 +544,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
             __syncwarp();
         } else {
             // ---------------- epilogue ----------------
-            // lane: point quarter * 32 + lane of the tile; columns 16 q + 8 colh + ...
+            // lane: point quarter * 32 + lane of the tile; columns 16 c + W colh + ...
             const int quarter = warp & 3, colh = warp >> 2, erow = quarter * 32 + lane;
             for (int q = 0, k = k0; q < count; ++q, ++k) {
                 const int tb = k % NTB;
@@ -547,23 +555,23 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                 tc::fence_after();
                 const int emax = sEmax[k & 3][erow] >> 8, bad = sEmax[k & 3][erow] & 255;
                 const uint32_t trow = tmem + ((uint32_t)(quarter * 32) << 16) +
-                                      (uint32_t)(tb * NACC * NP + 8 * colh);
-                const int nch = max(0, (nb - 8 * colh + 15) / 16);   // chunks of 8 columns
+                                      (uint32_t)(tb * NACC * NP + W * colh);
+                const int nch = max(0, (nb - W * colh + 15) / 16);
                 if (nch == 0) {
                     tc::fence_before();
                     arrive_warp(&emptyT[tb], lane);
                 }
 #pragma unroll 1
                 for (int c = 0; c < nch; ++c) {
-                    const int l0 = 16 * c + 8 * colh;
-                    uint32_t r[NACC][8];
+                    const int l0 = 16 * c + W * colh;
+                    uint32_t r[NACC][W];
                     __syncwarp();
 #pragma unroll
-                    for (int g = 0; g < NACC; ++g) tc::ld8(trow + (uint32_t)(g * NP + 16 * c), r[g]);
-                    double was[8];
+                    for (int g = 0; g < NACC; ++g) tmem_load(trow + (uint32_t)(g * NP + 16 * c), r[g]);
+                    double was[W];
                     if (upd && pe < V4)
 #pragma unroll
-                        for (int u = 0; u < 8; ++u)
+                        for (int u = 0; u < W; ++u)
                             if (l0 + u < nb) was[u] = upd[(long)sOut[l0 + u] * V4 + pe];
 #pragma unroll
                     for (int g = 0; g < NACC; ++g) tc::wait_ld(r[g]);
@@ -574,7 +582,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                     }
                     if (pe >= V4) continue;
 #pragma unroll
-                    for (int u = 0; u < 8; ++u) {
+                    for (int u = 0; u < W; ++u) {
                         if (l0 + u >= nb) break;
                         const int ex = sXe[l0 + u];
                         double x = 0.0;
@@ -607,7 +615,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                 }
                 if (ND == oz::kDigits64 && !kInPlace && pe < V4 && (bad != kNone || xbad))
                     // an infinity or a NaN at this point or in C: the plain sums
-                    for (int l = 8 * colh; l < nb; l += (l & 7) == 7 ? 9 : 1) {
+                    for (int l = W * colh; l < nb; l += (l & (W - 1)) == W - 1 ? 17 - W : 1) {
                         const double* C = coef + (long)b * bstride + l;
                         double x = 0.0;
 #pragma unroll 1
@@ -1055,7 +1063,7 @@ static int apply_launch(mg_ctx* c, int nblk, const double* coef, long bstride, i
     const long V4 = 4 * c->V;
     const int tpb = div_up(V4, kRows), ntiles = tpb * nblk;
     const int sms = c->tc_grid_cap > 0 ? std::min(c->tc_grid_cap, c->num_sms) : c->num_sms;
-    kernel<<<std::min(sms, ntiles), kRoleThreads, apply_smem(ND, NP), c->stream>>>(
+    kernel<<<std::min(sms, ntiles), apply_threads(NP), apply_smem(ND, NP), c->stream>>>(
         in, out, upd, bi, in_list, out_list, out_base, xd, xe, coef, bstride, ld, V4, tpb, ntiles,
         c->tc_status);
     MG_LAUNCHED(c);
@@ -1160,7 +1168,7 @@ int pair_field_tc(mg_ctx* c, bool f64) {
 
 // The same in the FP64 form, behind pair_field_tc, whose scratch basis takes the
 // factors Z.  Pairing field and gaps of 108 spwfs at 18^3 (blocks of 26 and 28): 136
-// and 152 us by FP64 FMAs, here 65 and 100.
+// and 152 us by FP64 FMAs, here 56 and 100.
 int gaps_tc64(mg_ctx* c, double* gsum) {
     Hfb& H = c->hfb;
     if (!mesh_tc_serves(c, H.hmax, true) || c->field_y == nullptr) return MG_ERR_STATE;
