@@ -90,8 +90,14 @@ __host__ __device__ constexpr int overlap_bufs(int nd, int np, bool two) {
     return (kSmemCap - 8192 - 128 - kOverlapTail) / overlap_stage(nd, np, two) >= 6
                ? 6 : (kSmemCap - 8192 - 128 - kOverlapTail) / overlap_stage(nd, np, two);
 }
+// (more than half of an SM's, so that no second CTA comes beside one that holds all
+// TMEM columns and waits for them)
+constexpr size_t kOneCtaSmem = 116 * 1024;
+__host__ __device__ constexpr size_t one_cta(size_t bytes) {
+    return bytes > kOneCtaSmem ? bytes : kOneCtaSmem;
+}
 __host__ __device__ constexpr size_t overlap_smem(int nd, int np, bool two) {
-    return (size_t)overlap_bufs(nd, np, two) * overlap_stage(nd, np, two) + kOverlapTail + 128;
+    return one_cta((size_t)overlap_bufs(nd, np, two) * overlap_stage(nd, np, two) + kOverlapTail + 128);
 }
 
 __device__ __forceinline__ bool wait_warp(uint64_t* mbar, uint32_t parity) {
@@ -394,7 +400,7 @@ __host__ __device__ constexpr int apply_bufs(int nd, int np) {
     return 2 * nd * apply_plane(np) + apply_coef(nd, np) + 128 <= kSmemCap ? 2 : 1;
 }
 __host__ __device__ constexpr size_t apply_smem(int nd, int np) {
-    return (size_t)apply_bufs(nd, np) * nd * apply_plane(np) + apply_coef(nd, np) + 128;
+    return one_cta((size_t)apply_bufs(nd, np) * nd * apply_plane(np) + apply_coef(nd, np) + 128);
 }
 
 template <int ND, int NP, bool kInPlace>
@@ -1141,20 +1147,43 @@ int gaps_tc(mg_ctx* c, double* gsum) {
     return MG_OK;
 }
 
+// Scratch of the pairing contractions.  False where the kernels of pairing.cu are the
+// ones to run, in the FP64 form also when the device has no room for the scratch.
+bool pair_tc_prepare(mg_ctx* c, bool f64) {
+    Hfb& H = c->hfb;
+    if (!mesh_tc_serves(c, H.hmax, f64)) return false;
+    if (c->field_ybase == nullptr) {
+        const int yb[4] = {0, H.hmax, 2 * H.hmax, 3 * H.hmax};
+        const auto room = [](auto** p, size_t bytes) {
+            return *p != nullptr || cudaMalloc(p, bytes) == cudaSuccess;
+        };
+        if (!room(&c->field_y, (size_t)4 * H.hmax * 4 * c->V * sizeof(double)) ||
+            !room(&c->field_xd, (size_t)4 * oz::kDigits64 * kXdStride * sizeof(uint16_t)) ||
+            !room(&c->field_xe, (size_t)4 * kMeshTcMax * sizeof(int)) ||
+            !room(&c->field_ybase, sizeof(yb)) ||
+            cudaMemcpy(c->field_ybase, yb, sizeof(yb), cudaMemcpyHostToDevice) != cudaSuccess) {
+            cudaGetLastError();
+            if (c->field_ybase) cudaFree(c->field_ybase);
+            c->field_ybase = nullptr;   // not complete
+            return !f64;                // mixed: the launch reports the missing scratch
+        }
+    }
+    if (f64 && c->gap_part64 == nullptr &&
+        cudaMalloc(&c->gap_part64, (size_t)4 * div_up(4 * c->V, chunk_for(oz::kDigits64)) * H.hmax *
+                                       H.hmax * sizeof(double)) != cudaSuccess) {
+        cudaGetLastError();
+        c->gap_part64 = nullptr;
+        return false;
+    }
+    return true;
+}
+
 // Pairing-field partials of the four blocks: Y = block apply of Ktilde
 // (tensor cores) into the scratch basis, then the pointwise contraction.
 int pair_field_tc(mg_ctx* c, bool f64) {
     Hfb& H = c->hfb;
-    if (!mesh_tc_serves(c, H.hmax, f64)) return MG_ERR_STATE;
+    if (c->field_ybase == nullptr) return MG_ERR_CUDA;   // pair_tc_prepare
     const long V = c->V;
-    if (c->field_y == nullptr) {
-        MG_CUDA(cudaMalloc(&c->field_y, (size_t)4 * H.hmax * 4 * V * sizeof(double)));
-        MG_CUDA(cudaMalloc(&c->field_xd, (size_t)4 * oz::kDigits64 * kXdStride * sizeof(uint16_t)));
-        MG_CUDA(cudaMalloc(&c->field_xe, (size_t)4 * kMeshTcMax * sizeof(int)));
-        MG_CUDA(cudaMalloc(&c->field_ybase, 4 * sizeof(int)));
-        const int yb[4] = {0, H.hmax, 2 * H.hmax, 3 * H.hmax};
-        MG_CUDA(cudaMemcpy(c->field_ybase, yb, sizeof(yb), cudaMemcpyHostToDevice));
-    }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
     MG_TRY(apply_tc(c, 4, H.hmax, f64, H.ktil, (long)H.hmax * H.hmax, 0, bi,
                     c->bas[MG_HF_BASIS].psi, c->field_y, nullptr, H.members, nullptr,
@@ -1171,11 +1200,9 @@ int pair_field_tc(mg_ctx* c, bool f64) {
 // and 152 us by FP64 FMAs, here 56 and 100.
 int gaps_tc64(mg_ctx* c, double* gsum) {
     Hfb& H = c->hfb;
-    if (!mesh_tc_serves(c, H.hmax, true) || c->field_y == nullptr) return MG_ERR_STATE;
+    if (c->field_y == nullptr || c->gap_part64 == nullptr) return MG_ERR_STATE;
     const long V = c->V;
     const int nchunk = div_up(4 * V, chunk_for(oz::kDigits64));
-    if (c->gap_part64 == nullptr)
-        MG_CUDA(cudaMalloc(&c->gap_part64, (size_t)4 * nchunk * H.hmax * H.hmax * sizeof(double)));
     const double* psi = c->bas[MG_HF_BASIS].psi;
     k_gaps_factor<<<dim3(div_up(V, 128), H.hmax, 4), 128, 0, c->stream>>>(
         psi, H.members, H.hsz, H.hmax, H.fre, H.fim, V, c->field_y);

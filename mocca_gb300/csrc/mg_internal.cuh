@@ -419,6 +419,7 @@ int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const i
 int can_transform_tc(mg_ctx* c, bool f64);
 int gaps_tc(mg_ctx* c, double* gsum);
 int gaps_tc64(mg_ctx* c, double* gsum);
+bool pair_tc_prepare(mg_ctx* c, bool f64);
 int pair_field_tc(mg_ctx* c, bool f64);
 int densities(mg_ctx* c);
 int moments(mg_ctx* c);

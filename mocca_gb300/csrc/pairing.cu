@@ -430,7 +430,7 @@ int pairing_mesh(mg_ctx* c) {
     MG_LAUNCHED(c);
     const size_t sm_f = (size_t)(hmax * hmax + hmax * 4 * kPts + 2 * kThreads) * sizeof(double);
     const bool mixed = c->cur_precision == MG_MIXED;
-    const bool tensor = mesh_tc_serves(c, hmax, !mixed);   // meshgemm_tc.cu
+    const bool tensor = pair_tc_prepare(c, !mixed);   // meshgemm_tc.cu
     if (tensor)
         MG_TRY(pair_field_tc(c, !mixed));
     else if (mixed)
