@@ -567,12 +567,11 @@ int tc_setup(mg_ctx* c) {
     MG_CUDA(cudaMemcpy(c->tcmats, h.data(), total * sizeof(uint16_t), cudaMemcpyHostToDevice));
     MG_CUDA(cudaMalloc(&c->tc_erow, he.size() * sizeof(int)));
     MG_CUDA(cudaMemcpy(c->tc_erow, he.data(), he.size() * sizeof(int), cudaMemcpyHostToDevice));
-    for (int form = 0; form < 2; ++form)
-        for (int kp : {16, 32, 48})
-            for (int xp = 0; xp < 2; ++xp)
-                MG_CUDA(cudaFuncSetAttribute(kernel_for(form == 1, kp, xp != 0),
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)kSmemCap));
+    // the kernels of this mesh (each is loaded when it is first touched)
+    for (int form = 0; form < (f64 ? 2 : 1); ++form)
+        for (int a = 0; a < 3; ++a)
+            MG_CUDA(cudaFuncSetAttribute(kernel_for(form == 1, kp_of(ns[a]), a == 0),
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemCap));
     c->tc_ok = true;
     c->tc_ok64 = f64;
     return MG_OK;
