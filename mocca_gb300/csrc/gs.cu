@@ -234,8 +234,9 @@ k_gs_apply(double* __restrict__ psi, double* __restrict__ upd, const int* __rest
 
 }  // namespace
 
-// Block lists (isospin, parity, signature) from the quantum numbers; they
-// are static for a run, so they are built once and kept on the device.
+// Block lists (isospin, parity, signature) from the quantum numbers, built when
+// these come (mg_upload_spinors) and kept on the device, with the scratch for blocks
+// of that number and size.
 static int gs_prepare(mg_ctx* c) {
     Basis& B = c->bas[MG_HF_BASIS];
     std::vector<int> keys;

@@ -1002,10 +1002,21 @@ bool mesh_tc_serves(const mg_ctx* c, int nbmax, bool f64) {
            (f64 ? nbmax >= kMeshTcMin64 && nbmax <= kMeshTcMax64 : nbmax <= kMeshTcMax);
 }
 
-// Buffers of the tensor-core Gram-Schmidt.  Returns false where the FP64 kernels of
-// gs.cu are the ones to run.
+static void gs_tc_free(mg_ctx* c) {
+    cudaFree(c->gs_Stc);
+    cudaFree(c->gs_xd);
+    cudaFree(c->gs_xe);
+    c->gs_Stc = nullptr;
+    c->gs_xd = nullptr;
+    c->gs_xe = nullptr;
+}
+
+// Buffers of the tensor-core Gram-Schmidt, for both forms; new quantum numbers can
+// change the number and the size of the blocks they are for.  Returns false where the
+// FP64 kernels of gs.cu are the ones to run.
 bool gs_tc_prepare(mg_ctx* c, bool f64) {
     if (!mesh_tc_serves(c, c->gs_nbmax, f64)) return false;
+    if (c->gs_tc_nblk != c->gs_nblk || c->gs_tc_nbmax != c->gs_nbmax) gs_tc_free(c);
     if (c->gs_xd == nullptr) {
         const int nblk = c->gs_nblk;
         const bool both = c->gs_nbmax <= kMeshTcMax64;   // the FP64 form's chunks are smaller
@@ -1016,6 +1027,8 @@ bool gs_tc_prepare(mg_ctx* c, bool f64) {
                 cudaSuccess ||
             cudaMalloc(&c->gs_xe, (size_t)nblk * kMeshTcMax * sizeof(int)) != cudaSuccess)
             return false;
+        c->gs_tc_nblk = nblk;
+        c->gs_tc_nbmax = c->gs_nbmax;
     }
     return true;
 }

@@ -270,8 +270,9 @@ struct mg_ctx {
     double* gs_R = nullptr;       // inverse Cholesky factors
     int* gs_index = nullptr;      // block lists + energy-ordered members
     int gs_nblk = 0, gs_nbmax = 0, gs_nchunk = 0, gs_lists_len = 0;
-    // tensor-core form (meshgemm_tc.cu): overlap partials per 256-point chunk, digit
-    // planes and row exponents of X = R^{-1}
+    // tensor-core form (meshgemm_tc.cu): overlap partials per 128- or 256-point chunk,
+    // digit planes and row exponents of X = R^{-1}, for blocks of this number and size
+    int gs_tc_nblk = 0, gs_tc_nbmax = 0;
     double* gs_Stc = nullptr;
     uint16_t* gs_xd = nullptr;
     int* gs_xe = nullptr;
