@@ -1013,7 +1013,7 @@ static void gs_tc_free(mg_ctx* c) {
 
 // Buffers of the tensor-core Gram-Schmidt, for both forms; new quantum numbers can
 // change the number and the size of the blocks they are for.  Returns false where the
-// FP64 kernels of gs.cu are the ones to run.
+// FP64 kernels of gs.cu are the ones to run, also when the device has no room for them.
 bool gs_tc_prepare(mg_ctx* c, bool f64) {
     if (!mesh_tc_serves(c, c->gs_nbmax, f64)) return false;
     if (c->gs_tc_nblk != c->gs_nblk || c->gs_tc_nbmax != c->gs_nbmax) gs_tc_free(c);
@@ -1025,8 +1025,11 @@ bool gs_tc_prepare(mg_ctx* c, bool f64) {
                                        sizeof(double)) != cudaSuccess ||
             cudaMalloc(&c->gs_xd, (size_t)nblk * oz::kDigits64 * kXdStride * sizeof(uint16_t)) !=
                 cudaSuccess ||
-            cudaMalloc(&c->gs_xe, (size_t)nblk * kMeshTcMax * sizeof(int)) != cudaSuccess)
+            cudaMalloc(&c->gs_xe, (size_t)nblk * kMeshTcMax * sizeof(int)) != cudaSuccess) {
+            cudaGetLastError();
+            gs_tc_free(c);
             return false;
+        }
         c->gs_tc_nblk = nblk;
         c->gs_tc_nbmax = c->gs_nbmax;
     }
@@ -1112,15 +1115,26 @@ int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const i
                     c->gs_xe);
 }
 
-// Canonical basis of the four pairing blocks (hsz[b] <= kMeshTcMax):
-// CanTransfo is stored densely per block (ld = h) at b * hmax^2.
+// Buffers of the tensor-core canonical transform.  False where the kernels of
+// pairing.cu are the ones to run, also when the device has no room for them.
+bool can_tc_prepare(mg_ctx* c, bool f64) {
+    if (!mesh_tc_serves(c, c->hfb.hmax, f64)) return false;
+    if (c->can_xe == nullptr) {   // allocated last
+        if ((c->can_xd == nullptr &&
+             cudaMalloc(&c->can_xd, (size_t)4 * oz::kDigits64 * kXdStride * sizeof(uint16_t)) !=
+                 cudaSuccess) ||
+            cudaMalloc(&c->can_xe, (size_t)4 * kMeshTcMax * sizeof(int)) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+    }
+    return true;
+}
+
+// Canonical basis of the four pairing blocks (hsz[b] <= kMeshTcMax), behind
+// can_tc_prepare: CanTransfo is stored densely per block (ld = h) at b * hmax^2.
 int can_transform_tc(mg_ctx* c, bool f64) {
     Hfb& H = c->hfb;
-    if (!mesh_tc_serves(c, H.hmax, f64)) return MG_ERR_STATE;
-    if (c->can_xd == nullptr) {
-        MG_CUDA(cudaMalloc(&c->can_xd, (size_t)4 * oz::kDigits64 * kXdStride * sizeof(uint16_t)));
-        MG_CUDA(cudaMalloc(&c->can_xe, (size_t)4 * kMeshTcMax * sizeof(int)));
-    }
     const BlockIdx bi{nullptr, H.hsz, H.hmax};
     return apply_tc(c, 4, H.hmax, f64, H.cantr, (long)H.hmax * H.hmax, 0, bi,
                     c->bas[MG_HF_BASIS].psi, c->bas[MG_CAN_BASIS].psi, nullptr, H.members,

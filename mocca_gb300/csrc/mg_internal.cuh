@@ -417,6 +417,7 @@ int gs_overlap_tc(mg_ctx* c, const double* psi, const int* d_lists, const int* d
                   int* nchunk);
 int gs_apply_tc(mg_ctx* c, double* psi, double* upd, const int* d_lists, const int* d_ordered,
                 bool f64);
+bool can_tc_prepare(mg_ctx* c, bool f64);
 int can_transform_tc(mg_ctx* c, bool f64);
 int gaps_tc(mg_ctx* c, double* gsum);
 int gaps_tc64(mg_ctx* c, double* gsum);

@@ -470,7 +470,7 @@ int canonical_transform(mg_ctx* c) {
     const long V4 = 4 * c->V;
     const size_t sm = (size_t)(H.hmax * H.hmax + H.hmax * kPts) * sizeof(double);
     const bool f64 = c->cur_precision != MG_MIXED;
-    if (mesh_tc_serves(c, H.hmax, f64)) return can_transform_tc(c, f64);   // meshgemm_tc.cu
+    if (can_tc_prepare(c, f64)) return can_transform_tc(c, f64);   // meshgemm_tc.cu
     if (c->cur_precision == MG_MIXED)
         k_can_transform_df<<<dim3(div_up(V4, kPts), 4), kThreads, sm, c->stream>>>(
             c->bas[MG_HF_BASIS].psi, H.members, H.hsz, H.cstart, H.hmax, H.cantr, V4,
