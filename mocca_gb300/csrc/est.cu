@@ -111,12 +111,11 @@ int estimate_parameters(mg_ctx* c) {
     const long V = c->V, V4 = 4 * V;
     const int nwt = c->p.nwt;
     double* psi = nullptr;
-    if (!c->est) {
+    if (!c->est)
         MG_CUDA(cudaMalloc(&c->est, (28 * V + 2 * kEstChunk) * sizeof(double) + sizeof(EstState)));
-        MG_CUDA(cudaMallocHost(&c->h_est, 2 * kEstChunk * sizeof(double)));
-        MG_CUDA(cudaMalloc(&c->est_jobs, 4 * sizeof(GridJob)));
-        MG_CUDA(cudaMalloc(&c->est_qn, 4 * sizeof(int)));
-    }
+    if (!c->h_est) MG_CUDA(cudaMallocHost(&c->h_est, 2 * kEstChunk * sizeof(double)));
+    if (!c->est_jobs) MG_CUDA(cudaMalloc(&c->est_jobs, 4 * sizeof(GridJob)));
+    if (!c->est_qn) MG_CUDA(cudaMalloc(&c->est_qn, 4 * sizeof(int)));
     psi = c->est;
     double* der = psi + V4;
     double* lap = der + 12 * V;

@@ -259,21 +259,24 @@ static int gs_prepare(mg_ctx* c) {
     }
     lists[nblk] = pos;
     if (2L * nbmax * nbmax * (long)sizeof(double) > 220L * 1024) return MG_ERR_ARG;
-    c->gs_nblk = nblk;
-    c->gs_nbmax = nbmax;
-    c->gs_nchunk = std::max(1, 2 * c->num_sms / nblk);
-    c->gs_lists_len = (int)lists.size();
-    if (c->gs_index) cudaFree(c->gs_index);
-    if (c->gs_S) cudaFree(c->gs_S);
-    if (c->gs_R) cudaFree(c->gs_R);
+    const int nchunk = std::max(1, 2 * c->num_sms / nblk);
+    cudaFree(c->gs_index);
+    cudaFree(c->gs_S);
+    cudaFree(c->gs_R);
+    c->gs_index = nullptr;
+    c->gs_S = c->gs_R = nullptr;
     MG_CUDA(cudaMalloc(&c->gs_index, (lists.size() + c->p.nwt) * sizeof(int)));
-    MG_CUDA(cudaMalloc(&c->gs_S, (size_t)nblk * c->gs_nchunk * nbmax * nbmax * sizeof(double)));
+    MG_CUDA(cudaMalloc(&c->gs_S, (size_t)nblk * nchunk * nbmax * nbmax * sizeof(double)));
     MG_CUDA(cudaMalloc(&c->gs_R, (size_t)nblk * nbmax * nbmax * sizeof(double)));
     MG_CUDA(cudaMemcpy(c->gs_index, lists.data(), lists.size() * sizeof(int),
                        cudaMemcpyHostToDevice));
     MG_CUDA(cudaFuncSetAttribute(k_gs_overlap, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     MG_CUDA(cudaFuncSetAttribute(k_gs_factor, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     MG_CUDA(cudaFuncSetAttribute(k_gs_apply, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    c->gs_nblk = nblk;   // complete
+    c->gs_nbmax = nbmax;
+    c->gs_nchunk = nchunk;
+    c->gs_lists_len = (int)lists.size();
     return MG_OK;
 }
 

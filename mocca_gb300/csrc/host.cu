@@ -344,8 +344,9 @@ extern "C" int mg_upload_spinors(mg_ctx* c, int b, const double* const* grids, c
         MG_CUDA(cudaMemcpyAsync(B.qn, B.h_qn.data(), B.h_qn.size() * sizeof(int),
                                 cudaMemcpyHostToDevice, c->stream));
         if (first + count == c->p.nwt || B.have_qn) {
-            B.have_qn = true;
+            B.have_qn = false;   // until the jobs are there
             MG_TRY(build_basis_jobs(c, b));
+            B.have_qn = true;
             if (b == MG_HF_BASIS) c->gs_nblk = 0;  // rebuild Gram-Schmidt blocks
         }
     }

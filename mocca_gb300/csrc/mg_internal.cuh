@@ -15,6 +15,7 @@
         if (e_ != cudaSuccess) {                                                   \
             fprintf(stderr, "mocca_gpu: %s failed at %s:%d: %s\n", #call, __FILE__, \
                     __LINE__, cudaGetErrorString(e_));                             \
+            cudaGetLastError(); /* reported: not the next launch's */              \
             return MG_ERR_CUDA;                                                    \
         }                                                                          \
     } while (0)

@@ -137,7 +137,69 @@ def canonical(room):
         assert relative(c2.T @ c2, can.T @ can) < 1e-9
 
 
+def refused(fn, status):
+    from mocca_gb300 import _abi
+    try:
+        fn()
+    except _abi.MgError as e:
+        assert e.status == status, e
+    else:
+        raise AssertionError("not refused")
+
+
+def retried(room):
+    """Set-ups that fail half way: the call is an error each time it is made
+    again, and once there is room it does its work."""
+    from mocca_gb300 import MG_FP64, SLY4, RunParams, _abi
+    from mocca_gb300.mesh import MeshState
+    nwt, n = 60, (9, 10, 8)
+    p = RunParams(nx=n[0], ny=n[1], nz=n[2], dx=0.8, nwt=nwt, neutrons=20, protons=20,
+                  precision=MG_FP64, parameter_estimation=1)
+    psi, qn, en = spinors(nwt, 4 * n[0] * n[1] * n[2], 2)
+
+    def prepare(g):
+        g.set_spinors(psi, qn)
+        g.set_energies(en)
+        g.GramSchmidt()
+        g.DeriveAll()
+        rng = np.random.default_rng(3)
+        g.set_potentials(U=rng.normal(size=2 * p.V), B=rng.uniform(10.0, 20.0, 2 * p.V),
+                         nablaB=rng.normal(size=6 * p.V), W=rng.normal(size=18 * p.V),
+                         divW=rng.normal(size=6 * p.V))
+
+    def step(g):
+        g.GradDesc(0.01, 0.3)
+        return g.get_spinors(), g.StepParameters()
+
+    with MeshState(p, SLY4) as g:
+        prepare(g)
+        want, dt = step(g)
+    lists = 4 * (2 + 1 + 2 * nwt)
+    with MeshState(p, SLY4) as g:
+        room.refuse(4 * 12 * nwt)           # the jobs sorted by their matrices
+        for _ in range(2):
+            refused(lambda: g.set_spinors(psi, qn), _abi.MG_ERR_CUDA)
+            refused(lambda: g.DeriveBasis(), _abi.MG_ERR_STATE)
+        room.refuse()
+        g.set_spinors(psi, qn)
+        g.set_energies(en)
+        for size in (lists, 2 * 30 * 30 * 8):   # member lists, factors
+            room.refuse(size)
+            for _ in range(2):
+                refused(g.GramSchmidt, _abi.MG_ERR_CUDA)
+            room.refuse()
+        prepare(g)
+        for size in (4 * 48, 4 * 4):        # the probe's jobs, its quantum numbers
+            room.refuse(size)
+            for _ in range(2):
+                refused(lambda: g.GradDesc(0.01, 0.3), _abi.MG_ERR_CUDA)
+            room.refuse()
+        got, dt2 = step(g)
+        assert dt2 == dt and np.array_equal(got, want)
+
+
 CASES = {
+    "retried": retried,
     "gram_schmidt_fp64": lambda room: gram_schmidt(room, 0, 1e-13),
     "gram_schmidt_mixed": lambda room: gram_schmidt(room, 1, 1e-11),
     "canonical": canonical,
