@@ -66,6 +66,8 @@ k_energy_partial(const double* __restrict__ rho, const double* __restrict__ tau,
                  const double* __restrict__ laprho, const double* __restrict__ nablaj,
                  const double* __restrict__ coul, const double* __restrict__ jm, ECoef k, long V,
                  double* __restrict__ part) {
+    // (below: no rank writes to the row's first block before that has started)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     double acc[kTerms];
 #pragma unroll
     for (int q = 0; q < kTerms; ++q) acc[q] = 0.0;
@@ -136,6 +138,7 @@ k_energy_partial(const double* __restrict__ rho, const double* __restrict__ tau,
     asm("mapa.shared::cluster.u32 %0, %1, 0;"
         : "=r"(to)
         : "r"((uint32_t)__cvta_generic_to_shared(&red[w][lane])));
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(x[0]) : "memory");
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

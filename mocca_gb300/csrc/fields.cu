@@ -141,6 +141,8 @@ __global__ void __cluster_dims__(kMomentCtas, 1, 1) __launch_bounds__(64)
 k_moments(const double* __restrict__ sh, const double* __restrict__ rho, long V, double dv,
           double* __restrict__ values) {
     __shared__ double red[2][kMomentCtas];   // of the first block
+    // (below: no rank writes to the first one before that has started)
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
     const int m = blockIdx.x / kMomentCtas, w = blockIdx.x % kMomentCtas;
     const int it = threadIdx.x / 32, lane = threadIdx.x % 32;
     const double* s = sh + (long)m * V;
@@ -170,6 +172,7 @@ k_moments(const double* __restrict__ sh, const double* __restrict__ rho, long V,
             if (v + (long)q * kThreads < V) a = fma(x0[q], y0[q], a);
     }
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (lane == 0) {
         uint32_t to;
         asm("mapa.shared::cluster.u32 %0, %1, 0;"
