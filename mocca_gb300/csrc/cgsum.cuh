@@ -46,6 +46,7 @@ struct ClusterSum {
     double warp[2][16];
     double result[2];
     int fail;                      // this block gives up
+    int late;                      // sums of other clusters did not come to this block
 };
 
 // The address of the same shared variable in the block `rank` of the cluster.
@@ -89,6 +90,8 @@ __device__ bool cluster_sum(ClusterSum& S, int turn, int rank, double& x, double
             for (int o = 8; o > 0; o >>= 1)
                 if (o < nw) v += __shfl_xor_sync(0xffffffffu, v, o);
         }
+    } else {
+        __syncwarp();   // `fail` of any lane
     }
     if (warp == 0) {
         // lane r of the lower half sends x, of the upper half y, to rank r

@@ -21,7 +21,9 @@
 // that carry a running number beside the halves of the value, so a reader sees
 // by itself whether the value is there: no counters, flags or fences.  The
 // waits are bounded: one that runs out of its cap sets the timeout status and
-// the kernel returns instead of hanging.
+// the kernel returns instead of hanging.  A block leaves with its cluster, after
+// a meeting that all eight attend (no rank writes to the shared memory of one
+// that is gone), and decides nothing from sums that did not come.
 // The kernel is a chain of latencies: an FP64 add or FMA takes 64 clocks, a
 // divide 549, a cluster barrier 400, a word written by one block and polled by
 // another about a thousand (but ten thousand where many blocks poll the lines
@@ -55,6 +57,8 @@ struct CgArgs {
     double prec;
     double rel;             // > 0: stop at |r| <= rel |src| instead of |r|^2 <= prec
     int maxit;
+    long long sum_wait;     // limit in clocks of the waits for the clusters' sums,
+    int sum_wait_from;      // from this iteration on (tests make single waits run out)
 };
 
 __device__ __forceinline__ double lap_at(const double* g, int i, int j, int k, int mx, int my,
@@ -98,9 +102,11 @@ __device__ __forceinline__ double value_of(const ulonglong2& w) {
 // `meanwhile` is work of warp 0 for the time that the cluster's barrier takes.
 // The tag's parity picks the turn: what is left for a turn has been read when
 // that turn comes again, because the call in between needed every block.
+// Waits for `limit` clocks.  False when this block gives up, which the other ranks
+// of its cluster learn at their next meeting, the one of the next tag.
 template <class Meanwhile, class Then>
-__device__ bool grid_sum(ClusterSum& S, ulonglong2* mail, int* status, unsigned tag, double x, double y,
-                         double& a, double& b, Meanwhile meanwhile, Then then) {
+__device__ bool grid_sum(ClusterSum& S, ulonglong2* mail, int* status, unsigned tag, long long limit,
+                         double x, double y, double& a, double& b, Meanwhile meanwhile, Then then) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int turn = (int)(tag & 1u);
     const int rank = (int)(blockIdx.x % kCluster), cluster = (int)(blockIdx.x / kCluster);
@@ -111,6 +117,7 @@ __device__ bool grid_sum(ClusterSum& S, ulonglong2* mail, int* status, unsigned 
         return false;
     }
     if (warp == 0) {
+        bool all = true;
         if (nclusters > 1) {
             ulonglong2* box = mail + (size_t)turn * gridDim.x * kMaxClusters * 2;
             if (rank == 0) {
@@ -132,26 +139,37 @@ __device__ bool grid_sum(ClusterSum& S, ulonglong2* mail, int* status, unsigned 
                         y = value_of(z);
                         break;
                     }
-                    if (clock64() - t0 > kWaitCycles) {
+                    if (clock64() - t0 > limit) {
                         ok = false;
                         break;
                     }
                 }
             }
-            if (!ok) S.fail = 1;   // read by warp 0 at the next call
-            __syncwarp();
+            all = __all_sync(0xffffffffu, ok) != 0;
             const double v = warp_sum2(x, y);
             x = __shfl_sync(0xffffffffu, v, 0);
             y = __shfl_sync(0xffffffffu, v, 16);
         }
-        double ra, rb;
-        then(x, y, ra, rb);
+        if (all) {
+            double ra, rb;
+            then(x, y, ra, rb);
+            if (lane == 0) {
+                S.result[0] = ra;
+                S.result[1] = rb;
+            }
+        }
         if (lane == 0) {
-            S.result[0] = ra;
-            S.result[1] = rb;
+            S.late = all ? 0 : 1;
+            if (!all) S.fail = 1;
         }
     }
     __syncthreads();
+    if (S.late) {
+        x = y = 0.0;
+        cluster_sum(S, turn ^ 1, rank, x, y, []() {});
+        if (threadIdx.x == 0) atomicExch(status, 2);
+        return false;
+    }
     a = S.result[0];
     b = S.result[1];
     return true;
@@ -224,6 +242,8 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(512, 1) k_cg(
     double sol[R], res[R], p[R], s[R];   // s = Lap(p)
     int ci[R], cj[R], ck[R];
 
+    long long limit = a.sum_wait_from > 0 ? kWaitCycles : a.sum_wait;
+
     // r0 = src - Lap(sol)
     double bb = 0.0, unused;
     if (a.rel > 0.0) ++tag;
@@ -245,7 +265,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(512, 1) k_cg(
     double prec = a.prec;
     if (a.rel > 0.0) {
         // |src|^2 over the stored box for the relative test
-        if (!grid_sum(S, a.mail, a.status, tag - 1, bb, 0.0, bb, unused, []() {},
+        if (!grid_sum(S, a.mail, a.status, tag - 1, limit, bb, 0.0, bb, unused, []() {},
                       [](double x, double, double& u, double& w) { u = x; w = 0.0; }))
             return;
         prec = a.rel * a.rel * bb;
@@ -257,6 +277,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(512, 1) k_cg(
     int it = 0;
     bool done = false;
     for (;; ++it) {
+        if (it == a.sum_wait_from) limit = a.sum_wait;
         double rr = 0.0, rw = 0.0, lap[R];
 #pragma unroll
         for (int q = 0; q < R; ++q) {
@@ -273,7 +294,7 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(512, 1) k_cg(
         // beta = rr / rr_old, alpha = rr / (rw - beta rr / alpha_old); a negative
         // beta says that the test is met (rr <= prec)
         if (!grid_sum(
-                S, a.mail, a.status, tag, rr, rw, alpha, beta,
+                S, a.mail, a.status, tag, limit, rr, rw, alpha, beta,
                 [&]() {
                     if (it == 0) return;
                     inv_rr = inverse(rr_old);
@@ -300,12 +321,18 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(512, 1) k_cg(
             res[q] = r;
         }
     }
+    // the last meeting: a rank whose last sums did not come is at it too
+    double none[2] = {0.0, 0.0};
+    if (!cluster_sum(S, (int)((tag + 1) & 1u), (int)(blockIdx.x % kCluster), none[0], none[1], []() {})) {
+        if (threadIdx.x == 0) atomicExch(a.status, 2);
+        return;
+    }
 #pragma unroll
     for (int q = 0; q < R; ++q)
         if (t0 + q * stride < V) a.sol[ci[q] + a.mx * (cj[q] + (long)a.my * ck[q])] = sol[q];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         a.status[1] = it;
-        if (!done && a.status[0] == 0) a.status[0] = 1;
+        if (!done) atomicCAS(a.status, 0, 1);
     }
 }
 
@@ -851,6 +878,8 @@ int coulomb_solve(mg_ctx* c, int* iters) {
     a.prec = 1.0e-9 / (c->p.dx * c->p.dx * c->p.dx * c->nx * c->ny * c->nz);
     a.rel = c->p.coulomb_prec > 0 ? c->p.coulomb_prec : 0.0;
     a.maxit = maxit;
+    a.sum_wait = c->cg_sum_wait > 0 ? c->cg_sum_wait : kWaitCycles;
+    a.sum_wait_from = c->cg_sum_wait_from;
     void* args[] = {&a};
     const CgShape shape = cg_shape(c);
     // cooperative: its blocks wait for one another
@@ -867,11 +896,19 @@ int coulomb_solve(mg_ctx* c, int* iters) {
     if (iters) {
         MG_CUDA(cudaStreamSynchronize(c->stream));
         *iters = c->h_cg_status[1];
-        if (c->h_cg_status[0] == 2) return MG_ERR_TIMEOUT;
-        if (c->h_cg_status[0] == 3) return MG_ERR_CUDA;
         if (c->h_cg_status[0] == 1) return MG_NOT_CONVERGED;
+        return coulomb_status(c);
     }
     return MG_OK;
+}
+
+// Whether a wait of the last CG solve ran out, read after a synchronisation behind it;
+// reported once.
+int coulomb_status(mg_ctx* c) {
+    const int st = c->h_cg_status[0];
+    if (st != 2 && st != 3) return MG_OK;
+    c->h_cg_status[0] = 0;
+    return st == 2 ? MG_ERR_TIMEOUT : MG_ERR_CUDA;
 }
 
 }  // namespace mg

@@ -279,6 +279,7 @@ extern "C" int mg_create(const mg_params* p, const mg_force* f, void* stream, mg
         cudaMemset(c->flags, 0, 16 * sizeof(int)) != cudaSuccess ||
         cudaMallocHost(&c->h_cg_status, 4 * sizeof(int)) != cudaSuccess)
         return fail(MG_ERR_CUDA);
+    std::fill(c->h_cg_status, c->h_cg_status + 4, 0);
     c->cur_precision = p->precision;
     if ((st = upload_matrices(c)) != MG_OK) return fail(st);
     if ((st = build_field_jobs(c)) != MG_OK) return fail(st);
@@ -661,7 +662,8 @@ extern "C" int mg_set_potentials(mg_ctx* c, const double* u, const double* b,
 
 extern "C" int mg_energy(mg_ctx* c, mg_energy_terms* out) {
     if (!c || !out) return MG_ERR_ARG;
-    return energy(c, out);
+    MG_TRY(energy(c, out));
+    return coulomb_status(c);   // of mg_construct_potentials without its iteration count
 }
 
 extern "C" int mg_set_pairing(mg_ctx* c, const mg_pairing_params* pp) {
@@ -853,6 +855,7 @@ extern "C" int mg_iterate(mg_ctx* c, int n_iter, double dt, double momentum,
         // the tensor-core status word comes back with the energy's readback
         if (k == n_iter - 1) MG_TRY(tc_status_async(c));
         MG_TRY(energy(c, out ? out : &e));
+        MG_TRY(coulomb_status(c));
         phase_mark(c, MG_PH_ENERGY);
         MG_TRY(phase_end(c));
     }

@@ -300,6 +300,8 @@ struct mg_ctx {
     ulonglong2* cg_tagged = nullptr;   // the CG kernel's residuals and partial sums
     unsigned cg_tag = 0;               // last tag its launches may have used
     int cg_clusters = 0;               // clusters of its blocks that run at once
+    long long cg_sum_wait = 0;         // limit of its waits for sums in clocks (0: ~2 s),
+    int cg_sum_wait_from = 0;          // ... from this iteration on
     int* cg_status = nullptr;          // [state, iterations]
     int* h_cg_status = nullptr;        // pinned host copy
     double* red = nullptr;             // reduction scratch
@@ -428,6 +430,7 @@ int densities(mg_ctx* c);
 int moments(mg_ctx* c);
 int coulomb_setup(mg_ctx* c);
 int coulomb_solve(mg_ctx* c, int* iters);
+int coulomb_status(mg_ctx* c);
 int coulomb_residual(mg_ctx* c, double* rel);
 int coulomb_reset(mg_ctx* c);
 int coulomb_multigrid(mg_ctx* c, double tol, int maxit, int* iters);
