@@ -37,7 +37,9 @@ extern "C" {
 #define MG_ERR_ARG         -1   /* invalid argument / unsupported mode    */
 #define MG_ERR_CUDA        -2   /* CUDA runtime error                     */
 #define MG_ERR_STATE       -3   /* call out of order (e.g. no spinors)    */
-#define MG_ERR_TIMEOUT     -4   /* a device-side wait ran out of its cap  */
+#define MG_ERR_TIMEOUT     -4   /* a device-side wait ran out of its cap, in
+                                    this call or one before it: reported once,
+                                    by the first call that waits for results */
 #define MG_ERR_NAN         -5   /* NaN detected (reference: x .eq. x+1)   */
 
 /* ---- precision modes ----------------------------------------------------- */

@@ -447,8 +447,7 @@ extern "C" int mg_get_constraint_fields(mg_ctx* c, double* cutoff, double* field
             for (long v = 0; v < 2 * V; ++v) dst[v] = 0.0;
         }
     }
-    MG_CUDA(cudaStreamSynchronize(c->stream));
-    return MG_OK;
+    return mg::sync_results(c);
 }
 
 extern "C" int mg_alternate_step(mg_ctx* c) {

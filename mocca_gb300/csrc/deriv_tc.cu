@@ -475,7 +475,7 @@ k_deriv_tc(TcPass P) {
             }
         }
     }
-    if (!ok) atomicExch(P.status, 1);
+    if (!ok) tc::report_timeout(P.status);
     tc::fence_before();
     __syncthreads();
     if (warp == 0) tc::dealloc(tmem, tmem_cols(KP, NACC));
@@ -516,12 +516,11 @@ int tc_setup(mg_ctx* c) {
     c->tc_ok = c->tc_ok64 = false;
     // the mesh-sized GEMMs of meshgemm_tc.cu need no Lagrange planes: they
     // run on any mesh
-    if (!c->tc_status) {
-        MG_CUDA(cudaMalloc(&c->tc_status, sizeof(int)));
-        MG_CUDA(cudaMemset(c->tc_status, 0, sizeof(int)));
-        MG_CUDA(cudaMallocHost(&c->h_tc_status, sizeof(int)));
+    if (!c->h_tc_status) {
+        MG_CUDA(cudaHostAlloc(&c->h_tc_status, sizeof(int), cudaHostAllocMapped));
         *c->h_tc_status = 0;
     }
+    MG_CUDA(cudaHostGetDevicePointer(&c->tc_status, c->h_tc_status, 0));
     c->tc_mesh_ok = true;
     const int nmax = std::max(ns[0], std::max(ns[1], ns[2]));
     if (nmax > kMaxLine) return MG_OK;
@@ -633,27 +632,16 @@ int derive_basis_tc(mg_ctx* c, int b, bool f64) {
     return MG_OK;
 }
 
-// Status of the tensor-core waits since the last call (MG_ERR_TIMEOUT when an
-// MMA completion wait ran out of its cap, in the derivatives or the mesh
-// GEMMs); synchronises the stream.
-int tc_status_async(mg_ctx* c) {
-    if (!c->tc_ok && !c->tc_mesh_ok) return MG_OK;
-    MG_CUDA(cudaMemcpyAsync(c->h_tc_status, c->tc_status, sizeof(int), cudaMemcpyDeviceToHost,
-                            c->stream));
-    return MG_OK;
+int tc_result(mg_ctx* c) {
+    volatile int* word = c->h_tc_status;
+    if (*word == 0) return MG_OK;
+    *word = 0;
+    return MG_ERR_TIMEOUT;
 }
 
-int tc_status_result(mg_ctx* c) {
-    if (!c->tc_ok && !c->tc_mesh_ok) return MG_OK;
-    return *c->h_tc_status ? MG_ERR_TIMEOUT : MG_OK;
-}
-
-int tc_check(mg_ctx* c) {
-    if (!c->tc_ok && !c->tc_mesh_ok) return MG_OK;
-    int h = 0;
-    MG_CUDA(cudaMemcpyAsync(&h, c->tc_status, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+int sync_results(mg_ctx* c) {
     MG_CUDA(cudaStreamSynchronize(c->stream));
-    return h ? MG_ERR_TIMEOUT : MG_OK;
+    return tc_result(c);
 }
 
 }  // namespace mg

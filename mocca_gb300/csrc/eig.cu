@@ -287,11 +287,12 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
                 peer_arrive(peer_addr(&ring.empty[slot], 0));
             }
         }
-        if (!ok && flag) atomicExch(flag, 1);
+        // rounds that did not come: no vectors, so that nobody takes these for some
+        const float lost = ok ? 0.0f : __int_as_float(0x7FC00000);
         pair_barrier();   // side 0 has written perm
         for (int q = tid; q < n0 * n0; q += kJThreads) {
             const int i = q / n0, col = q % n0;
-            X[b * xstride + (long)i * ldx + col] = (double)v[i * ld + perm[col]];
+            X[b * xstride + (long)i * ldx + col] = (double)(v[i * ld + perm[col]] + lost);
         }
         return;
     }
@@ -410,7 +411,7 @@ k_jacobi32(const double* __restrict__ A, long astride, int lda, const int* __res
         }
     }
     send(-1, 1.0f, 0.0f);
-    if ((sweep == max_sweeps && tid == 0 || !sending) && flag) atomicExch(flag, 1);
+    if (sweep == max_sweeps && tid == 0 && flag) atomicExch(flag, 1);
     // sort the n0 real eigenpairs ascending, ties by index (the padding row
     // stays last): rank of each diagonal entry; perm starts as the identity
     // so that it stays a valid index table whatever the values

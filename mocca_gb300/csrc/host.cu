@@ -27,7 +27,6 @@ void free_all(mg_ctx* c) {
     F(c->mats32);
     F(c->tcmats);
     F(c->tc_erow);
-    F(c->tc_status);
     F(c->gs_Stc); F(c->gs_xd); F(c->gs_xe); F(c->can_xd); F(c->can_xe); F(c->gap_part); F(c->gap_part64); F(c->fields_df);
     F(c->field_y); F(c->field_xd); F(c->field_xe); F(c->field_ybase);
     F(c->est); F(c->est_jobs); F(c->est_qn);
@@ -309,7 +308,7 @@ extern "C" int mg_destroy(mg_ctx* c) {
 
 extern "C" int mg_synchronize(mg_ctx* c) {
     if (!c) return MG_ERR_ARG;
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
@@ -367,7 +366,7 @@ extern "C" int mg_download_spinors(mg_ctx* c, int b, double* const* grids, int f
                                 c->stream));
         i = j;
     }
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
@@ -384,7 +383,7 @@ extern "C" int mg_download_derivatives(mg_ctx* c, int b, double* const* der, dou
             MG_CUDA(cudaMemcpyAsync(lap[i], c->bas[b].lap + (long)(first + i) * 4 * V,
                                     4 * V * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     }
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     if (c->bas[b].der_df) {
         // mixed form: {hi, lo} float pairs -> FP64 in place
         auto widen = [](double* p, long n) {
@@ -415,7 +414,7 @@ extern "C" int mg_get_occupations(mg_ctx* c, int b, double* occ) {
     if (!c || !valid_basis(c, b) || !occ) return MG_ERR_ARG;
     MG_CUDA(cudaMemcpyAsync(occ, c->bas[b].occ, c->p.nwt * sizeof(double), cudaMemcpyDeviceToHost,
                             c->stream));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
@@ -435,7 +434,7 @@ extern "C" int mg_get_energies(mg_ctx* c, int b, double* e, double* disp) {
     if (disp)
         MG_CUDA(cudaMemcpyAsync(disp, c->bas[b].disp, c->p.nwt * sizeof(double),
                                 cudaMemcpyDeviceToHost, c->stream));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
@@ -451,7 +450,7 @@ extern "C" int mg_derive_all(mg_ctx* c) {
     if (!c) return MG_ERR_ARG;
     MG_TRY(derive_basis(c, MG_HF_BASIS));
     if (c->p.pairing == MG_PAIRING_HFB) MG_TRY(derive_basis(c, MG_CAN_BASIS));
-    return tc_check(c);
+    return sync_results(c);
 }
 
 extern "C" int mg_hpsi(mg_ctx* c, int b, double* hpsi, double* e, double* disp) {
@@ -549,14 +548,14 @@ extern "C" int mg_get_densities(mg_ctx* c, double* rho, double* tau, double* nab
     MG_TRY(copy_out(c, nablaj, c->nablaj, 2 * V));
     MG_TRY(copy_out(c, derrho, c->derrho, 6 * V));
     MG_TRY(copy_out(c, laprho, c->laprho, 2 * V));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
 extern "C" int mg_get_jmunu(mg_ctx* c, double* jmunu) {
     if (!c || !jmunu || !c->tensor) return MG_ERR_ARG;
     MG_TRY(copy_out(c, jmunu, c->jmunu, 18 * c->V));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
@@ -590,6 +589,8 @@ extern "C" int mg_solve_coulomb(mg_ctx* c, int* iters) {
     int it = 0;
     const int st = coulomb_solve(c, &it);
     if (iters) *iters = it;
+    MG_TRY(st);
+    MG_TRY(tc_result(c));   // of the density
     return st;
 }
 
@@ -642,7 +643,7 @@ extern "C" int mg_get_potentials(mg_ctx* c, double* u, double* b, double* nablab
     MG_TRY(copy_out(c, divw, c->divW, 6 * V));
     MG_TRY(copy_out(c, coul, c->coulomb, V));
     MG_TRY(copy_out(c, coulex, c->coulex, V));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
@@ -663,6 +664,7 @@ extern "C" int mg_set_potentials(mg_ctx* c, const double* u, const double* b,
 extern "C" int mg_energy(mg_ctx* c, mg_energy_terms* out) {
     if (!c || !out) return MG_ERR_ARG;
     MG_TRY(energy(c, out));
+    MG_TRY(tc_result(c));
     return coulomb_status(c);   // of mg_construct_potentials without its iteration count
 }
 
@@ -682,7 +684,10 @@ extern "C" int mg_solve_pairing(mg_ctx* c, mg_pairing_info* info) {
     if (!c || c->p.pairing != MG_PAIRING_HFB) return MG_ERR_ARG;
     if (!(c->hfb.pp.rhosat > 0)) return MG_ERR_STATE;  // mg_set_pairing first
     if (!c->bas[MG_HF_BASIS].have_qn) return MG_ERR_STATE;
-    return hfb_solve(c, info);
+    const int st = hfb_solve(c, info);
+    MG_TRY(st);
+    MG_TRY(tc_result(c));   // of what it has waited for
+    return st;
 }
 
 extern "C" int mg_get_hfb_block(mg_ctx* c, int b, double* rho, double* kappa, double* delta) {
@@ -693,7 +698,7 @@ extern "C" int mg_get_hfb_block(mg_ctx* c, int b, double* rho, double* kappa, do
     if (rho) MG_CUDA(cudaMemcpyAsync(rho, H.rho + off, (size_t)N * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (kappa) MG_CUDA(cudaMemcpyAsync(kappa, H.kappa + off, (size_t)N * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (delta) MG_CUDA(cudaMemcpyAsync(delta, H.delta + off, (size_t)N * N * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return N;
 }
 
@@ -703,7 +708,7 @@ extern "C" int mg_get_pairing_field(mg_ctx* c, double* re, double* im, double* d
     MG_TRY(copy_out(c, re, c->hfb.fre, 2 * V));
     MG_TRY(copy_out(c, im, c->hfb.fim, 2 * V));
     MG_TRY(copy_out(c, dfac, c->hfb.dfac, 2 * V));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     return MG_OK;
 }
 
@@ -825,8 +830,8 @@ extern "C" int mg_iterate(mg_ctx* c, int n_iter, double dt, double momentum,
             c->side_derive_pending = true;
             const int sp = mg_solve_pairing(c, nullptr);
             if (c->side_derive_pending) MG_TRY(side_derive_hf(c));   // not forked
-            MG_TRY(sp);
             MG_CUDA(cudaStreamWaitEvent(c->stream, c->ev_join, 0));
+            MG_TRY(sp);
             MG_TRY(derive_basis(c, MG_CAN_BASIS));
         } else {
             MG_TRY(mg_hf_fill(c));
@@ -852,14 +857,13 @@ extern "C" int mg_iterate(mg_ctx* c, int n_iter, double dt, double momentum,
         // CompEnergy every pass (src/Main.f90:309): it also keeps the energy
         // history of the convergence check
         mg_energy_terms e{};
-        // the tensor-core status word comes back with the energy's readback
-        if (k == n_iter - 1) MG_TRY(tc_status_async(c));
         MG_TRY(energy(c, out ? out : &e));
+        MG_TRY(tc_result(c));
         MG_TRY(coulomb_status(c));
         phase_mark(c, MG_PH_ENERGY);
         MG_TRY(phase_end(c));
     }
-    MG_TRY(n_iter > 0 ? tc_status_result(c) : tc_check(c));
+    if (n_iter == 0) MG_TRY(sync_results(c));
     return st;
 }
 

@@ -325,7 +325,7 @@ k_gs_overlap_tc(const double* __restrict__ psi, const double* __restrict__ z, Bl
         }
     }
     ok = __syncthreads_and(ok) != 0;
-    if (!ok && tid == 0) atomicExch(status, 1);
+    if (!ok && tid == 0) tc::report_timeout(status);
     tc::fence_before();
     __syncthreads();
     if (warp == 0) tc::dealloc(tmem_slot, 512u);
@@ -635,7 +635,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
         ok = __syncthreads_and(ok) != 0;
         if (!ok) break;
     }
-    if (!ok && tid == 0) atomicExch(status, 1);
+    if (!ok && tid == 0) tc::report_timeout(status);
     tc::fence_before();
     __syncthreads();
     if (warp == 0) tc::dealloc(tmem_slot, 512u);
@@ -872,7 +872,7 @@ k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
         }
     }
     ok = __syncthreads_and(ok) != 0;
-    if (!ok && tid == 0) atomicExch(status, 1);
+    if (!ok && tid == 0) tc::report_timeout(status);
     tc::fence_before();
     __syncthreads();
     if (warp == 0) tc::dealloc(tmem_slot, 512u);

@@ -238,12 +238,14 @@ struct mg_ctx {
     // (deriv_tc.cu), bf16: per (axis, slot) six planes, for the FP64 form seven
     uint16_t* tcmats = nullptr;
     int* tc_erow = nullptr;       // [axis][slot] row exponents
-    int* tc_status = nullptr;     // set when an MMA completion wait ran out
+    // set by a tensor-core kernel one of whose waits ran out: a word of host memory, by
+    // its address there and on the device
+    int* h_tc_status = nullptr;
+    int* tc_status = nullptr;
     long tc_off[2][3][2];         // [0 mixed, 1 FP64][axis][slot]
     bool tc_ok = false;           // every line length <= 48: the mixed form's derivatives
     bool tc_ok64 = false;         // every line length <= 32: the FP64 form's
     bool tc_mesh_ok = false;      // mesh-sized GEMMs on the tensor cores (blocks <= kMeshTcMax)
-    int* h_tc_status = nullptr;   // pinned copy of tc_status, read with the energy's sync
     // largest grid of the persistent tensor-core derivative kernel (0: one CTA
     // per SM); set while it runs beside other work on the side stream
     int tc_grid_cap = 0;
@@ -403,10 +405,11 @@ int run_jobs(mg_ctx* c, const GridJob* jobs, int njobs, bool out_df = false);
 int derive_basis(mg_ctx* c, int b);
 int tc_setup(mg_ctx* c);
 int derive_basis_tc(mg_ctx* c, int b, bool f64);
-int tc_check(mg_ctx* c);
-// tc_check in two halves: enqueue the status copy, read it after a later sync
-int tc_status_async(mg_ctx* c);
-int tc_status_result(mg_ctx* c);
+// Whether a wait of a tensor-core kernel ran out (MG_ERR_TIMEOUT), read after a
+// synchronisation behind it; reported once.
+int tc_result(mg_ctx* c);
+// Waits for the stream, then that: what every call does that hands out results.
+int sync_results(mg_ctx* c);
 
 int hpsi_basis(mg_ctx* c, int b, double* out, bool grad_step, double fac, double mom);
 int hpsi_single(mg_ctx* c, double* psi, const double* der, const double* lap, const int* qn_dev,

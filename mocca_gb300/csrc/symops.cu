@@ -179,7 +179,7 @@ extern "C" int mg_symmetry_operators(mg_ctx* c, int b, double* out) {
     std::vector<double> h((size_t)nwt * nch * kQ);
     MG_CUDA(cudaMemcpyAsync(h.data(), c->red, h.size() * sizeof(double), cudaMemcpyDeviceToHost,
                             c->stream));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     for (int i = 0; i < nwt; ++i) {
         double s[kQ] = {0, 0, 0, 0, 0};
         for (int q = 0; q < nch; ++q)
@@ -218,7 +218,7 @@ extern "C" int mg_angular_momentum(mg_ctx* c, int b, double* out) {
     std::vector<double> h((size_t)nwt * nch * kJ);
     MG_CUDA(cudaMemcpyAsync(h.data(), c->red, h.size() * sizeof(double), cudaMemcpyDeviceToHost,
                             c->stream));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
+    MG_TRY(sync_results(c));
     for (int i = 0; i < nwt; ++i) {
         double s[kJ] = {0, 0, 0};
         for (int q = 0; q < nch; ++q)

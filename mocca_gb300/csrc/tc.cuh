@@ -123,6 +123,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mbar, uint32_t parity, long 
     return true;
 }
 
+// The context's status word, in host memory: a wait ran out.
+__device__ __forceinline__ void report_timeout(int* status) {
+    asm volatile("st.relaxed.sys.global.s32 [%0], 1;" ::"l"(status) : "memory");
+}
+
 __device__ __forceinline__ void mbar_arrive(uint64_t* mbar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(mbar)) : "memory");
 }

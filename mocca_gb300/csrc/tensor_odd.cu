@@ -474,6 +474,5 @@ extern "C" int mg_get_time_odd_tensor(mg_ctx* c, double* vect, double* vecf, dou
         if (dst[q])
             MG_CUDA(cudaMemcpyAsync(dst[q], src[q], (q == 6 ? 2 : 6) * V * sizeof(double),
                                     cudaMemcpyDeviceToHost, c->stream));
-    MG_CUDA(cudaStreamSynchronize(c->stream));
-    return MG_OK;
+    return mg::sync_results(c);
 }

@@ -71,7 +71,7 @@ extern "C" int mg_break_symmetries(mg_ctx* ev8, mg_ctx* full) {
     if (!S.have_qn) return MG_ERR_STATE;
     const int nwt = a.nwt;
     // the EV8 context's work is done before the other stream reads it
-    MG_CUDA(cudaStreamSynchronize(ev8->stream));
+    MG_TRY(sync_results(ev8));
     if (nwt > 0) {
         const long V8 = 8 * ev8->V;
         k_unfold<<<dim3(std::max(1, std::min(1024, div_up(V8, kThreads * 4))), nwt, 4), kThreads,

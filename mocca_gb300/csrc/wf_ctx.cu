@@ -307,7 +307,7 @@ int from_context(mg_ctx* c, const char* force_name, mg_wf& w) {
     if (hfb) {
         MG_CUDA(cudaMemcpyAsync(w.d[MG_WF_CUTOFFS].data(), c->hfb.pcut, nwt * sizeof(double),
                                 cudaMemcpyDeviceToHost, c->stream));
-        MG_CUDA(cudaStreamSynchronize(c->stream));
+        MG_TRY(sync_results(c));
         MG_TRY(hfb_matrices(c, w));
     } else {
         guess_hf_matrices(w, B.h_qn, nwt);

@@ -16,6 +16,8 @@ void poke_cg_sum_wait(mg_ctx* c, long long clocks, int from) {
     c->cg_sum_wait = clocks;
     c->cg_sum_wait_from = from;
 }
+// a wait of a tensor-core kernel has run out
+void poke_tc_timeout(mg_ctx* c) { *c->h_tc_status = 1; }
 }
 """
 
@@ -31,4 +33,6 @@ def load():
     lib = C.CDLL(str(d / "poke.so"))
     lib.poke_cg_sum_wait.argtypes = [C.c_void_p, C.c_longlong, C.c_int]
     lib.poke_cg_sum_wait.restype = None
+    lib.poke_tc_timeout.argtypes = [C.c_void_p]
+    lib.poke_tc_timeout.restype = None
     return lib
