@@ -846,9 +846,7 @@ void multigrid_free(Multigrid* M) {
     delete M;
 }
 
-static int multigrid_setup(mg_ctx* c) {
-    Multigrid* M = new Multigrid();
-    c->mgrid = M;
+static int multigrid_build(mg_ctx* c, Multigrid* M) {
     int n[3] = {c->nx, c->ny, c->nz};
     double h = c->p.dx;
     long total = 0;
@@ -916,6 +914,18 @@ static int multigrid_setup(mg_ctx* c) {
     }
     MG_CUDA(cudaMallocHost(&M->h_S, 2 * sizeof(PcgScalars)));
     for (cudaEvent_t& e : M->read) MG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return MG_OK;
+}
+
+// The context's hierarchy; none when it cannot be had (MG_ERR_ARG: a mesh without one).
+static int multigrid_setup(mg_ctx* c) {
+    Multigrid* M = new Multigrid();
+    const int st = multigrid_build(c, M);
+    if (st != MG_OK) {
+        multigrid_free(M);
+        return st;
+    }
+    c->mgrid = M;
     return MG_OK;
 }
 

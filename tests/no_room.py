@@ -198,7 +198,45 @@ def retried(room):
         assert dt2 == dt and np.array_equal(got, want)
 
 
+def multigrid(room):
+    """A Coulomb multigrid that cannot be set up, for want of room or because the
+    mesh has none, is refused as often as it is asked for."""
+    from mocca_gb300 import MG_FP64, SLY4, RunParams, _abi
+    from mocca_gb300.mesh import MeshState
+
+    def state(n):
+        p = RunParams(nx=n[0], ny=n[1], nz=n[2], dx=0.8, nwt=2, neutrons=20, protons=20,
+                      precision=MG_FP64, coulomb_solver=2)
+        g = MeshState(p, SLY4)
+        g.set_densities(rho=np.random.default_rng(4).uniform(0.0, 0.08, 2 * p.V))
+        g.CalculateAllMoments()
+        return g
+
+    with state((17, 17, 17)) as g:
+        for _ in range(3):
+            refused(g.SolveCoulomb, _abi.MG_ERR_ARG)
+    n = (24, 20, 28)
+    V = n[0] * n[1] * n[2]
+    with state(n) as g:
+        its = g.SolveCoulomb()
+        want = g.get_potentials()["coulomb"]
+    with state(n) as g:
+        # a double per point, the levels' floats, the partials, the sweep matrix
+        parts = max(3 * 3 * 7, 256)
+        coarse = 6 * 5 * 7
+        for size in (8 * V, 4 * 3 * (V + V // 8 + V // 64), 3 * 8 * parts, 4 * coarse ** 2):
+            seen = room.refusals()
+            room.refuse(size)
+            for _ in range(2):
+                refused(g.SolveCoulomb, _abi.MG_ERR_CUDA)
+            room.refuse()
+            assert room.refusals() == seen + 2, size
+        assert g.SolveCoulomb() == its
+        assert np.array_equal(g.get_potentials()["coulomb"], want)
+
+
 CASES = {
+    "multigrid": multigrid,
     "retried": retried,
     "gram_schmidt_fp64": lambda room: gram_schmidt(room, 0, 1e-13),
     "gram_schmidt_mixed": lambda room: gram_schmidt(room, 1, 1e-11),
