@@ -11,10 +11,10 @@
 //   mixed form  six digits (47-bit operands), four accumulators, stored as
 //               {hi, lo} float pairs, the format the double-float consumers
 //               read;
-//   FP64 form   eight digits (62-bit operands), seven accumulators, rounded once
+//   FP64 form   eight digits (62-bit operands), eight accumulators, rounded once
 //               to FP64.  Its error is below that of the FP64 FMA chain it
 //               replaces (ozaki.cuh), which is bound by the FP64 pipe: 2104 us
-//               against 336 us here at 24^3 with 160 spwfs.
+//               against 327 us here at 24^3 with 160 spwfs.
 //
 // One persistent CTA per SM walks 128-line tiles of one matrix slot (the
 // basis' jobs are sorted by slot, the CTAs divided between the two slots by
@@ -22,8 +22,9 @@
 // warp-specialised roles:
 //   warps 0-7   slicers: two lanes per line (lanes l and l + 16 of a warp),
 //               each with every other chunk of four points; they prefetch the
-//               next tile's points with cp.async into slots of their own while
-//               they turn the current ones into digit planes;
+//               next tile's points with cp.async into slots of their own, before
+//               they turn the current ones into digit planes or, where shared
+//               memory has one slot only, behind their last reads of it;
 //   warp 8      MMA issue (one thread): the digit pairs of both derivatives'
 //               columns together (mixed form), or of the first's, then of the
 //               second's, with a commit each (FP64 form, whose accumulators
@@ -34,10 +35,10 @@
 //               to are loaded while the chunk before it is worked on.
 // The kernel is bound by instruction issue (63% of the slots at 24^3; HBM and
 // the tensor pipe below 30%).  Two things brought it there.  The digit planes
-// of a column block's matrix are stacked, so that one MMA of up to 256 columns
-// serves every pair of a line digit (issue_stacked in ozaki.cuh): with one MMA
+// of a column block's matrix are stacked, so that an MMA of up to 192 columns
+// serves several pairs of a line digit (stacked_pairs in ozaki.cuh): with one MMA
 // of 32 columns per pair, about 125 clocks each, the MMAs bound the kernel
-// (FP64 form 660 us, now 336).  And separate column blocks give the two
+// (FP64 form 660 us, now 327).  And separate column blocks give the two
 // epilogue groups straight code and let one block's MMAs run under the other's
 // epilogue, while every plane, slot and address that one thread alone uses
 // needs no barrier.  DeriveAll of one basis, mixed form, against one epilogue
@@ -76,11 +77,20 @@ constexpr int kBlockWarps = 8;                  // epilogue warps of one column 
 constexpr int kThreads = kSlicers + 32 + 2 * 32 * kBlockWarps;   // 800
 constexpr long long kWaitCycles = 4000000000LL; // ~2 s at the top SM clock
 constexpr int kMaxLine = 48;                    // mixed form
-constexpr int kMaxLine64 = 32;                  // FP64 form (seven accumulators of 2 x 32 columns)
+constexpr int kMaxLine64 = 32;                  // FP64 form (eight accumulators of 2 x 32 columns)
 
-// Buffers by K: up to 32 points two plane buffers and two staging slots, at
-// 48 one of each (the planes of 128 x 48 digits take 74 KB).
+// Buffers by K: up to 32 points two plane buffers, at 48 one (the planes of 128 x 48
+// digits take 74 KB); a second staging slot where there is room for it beside them and
+// the matrices with their planes of zeros.
 constexpr int nbuf_of(int kp) { return kp <= 32 ? 2 : 1; }
+constexpr int nslot_of(int kp, bool f64) { return kp == 48 || (f64 && kp == 32) ? 1 : 2; }
+constexpr int blocks_of(bool f64) { return f64 ? 2 : 1; }   // MMA blocks, see k_deriv_tc
+constexpr int digits_of_form(bool f64) { return f64 ? oz::kDigits64 : oz::kDigits; }
+// bytes of a matrix plane of a block, planes of both derivatives with their zeros
+constexpr int plane_bytes(int kp, bool f64) { return 2 * kp / blocks_of(f64) * kp * 2; }
+constexpr int matrix_planes(int kp, bool f64) {
+    return blocks_of(f64) * oz::stack_planes(digits_of_form(f64), 2 * kp / blocks_of(f64));
+}
 constexpr int accs_of(bool f64) { return f64 ? oz::kAccs64 : (int)oz::kAccs; }
 // TMEM accumulator sets: two where 512 columns hold them
 constexpr int tbuf_of(int kp, int nacc) { return 4 * nacc * kp <= 512 ? 2 : 1; }
@@ -171,17 +181,18 @@ __device__ __forceinline__ void store4(double* p, const double (&o)[4], int left
 template <int KP, bool F64, bool XP>
 __global__ void __launch_bounds__(kThreads, 1)
 k_deriv_tc(TcPass P) {
-    constexpr int ND = F64 ? oz::kDigits64 : oz::kDigits;
+    constexpr int ND = digits_of_form(F64);
     constexpr int NACC = accs_of(F64);
     static_assert(!F64 || KP <= kMaxLine64, "combine64 holds sums of at most 32 terms");
-    constexpr int NBUF = nbuf_of(KP), NTB = tbuf_of(KP, NACC);
+    constexpr int NBUF = nbuf_of(KP), NSLOT = nslot_of(KP, F64), NTB = tbuf_of(KP, NACC);
     // FP64 form: the two derivatives' columns are two MMA blocks with commits of
     // their own; mixed form: one block of 2 KP columns
-    constexpr int NBLK = F64 ? 2 : 1, COLS = 2 * KP / NBLK;
+    constexpr int NBLK = blocks_of(F64), COLS = 2 * KP / NBLK;
     constexpr int kPlane = kTile * KP * 2;     // bytes of one digit plane of a tile
     constexpr int kKg = KP / 8;                // K groups of 8
     constexpr uint32_t kSboK = 128u * kKg;     // stride byte offset of the planes
-    constexpr int kBlockB = ND * KP * KP * 2;  // bytes of a column block's matrix planes
+    constexpr int kPlaneB = plane_bytes(KP, F64);
+    constexpr int kZerosB = oz::stack_zeros(ND, COLS) * kPlaneB, kBlockB = ND * kPlaneB;
     extern __shared__ uint8_t smraw[];
     __shared__ TcShared<NBUF, NTB, NBLK> S;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -194,8 +205,8 @@ k_deriv_tc(TcPass P) {
 
     const uint32_t s0 = tc::smem_u32(smraw);
     uint8_t* sA = smraw + ((128u - (s0 & 127u)) & 127u);        // NBUF x ND planes
-    uint8_t* sB = sA + NBUF * ND * kPlane;                      // 2 x ND planes of KP rows
-    uint8_t* sIn = sB + 2 * kBlockB;                            // NBUF x nch8 x 2 x kSlicers x 16
+    uint8_t* sB = sA + NBUF * ND * kPlane;                      // per block zeros, ND planes
+    uint8_t* sIn = sB + NBLK * (kZerosB + kBlockB);             // NSLOT x nch8 x 2 x kSlicers x 16
 
     if (warp == 0) tc::alloc(&S.tmem, tmem_cols(KP, NACC));
     if (tid == 0) {
@@ -211,9 +222,12 @@ k_deriv_tc(TcPass P) {
         for (int b = 0; b < 4; ++b) tc::mbar_init(&S.emaxReady[b], kSliceWarps);
     }
     {
-        const uint4* src = reinterpret_cast<const uint4*>(P.bmat[slot]);
-        uint4* dst = reinterpret_cast<uint4*>(sB);
-        for (int t = tid; t < 2 * kBlockB / 16; t += kThreads) dst[t] = src[t];
+        for (int h = 0; h < NBLK; ++h) {
+            const uint4* src = reinterpret_cast<const uint4*>(P.bmat[slot]) + h * (kBlockB / 16);
+            uint4* dst = reinterpret_cast<uint4*>(sB + h * (kZerosB + kBlockB));
+            for (int t = tid; t < (kZerosB + kBlockB) / 16; t += kThreads)
+                dst[t] = t < kZerosB / 16 ? make_uint4(0u, 0u, 0u, 0u) : src[t - kZerosB / 16];
+        }
         // K columns past the line stay zero
         uint4* a = reinterpret_cast<uint4*>(sA);
         for (int t = tid; t < NBUF * ND * kPlane / 16; t += kThreads)
@@ -245,41 +259,48 @@ k_deriv_tc(TcPass P) {
             return reinterpret_cast<double*>(
                 sIn + ((size_t)((sbuf * nch8 + i) * 2 + pair) * kSlicers + tid) * 16);
         };
-        // whether this lane's line of the tile exists
-        auto prefetch = [&](int T, int sbuf) {
+        // this lane's first point of the tile, null where its line does not exist
+        auto first_point = [&](int T) -> const double* {
+            if (T >= ntiles) return nullptr;
             const int job = quotient(T, P.tpj_inv), l = (T - job * P.tpj) * kTile + row;
-            if (l >= P.nlines) return false;
-            const double* in = P.jobs[perm[job]].in + line_offset(P, l) + 4 * h * lstride;
-#pragma unroll 1
-            for (int i = 0, k0 = 4 * h; k0 < n; ++i, k0 += 8) {
-                if (XP && (n & 1) == 0) {
-                    // even lines: 16-byte copies (line starts and k0 are even)
-                    cp_async16(slot_at(sbuf, i, 0), in);
-                    if (k0 + 2 < n) cp_async16(slot_at(sbuf, i, 1), in + 2);
-                    in += 8;
-                } else {
+            if (l >= P.nlines) return nullptr;
+            return P.jobs[perm[job]].in + line_offset(P, l) + 4 * h * lstride;
+        };
+        // copies chunk i (points k0 = 4 h + 8 i, ...) at `in`, which moves on to the next
+        auto prefetch = [&](const double*& in, int sbuf, int i) {
+            const int k0 = 4 * h + 8 * i;
+            if (XP && (n & 1) == 0) {
+                // even lines: 16-byte copies (line starts and k0 are even)
+                cp_async16(slot_at(sbuf, i, 0), in);
+                if (k0 + 2 < n) cp_async16(slot_at(sbuf, i, 1), in + 2);
+                in += 8;
+            } else {
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        if (k0 + u < n) tc::cp_async8(slot_at(sbuf, i, u >> 1) + (u & 1), in);
-                        in += lstride;
-                    }
-                    in += 4 * lstride;
+                for (int u = 0; u < 4; ++u) {
+                    if (k0 + u < n) tc::cp_async8(slot_at(sbuf, i, u >> 1) + (u & 1), in);
+                    in += lstride;
                 }
+                in += 4 * lstride;
             }
-            return true;
+        };
+        auto prefetch_all = [&](const double* in, int sbuf) {
+            if (in)
+#pragma unroll 1
+                for (int i = 0; 4 * h + 8 * i < n; ++i) prefetch(in, sbuf, i);
         };
         int T = cta;
-        bool next_live = T < ntiles && prefetch(T, 0);
+        const double* next = first_point(T);
+        prefetch_all(next, 0);
         tc::cp_async_commit();
         for (int k = 0; T < ntiles; T += nctas, ++k) {
-            const int buf = k % NBUF;
-            const bool live = next_live;
+            const int buf = k % NBUF, sbuf = k % NSLOT;
+            const bool live = next != nullptr;
             tc::cp_async_wait_all();
             // the points of chunk i, zero past the line's end
             auto chunk = [&](int i, double (&v)[4]) {
 #pragma unroll
                 for (int pair = 0; pair < 2; ++pair) {
-                    const double2 x = *reinterpret_cast<const double2*>(slot_at(buf, i, pair));
+                    const double2 x = *reinterpret_cast<const double2*>(slot_at(sbuf, i, pair));
                     const int q = 4 * (2 * i + h) + 2 * pair;
                     v[2 * pair] = live && q < n ? x.x : 0.0;
                     v[2 * pair + 1] = live && q + 1 < n ? x.y : 0.0;
@@ -295,10 +316,11 @@ k_deriv_tc(TcPass P) {
             }
             top = max(top, __shfl_xor_sync(0xffffffffu, top, 16));
             const int emax = (int)(top >> 20);
-            const int Tn = T + nctas;
-            if (NBUF == 2) {
+            next = first_point(T + nctas);
+            const double* ahead = next;
+            if (NSLOT == 2) {
                 // the other staging slot was read in the iteration before
-                next_live = Tn < ntiles && prefetch(Tn, buf ^ 1);
+                prefetch_all(next, sbuf ^ 1);
                 tc::cp_async_commit();
             }
             if (k >= NBUF) {
@@ -314,6 +336,7 @@ k_deriv_tc(TcPass P) {
             for (int i = 0; 4 * (2 * i + h) < n; ++i) {
                 double v[4];
                 chunk(i, v);
+                if (NSLOT == 1 && NBUF == 2 && ahead) prefetch(ahead, 0, i);
                 uint2 w[ND];
                 oz::digits4<ND>(v, fixed, w);
 #pragma unroll
@@ -322,9 +345,11 @@ k_deriv_tc(TcPass P) {
             }
             tc::fence_proxy_async();
             arrive_warp(&S.fullA[buf], lane);
-            if (NBUF == 1) {
-                // one staging slot: the next tile's points once these are sliced
-                next_live = Tn < ntiles && prefetch(Tn, 0);
+            if (NSLOT == 1) {
+                // with one plane buffer the MMAs leave time for all of the next tile's
+                // points (36^3: 1016 us this way, 1072 chunk by chunk; FP64 at 24^3 with
+                // two buffers 335 and 328)
+                if (NBUF == 1) prefetch_all(next, 0);
                 tc::cp_async_commit();
             }
         }
@@ -341,10 +366,10 @@ k_deriv_tc(TcPass P) {
                         ok = tc::mbar_wait(&S.emptyT[h][tb], ((k - NTB) / NTB) & 1, kWaitCycles);
                     if (!ok) break;
                     tc::fence_after();
-                    oz::issue_stacked<ND, NACC, COLS, KP / 16>(
+                    oz::issue_stacked<ND, COLS, KP / 16>(
                         tmem + (uint32_t)((tb * NBLK + h) * NACC * COLS),
                         tc::smem_u32(sA + buf * ND * kPlane), kPlane,
-                        tc::smem_u32(sB) + (uint32_t)h * (ND * COLS * KP * 2), kSboK);
+                        tc::smem_u32(sB + h * (kZerosB + kBlockB) + kZerosB), kSboK);
                     if (h == NBLK - 1) tc::commit(&S.emptyA[buf]);
                     tc::commit(&S.fullT[h][tb]);
                 }
@@ -484,9 +509,10 @@ k_deriv_tc(TcPass P) {
 int kp_of(int n) { return n <= 16 ? 16 : (n <= 32 ? 32 : 48); }
 
 size_t smem_bytes(int n, bool f64) {
-    const int kp = kp_of(n), nd = f64 ? oz::kDigits64 : oz::kDigits;
-    return 128 + (size_t)nbuf_of(kp) * nd * kTile * kp * 2 + (size_t)nd * 2 * kp * kp * 2 +
-           (size_t)nbuf_of(kp) * ((n + 7) / 8) * 2 * kSlicers * 16;
+    const int kp = kp_of(n);
+    return 128 + (size_t)nbuf_of(kp) * digits_of_form(f64) * kTile * kp * 2 +
+           (size_t)matrix_planes(kp, f64) * plane_bytes(kp, f64) +
+           (size_t)nslot_of(kp, f64) * ((n + 7) / 8) * 2 * kSlicers * 16;
 }
 
 template <bool F64>

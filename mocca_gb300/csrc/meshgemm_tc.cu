@@ -25,9 +25,9 @@
 //                     GradDesc history upd_l = out_l - upd_l.  Canonical basis
 //                     (HFBOccupations, src/HFB.f90:3448-3487): C = CanTransfo,
 //                     HF basis in, canonical basis out.
-// A chunk keeps the digit-weight groups of the overlap that have an accumulator of
-// their own below 2^24 (at most 3 pairs x 256 points x 2^14, in the FP64 form 6 x 128),
-// so their FP32 sums are exact.
+// A chunk keeps the digit weights of the overlap that have an accumulator of their own
+// within 2^24 (at most 3 pairs x 256 points x 2^14, in the FP64 form 8 x 128), so their
+// FP32 sums are exact.
 #include <algorithm>
 #include <vector>
 
@@ -69,10 +69,11 @@ __device__ __forceinline__ double pow2d(int x) {
 // the roles of k_apply_tc: the slicers cut stages of kStage points into a ring of
 // plane buffers, one thread issues a stage's MMAs, the epilogue writes a unit's sums
 // while the next unit's stages go on.  A's rows are the planes' own, one after the
-// other, so that the planes are B's stacked columns too; what A reads past a plane's
-// NP rows gives rows of D that nothing reads.  The tensor pipe bounds it (36 MMAs of
-// ~130 clocks a stage of 32 points): 300 spwfs of 36^3 (blocks of 75) 566 us, 834
-// with a CTA per chunk; the FP64 form for 160 of 24^3 (40) 156, 512 by FP64 FMAs.
+// other, so that the planes are B's stacked columns too, behind the planes of zeros that
+// the stack begins with; what A reads past a plane's NP rows gives rows of D that
+// nothing reads.  300 spwfs of 36^3 (blocks of 75, 38 MMAs a stage of 32 points) 566
+// us, 834 with a CTA per chunk; the FP64 form for 160 of 24^3 (40, 24 MMAs) 150, 512
+// by FP64 FMAs.
 constexpr int kRoleWarps = 8;                       // epilogue: warps 0-7, slicers: 8-15
 constexpr int kRoleThreads = 2 * kRoleWarps * 32 + 32;   // and the MMA warp
 constexpr int kSmemCap = 225 * 1024;
@@ -81,14 +82,22 @@ constexpr int kNone = 255;
 __host__ __device__ constexpr int accs_for(int nd) { return nd == oz::kDigits64 ? oz::kAccs64 : (int)oz::kAccs; }
 __host__ __device__ constexpr int chunk_for(int nd) { return nd == oz::kDigits64 ? 128 : kChunk; }
 __host__ __device__ constexpr int tbufs_for(int nd, int np) { return 2 * accs_for(nd) * np <= 512 ? 2 : 1; }
-__host__ __device__ constexpr int overlap_stage(int nd, int np, bool two) {
-    return (two ? 2 : 1) * nd * np * kStage * 2;
+// A stage's planes: of two operands A's, zeros, B's; of one zeros and the planes of both.
+__host__ __device__ constexpr int overlap_a(int nd, int np, bool two) {
+    return two ? 0 : oz::stack_zeros(nd, np);
 }
-constexpr int kOverlapTail = kRows * kStage * 2;    // A's reads past the last plane
+__host__ __device__ constexpr int overlap_b(int nd, int np, bool two) {
+    return (two ? nd : 0) + oz::stack_zeros(nd, np);
+}
+__host__ __device__ constexpr int overlap_stage(int nd, int np, bool two) {
+    return (overlap_b(nd, np, two) + nd) * np * kStage * 2;
+}
+// A's reads past its last plane: of two operands they end in the planes behind it
+__host__ __device__ constexpr int overlap_tail(bool two) { return two ? 0 : kRows * kStage * 2; }
 __host__ __device__ constexpr int overlap_bufs(int nd, int np, bool two) {
     // (8 KB left for the kernels' static shared memory)
-    return (kSmemCap - 8192 - 128 - kOverlapTail) / overlap_stage(nd, np, two) >= 6
-               ? 6 : (kSmemCap - 8192 - 128 - kOverlapTail) / overlap_stage(nd, np, two);
+    const int n = (kSmemCap - 8192 - 128 - overlap_tail(two)) / overlap_stage(nd, np, two);
+    return n >= 6 ? 6 : n;
 }
 // (more than half of an SM's, so that no second CTA comes beside one that holds all
 // TMEM columns and waits for them)
@@ -97,7 +106,8 @@ __host__ __device__ constexpr size_t one_cta(size_t bytes) {
     return bytes > kOneCtaSmem ? bytes : kOneCtaSmem;
 }
 __host__ __device__ constexpr size_t overlap_smem(int nd, int np, bool two) {
-    return one_cta((size_t)overlap_bufs(nd, np, two) * overlap_stage(nd, np, two) + kOverlapTail + 128);
+    return one_cta((size_t)overlap_bufs(nd, np, two) * overlap_stage(nd, np, two) +
+                   overlap_tail(two) + 128);
 }
 
 __device__ __forceinline__ bool wait_warp(uint64_t* mbar, uint32_t parity) {
@@ -117,6 +127,8 @@ k_gs_overlap_tc(const double* __restrict__ psi, const double* __restrict__ z, Bl
     constexpr int NACC = accs_for(ND), NBUF = overlap_bufs(ND, NP, kTwo), NTB = tbufs_for(ND, NP);
     constexpr int CH = chunk_for(ND), kPlane = NP * kStage * 2, kBuf = overlap_stage(ND, NP, kTwo);
     constexpr int kArr = kTwo ? 2 : 1;
+    constexpr int kA = overlap_a(ND, NP, kTwo) * kPlane, kB = overlap_b(ND, NP, kTwo) * kPlane;
+    static_assert(!kTwo || kBuf >= (ND - 1) * kPlane + kRows * kStage * 2, "A's reads past its planes");
     constexpr int kPasses = (NP + 63) / 64;   // rows of a slicer: row0, row0 + 64
     extern __shared__ uint8_t smraw[];
     __shared__ __align__(8) uint64_t full[6], empty[6], fullT[2], emptyT[2], expReady[8];
@@ -125,7 +137,7 @@ k_gs_overlap_tc(const double* __restrict__ psi, const double* __restrict__ z, Bl
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t s0a = tc::smem_u32(smraw);
     uint8_t* base = smraw + ((128u - (s0a & 127u)) & 127u);
-    for (int t = tid; t < (NBUF * kBuf + kOverlapTail) / 16; t += kRoleThreads)
+    for (int t = tid; t < (NBUF * kBuf + overlap_tail(kTwo)) / 16; t += kRoleThreads)
         reinterpret_cast<uint4*>(base)[t] = make_uint4(0u, 0u, 0u, 0u);
     if (warp == 0) tc::alloc(&tmem_slot, 512u);
     if (tid == 0) {
@@ -227,7 +239,7 @@ k_gs_overlap_tc(const double* __restrict__ psi, const double* __restrict__ z, Bl
                             oz::digits4<ND>(v4, fixed, w);
 #pragma unroll
                             for (int a = 0; a < ND; ++a)
-                                *reinterpret_cast<uint2*>(planes + (y * ND + a) * kPlane +
+                                *reinterpret_cast<uint2*>(planes + (y == 0 ? kA : kB) + a * kPlane +
                                                           tc::kmajor_off(row, 8 * g + 4 * h)) = w[a];
                         }
                     }
@@ -252,9 +264,8 @@ k_gs_overlap_tc(const double* __restrict__ psi, const double* __restrict__ z, Bl
                     if (!ok) break;
                     tc::fence_after();
                     const uint32_t pa = tc::smem_u32(base + buf * kBuf);
-                    oz::issue_stacked<ND, NACC, NP, kStage / 16>(
-                        tmem + (uint32_t)(tb * NACC * NP), pa, kPlane,
-                        kTwo ? pa + ND * kPlane : pa, tc::kSbo, s > 0);
+                    oz::issue_stacked<ND, NP, kStage / 16>(tmem + (uint32_t)(tb * NACC * NP), pa + kA,
+                                                           kPlane, pa + kB, tc::kSbo, s > 0);
                     tc::commit(&empty[buf]);
                 }
                 if (!ok) break;
@@ -382,8 +393,8 @@ k_coef_digits(const double* __restrict__ coef, long bstride, int ld, BlockIdx bi
 // MMAs, the epilogue takes the accumulators to registers, gives them back and
 // writes.  The integer and FP32 work of cutting and combining bounds it (about 160
 // instructions per entry, 51% of the issue slots), the MMAs come next (one of up to
-// 256 columns holds the tensor pipe ~130 clocks: 54 of them for a tile of 48
-// spinors, 90 for 80).  A CTA per tile went through the same steps one after the
+// 192 columns holds the tensor pipe ~130 clocks: 54 of them for a tile of 48
+// spinors, 95 for 80).  A CTA per tile went through the same steps one after the
 // other: 1628 us for the 300 spwfs of 36^3 (blocks of 75), now 573; 110 for the 160
 // of 24^3 (40), now 77.
 // Epilogue warps.  Up to 48 spinors a slicer's values leave the registers for sixteen:
@@ -394,7 +405,9 @@ __host__ __device__ constexpr int apply_threads(int np) { return 32 * (apply_epi
 __device__ __forceinline__ void tmem_load(uint32_t t, uint32_t (&r)[4]) { tc::ld4(t, r); }
 __device__ __forceinline__ void tmem_load(uint32_t t, uint32_t (&r)[8]) { tc::ld8(t, r); }
 __host__ __device__ constexpr int apply_plane(int np) { return kRows * np * 2; }
-__host__ __device__ constexpr int apply_coef(int nd, int np) { return nd * np * np * 2; }
+// the coefficients' planes behind the zeros that their stack begins with
+__host__ __device__ constexpr int apply_zeros(int nd, int np) { return oz::stack_zeros(nd, np) * np * np * 2; }
+__host__ __device__ constexpr int apply_coef(int nd, int np) { return oz::stack_planes(nd, np) * np * np * 2; }
 // operand and accumulator buffers that fit
 __host__ __device__ constexpr int apply_bufs(int nd, int np) {
     return 2 * nd * apply_plane(np) + apply_coef(nd, np) + 128 <= kSmemCap ? 2 : 1;
@@ -411,7 +424,9 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
            const int* __restrict__ xe, const double* __restrict__ coef, long bstride, int ld,
            long V4, int tpb, int ntiles, int* __restrict__ status) {
     constexpr int NACC = accs_for(ND), NBUF = apply_bufs(ND, NP), NTB = tbufs_for(ND, NP);
-    constexpr int kg = NP / 8, kPlane = apply_plane(NP), EW = apply_epilogue(NP);
+    constexpr int kg = NP / 8, kPlane = apply_plane(NP), kZeros = apply_zeros(ND, NP);
+    constexpr int EW = apply_epilogue(NP);
+    static_assert(apply_smem(ND, NP) <= kSmemCap, "operands");
     constexpr int W = 64 / EW;   // columns of an epilogue chunk, 16 / W warps side by side
     extern __shared__ uint8_t smraw[];
     __shared__ __align__(8) uint64_t fullA[2], emptyA[2], fullT[2], emptyT[2], emaxReady[4];
@@ -448,7 +463,8 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
         {
             const uint4* src = reinterpret_cast<const uint4*>(xd + (long)b * ND * kXdStride);
             uint4* dst = reinterpret_cast<uint4*>(sB);
-            for (int t = tid; t < apply_coef(ND, NP) / 16; t += apply_threads(NP)) dst[t] = src[t];
+            for (int t = tid; t < apply_coef(ND, NP) / 16; t += apply_threads(NP))
+                dst[t] = t < kZeros / 16 ? make_uint4(0u, 0u, 0u, 0u) : src[t - kZeros / 16];
             // K groups past the block's spinors stay zero
             uint4* a = reinterpret_cast<uint4*>(sA);
             for (int t = tid; t < NBUF * ND * kPlane / 16; t += apply_threads(NP))
@@ -538,9 +554,9 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                         ok = tc::mbar_wait(&emptyT[tb], ((k - NTB) / NTB) & 1, kWaitCycles);
                     if (!ok) break;
                     tc::fence_after();
-                    oz::issue_stacked<ND, NACC, NP, NP / 16>(
+                    oz::issue_stacked<ND, NP, NP / 16>(
                         tmem + (uint32_t)(tb * NACC * NP), tc::smem_u32(sA + buf * ND * kPlane),
-                        kPlane, tc::smem_u32(sB), (uint32_t)kg * 128u);
+                        kPlane, tc::smem_u32(sB + kZeros), (uint32_t)kg * 128u);
                     tc::commit(&emptyA[buf]);
                     tc::commit(&fullT[tb]);
                 }
@@ -597,7 +613,8 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
 #pragma unroll
                             for (int g = 0; g < NACC; ++g) acc[g] = r[g][u];
                             const int e = emax - 1023 + ex - 1023 - oz::kUnit64;
-                            // 6 pairs x 42 x 2^14 < 2^22: the magic numbers' range
+                            // 6 pairs x 42 x 2^14 < 2^22: the magic numbers' range (weights
+                            // 6 and 7 are taken far below theirs)
                             if (nb <= 42 && e >= -900 && e <= 900)
                                 x = oz::combine64(acc, e);
                             else
@@ -663,7 +680,9 @@ k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
           int* __restrict__ status) {
     constexpr int NACC = oz::kAccs, NBUF = overlap_bufs(kDigits, NP, true),
                   NTB = tbufs_for(kDigits, NP);
-    constexpr int kPlane = NP * kStage * 2, kBuf = 2 * kDigits * kPlane, nst = kGapPts / 8;
+    constexpr int kPlane = NP * kStage * 2, kBuf = overlap_stage(kDigits, NP, true), nst = kGapPts / 8;
+    constexpr int kB = overlap_b(kDigits, NP, true) * kPlane;
+    static_assert(kBuf >= (kDigits - 1) * kPlane + kRows * kStage * 2, "A's reads past its planes");
     constexpr int kPasses = (NP + 63) / 64;   // rows of a slicer: row0, row0 + 64
     extern __shared__ uint8_t smraw[];
     __shared__ __align__(8) uint64_t full[6], empty[6], fullT[2], emptyT[2], expReady[8];
@@ -674,7 +693,7 @@ k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t s0a = tc::smem_u32(smraw);
     uint8_t* base = smraw + ((128u - (s0a & 127u)) & 127u);
-    for (int t = tid; t < (NBUF * kBuf + kOverlapTail) / 16; t += kGapThreads)
+    for (int t = tid; t < NBUF * kBuf / 16; t += kGapThreads)
         reinterpret_cast<uint4*>(base)[t] = make_uint4(0u, 0u, 0u, 0u);
     if (warp == 0) tc::alloc(&tmem_slot, 512u);
     if (tid == 0) {
@@ -790,7 +809,7 @@ k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
                     oz::digits4_fixed(zx, w);
 #pragma unroll
                     for (int d = 0; d < kDigits; ++d)
-                        *reinterpret_cast<uint2*>(planes + (kDigits + d) * kPlane + o) = w[d];
+                        *reinterpret_cast<uint2*>(planes + kB + d * kPlane + o) = w[d];
                 }
                 tc::fence_proxy_async();
                 arrive_warp(&full[buf], lane);
@@ -810,9 +829,8 @@ k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
                     if (!ok) break;
                     tc::fence_after();
                     const uint32_t pa = tc::smem_u32(base + buf * kBuf);
-                    oz::issue_stacked<kDigits, NACC, NP, kStage / 16>(
-                        tmem + (uint32_t)(tb * NACC * NP), pa, kPlane, pa + kDigits * kPlane,
-                        tc::kSbo, s > 0);
+                    oz::issue_stacked<kDigits, NP, kStage / 16>(
+                        tmem + (uint32_t)(tb * NACC * NP), pa, kPlane, pa + kB, tc::kSbo, s > 0);
                     tc::commit(&empty[buf]);
                 }
                 if (!ok) break;
@@ -988,7 +1006,7 @@ k_gaps_factor(const double* __restrict__ psi, const int* __restrict__ members,
 
 }  // namespace
 
-// Largest and smallest blocks of the FP64 form.  Above 64 its seven accumulators do
+// Largest and smallest blocks of the FP64 form.  Above 64 its eight accumulators do
 // not fit the 512 TMEM columns.  Below 24 the FP64 kernels of gs.cu are as fast or
 // faster; the whole Gram-Schmidt of four blocks at 10^3 / 16^3 / 24^3 in us, there and
 // here: blocks of 16: 54 / 83 / 167 and 64 / 89 / 166, of 24: 83 / 149 / 336 and

@@ -235,7 +235,7 @@ struct mg_ctx {
     long mat32_off[3][2][2];
     int cur_precision = MG_FP64;  // precision of the next kernels (MG_FP64 / MG_MIXED)
     // digit planes of the Lagrange blocks for the tensor-core derivatives
-    // (deriv_tc.cu), bf16: per (axis, slot) six planes, for the FP64 form seven
+    // (deriv_tc.cu), bf16: per (axis, slot) six planes, for the FP64 form eight
     uint16_t* tcmats = nullptr;
     int* tc_erow = nullptr;       // [axis][slot] row exponents
     // set by a tensor-core kernel one of whose waits ran out: a word of host memory, by

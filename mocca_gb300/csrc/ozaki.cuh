@@ -101,15 +101,13 @@ __device__ __forceinline__ void digits4_fixed(const long long (&X)[4], uint2 (&w
 
 // ---- eight digits: operands of 62 bits, results rounded once to FP64 -----------
 //
-// The FP64 form of a contraction over at most 32 terms.  Every entry is
-// rounded to 62 bits of its row's largest (FP64 carries 53 of its own), the
-// 36 digit pairs of weight 0..7 are kept, those of weight 0..5 in six exact
-// accumulators (6 pairs x 32 terms x 2^14 < 2^22) and those of weight 6 and 7
-// in a seventh, rounded near 2^-70 of the row's largest products; the
-// epilogue adds them as one 64-bit integer and rounds it once to FP64.  (An
-// eighth accumulator saves MMAs but not time: 356 us against 336 for DeriveAll
-// at 24^3 with 160 spwfs, the epilogue's loads and registers being the limit.)  A
-// chain of FP64 FMAs rounds every partial sum.  Norm-wise errors against
+// The FP64 form of a contraction over at most 128 terms.  Every entry is rounded to
+// 62 bits of its row's largest (FP64 carries 53 of its own) and the 36 digit pairs of
+// weight 0..7 are kept, each weight in an accumulator of its own, whose sums are exact
+// (8 pairs x 128 terms x 2^14 = 2^24).  The epilogue adds weights 6 and 7 in FP32
+// (rounded at 2^-61 of the largest product of the two rows, which is 2^12 in these
+// units), takes all to a 64-bit integer in units of 2^-56 of it, and rounds that to
+// FP64.  A chain of FP64 FMAs rounds every partial sum.  Norm-wise errors against
 // extended-precision sums on Lagrange lines (5 to 32 points, folded and full):
 // first derivatives 0.5e-16 to 1.1e-16 (the chain: 1.3e-16 to 2.8e-16),
 // Laplacians 0.8e-16 to 2.4e-16 (1.5e-16 to 3.0e-16).
@@ -118,7 +116,7 @@ __device__ __forceinline__ void digits4_fixed(const long long (&X)[4], uint2 (&w
 // 2.6e-16.)
 
 constexpr int kDigits64 = 8;
-constexpr int kAccs64 = 7;
+constexpr int kAccs64 = 8;
 // product units: 2^(E_row + E_col - kUnit64), E as above
 constexpr int kUnit64 = 10;
 
@@ -248,7 +246,7 @@ __device__ __forceinline__ double round64(unsigned long long I, int x) {
     return __hiloint2double((int)(rh | (sgn & 0x80000000u)), (int)(uint32_t)r);
 }
 
-// The seven accumulators' sum times 2^x as FP64: a 64-bit integer in units
+// The eight accumulators' sum times 2^x as FP64: a 64-bit integer in units
 // of 2^-44 (top digits are at most 64, so 32 products stay below 2^18 and the
 // integer below 2^62), rounded once.  The accumulators' magic numbers are carried
 // along and taken off once.
@@ -256,7 +254,7 @@ __device__ __forceinline__ double combine64(const uint32_t (&a)[kAccs64], int x)
     const uint32_t hi = units<0>(a[0]) * 256u + units<8>(a[1]);     // 2^-8
     const uint32_t mid = units<16>(a[2]) * 256u + units<24>(a[3]);  // 2^-24, with its magic >= 0
     const uint32_t low = units<32>(a[4]) * 256u + units<40>(a[5]);  // 2^-40, with its magic >= 0
-    const uint32_t tail = units<44>(a[6]);
+    const uint32_t tail = units<44>(__float_as_uint(__fadd_rn(__uint_as_float(a[6]), __uint_as_float(a[7]))));
     constexpr uint32_t mhi = magic_bits(0) * 256u + magic_bits(8);
     constexpr uint32_t mmid = magic_bits(16) * 256u + magic_bits(24);
     constexpr uint32_t mlow = magic_bits(32) * 256u + magic_bits(40);
@@ -273,14 +271,16 @@ __device__ __forceinline__ double combine64(const uint32_t (&a)[kAccs64], int x)
 // FP32 but past the magic numbers' range; the whole sum is below 2^63 units), and for
 // any x.
 __device__ __forceinline__ double combine64_any(const uint32_t (&a)[kAccs64], int x) {
-    const auto part = [&a](int g, int up, int shift) {
+    const auto part = [](float x, int up, int shift) {
         // a multiple of 2^-up below 2^(31 - up) as an integer, shifted
-        const float f = __uint_as_float(a[g]) * __int_as_float((up + 127) << 23);
+        const float f = x * __int_as_float((up + 127) << 23);
         return (unsigned long long)(long long)__float2int_rn(f) << shift;
     };
-    const unsigned long long I = part(0, 0, 44) + part(1, 8, 36) + part(2, 16, 28) +
-                                 part(3, 24, 20) + part(4, 32, 12) + part(5, 40, 4) +
-                                 part(6, 44, 0);
+    const auto acc = [&a](int g) { return __uint_as_float(a[g]); };
+    const unsigned long long I = part(acc(0), 0, 44) + part(acc(1), 8, 36) +
+                                 part(acc(2), 16, 28) + part(acc(3), 24, 20) +
+                                 part(acc(4), 32, 12) + part(acc(5), 40, 4) +
+                                 part(__fadd_rn(acc(6), acc(7)), 44, 0);
     if (x >= -900 && x <= 900) return round64(I, x);
     // past the exponent range of one step: two exact ones and a rounding
     const int first = x < 0 ? max(x, -1960) / 2 : min(x, 1960) / 2;
@@ -308,55 +308,75 @@ __device__ __forceinline__ float pow2f(int x) {
     return x < -126 ? 0.0f : __int_as_float((min(x, 127) + 127) << 23);
 }
 
-// The digit-pair MMAs of a block of COLS columns with ND digits and NACC
-// accumulators side by side at tmem (COLS columns each): A planes at aBase + a
-// aPlane, the B planes of the block stacked row below row at bBase.  Plane a
-// times the stacked planes 0, 1, ... fills accumulators a, a + 1, ..., so one
-// MMA of up to 256 columns serves all pairs of digit a that have an
-// accumulator of their own; the pairs of the last accumulator's weights follow
-// one by one, in order of weight and a.  (An MMA of 32 columns holds the
-// tensor pipe for as long as one of 192: with a pair per MMA and column block
-// the issue of 84 to 144 MMAs per tile bound the derivative kernel.)
-template <int ND, int NACC, int COLS, int KSTEPS>
+// ---- digit-pair MMAs ------------------------------------------------------------
+//
+// The pairs of a block of `cols` columns with nd digits go into accumulators side by
+// side, `cols` columns each: a weight a + b its own one, in the mixed form the weights
+// from 3 on the last one together.  The B planes of the block are stacked row below
+// row, so that plane a times planes b, b + 1, ... is one MMA of up to 256 columns over
+// accumulators a + b, a + b + 1, ...: an MMA of 32 columns holds the tensor pipe for
+// as long as one of 256 (~130 clocks), and with a pair per MMA the issue of 84 to 144
+// of them per tile bound the derivative kernel.
+//
+// The order of two MMAs into one accumulator is only given where both have the same
+// accumulator columns and the same shape.  So the accumulators come in groups of
+// `width`, and every MMA into a group covers all of it: for the accumulators before a,
+// which have no pair of digit a, the stack begins with planes of zeros.
+__host__ __device__ constexpr int own_accs(int nd) {   // accumulators of one weight
+    return nd == kDigits64 ? kAccs64 : (int)kAccs - 1;
+}
+constexpr int kStackCols = 192;
+// the fewest groups that this allows, of even width (what is left over: the first)
+__host__ __device__ constexpr int stack_width(int nd, int cols) {
+    const int own = own_accs(nd), most = kStackCols / cols < own ? kStackCols / cols : own;
+    const int groups = (own + most - 1) / most;
+    return (own + groups - 1) / groups;
+}
+__host__ __device__ constexpr int stack_zeros(int nd, int cols) { return stack_width(nd, cols) - 1; }
+// planes of a block with its zeros
+__host__ __device__ constexpr int stack_planes(int nd, int cols) { return stack_zeros(nd, cols) + nd; }
+
+// mma(a, b, ks, acc, count, first): plane a times planes b .. b + count - 1 (zeros where
+// negative), K step ks, into accumulators acc .. acc + count - 1; `first`: the first MMA
+// into them.
+template <int ND, int COLS, int KSTEPS, class Mma>
+__host__ __device__ __forceinline__ void stacked_pairs(Mma mma) {
+    constexpr int own = own_accs(ND), width = stack_width(ND, COLS);
+    constexpr int rest = (own - 1) % width + 1;   // the first group: as many MMAs as its end
+#pragma unroll
+    for (int ks = 0; ks < KSTEPS; ++ks)
+#pragma unroll
+        for (int a = 0; a < own; ++a)
+#pragma unroll
+            for (int end = rest; end <= own; end += width) {
+                const int count = end == rest ? rest : width;
+                if (end > a) mma(a, end - count - a, ks, end - count, count, ks == 0 && a == 0);
+            }
+    // the weights that share the last accumulator, one pair at a time in order of weight and a
+#pragma unroll
+    for (int c = own; c < ND; ++c)
+#pragma unroll
+        for (int a = 0; a <= c; ++a)
+#pragma unroll
+            for (int ks = 0; ks < KSTEPS; ++ks)
+                mma(a, c - a, ks, own, 1, c == own && a == 0 && ks == 0);
+}
+
+// A planes at aBase + a aPlane, the stacked B planes at bBase, behind stack_zeros(ND,
+// COLS) planes of zeros.  accumulate: the accumulators hold an earlier K stage's sums.
+template <int ND, int COLS, int KSTEPS>
 __device__ __forceinline__ void issue_stacked(uint32_t tmem, uint32_t aBase, uint32_t aPlane,
                                               uint32_t bBase, uint32_t sbo,
                                               bool accumulate = false) {
     constexpr uint32_t bPlane = COLS * KSTEPS * 32;
-    constexpr int most = 256 / COLS;   // stacked planes of one MMA
-    // accumulators filled by stacked planes; the FP64 form's last one takes its
-    // own weight that way too (its sums are not exact, but far below the result)
-    constexpr int own = ND == kDigits64 ? NACC : NACC - 1;
-    const uint64_t da = tc::desc_sbo(aBase, sbo), db = tc::desc_sbo(bBase, sbo);
+    constexpr int zeros = stack_zeros(ND, COLS);
+    const uint64_t da = tc::desc_sbo(aBase, sbo), db = tc::desc_sbo(bBase - zeros * bPlane, sbo);
     // the descriptors' address field counts 16 bytes
-    const auto mma = [&](int a, int b, int ks, int acc, int count, uint32_t add) {
+    stacked_pairs<ND, COLS, KSTEPS>([&](int a, int b, int ks, int acc, int count, bool first) {
         tc::mma_bf16(tmem + (uint32_t)(acc * COLS), da + ((a * aPlane + ks * tc::kKStep) >> 4),
-                     db + ((b * bPlane + ks * tc::kKStep) >> 4),
-                     tc::idesc_bf16(128, count * COLS), add);
-    };
-#pragma unroll
-    for (int ks = 0; ks < KSTEPS; ++ks)
-#pragma unroll
-        for (int a = 0; a < ND; ++a) {
-#pragma unroll
-            for (int b = 0; b < own - a; b += most) {
-                const int left = own - a - b;
-                // digit 0 is the first to reach each of these accumulators
-                mma(a, b, ks, a + b, left < most ? left : most, ks == 0 && a == 0 && !accumulate ? 0u : 1u);
-            }
-            // the pairs past the last weight, between MMAs that do not wait for them
-            if (own == NACC)
-#pragma unroll
-                for (int b = own - a > 0 ? own - a : 0; b < ND - a; ++b) mma(a, b, ks, NACC - 1, 1, 1u);
-        }
-    if (own < NACC) {
-#pragma unroll
-        for (int c = own; c < ND; ++c)
-#pragma unroll
-            for (int a = 0; a <= c; ++a)
-#pragma unroll
-                for (int ks = 0; ks < KSTEPS; ++ks)
-                    mma(a, c - a, ks, NACC - 1, 1, c == own && a == 0 && ks == 0 && !accumulate ? 0u : 1u);
-    }
+                     db + (((b + zeros) * bPlane + ks * tc::kKStep) >> 4),
+                     tc::idesc_bf16(128, count * COLS), first && !accumulate ? 0u : 1u);
+    });
 }
 
 // Host form of the digits: BF16 bit patterns of the pre-scaled digits of
