@@ -485,6 +485,7 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
             // thread: point `row`, K groups half, half + 2, ...
             const int st = tid - 32 * EW, row = st & (kRows - 1), half = st >> 7;
             constexpr int own = (kg + 1) / 2;
+            // (a warp whose wait has run out stays in the loop: the barrier below counts it)
             for (int q = 0, k = k0; q < count; ++q, ++k) {
                 const int buf = k % NBUF;
                 const long p = first + (long)q * kRows + row;
@@ -516,10 +517,8 @@ k_apply_tc(const double* in, double* out, double* __restrict__ upd, BlockIdx bi,
                     emax = max(e0 >> 8, e1 >> 8);
                     bad = min(e0 & 255, e1 & 255);
                 }
-                if (k >= NBUF) {
-                    ok = wait_warp(&emptyA[buf], ((k - NBUF) / NBUF) & 1);
-                    if (!ok) break;
-                }
+                if (ok && k >= NBUF) ok = wait_warp(&emptyA[buf], ((k - NBUF) / NBUF) & 1);
+                if (!ok) continue;
                 if (half == 0) sEmax[k & 3][row] = emax * 256 + bad;
                 arrive_warp(&emaxReady[k & 3], lane);
                 const oz::FixedRow<ND> fixed(emax);
@@ -720,7 +719,8 @@ k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
         // ------- slicers: rows row0 and row0 + 64, component c, half of the points -------
         const int st = tid - 32 * kRoleWarps, row0 = st >> 3, c = (st >> 1) & 3, half = st & 1;
         int stage = 0;
-        for (int unit = u0, k = 0; unit < u1 && ok; ++unit) {
+        // (a warp whose wait has run out stays in the loop: the barrier below counts it)
+        for (int unit = u0, k = 0; unit < u1; ++unit) {
             const int b = unit / nchunk, it = b >> 1, h = hsz[b];
             if (h == 0) continue;
             const long p0 = (long)(unit - b * nchunk) * kGapPts;
@@ -768,7 +768,7 @@ k_gaps_tc(const double* __restrict__ psi, const int* __restrict__ members,
             arrive_warp(&expReady[k & 7], lane);
             const float4* F = sF[k & 1];
             ++k;
-            for (int s = 0; s < nst; ++s, ++stage) {
+            for (int s = 0; s < nst && ok; ++s, ++stage) {
                 const int buf = stage % NBUF;
                 uint8_t* planes = base + buf * kBuf;
                 double a[kPasses][4], ap[kPasses][4];
