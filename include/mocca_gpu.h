@@ -44,8 +44,8 @@ extern "C" {
 
 /* ---- precision modes ----------------------------------------------------- */
 #define MG_FP64   0   /* FP64 data and accuracy; the contractions of large
-                         bases as exact digit products rounded once to FP64,
-                         with a smaller error than a chain of FP64 FMAs    */
+                         bases as digit products of 62-bit operands, with
+                         a smaller error than a chain of FP64 FMAs         */
 #define MG_MIXED  1   /* tensor-core digit GEMMs, double-float mesh work  */
 
 /* ---- bases --------------------------------------------------------------- */

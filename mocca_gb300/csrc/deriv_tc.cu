@@ -33,8 +33,8 @@
 //               quarter, alternating chunks of four columns), combine the
 //               accumulators, scale, store.  The Laplacian values a chunk adds
 //               to are loaded while the chunk before it is worked on.
-// The kernel is bound by instruction issue (63% of the slots at 24^3; HBM and
-// the tensor pipe below 30%).  Two things brought it there.  The digit planes
+// The kernel is bound by instruction issue (58 to 66% of the slots at 24^3; HBM
+// below 34%, the tensor pipe below 36%).  Two things brought it there.  The digit planes
 // of a column block's matrix are stacked, so that an MMA of up to 192 columns
 // serves several pairs of a line digit (stacked_pairs in ozaki.cuh): with one MMA
 // of 32 columns per pair, about 125 clocks each, the MMAs bound the kernel
@@ -43,7 +43,7 @@
 // epilogue, while every plane, slot and address that one thread alone uses
 // needs no barrier.  DeriveAll of one basis, mixed form, against one epilogue
 // group, both slots' matrices per CTA, a pair per MMA and eight-byte stores
-// on every axis: 241 us (336 before) at 24^3 with 160 spwfs, 25 us (37) at
+// on every axis: 240 us (336 before) at 24^3 with 160 spwfs, 25 us (37) at
 // 10^3 with 40, 1.50 ms (3.03) at 36^3 with 300.
 //
 // Hand-offs are mbarriers: fullA (one arrival per slicer warp), emptyA and

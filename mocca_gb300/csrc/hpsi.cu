@@ -48,9 +48,10 @@ __device__ __forceinline__ void pauli(const double* p, int dir, double* o) {
     else { o[0] = p[0]; o[1] = p[1]; o[2] = -p[2]; o[3] = -p[3]; }
 }
 
-// Bound by the FP64 pipe (a warp's instruction takes 16 clocks of the SM): 83 FP64
-// instructions a point, 95 with the GradDesc step.  200 spwfs at 32^3: 927 us (1180
-// with 101, the terms summed one by one), 160 at 24^3 with the step 466 (510).
+// Bound by the FP64 pipe (a warp's instruction takes 16 clocks of the SM; 69% active
+// with the GradDesc step, whose loads are waited for the rest): 83 FP64 instructions a
+// point, 95 with the step.  200 spwfs at 32^3: 927 us (1180 with 101, the terms summed
+// one by one), 160 at 24^3 with the step 478 (510).
 // Blocks of kT threads: 128, or 64 for the few points of a single spinor.
 template <bool kGradStep, int kT>
 __global__ void __launch_bounds__(kT, 768 / kT)

@@ -71,7 +71,9 @@ __device__ __forceinline__ double pow2d(int x) {
 // while the next unit's stages go on.  A's rows are the planes' own, one after the
 // other, so that the planes are B's stacked columns too, behind the planes of zeros that
 // the stack begins with; what A reads past a plane's NP rows gives rows of D that
-// nothing reads.  300 spwfs of 36^3 (blocks of 75, 38 MMAs a stage of 32 points) 566
+// nothing reads.  Bound by the latency of the slicers' loads (160 spwfs of 24^3: a
+// quarter of the issue slots used, the tensor pipe active 27% in the mixed form, 40% in
+// the FP64 form).  300 spwfs of 36^3 (blocks of 75, 38 MMAs a stage of 32 points) 572
 // us, 834 with a CTA per chunk; the FP64 form for 160 of 24^3 (40, 24 MMAs) 150, 512
 // by FP64 FMAs.
 constexpr int kRoleWarps = 8;                       // epilogue: warps 0-7, slicers: 8-15
@@ -392,7 +394,7 @@ k_coef_digits(const double* __restrict__ coef, long bstride, int ld, BlockIdx bi
 // and cut them once the planes of the tile before are free, one thread issues the
 // MMAs, the epilogue takes the accumulators to registers, gives them back and
 // writes.  The integer and FP32 work of cutting and combining bounds it (about 160
-// instructions per entry, 51% of the issue slots), the MMAs come next (one of up to
+// instructions per entry, 55 to 61% of the issue slots at 24^3), the MMAs come next (one of up to
 // 192 columns holds the tensor pipe ~130 clocks: 54 of them for a tile of 48
 // spinors, 95 for 80).  A CTA per tile went through the same steps one after the
 // other: 1628 us for the 300 spwfs of 36^3 (blocks of 75), now 573; 110 for the 160
@@ -1008,10 +1010,10 @@ k_gaps_factor(const double* __restrict__ psi, const int* __restrict__ members,
 
 // Largest and smallest blocks of the FP64 form.  Above 64 its eight accumulators do
 // not fit the 512 TMEM columns.  Below 24 the FP64 kernels of gs.cu are as fast or
-// faster; the whole Gram-Schmidt of four blocks at 10^3 / 16^3 / 24^3 in us, there and
-// here: blocks of 16: 54 / 83 / 167 and 64 / 89 / 166, of 24: 83 / 149 / 336 and
-// 83 / 119 / 216, of 40: 155 / 318 / 785 and 130 / 193 / 360, of 64: 317 / 709 / 1851
-// and 217 / 301 / 546.
+// faster, but on large meshes; the whole Gram-Schmidt of four blocks at 10^3 / 16^3 /
+// 24^3 in us, there and here: blocks of 16: 44 / 73 / 158 and 52 / 77 / 143, of 20: 53 /
+// 96 / 220 and 59 / 88 / 163, of 24: 66 / 131 / 320 and 64 / 92 / 171, of 40: 118 / 280 /
+// 750 and 92 / 146 / 297, of 64: 243 / 636 / 1776 and 144 / 230 / 480.
 constexpr int kMeshTcMax64 = 64, kMeshTcMin64 = 24;
 
 // Whether blocks of up to nbmax spinors go to the kernels of this file.
