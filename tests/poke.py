@@ -10,14 +10,20 @@ ROOT = Path(__file__).resolve().parents[1]
 
 SOURCE = r"""
 #include "mg_internal.cuh"
+#include "tc.cuh"
+__global__ void k_report(int* status) { mg::tc::report_timeout(status); }
 extern "C" {
 // the waits for the Coulomb CG's sums give up after so many clocks, from an iteration on
 void poke_cg_sum_wait(mg_ctx* c, long long clocks, int from) {
     c->cg_sum_wait = clocks;
     c->cg_sum_wait_from = from;
 }
-// a wait of a tensor-core kernel has run out
-void poke_tc_timeout(mg_ctx* c) { *c->h_tc_status = 1; }
+// a kernel on the context's stream that reports what a tensor-core kernel reports whose
+// wait has run out
+int poke_tc_timeout(mg_ctx* c) {
+    k_report<<<1, 1, 0, c->stream>>>(c->tc_status);
+    return (int)cudaGetLastError();
+}
 }
 """
 
@@ -34,5 +40,5 @@ def load():
     lib.poke_cg_sum_wait.argtypes = [C.c_void_p, C.c_longlong, C.c_int]
     lib.poke_cg_sum_wait.restype = None
     lib.poke_tc_timeout.argtypes = [C.c_void_p]
-    lib.poke_tc_timeout.restype = None
+    lib.poke_tc_timeout.restype = C.c_int
     return lib

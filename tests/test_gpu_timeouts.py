@@ -1,6 +1,6 @@
-"""A wait of a tensor-core kernel that ran out (the word such a kernel leaves behind,
-set by hand) is reported by whichever call hands out results next, in both forms,
-and by that one only."""
+"""A wait of a tensor-core kernel that ran out (here a kernel that does nothing but
+leave the word which such a kernel leaves behind) is reported by whichever call hands
+out results next, in both forms, and by that one only."""
 import ctypes as C
 
 import numpy as np
@@ -56,7 +56,7 @@ CALLS = {
 
 @pytest.mark.parametrize("call", sorted(CALLS))
 def test_reported_once(state, call):
-    poke.load().poke_tc_timeout(state.h)
+    assert poke.load().poke_tc_timeout(state.h) == 0
     # the calls that only queue work leave it to the next
     state.DeriveBasis(MG_HF_BASIS)
     state.UpdateDensities()
